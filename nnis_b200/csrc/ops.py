@@ -698,6 +698,48 @@ def attention_prefill_mma(q: torch.Tensor, q_stride: int, k_cache: torch.Tensor,
         "attention_prefill_mma")
 
 
+def attention_tile_f32_takes(head_dim: int, page_size: int, q_stride: int) -> bool:
+    """Whether a float32 prompt step's attention runs as tiles of 64 queries."""
+    return 0 < head_dim <= 128 and head_dim % 4 == 0 and page_size == 64 and q_stride % 4 == 0
+
+
+def attention_tile_f32_splits(n_tiles: int, heads: int, max_context: int, device=None) -> int:
+    """Slices of a tile's key range: enough CTAs for two per SM, at least four pages a slice."""
+    want = -(-2 * sm_count(device) // max(1, n_tiles * heads))
+    return int(max(1, min(want, -(-max_context // 64) // 4, 64)))
+
+
+def attention_tile_f32(q: torch.Tensor, q_stride: int, k_cache: torch.Tensor, v_cache: torch.Tensor,
+                       tiles: torch.Tensor, seq_first_row: torch.Tensor, seq_start: torch.Tensor,
+                       seq_count: torch.Tensor, page_table: torch.Tensor, out: torch.Tensor, heads: int,
+                       kv_heads: int, head_dim: int, window: int, scale: float, n_splits: int = 1,
+                       partial: Optional[torch.Tensor] = None) -> None:
+    """Prompt attention in true float32: packed query tokens, 64 per tile, each over its own
+    sequence's keys in the paged cache."""
+    _cuda(k_cache, v_cache, tiles, seq_first_row, seq_start, seq_count, page_table, out, partial)
+    _need(q.is_cuda and q.dtype == torch.float32 == k_cache.dtype == v_cache.dtype == out.dtype,
+          "attention_tile_f32: float32 tensors")
+    pages, nkv, page_size, d = k_cache.shape
+    n = out.shape[0]
+    _need(nkv == kv_heads and d == head_dim, "cache shape differs from the heads given")
+    _need(attention_tile_f32_takes(head_dim, page_size, q_stride),
+          f"attention_tile_f32: head_dim {head_dim} / page {page_size} is not taken")
+    _need(heads % kv_heads == 0, "attention: heads is not a multiple of kv_heads")
+    _need(pages * nkv * page_size < 2 ** 31, "attention: the cache has too many rows")
+    _need(out.shape[1] == heads * head_dim, "attention: out [n, heads * d]")
+    for t in (tiles, seq_first_row, seq_start, seq_count):
+        _need(t.dtype == torch.int32, "attention_tile_f32: int32 tables")
+    _need(tiles.dim() == 2 and tiles.shape[1] == 2 and tiles.shape[0] > 0, "tiles: int32 [n_tiles, 2]")
+    if n_splits > 1:
+        _need(partial is not None and partial.dtype == torch.float32
+              and partial.numel() >= n * heads * n_splits * (head_dim + 2), "attention: partial scratch too small")
+    _check(_lib().nnis_attention_tile_f32(
+        _ptr(q), q_stride, _ptr(k_cache), _ptr(v_cache), _ptr(tiles), tiles.shape[0], _ptr(seq_first_row),
+        _ptr(seq_start), _ptr(seq_count), _ptr(page_table), page_table.shape[1], _ptr(out), _ptr(partial), n, heads,
+        kv_heads, head_dim, page_size, window, ctypes.c_float(scale), n_splits, _stream()),
+        "attention_tile_f32", 2 if n_splits > 1 else 1)
+
+
 WIDE_QUERY_TILE = 128  # queries per CTA of attention_prefill_tc
 TC_ATTENTION = 0 if os.environ.get("NNIS_TC_ATTENTION", "1") == "0" else 1
 
