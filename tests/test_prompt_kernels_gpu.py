@@ -25,6 +25,23 @@ def stored(case, dtype, empty):
     return kc.to(dtype).to(DEV), vc.to(dtype).to(DEV)
 
 
+@pytest.mark.parametrize("m", [63, 64, 65, 129])
+@pytest.mark.parametrize("n,k", [(64, 32), (63, 31), (65, 33), (130, 576), (4, 1)])
+def test_float32_product_at_the_edges_of_its_tiles(m, n, k):
+    o = ops()
+    g = torch.Generator().manual_seed(m + 10 * n + 100 * k)
+    a, w = torch.randn(m, k, generator=g), torch.randn(n, k, generator=g) / math.sqrt(k)
+    bias = torch.randn(n, generator=g)
+    want = P.linear(a, w, bias)
+    room = torch.full((m * n + 1,), 7.0, device=DEV)
+    for off in (0, 1):  # (a destination that is not 16-byte aligned)
+        out = room[off:off + m * n].view(m, n)
+        o.gemm_simt(a.to(DEV), w.to(DEV), bias.to(DEV), out, o.STORE)
+        close(out, want, "float32", f"store at {off}")
+        o.gemm_simt(a.to(DEV), w.to(DEV), None, out, o.ADD_F32)
+        close(out, want + P.linear(a, w), "float32", f"add at {off}")
+
+
 @pytest.mark.parametrize("nq,nkv,d", [(3, 3, 64), (6, 2, 48), (4, 1, 128), (2, 2, 4), (3, 1, 100)])
 @pytest.mark.parametrize("window", [0, 1, 70])
 @pytest.mark.parametrize("splits", [1, 3])
