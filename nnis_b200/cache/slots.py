@@ -13,6 +13,7 @@ batched form of that.
 """
 from __future__ import annotations
 
+import heapq
 from typing import List
 
 
@@ -32,7 +33,9 @@ class FreeList:
             raise ValueError(f"a pool of {what}s needs a positive count; got {count}")
         self.count = count
         self.what = what
-        self._free: List[int] = list(range(count - 1, -1, -1))
+        # a heap: giving back one of 4,096 pages into a list that was sorted again each time cost 10 us, half a
+        # millisecond for a prompt of 3,000 tokens
+        self._free: List[int] = list(range(count))
         self._held = [False] * count
 
     @property
@@ -49,7 +52,7 @@ class FreeList:
     def take(self) -> int:
         if not self._free:
             raise CacheFull(f"no free {self.what} (all {self.count} are held)")
-        index = self._free.pop()
+        index = heapq.heappop(self._free)
         self._held[index] = True
         return index
 
@@ -64,9 +67,7 @@ class FreeList:
         if not self._held[index]:
             raise SlotError(f"{self.what} {index} is not held (freed twice?)")
         self._held[index] = False
-        self._free.append(index)
-        # keep "lowest first": the list is popped from its end
-        self._free.sort(reverse=True)
+        heapq.heappush(self._free, index)
 
     def check(self) -> None:
         """Every index is either free once or held, never both."""
