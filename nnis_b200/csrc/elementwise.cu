@@ -269,8 +269,8 @@ __global__ void relu2_gate_kernel(const float* __restrict__ u, T* __restrict__ o
 // (float32), the rest pass.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void rope_part_kernel(const T* __restrict__ src, long long src_row, int src_head,
-                                 int src_off, T* __restrict__ dst, long long dst_row, int dst_head,
+__global__ void rope_part_kernel(const T* src, long long src_row, int src_head,  // (src may be dst itself)
+                                 int src_off, T* dst, long long dst_row, int dst_head,
                                  int dst_off, const int* __restrict__ token_pos,
                                  const float* __restrict__ freq, int heads, int len, int dims,
                                  int neighbours) {

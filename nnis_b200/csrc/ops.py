@@ -858,6 +858,117 @@ def attention_prefill_tc(q: torch.Tensor, q_stride: int, k_cache: torch.Tensor, 
         "attention_prefill_tc")
 
 
+def attention_wide_tc_takes(head_dim: int, page_size: int, q_stride: int) -> bool:
+    """Head size 128 on the tcgen05 kernel for wide heads."""
+    return bool(TC_ATTENTION) and head_dim == 128 and page_size == 64 and q_stride % 8 == 0
+
+
+def attention_wide_tc_takes_expanded(dim: int, rot: int, vdim: int, kv_rank: int) -> bool:
+    """Latent attention's sizes that the same kernel runs with keys and values multiplied out."""
+    return bool(TC_ATTENTION) and (dim, rot, vdim) in ((128, 64, 128), (64, 32, 64)) and kv_rank % 8 == 0
+
+
+def attention_wide_plan(counts, starts, window: int, heads: int, sms: int):
+    """Work list of attention_wide_tc: int32 [n, 4] = (sequence, first query of a tile of 128, first query of a
+    second tile or -1, 0), most pages first.
+
+    With no more tiles than SMs (tiles x heads) every tile has a CTA of its own; else two tiles of a sequence
+    share one: the first with the last, the second with the last but one, so that every pair has the same number
+    of pages; within a window, where neighbours see the same pages, neighbours."""
+    import numpy as np
+    tiles = []  # per sequence: (first query, pages)
+    for c, st in zip(counts, starts):
+        mine = []
+        for q0 in range(0, int(c), WIDE_QUERY_TILE):
+            last = int(st) + min(int(c), q0 + WIDE_QUERY_TILE) - 1
+            lo = max(0, int(st) + q0 - window + 1) if window > 0 else 0
+            mine.append((q0, last // 64 - lo // 64 + 1))
+        tiles.append(mine)
+    units = []
+    single = sum(len(m) for m in tiles) * heads <= sms
+    for i, mine in enumerate(tiles):
+        n = len(mine)
+        if single:
+            pairs = [(t, None) for t in mine]
+        elif window > 0:
+            pairs = [(mine[j], mine[j + 1] if j + 1 < n else None) for j in range(0, n, 2)]
+        else:
+            pairs = [(mine[n - 1 - j], mine[j] if j < n - 1 - j else None) for j in range((n + 1) // 2)]
+        units += [(a[1] + (b[1] if b else 0), i, a[0], b[0] if b else -1, 0) for a, b in pairs]
+    units.sort(key=lambda u: -u[0])
+    return np.asarray([u[1:] for u in units], dtype=np.int32).reshape(-1, 4)
+
+
+def _wide_tables(units, *tables):
+    _need(units.dtype == torch.int32 and units.dim() == 2 and units.shape[1] == 4 and units.shape[0] > 0
+          and units.is_contiguous(), "units: int32 [n_units, 4]")
+    for t in tables:
+        _need(t.dtype == torch.int32, "attention_wide_tc: int32 tables")
+
+
+def attention_wide_tc(q: torch.Tensor, q_stride: int, k_cache: torch.Tensor, v_cache: torch.Tensor,
+                      units: torch.Tensor, seq_first_row: torch.Tensor, seq_start: torch.Tensor,
+                      seq_count: torch.Tensor, page_table: torch.Tensor, out: torch.Tensor, heads: int,
+                      kv_heads: int, head_dim: int, window: int, scale: float) -> None:
+    """Prompt attention on tcgen05 (head size 128): packed query tokens, each over its own sequence's keys in the
+    paged cache.  ``units`` comes from ``attention_wide_plan``."""
+    _cuda(k_cache, v_cache, units, seq_first_row, seq_start, seq_count, page_table, out)
+    _need(q.is_cuda and q.dtype == torch.bfloat16 == k_cache.dtype == v_cache.dtype == out.dtype,
+          "attention_wide_tc: bfloat16 tensors")
+    pages, nkv, page_size, d = k_cache.shape
+    _need(nkv == kv_heads and d == head_dim and v_cache.shape == k_cache.shape, "cache shape differs from the heads given")
+    _need(attention_wide_tc_takes(head_dim, page_size, q_stride),
+          f"attention_wide_tc: head_dim {head_dim} / page {page_size} / stride {q_stride} is not taken")
+    _need(heads % kv_heads == 0, "attention: heads is not a multiple of kv_heads")
+    _need(pages * nkv * page_size < 2 ** 31, "attention: the cache has too many rows")
+    _need(out.shape[1] == heads * head_dim and out.is_contiguous(), "attention: out [n, heads * d]")
+    _wide_tables(units, seq_first_row, seq_start, seq_count, page_table)
+    _check(_lib().nnis_attention_wide_tc(
+        _ptr(q), q_stride, out.shape[0], _ptr(k_cache), _ptr(v_cache), ctypes.c_longlong(pages * nkv * page_size),
+        _ptr(units), units.shape[0], _ptr(seq_first_row), _ptr(seq_start), _ptr(seq_count), _ptr(page_table),
+        page_table.shape[1], _ptr(out), heads, kv_heads, head_dim, page_size, window, ctypes.c_float(scale),
+        _ptr(status_word(out.device)), PDL, _stream()), "attention_wide_tc")
+
+
+def attention_wide_tc_expanded(q: torch.Tensor, kv: torch.Tensor, kr: torch.Tensor, units: torch.Tensor,
+                               key_base: torch.Tensor, seq_first_row: torch.Tensor, seq_start: torch.Tensor,
+                               seq_count: torch.Tensor, out: torch.Tensor, heads: int, dim: int, rot: int, vdim: int,
+                               window: int, scale: float) -> None:
+    """The same over keys and values multiplied out: kv [R, heads * (dim + vdim)] (all heads' plain keys, then all
+    heads' values), kr [R, 64] the key part that the heads share; a sequence's rows from ``key_base`` on."""
+    _cuda(q, kv, kr, units, key_base, seq_first_row, seq_start, seq_count, out)
+    _need(q.dtype == torch.bfloat16 == kv.dtype == kr.dtype == out.dtype, "attention_wide_tc: bfloat16 tensors")
+    n = out.shape[0]
+    _need(tuple(q.shape) == (n, heads * (dim + rot)) and out.shape[1] == heads * vdim
+          and kv.shape[1] == heads * (dim + vdim) and tuple(kr.shape) == (kv.shape[0], 64),
+          "attention_wide_tc: shapes of q, kv, kr and out")
+    for t in (q, kv, kr, out):
+        _need(t.is_contiguous(), "attention_wide_tc: contiguous tensors")
+    _wide_tables(units, key_base, seq_first_row, seq_start, seq_count)
+    _check(_lib().nnis_attention_wide_tc_expanded(
+        _ptr(q), n, _ptr(kv), _ptr(kr), ctypes.c_longlong(kv.shape[0]), _ptr(units), units.shape[0], _ptr(key_base),
+        _ptr(seq_first_row), _ptr(seq_start), _ptr(seq_count), _ptr(out), heads, dim, rot, vdim, window,
+        ctypes.c_float(scale), _ptr(status_word(out.device)), PDL, _stream()), "attention_wide_tc_expanded")
+
+
+def latent_rows(cache: torch.Tensor, blocks: torch.Tensor, seq_start: torch.Tensor, seq_count: torch.Tensor,
+                page_table: torch.Tensor, c_out: torch.Tensor, r_out: torch.Tensor) -> None:
+    """The cached rows [latent | rotated part] of whole sequences into c_out [R, kv_rank] and r_out [R, 64]
+    (zeros beyond the rotated part); ``blocks`` int32 [R / 64, 2] = (sequence, page)."""
+    _cuda(cache, blocks, seq_start, seq_count, page_table, c_out, r_out)
+    _need(cache.dtype == torch.bfloat16 == c_out.dtype == r_out.dtype, "latent_rows: bfloat16 tensors")
+    rows, rank = c_out.shape
+    _need(cache.shape[1] == 1 and cache.shape[2] == 64 and rank <= cache.shape[3] <= rank + 64,
+          "latent_rows: cache [pages, 1, 64, rank + rot]")
+    _need(tuple(r_out.shape) == (rows, 64) and tuple(blocks.shape) == (rows // 64, 2) and rows % 64 == 0,
+          "latent_rows: c_out [R, rank], r_out [R, 64], blocks [R / 64, 2]")
+    for t in (blocks, seq_start, seq_count, page_table):
+        _need(t.dtype == torch.int32, "latent_rows: int32 tables")
+    _check(_lib().nnis_latent_rows(_ptr(cache), _ptr(blocks), blocks.shape[0], _ptr(seq_start), _ptr(seq_count),
+                                   _ptr(page_table), page_table.shape[1], _ptr(c_out), _ptr(r_out), rank,
+                                   cache.shape[3] - rank, _stream()), "latent_rows")
+
+
 def mma_ticket_count(n: int, heads: int, kv_heads: int) -> int:
     return n * kv_heads * (-(-(heads // kv_heads) // 16))
 

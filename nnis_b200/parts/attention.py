@@ -105,12 +105,15 @@ class Attention(Part):
     def _tc_plan_name(self) -> str:
         return f"prefill_tc/window{self.window}/heads{self.heads}"
 
+    def _wide_plan_name(self) -> str:
+        return f"prefill_wide/window{self.window}/heads{self.heads}"
+
     TILES_64 = "prefill_mma/tiles64"  # (sequence, first query) per 64 queries of the step
 
     def step_tables(self, counts, starts, have=()):
         """Work lists of the bfloat16 prompt attention kernels: the units of the
-        tcgen05 kernel (head size 64), shared by all layers with this window and
-        number of heads, where that kernel pays; else the 64-query tiles of the
+        tcgen05 kernels (head sizes 64 and 128), shared by all layers with this window
+        and number of heads, where they pay; else the 64-query tiles of the
         mma.sync kernel (head sizes 64 and 128), the same for every layer.  In float32
         the same 64-query tiles, the ones with the most keys first."""
         if self.dtype != torch.bfloat16:
@@ -127,6 +130,11 @@ class Attention(Part):
             units, slots = ops.prefill_tc_plan(counts, starts, self.window, self.heads,
                                                ops.sm_count(self.device))
             return {name + "/units": units, name + "/slots": np.asarray([slots], dtype=np.int32)}
+        if ops.attention_wide_tc_takes(self.head_dim, PAGE_SIZE, self.heads * self.head_dim) \
+                and ops.prefill_tc_pays(counts, starts, self.window):
+            name = self._wide_plan_name()
+            return {} if name in have else {
+                name: ops.attention_wide_plan(counts, starts, self.window, self.heads, ops.sm_count(self.device))}
         if ops.attention_decode_mma_takes(self.head_dim, PAGE_SIZE) and self.TILES_64 not in have:
             tiles = [(i, q0) for i, c in enumerate(counts) for q0 in range(0, int(c), 64)]
             return {self.TILES_64: np.asarray(tiles, dtype=np.int32).reshape(-1, 2)}
@@ -274,6 +282,11 @@ class Attention(Part):
             ops.attention_prefill_tc(q_buf, q_stride, cache.k, cache.v, ctx.tables[name + "/units"],
                                      partial, tickets, ctx.seq_first_row, ctx.seq_start, ctx.seq_count,
                                      table, attn, nq, nkv, d, self.window, self.scale)
+        elif not ctx.decode and self._wide_plan_name() in ctx.tables \
+                and ops.attention_wide_tc_takes(d, cache.page_size, q_stride):
+            ops.attention_wide_tc(q_buf, q_stride, cache.k, cache.v, ctx.tables[self._wide_plan_name()],
+                                  ctx.seq_first_row, ctx.seq_start, ctx.seq_count, table, attn, nq, nkv, d,
+                                  self.window, self.scale)
         elif self.dtype == torch.bfloat16 and not ctx.decode and self.TILES_64 in ctx.tables \
                 and ops.attention_decode_mma_takes(d, cache.page_size):
             ops.attention_prefill_mma(q_buf, q_stride, cache.k, cache.v, ctx.tables[self.TILES_64],

@@ -24,7 +24,12 @@ the queries are carried into the latent's space (one small product per head,
 ``W_uk`` transposed per head at load) and attention runs there: a score is one dot
 product with the cached row, the output is a weighted sum of the rows' ``c`` part,
 and the heads' values are made from that sum (``W_uv`` per head) before ``W_o`` adds
-into the residual stream.  Prompts, later chunks and single tokens take the same way.
+into the residual stream.  Single tokens, and prompts of any size, can take this way.
+
+A prompt multiplies the latents out instead where that is fewer operations and the sizes
+are those of the tcgen05 kernel: ``W_uk c`` and ``W_uv c`` of every position the step's queries
+see, once, in one product, and then attention in the heads' own spaces (``dim + rot_dim`` and
+``vdim`` operations a pair of positions instead of ``kv_rank + rot_dim`` and ``kv_rank``).
 
 params: hidden_size, heads, dim, rot_dim, vdim, q_rank, kv_rank, scale, eps, window, gate, sink,
 position (a ``rope_frequencies`` PartSpec, either pairing), names {dq, dq_norm, uq (or q), dkv,
@@ -34,6 +39,7 @@ from __future__ import annotations
 
 from typing import Dict, Mapping, Optional
 
+import numpy as np
 import torch
 
 from ..cache import PAGE_SIZE, KVRequest, KVView
@@ -85,6 +91,7 @@ class LatentAttention(Part):
         self.row = self.kv_rank + self.rot  # a cached row, and a query in the latent's space
         self.q_cols = self.heads * (self.dim + self.rot)
         self.w_down = self.w_uq = self.w_ukt = self.w_uv = self.w_o = None
+        self.w_kv = None  # [W_uk; W_uv], where a prompt may multiply the latents out
         self.norm_q = self.norm_kv = self.sink = None
 
     # -- weights ----------------------------------------------------------
@@ -130,7 +137,11 @@ class LatentAttention(Part):
             self.sink = tensors[self._name("sink")]
         # per head [kv_rank, dim]: the product that carries q_plain into the latent's space
         self.w_ukt = tensors[self._name("uk")].view(H, self.dim, self.kv_rank).transpose(1, 2).contiguous()
-        self.w_uv = tensors[self._name("uv")].view(H, self.vdim, self.kv_rank).contiguous()
+        if self._expandable():
+            self.w_kv = torch.cat([tensors[self._name("uk")], tensors[self._name("uv")]], 0).contiguous()
+            self.w_uv = self.w_kv[H * self.dim:].view(H, self.vdim, self.kv_rank)
+        else:
+            self.w_uv = tensors[self._name("uv")].view(H, self.vdim, self.kv_rank).contiguous()
         self.w_o = tensors[self._name("o")]
 
     def parameter_bytes(self) -> int:
@@ -161,9 +172,43 @@ class LatentAttention(Part):
     def _tensor_cores(self) -> bool:
         return self.dtype == torch.bfloat16 and ops.attention_latent_mma_takes(self.row, self.kv_rank, PAGE_SIZE)
 
+    def _expandable(self) -> bool:
+        """Whether the tcgen05 kernel takes this layer's sizes and options."""
+        return (self.dtype == torch.bfloat16 and self.q_rank > 0 and not self.window and not self.has_gate
+                and not self.has_sink and ops.attention_wide_tc_takes_expanded(self.dim, self.rot, self.vdim, self.kv_rank))
+
+    def _expand_name(self) -> str:
+        return f"latent_wide/{self.heads}x{self.dim}+{self.rot}+{self.vdim}/rank{self.kv_rank}"
+
+    def _expands(self, counts, starts) -> bool:
+        """Whether a prompt step multiplies the latents out.  The operations of either way, those of the way through
+        the latent's space four times: its kernels (mma.sync) run at 145 to 200 TFLOP/s, the tcgen05 ones at 600 to 800.
+        A portion of a few tokens after a long past keeps the latent's space (every position of the past would be
+        multiplied out for them), and so does a step whose keys and values would take over half a gigabyte."""
+        if not self._expandable():
+            return False
+        rows = sum(-(-(int(c) + int(st)) // PAGE_SIZE) * PAGE_SIZE for c, st in zip(counts, starts))
+        pairs = sum(int(c) * int(st) + int(c) * (int(c) + 1) // 2 for c, st in zip(counts, starts))
+        up = self.kv_rank * (self.dim + self.vdim)
+        return (rows * self.heads * (self.dim + self.vdim) * 2 <= 1 << 29
+                and rows * up + pairs * (self.dim + self.rot + self.vdim)
+                <= 4 * (sum(int(c) for c in counts) * up + pairs * (2 * self.kv_rank + self.rot)))
+
     def step_tables(self, counts, starts, have=()):
         """The tiles of the tensor-core kernel for a prompt step: 64 or 128 stacked (token,
-        head) rows each; the same for every layer with this number of heads and tile."""
+        head) rows each; the same for every layer with this number of heads and tile.  Where the
+        latents are multiplied out, the units of that kernel, the pages of every sequence and
+        where a sequence's rows begin."""
+        if self._expands(counts, starts):
+            name = self._expand_name()
+            if name + "/units" in have:
+                return {}
+            pages = [-(-(int(c) + int(st)) // PAGE_SIZE) for c, st in zip(counts, starts)]
+            blocks = [(i, p) for i, n in enumerate(pages) for p in range(n)]
+            base = np.concatenate([[0], np.cumsum(pages)[:-1]]) * PAGE_SIZE
+            return {name + "/units": ops.attention_wide_plan(counts, starts, 0, self.heads, ops.sm_count(self.device)),
+                    name + "/blocks": np.asarray(blocks, dtype=np.int32).reshape(-1, 2),
+                    name + "/key_base": base.astype(np.int32)}
         if not self._tensor_cores() or self._tiles_name() in have:
             return {}
         return {self._tiles_name(): ops.latent_tiles(counts, starts, self.heads,
@@ -186,6 +231,9 @@ class LatentAttention(Part):
         freq = self.position.frequencies()
         down = ws.get("latent_down", (n, self.w_down.shape[0]), torch.float32)
         linear(x, self.w_down, None, down, STORE_F32, decode=ctx.decode)
+        if not ctx.decode and self._expand_name() + "/units" in ctx.tables:
+            self._forward_expanded(ctx, down, freq, table, residual, cache)
+            return
         q_lat = ws.get("latent_q_abs", (n, H * self.row), self.dtype)
         # (a gate per head multiplies inside the attention kernel, one per value after W_uv)
         gate = ws.get("latent_gate", (n, H), torch.float32) if self.has_gate and not self.gate_by_value else None
@@ -224,15 +272,41 @@ class LatentAttention(Part):
                            gate_off=self.q_cols + self.row if self.gate_by_value else 0)
         linear(attn, self.w_o, None, residual, ADD_F32, ws, decode=ctx.decode)
 
-    def _queries_from_latent(self, ctx, down, q_lat, freq, table, cache) -> None:
-        """Queries by way of their own latent: norm, up-projection, into the latent's space."""
-        n, H, ws = down.shape[0], self.heads, ctx.workspace
+    def _forward_expanded(self, ctx, down, freq, table, residual, cache) -> None:
+        """A prompt with the latents multiplied out: keys and values of every position that is seen, in one product,
+        and attention in the heads' own spaces."""
+        n, H, ws, name = down.shape[0], self.heads, ctx.workspace, self._expand_name()
+        q = self._queries(ctx, down, freq, table, cache)
+        if self.rot:
+            ops.rope_part(q, self.dim + self.rot, self.dim, q, self.dim + self.rot, self.dim, ctx.token_pos, freq, H,
+                          self.rot, self.position.dims, pairing=self.pairing)
+        blocks = ctx.tables[name + "/blocks"]
+        rows = blocks.shape[0] * PAGE_SIZE
+        c = ws.get("latent_rows_c", (rows, self.kv_rank), self.dtype)
+        kr = ws.get("latent_rows_r", (rows, 64), self.dtype)
+        ops.latent_rows(cache.k, blocks, ctx.seq_start, ctx.seq_count, table, c, kr)
+        kv = ws.get("latent_kv", (rows, H * (self.dim + self.vdim)), self.dtype)
+        linear(c, self.w_kv, None, kv, STORE)
+        attn = ws.get("attn", (n, H * self.vdim), self.dtype)
+        ops.attention_wide_tc_expanded(q, kv, kr, ctx.tables[name + "/units"], ctx.tables[name + "/key_base"],
+                                       ctx.seq_first_row, ctx.seq_start, ctx.seq_count, attn, H, self.dim, self.rot,
+                                       self.vdim, 0, self.scale)
+        linear(attn, self.w_o, None, residual, ADD_F32, ws)
+
+    def _queries(self, ctx, down, freq, table, cache) -> torch.Tensor:
+        """Queries by way of their own latent: norm, up-projection; the step's rows go to the cache."""
+        n, ws = down.shape[0], ctx.workspace
         cq = ws.get("latent_cq", (n, self.q_rank), self.dtype)
         ops.latent_prep(down, self.norm_q, self.norm_kv, freq, ctx.token_pos, ctx.token_seq, table, cq,
                         cache.k, self.q_rank, self.kv_rank, self.rot, self.position.dims, self.eps,
                         pairing=self.pairing)
         q = ws.get("latent_q", (n, self.q_cols), self.dtype)
         linear(cq, self.w_uq, None, q, STORE, decode=ctx.decode)
+        return q
+
+    def _queries_from_latent(self, ctx, down, q_lat, freq, table, cache) -> None:
+        """... and on into the latent's space."""
+        H, q = self.heads, self._queries(ctx, down, freq, table, cache)
         ops.batched_linear(q, self.dim + self.rot, self.w_ukt, q_lat, self.row)
         if self.rot:
             ops.rope_part(q, self.dim + self.rot, self.dim, q_lat, self.row, self.kv_rank, ctx.token_pos,

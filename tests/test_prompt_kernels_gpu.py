@@ -66,3 +66,87 @@ def test_float32_prompt_attention_in_tiles(nq, nkv, d, window, splits):
         full = P.causal_attention(case.q[s], case.k[s], case.v[s], window)
         close(out[r:r + new[s]], full[L - new[s]:].reshape(new[s], -1), "float32", f"sequence {s}")
         r += new[s]
+
+
+def wide_inputs(new, lengths):
+    starts = [L - c for L, c in zip(lengths, new)]
+    return i32([sum(new[:i]) for i in range(len(new))]), i32(starts), i32(new), starts
+
+
+@pytest.mark.parametrize("nq,nkv", [(4, 1), (2, 2), (6, 3)])
+@pytest.mark.parametrize("window", [0, 70, 300])
+@pytest.mark.parametrize("pad,sms", [(0, 1000), (24, 1)])
+def test_wide_prompt_attention_on_tcgen05(nq, nkv, window, pad, sms):
+    """Head size 128: whole prompts and later portions, one tile of queries a CTA and two, more pages than the ring holds."""
+    o = ops()
+    d, lengths, new = 128, [70, 1, 200, 64, 333, 129, 1500], [70, 1, 5, 64, 200, 65, 1500]
+    case = PagedCase(lengths, new, nq, nkv, d, "bfloat16", seed=5 * nq + window)
+    kc, vc = stored(case, torch.bfloat16, 50.0)
+    q = case.packed()[2]
+    n, stride = q.shape[0], nq * d + pad
+    qd = torch.full((n, stride), 3.0, dtype=torch.bfloat16, device=DEV)
+    qd[:, :nq * d] = q.reshape(n, -1).bfloat16().to(DEV)
+    first, start, count, starts = wide_inputs(new, lengths)
+    units = o.attention_wide_plan(new, starts, window, nq, sms)
+    out = torch.full((n, nq * d), 5.0, dtype=torch.bfloat16, device=DEV)
+    o.attention_wide_tc(qd, stride, kc, vc, torch.from_numpy(units).to(DEV), first, start, count, case.table.to(DEV), out,
+                        nq, nkv, d, window, 1.0 / math.sqrt(d))
+    o.check_status(DEV)
+    r = 0
+    for s, L in enumerate(lengths):
+        full = P.causal_attention(case.q[s], case.k[s], case.v[s], window)
+        close(out[r:r + new[s]], full[L - new[s]:].reshape(new[s], -1), "bfloat16", f"sequence {s}")
+        r += new[s]
+
+
+@pytest.mark.parametrize("dim,rot", [(128, 64), (64, 32)])
+@pytest.mark.parametrize("heads,sms,sharp", [(1, 1000, 1.0), (3, 1, 1.0), (2, 1, 6.0)])
+def test_wide_prompt_attention_over_expanded_latents(dim, rot, heads, sms, sharp):
+    """Keys whose last part all heads share; ``sharp`` scores make the running maximum rise from page to page."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim + heads)
+    lengths, new = [64, 1, 200, 333, 1000], [64, 1, 5, 200, 1000]
+    first, start, count, starts = wide_inputs(new, lengths)
+    pages = [-(-L // 64) for L in lengths]
+    rows, base = 64 * sum(pages), [64 * sum(pages[:i]) for i in range(len(pages))]
+    n = sum(new)
+    q = (torch.randn(n, heads, dim + rot, generator=g) * sharp).bfloat16()
+    kv = torch.randn(rows, heads * 2 * dim, generator=g).bfloat16()
+    kr = torch.zeros(rows, 64)
+    kr[:, :rot] = torch.randn(rows, rot, generator=g)
+    kr = kr.bfloat16()
+    units = torch.from_numpy(o.attention_wide_plan(new, starts, 0, heads, sms)).to(DEV)
+    out = torch.full((n, heads * dim), 5.0, dtype=torch.bfloat16, device=DEV)
+    scale = (dim + rot) ** -0.5
+    o.attention_wide_tc_expanded(q.reshape(n, -1).to(DEV), kv.to(DEV), kr.to(DEV), units, i32(base), first, start, count,
+                                 out, heads, dim, rot, dim, 0, scale)
+    o.check_status(DEV)
+    r = 0
+    for s, L in enumerate(lengths):
+        part = slice(base[s], base[s] + L)
+        k = torch.cat([kv[part, :heads * dim].view(L, heads, dim), kr[part, None, :rot].expand(L, heads, rot)], -1).double()
+        v = kv[part, heads * dim:].view(L, heads, dim).double()
+        qs = q[r:r + new[s]].double()
+        scores = torch.einsum("thd,shd->hts", qs, k) * scale
+        hidden = torch.arange(L)[None, :] > torch.arange(L - new[s], L)[:, None]
+        want = torch.einsum("hts,shd->thd", torch.softmax(scores.masked_fill(hidden, -math.inf), -1), v)
+        close(out[r:r + new[s]], want.reshape(new[s], -1), "bfloat16", f"sequence {s}")
+        r += new[s]
+
+
+@pytest.mark.parametrize("rank,rot", [(256, 32), (24, 64), (512, 0)])
+def test_cached_latent_rows_one_after_another(rank, rot):
+    o = ops()
+    g = torch.Generator().manual_seed(rank)
+    lengths, new = [64, 1, 130], [3, 1, 130]
+    cache = torch.randn(9, 1, 64, rank + rot, generator=g).bfloat16()
+    table = torch.tensor([[4, -1, -1], [7, -1, -1], [2, 8, 0]], dtype=torch.int32)
+    blocks = [(0, 0), (1, 0), (2, 0), (2, 1), (2, 2)]
+    c, r = (torch.full((320, w), 9.0, dtype=torch.bfloat16, device=DEV) for w in (rank, 64))
+    _, start, count, _ = wide_inputs(new, lengths)
+    o.latent_rows(cache.to(DEV), i32(blocks), start, count, table.to(DEV), c, r)
+    want = torch.zeros(320, rank + 64, dtype=torch.bfloat16)
+    for b, (s, p) in enumerate(blocks):
+        rows = min(64, lengths[s] - 64 * p)
+        want[64 * b:64 * b + rows, :rank + rot] = cache[int(table[s, p]), 0, :rows]
+    assert torch.equal(torch.cat([c, r], 1).cpu(), want)
