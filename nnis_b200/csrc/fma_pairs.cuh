@@ -1,0 +1,41 @@
+// Pairs of float32 multiply-adds and 16-byte asynchronous copies: what the tiled float32 products share.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace nnis {
+
+// Two float32 multiply-adds in one instruction, each rounded as fmaf rounds.
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+// The same value in both halves of a pair.
+__device__ __forceinline__ unsigned long long both(float x) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float2 halves(unsigned long long p) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ unsigned long long pair_of(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// 16 bytes to shared memory, or 16 zero bytes where the source does not exist (`src` is any valid address then).
+__device__ __forceinline__ void copy16_or_zero(float* dst, const float* src, bool there) {
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+}  // namespace nnis

@@ -10,6 +10,7 @@
 // NNIS: crates/nnis-kernels/src/gemm.rs:16-64 (tiled product),
 // crates/nnis-kernels/src/gemv.rs:45-61 (one-token projection).
 #include "common.cuh"
+#include "fma_pairs.cuh"
 
 namespace nnis {
 
@@ -18,18 +19,6 @@ __device__ __forceinline__ void emit(void* C, size_t idx, float v) {
     if (MODE == 0) reinterpret_cast<T*>(C)[idx] = from_float<T>(v);
     else if (MODE == 1) reinterpret_cast<float*>(C)[idx] = v;
     else reinterpret_cast<float*>(C)[idx] += v;
-}
-
-// Two float32 multiply-adds in one instruction, each rounded as fmaf rounds.
-__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-
-// The same value in both halves of a pair.
-__device__ __forceinline__ unsigned long long both(float x) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
-    return r;
 }
 
 // ---- 64 x 64 tile, 256 threads: four groups of 64 threads share K, 8 x 8 outputs per thread ----

@@ -1329,30 +1329,34 @@ def retention(qkvg: torch.Tensor, freq: torch.Tensor, decay: torch.Tensor, state
               token_pos: torch.Tensor, token_seq: torch.Tensor, seq_slots: torch.Tensor,
               seq_first_row: Optional[torch.Tensor], seq_start: Optional[torch.Tensor],
               seq_count: Optional[torch.Tensor], o_raw: torch.Tensor, out: torch.Tensor, heads: int,
-              dim: int, vdim: int, rot_dims: int, eps: float, segments: Optional[torch.Tensor] = None,
-              seq_first_segment: Optional[torch.Tensor] = None, seg_state: Optional[torch.Tensor] = None,
-              seg_len: int = 0, activation: bool = False, key_scale: Optional[float] = None,
+              dim: int, vdim: int, rot_dims: int, eps: float, chunks: Optional[torch.Tensor] = None,
+              seq_first_chunk: Optional[torch.Tensor] = None, packed: Optional[torch.Tensor] = None,
+              chunk_state: Optional[torch.Tensor] = None, activation: bool = False, key_scale: Optional[float] = None,
               norm_weight: Optional[torch.Tensor] = None, gate: str = "silu") -> None:
     """Retention of packed rows [q | k | v | g] from and into the per-slot state
     [slots, heads, dim, vdim] (float32); out [n, heads * vdim] = o / rms(o) * silu(g).
     ``activation``: q, k and v pass silu as they are read; ``key_scale``: what multiplies k
     (dim^-1/2 unless given); ``norm_weight`` (float32 [heads * vdim]): one norm over a token's
     joined heads, times this weight, instead of a norm per head; ``gate``: "silu" or "sigmoid".
-    Without ``seq_first_row`` every row is one token of a sequence of its own.  With
-    ``segments`` (``retention_segments``) a prompt step's sequences are cut into runs of
-    ``seg_len`` tokens that are worked side by side (``retention_takes_segments``)."""
+    Without ``seq_first_row`` every row is one token of a sequence of its own.  With ``chunks`` (``scan_segments`` of
+    RETENTION_CHUNK tokens) and the scratch that ``retention_scratch`` names a prompt step's chunks are worked side by
+    side (``retention_takes_chunks``)."""
     _cuda(qkvg, freq, decay, state, token_pos, token_seq, seq_slots, seq_first_row, seq_start, seq_count,
-          o_raw, out, segments, seq_first_segment, seg_state, norm_weight)
+          o_raw, out, chunks, seq_first_chunk, packed, chunk_state, norm_weight)
     _need(gate in ("silu", "sigmoid"), "retention: the gate is silu or sigmoid")
     _need(norm_weight is None or (norm_weight.dtype == torch.float32 and norm_weight.numel() == heads * vdim),
           "retention: norm_weight float32 [heads * vdim]")
-    n_segments = 0
-    if segments is not None:
-        n_segments = segments.shape[0]
-        _need(retention_takes_segments(dim) and seq_first_row is not None and seq_first_segment is not None
-              and seg_state is not None and seg_state.dtype == torch.float32
-              and seg_state.numel() >= n_segments * heads * dim * vdim and seg_len > 0,
-              "retention: segments need a prompt step, their tables and scratch")
+    n_chunks = 0
+    if chunks is not None:
+        n_chunks = chunks.shape[0]
+        sizes = retention_scratch(n_chunks, heads, dim, vdim)
+        _need(retention_takes_chunks(dim) and seq_first_row is not None and seq_first_chunk is not None
+              and packed is not None and packed.dtype == torch.float32 and packed.numel() >= sizes[0]
+              and chunk_state is not None and chunk_state.dtype == torch.float32 and chunk_state.numel() >= sizes[1],
+              "retention: chunks need a prompt step, their tables and scratch")
+        _need(chunks.dtype == torch.int32 and chunks.dim() == 2 and chunks.shape[1] == 2
+              and seq_first_chunk.dtype == torch.int32 and seq_first_chunk.numel() == seq_first_row.numel() + 1,
+              "retention: chunks int32 [n, 2], seq_first_chunk int32 [sequences + 1]")
     n = out.shape[0]
     _need(qkvg.shape[0] >= n and qkvg.shape[1] == 2 * heads * (dim + vdim) and qkvg.dtype == out.dtype,
           "retention: rows [n, 2 heads (dim + vdim)]")
@@ -1365,31 +1369,26 @@ def retention(qkvg: torch.Tensor, freq: torch.Tensor, decay: torch.Tensor, state
     units = seq_first_row.numel() if seq_first_row is not None else n
     _check(_lib().nnis_retention(_ptr(qkvg), _ptr(freq), _ptr(decay), _ptr(state), _ptr(token_pos),
                                  _ptr(token_seq), _ptr(seq_slots), _ptr(seq_first_row), _ptr(seq_start),
-                                 _ptr(seq_count), _ptr(segments), n_segments, _ptr(seq_first_segment), seg_len,
-                                 _ptr(seg_state), _ptr(o_raw), _ptr(out), n, units, heads, dim, vdim,
+                                 _ptr(seq_count), _ptr(chunks), n_chunks, _ptr(seq_first_chunk), _ptr(packed),
+                                 _ptr(chunk_state), _ptr(o_raw), _ptr(out), n, units, heads, dim, vdim,
                                  rot_dims, ctypes.c_float(eps), 1 if activation else 0,
                                  ctypes.c_float(dim ** -0.5 if key_scale is None else key_scale),
                                  _ptr(norm_weight), 1 if gate == "sigmoid" else 0, code_of(out.dtype), _stream()),
-           "retention", 4 if segments is not None else 2)
+           "retention", 5 if chunks is not None else 2)
 
 
-RETENTION_SEGMENT = int(os.environ.get("NNIS_RETENTION_SEGMENT", "256"))  # tokens of a run; 0: no runs
+RETENTION_CHUNK = 64  # tokens of a chunk
 
 
-def retention_takes_segments(dim: int) -> bool:
-    """Whether prompts of these key sizes can be cut into runs worked side by side."""
-    return RETENTION_SEGMENT > 0 and RETENTION_SEGMENT % 32 == 0 and dim in (32, 64, 128, 256)
+def retention_takes_chunks(dim: int) -> bool:
+    """Whether prompts of this key size are worked a chunk of tokens at a time, chunks side by side."""
+    return dim in (32, 64, 128, 256)
 
 
-def retention_segments(counts, seg_len: int):
-    """(segments [n, 2] = (sequence, first token of the run), first segment of every
-    sequence [sequences + 1]) for a prompt step whose sequences bring ``counts`` tokens."""
-    import numpy as np
-    segments, first = [], [0]
-    for i, c in enumerate(counts):
-        segments += [(i, t) for t in range(0, int(c), seg_len)]
-        first.append(len(segments))
-    return np.asarray(segments, dtype=np.int32).reshape(-1, 2), np.asarray(first, dtype=np.int32)
+def retention_scratch(n_chunks: int, heads: int, dim: int, vdim: int):
+    """Float32 values of ``packed`` and ``chunk_state`` for a prompt step of ``n_chunks`` chunks."""
+    vp = -(-vdim // 4) * 4
+    return n_chunks * heads * RETENTION_CHUNK * (3 * dim + vp), n_chunks * heads * dim * vp
 
 
 def moe_route(h: torch.Tensor, w_router: torch.Tensor, b_router: Optional[torch.Tensor],
@@ -1774,7 +1773,12 @@ SCAN_SEGMENT = int(os.environ.get("NNIS_SCAN_SEGMENT", "64"))  # tokens of a run
 def scan_segments(counts, seg_len: int):
     """(segments [n, 2] = (sequence, first token of the run), first run of every sequence
     [sequences + 1]) for a prompt step whose sequences bring ``counts`` tokens."""
-    return retention_segments(counts, seg_len)
+    import numpy as np
+    segments, first = [], [0]
+    for i, c in enumerate(counts):
+        segments += [(i, t) for t in range(0, int(c), seg_len)]
+        first.append(len(segments))
+    return np.asarray(segments, dtype=np.int32).reshape(-1, 2), np.asarray(first, dtype=np.int32)
 
 
 def qkv_prep(a: torch.Tensor, wq: Optional[torch.Tensor], wk: Optional[torch.Tensor],

@@ -8,10 +8,8 @@
 //   retention_scan   a CTA per (sequence, head, 32 columns of vdim) walks the step's
 //                    tokens of that sequence in order; warp w holds rows w, w+8, ...
 //                    of the state tile in registers.  Steps of single tokens.
-//   retention_chunk  prompts and later chunks of them (the state says where a sequence
-//                    stands): 32 tokens at a time, see below.
-//   retention_prefix, retention_carry   long prompts cut into runs that are worked side by
-//                    side: the states between the runs, and what they give each token.
+//   retention_pack, retention_update, retention_carry, retention_read   prompts and later
+//                    portions of them, key sizes 32, 64, 128 and 256: chunks of 64 tokens side by side, see below.
 //   retention_gate   o / rms(o) per head, times silu(g) (or sigmoid(g)), rounded once;
 //   retention_gate_joined   the same with one norm over a token's joined heads and a weight per value.
 //
@@ -21,6 +19,7 @@
 // Packed input rows: [q (H dim) | k (H dim) | v (H vdim) | g (H vdim)].
 #include "async_copy.cuh"
 #include "common.cuh"
+#include "linear_chunks.cuh"
 
 namespace nnis {
 
@@ -118,277 +117,240 @@ retention_scan_kernel(const T* __restrict__ qkvg, const float* __restrict__ freq
     }
 }
 
-// Prompts: the same recurrence a chunk of 32 tokens at a time.  Within a chunk, with
-// A[i][j] = (q_i . k_j) g^(i-j) for j <= i:
+// Prompts: the same recurrence a chunk of 64 tokens at a time.  Within a chunk of C tokens, with
+// A[i][j] = (q_i . k_j) g^(i-j) for j <= i and S the state before it:
 //     o_i = sum_j A[i][j] v_j + g^(i+1) S^T q_i        S <- g^C S + sum_j g^(C-1-j) k_j v_j^T
-// (C tokens in the chunk, S the state before it), all in float32 on the CUDA cores.  A CTA
-// owns (sequence, head, 32 columns of vdim) and walks the chunks in order with its tile of
-// S in shared memory; q and k of the chunk are rotated once into shared memory.
-constexpr int kRetChunk = 32;
+// all in float32 on the CUDA cores.  Four kernels: `pack` turns q, k and v of every (chunk, head) into the layouts that
+// the products read (rotated once, not once per tile of columns); `update` makes what every chunk adds to the state, all
+// chunks side by side; `carry` walks a sequence's chunks in order and leaves the state before each of them, and the
+// slot's state; `read` makes the outputs, all chunks side by side.  The products are linear_chunks.cuh's.
+// Before, chunks of 32 in runs of 256 tokens from zero, 32 columns a CTA with A made again for each, 2 x 2 entries of A
+// and 4 x 1 of the output a thread, took 495 us for 2,048 tokens and 8 heads of 128 x 256 on a B200 (chunk 351, prefix
+// 30, carry 114); now 143 (pack 39, update 25, carry 12, read 68: 22 TFLOP/s of multiply-adds).
 
-// DR4: dim / 32 (the kernel takes dim = 32, 64, 128, 256; a warp owns dim / 8 rows of the
-// state in the update).  The three products are tiled in registers: 2 x 2 entries of A per
-// thread, four rows of the output per thread, dim / 8 rows of the state per thread, with
-// q and k read as float4 along dim.
-template <typename T, int DR4>
-__global__ void __launch_bounds__(256)
-retention_chunk_kernel(const T* __restrict__ qkvg, const float* __restrict__ freq,
-                       const float* __restrict__ decay, float* __restrict__ state,
-                       const int* __restrict__ seq_slots, const int* __restrict__ seq_first_row,
-                       const int* __restrict__ seq_start, const int* __restrict__ seq_count,
-                       const int* __restrict__ segments, int seg_len, float* __restrict__ seg_state,
-                       float* __restrict__ o_raw, int heads, int vdim, int rot_dims, int act, float k_scale) {
-    constexpr int C = kRetChunk, dim = 32 * DR4, ld = dim + 4, DR = 4 * DR4;
-    extern __shared__ __align__(16) float smem[];
-    float* qs = smem;                  // [C][dim + 4]
-    float* ks = qs + C * ld;           // [C][dim + 4]
-    float* Ss = ks + C * ld;           // [dim][32]
-    float* As = Ss + dim * 32;         // [C][C + 1]
-    float* vs = As + C * (C + 1);      // [C][32]
-    float* pw = vs + C * 32;           // [C + 1]: g^n
-    const int h = blockIdx.y;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
-    const int col = blockIdx.z * 32 + lane;
-    // a unit is a sequence, from and into its state; or, with `segments`, a run of seg_len
-    // tokens of a sequence from a zero state into a state of its own (retention_carry adds
-    // what the tokens before the run contribute)
-    const int unit = segments ? segments[2 * blockIdx.x] : (int)blockIdx.x;
-    const int begin = segments ? segments[2 * blockIdx.x + 1] : 0;
-    const int first = seq_first_row[unit] + begin, start = seq_start[unit] + begin;
-    const int count = segments ? min(seg_len, seq_count[unit] - begin) : seq_count[unit];
-    if (count <= 0) return;
-    const bool live = col < vdim;
-    const float g = decay[h];
-    float* S = segments ? seg_state + (((size_t)blockIdx.x * heads + h) * dim) * vdim
-                        : state + (((size_t)seq_slots[unit] * heads + h) * dim) * vdim;
-    for (int d = warp; d < dim; d += 8) Ss[d * 32 + lane] = live && !segments ? S[(size_t)d * vdim + col] : 0.f;
-    for (int it = tid; it < 2 * C * ld; it += 256) qs[it] = 0.f;  // (rows beyond a short chunk)
-    if (tid == 0) {
+// A packed (chunk, head): queries [dim][64], keys [dim][64], keys times g^(C-1-j) [64][dim], values [64][vp].
+__host__ __device__ __forceinline__ size_t packed_floats(int dim, int vp) {
+    return (size_t)kChunkTokens * (3 * dim + vp);
+}
+
+struct RetChunk {
+    int seq, begin, first, start, count;  // of the batch; first token among the step's of the sequence; its row; position; tokens
+};
+__device__ __forceinline__ RetChunk ret_chunk(const int* chunks, const int* seq_first_row, const int* seq_start,
+                                              const int* seq_count, int c) {
+    RetChunk m;
+    m.seq = chunks[2 * c];
+    m.begin = chunks[2 * c + 1];
+    m.first = seq_first_row[m.seq] + m.begin;
+    m.start = seq_start[m.seq] + m.begin;
+    m.count = min(kChunkTokens, seq_count[m.seq] - m.begin);
+    return m;
+}
+
+// g^0 .. g^64 as a chain of products; every thread of the block calls it
+__device__ __forceinline__ void decay_powers(float g, float* pw) {
+    if (threadIdx.x == 0) {
         float p = 1.f;
-        for (int n = 0; n <= C; ++n) {
+        for (int n = 0; n <= kChunkTokens; ++n) {
             pw[n] = p;
             p *= g;
-        }
-    }
-    const size_t row_len = (size_t)2 * heads * dim + (size_t)2 * heads * vdim;
-    const int half = rot_dims >> 1, per_tok = dim - half;
-    for (int t0 = 0; t0 < count; t0 += C) {
-        const int cnt = min(C, count - t0);
-        __syncthreads();  // the chunk before is done with qs, ks, vs, As; Ss is up to date
-        for (int it = tid; it < cnt * per_tok; it += 256) {
-            int i = it / per_tok, j = it - i * per_tok;
-            const T* row = qkvg + (size_t)(first + t0 + i) * row_len;
-            const T* qh = row + (size_t)h * dim;
-            const T* kh = row + (size_t)heads * dim + (size_t)h * dim;
-            if (j < half) {
-                float ang = (float)(start + t0 + i) * freq[j];
-                float c = cosf(ang), sn = sinf(ang);
-                float u = pre(qh[j], act), v = pre(qh[j + half], act);
-                qs[i * ld + j] = u * c - v * sn;
-                qs[i * ld + j + half] = v * c + u * sn;
-                u = pre(kh[j], act);
-                v = pre(kh[j + half], act);
-                ks[i * ld + j] = (u * c - v * sn) * k_scale;
-                ks[i * ld + j + half] = (v * c + u * sn) * k_scale;
-            } else {
-                qs[i * ld + j + half] = pre(qh[j + half], act);
-                ks[i * ld + j + half] = pre(kh[j + half], act) * k_scale;
-            }
-        }
-        for (int it = tid; it < C * 32; it += 256) {
-            int i = it >> 5;
-            float v = 0.f;
-            if (i < cnt && live)
-                v = pre(qkvg[(size_t)(first + t0 + i) * row_len + (size_t)2 * heads * dim +
-                             (size_t)h * vdim + col], act);
-            vs[it] = v;
-        }
-        __syncthreads();
-        {   // A[i][j] = (q_i . k_j) g^(i - j) for j <= i: a 2 x 2 tile per thread
-            const int i0 = (tid >> 4) * 2, j0 = (tid & 15) * 2;
-            float a00 = 0.f, a01 = 0.f, a10 = 0.f, a11 = 0.f;
-            if (j0 <= i0 + 1) {
-                const float4* q0 = reinterpret_cast<const float4*>(qs + i0 * ld);
-                const float4* q1 = reinterpret_cast<const float4*>(qs + (i0 + 1) * ld);
-                const float4* k0 = reinterpret_cast<const float4*>(ks + j0 * ld);
-                const float4* k1 = reinterpret_cast<const float4*>(ks + (j0 + 1) * ld);
-#pragma unroll 4
-                for (int d = 0; d < dim / 4; ++d) {
-                    float4 x0 = q0[d], x1 = q1[d], y0 = k0[d], y1 = k1[d];
-                    a00 = fmaf(x0.x, y0.x, fmaf(x0.y, y0.y, fmaf(x0.z, y0.z, fmaf(x0.w, y0.w, a00))));
-                    a01 = fmaf(x0.x, y1.x, fmaf(x0.y, y1.y, fmaf(x0.z, y1.z, fmaf(x0.w, y1.w, a01))));
-                    a10 = fmaf(x1.x, y0.x, fmaf(x1.y, y0.y, fmaf(x1.z, y0.z, fmaf(x1.w, y0.w, a10))));
-                    a11 = fmaf(x1.x, y1.x, fmaf(x1.y, y1.y, fmaf(x1.z, y1.z, fmaf(x1.w, y1.w, a11))));
-                }
-            }
-            As[i0 * (C + 1) + j0] = j0 <= i0 ? a00 * pw[i0 - j0] : 0.f;
-            As[i0 * (C + 1) + j0 + 1] = j0 + 1 <= i0 ? a01 * pw[i0 - j0 - 1] : 0.f;
-            As[(i0 + 1) * (C + 1) + j0] = j0 <= i0 + 1 ? a10 * pw[i0 + 1 - j0] : 0.f;
-            As[(i0 + 1) * (C + 1) + j0 + 1] = j0 <= i0 ? a11 * pw[i0 - j0] : 0.f;
-        }
-        __syncthreads();
-        {   // outputs: rows 4 warp .. 4 warp + 3, column = lane
-            const int i0 = warp * 4;
-            float inter[4] = {0.f, 0.f, 0.f, 0.f}, intra[4] = {0.f, 0.f, 0.f, 0.f};
-            if (i0 < cnt) {
-#pragma unroll 2
-                for (int d = 0; d < dim; d += 4) {
-                    float s0 = Ss[d * 32 + lane], s1 = Ss[(d + 1) * 32 + lane];
-                    float s2 = Ss[(d + 2) * 32 + lane], s3 = Ss[(d + 3) * 32 + lane];
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        float4 x = *reinterpret_cast<const float4*>(qs + (i0 + r) * ld + d);
-                        inter[r] = fmaf(x.x, s0, fmaf(x.y, s1, fmaf(x.z, s2, fmaf(x.w, s3, inter[r]))));
-                    }
-                }
-                for (int j = 0; j <= i0 + 3; ++j) {  // (A is zero above its diagonal)
-                    float v = vs[j * 32 + lane];
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) intra[r] = fmaf(As[(i0 + r) * (C + 1) + j], v, intra[r]);
-                }
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-                    if (live && i0 + r < cnt)
-                        o_raw[((size_t)(first + t0 + i0 + r) * heads + h) * vdim + col] =
-                            fmaf(pw[i0 + r + 1], inter[r], intra[r]);
-            }
-        }
-        __syncthreads();
-        {   // the state after the chunk: rows warp * DR .. + DR - 1, column = lane
-            const int d0 = warp * DR;
-            float acc[DR];
-#pragma unroll
-            for (int r = 0; r < DR; ++r) acc[r] = 0.f;
-            for (int j = 0; j < cnt; ++j) {
-                float v = pw[cnt - 1 - j] * vs[j * 32 + lane];
-#pragma unroll
-                for (int r4 = 0; r4 < DR4; ++r4) {
-                    float4 k = *reinterpret_cast<const float4*>(ks + j * ld + d0 + 4 * r4);
-                    acc[4 * r4] = fmaf(k.x, v, acc[4 * r4]);
-                    acc[4 * r4 + 1] = fmaf(k.y, v, acc[4 * r4 + 1]);
-                    acc[4 * r4 + 2] = fmaf(k.z, v, acc[4 * r4 + 2]);
-                    acc[4 * r4 + 3] = fmaf(k.w, v, acc[4 * r4 + 3]);
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < DR; ++r) Ss[(d0 + r) * 32 + lane] = fmaf(pw[cnt], Ss[(d0 + r) * 32 + lane], acc[r]);
         }
     }
     __syncthreads();
-    for (int d = warp; d < dim; d += 8)
-        if (live) S[(size_t)d * vdim + col] = Ss[d * 32 + lane];
 }
 
-// Long prompts run as runs of seg_len tokens side by side (retention_chunk with `segments`),
-// each from a zero state.  This kernel then walks a sequence's runs in order, per element of
-// the state: the state before a run replaces the run's own in `seg_state`, and the state
-// after the last run goes to the sequence's slot.  S_before(r + 1) = g^len(r) S_before(r) + U(r).
+template <typename T>
 __global__ void __launch_bounds__(256)
-retention_prefix_kernel(float* __restrict__ seg_state, float* __restrict__ state,
-                        const float* __restrict__ decay, const int* __restrict__ seq_slots,
-                        const int* __restrict__ seq_count, const int* __restrict__ seq_first_segment,
-                        int seg_len, int heads, int per_head) {
-    const int b = blockIdx.x, h = blockIdx.y;
-    const int e = blockIdx.z * 256 + threadIdx.x;
-    if (e >= per_head) return;
-    const int s0 = seq_first_segment[b], s1 = seq_first_segment[b + 1], count = seq_count[b];
+retention_pack_kernel(const T* __restrict__ qkvg, const float* __restrict__ freq, const float* __restrict__ decay,
+                      const int* __restrict__ chunks, const int* __restrict__ seq_first_row,
+                      const int* __restrict__ seq_start, const int* __restrict__ seq_count, float* __restrict__ packed,
+                      int heads, int dim, int vdim, int vp, int rot_dims, int act, float k_scale) {
+    constexpr int C = kChunkTokens;
+    extern __shared__ float pack_smem[];
+    __shared__ float pw[C + 1];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int ld = dim + 1, tid = threadIdx.x, h = blockIdx.y;
+    float* qs = pack_smem;    // [64][dim + 1]
+    float* ks = qs + C * ld;  // [64][dim + 1]
+    const RetChunk ch = ret_chunk(chunks, seq_first_row, seq_start, seq_count, blockIdx.x);
+    const size_t row_len = (size_t)2 * heads * (dim + vdim);
+    const T* rows = qkvg + (size_t)ch.first * row_len + (size_t)h * dim;
+    for (int it = tid; it < C * dim; it += 256) {
+        const int t = it / dim, d = it - t * dim;
+        const bool in = t < ch.count;
+        qs[t * ld + d] = in ? pre(rows[(size_t)t * row_len + d], act) : 0.f;
+        ks[t * ld + d] = in ? pre(rows[(size_t)t * row_len + (size_t)heads * dim + d], act) * k_scale : 0.f;
+    }
+    decay_powers(decay[h], pw);
+    const int half = rot_dims >> 1;
+    for (int it = tid; it < C * half; it += 256) {
+        const int t = it & (C - 1), j = it >> 6;
+        const float ang = (float)(ch.start + t) * freq[j];
+        const float c = cosf(ang), sn = sinf(ang);
+        float* q = qs + t * ld + j;
+        float* k = ks + t * ld + j;
+        const float q0 = q[0], q1 = q[half], k0 = k[0], k1 = k[half];
+        q[0] = q0 * c - q1 * sn;
+        q[half] = q1 * c + q0 * sn;
+        k[0] = k0 * c - k1 * sn;
+        k[half] = k1 * c + k0 * sn;
+    }
+    __syncthreads();
+    float* to = packed + ((size_t)blockIdx.x * heads + h) * packed_floats(dim, vp);
+    for (int it = tid; it < C * dim; it += 256) {
+        const int t = it & (C - 1), d = it >> 6;
+        to[it] = qs[t * ld + d];
+        to[C * dim + it] = ks[t * ld + d];
+    }
+    to += (size_t)2 * C * dim;
+    for (int it = tid; it < C * dim; it += 256) {
+        const int t = it / dim, d = it - t * dim;
+        to[it] = t < ch.count ? ks[t * ld + d] * pw[ch.count - 1 - t] : 0.f;
+    }
+    to += (size_t)C * dim;
+    const T* v = qkvg + (size_t)ch.first * row_len + (size_t)2 * heads * dim + (size_t)h * vdim;
+    for (int it = tid; it < C * vp; it += 256) {
+        const int t = it / vp, j = it - t * vp;
+        to[it] = t < ch.count && j < vdim ? pre(v[(size_t)t * row_len + j], act) : 0.f;
+    }
+}
+
+template <int BV>
+__global__ void __launch_bounds__(128)
+retention_update_kernel(const float* __restrict__ packed, float* __restrict__ chunk_state, int heads, int dim, int vp) {
+    extern __shared__ __align__(16) float update_smem[];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int v_tiles = (vp + BV - 1) / BV;
+    const size_t unit = (size_t)blockIdx.x * heads + blockIdx.y;
+    const float* from = packed + unit * packed_floats(dim, vp) + (size_t)2 * kChunkTokens * dim;
+    chunk_update_tile<BV>(from, from + (size_t)kChunkTokens * dim, chunk_state + unit * dim * vp, dim, vp,
+                          (int)(blockIdx.z / v_tiles) * 64, (int)(blockIdx.z % v_tiles) * BV, update_smem);
+}
+
+// The state before every chunk in place of what the chunk adds, in order, a thread per four values of a row, eight
+// chunks fetched ahead; the state after the last goes to the slot (whose rows have vdim values and no alignment).
+__global__ void __launch_bounds__(128)
+retention_carry_kernel(float* chunk_state, float* state, const float* __restrict__ decay,
+                       const int* __restrict__ seq_slots, const int* __restrict__ seq_start,
+                       const int* __restrict__ seq_count, const int* __restrict__ seq_first_chunk, int heads, int dim,
+                       int vdim, int vp) {
+    constexpr int AHEAD = 8;
+    pdl_wait();
+    pdl_launch_dependents();
+    const int seq = blockIdx.x, h = blockIdx.y, quads = vp >> 2;
+    const int e = blockIdx.z * 128 + threadIdx.x;
+    if (e >= dim * quads) return;
+    const int d = e / quads, j = (e - d * quads) * 4;
+    const int c0 = seq_first_chunk[seq], c1 = seq_first_chunk[seq + 1], count = seq_count[seq];
+    if (c1 <= c0) return;
     const float g = decay[h];
-    float* cell = state + ((size_t)seq_slots[b] * heads + h) * per_head + e;
-    float run = *cell;
-    // g^32 and g^seg_len as the chunk kernel's chain of products makes them
-    float g32 = 1.f;
-    for (int n = 0; n < 32; ++n) g32 *= g;
-    float g_run = 1.f;
-    for (int n = 0; n < seg_len / 32; ++n) g_run *= g32;
-    for (int s = s0; s < s1; ++s) {
-        int len = min(seg_len, count - (s - s0) * seg_len);
-        float p = g_run;
-        if (len < seg_len) {  // the last, shorter run: whole chunks, then the rest
-            p = 1.f;
-            for (int n = 0; n < len / 32; ++n) p *= g32;
-            float rest = 1.f;
-            for (int n = 0; n < len % 32; ++n) rest *= g;
-            p *= rest;
-        }
-        float* u = seg_state + ((size_t)s * heads + h) * per_head + e;
-        float after = fmaf(p, run, *u);
-        *u = run;
-        run = after;
+    float g_chunk = 1.f, g_last = 1.f;  // as decay_powers makes them
+    const int last = count - (c1 - c0 - 1) * kChunkTokens;
+    for (int n = 0; n < kChunkTokens; ++n) {
+        g_chunk *= g;
+        if (n < last) g_last *= g;
     }
-    *cell = run;
+    float* own = chunk_state + ((size_t)c0 * heads + h) * dim * vp + (size_t)d * vp + j;
+    const size_t step = (size_t)heads * dim * vp;
+    float* slot = state + ((size_t)seq_slots[seq] * heads + h) * dim * vdim + (size_t)d * vdim + j;
+    float run[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) run[v] = j + v < vdim ? slot[v] : 0.f;
+    for (int c = c0; c < c1; c += AHEAD) {
+        float4 add[AHEAD];
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k)
+            if (c + k < c1) add[k] = load4(own + (size_t)(c - c0 + k) * step);
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k) {
+            if (c + k >= c1) break;
+            store4(own + (size_t)(c - c0 + k) * step, make_float4(run[0], run[1], run[2], run[3]));
+            const float f = c + k == c1 - 1 ? g_last : g_chunk;
+            run[0] = fmaf(f, run[0], add[k].x);
+            run[1] = fmaf(f, run[1], add[k].y);
+            run[2] = fmaf(f, run[2], add[k].z);
+            run[3] = fmaf(f, run[3], add[k].w);
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+        if (j + v < vdim) slot[v] = run[v];
 }
 
-// ... and this one adds to every token of a run what the state before the run gives it:
-// o_i += g^(i + 1) S_before^T q_i, i counted within the run.
-template <typename T, int DR4>
-__global__ void __launch_bounds__(256)
-retention_carry_kernel(const T* __restrict__ qkvg, const float* __restrict__ freq,
-                       const float* __restrict__ decay, const float* __restrict__ seg_state,
-                       const int* __restrict__ seq_first_row, const int* __restrict__ seq_start,
-                       const int* __restrict__ seq_count, const int* __restrict__ segments, int seg_len,
-                       float* __restrict__ o_raw, int heads, int vdim, int rot_dims, int act, float k_scale) {
-    constexpr int C = kRetChunk, dim = 32 * DR4, ld = dim + 4;
-    extern __shared__ __align__(16) float smem[];
-    float* qs = smem;             // [C][dim + 4]
-    float* Ss = qs + C * ld;      // [dim][32]
-    float* pw = Ss + dim * 32;    // [seg_len + 1]
-    const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
-    const int col = blockIdx.z * 32 + lane;
-    const int unit = segments[2 * blockIdx.x], begin = segments[2 * blockIdx.x + 1];
-    const int first = seq_first_row[unit] + begin, start = seq_start[unit] + begin;
-    const int count = min(seg_len, seq_count[unit] - begin);
-    if (count <= 0 || (begin == 0 && seq_start[unit] == 0)) return;  // (nothing before a sequence's start)
-    const bool live = col < vdim;
-    const float* S = seg_state + (((size_t)blockIdx.x * heads + h) * dim) * vdim;
-    for (int d = warp; d < dim; d += 8) Ss[d * 32 + lane] = live ? S[(size_t)d * vdim + col] : 0.f;
-    for (int it = tid; it < C * ld; it += 256) qs[it] = 0.f;
-    if (tid == 0) {
-        float p = 1.f, g = decay[h];
-        for (int n = 0; n <= seg_len; ++n) {
-            pw[n] = p;
-            p *= g;
-        }
-    }
-    const size_t row_len = (size_t)2 * heads * dim + (size_t)2 * heads * vdim;
-    const int half = rot_dims >> 1, per_tok = dim - half;
-    for (int t0 = 0; t0 < count; t0 += C) {
-        const int cnt = min(C, count - t0);
-        __syncthreads();
-        for (int it = tid; it < cnt * per_tok; it += 256) {
-            int i = it / per_tok, j = it - i * per_tok;
-            const T* qh = qkvg + (size_t)(first + t0 + i) * row_len + (size_t)h * dim;
-            if (j < half) {
-                float ang = (float)(start + t0 + i) * freq[j];
-                float c = cosf(ang), sn = sinf(ang);
-                float u = pre(qh[j], act), v = pre(qh[j + half], act);
-                qs[i * ld + j] = u * c - v * sn;
-                qs[i * ld + j + half] = v * c + u * sn;
+template <int BV>
+__global__ void __launch_bounds__(128, 3)
+retention_read_kernel(const float* __restrict__ packed, const float* __restrict__ chunk_state,
+                      const float* __restrict__ decay, const int* __restrict__ chunks,
+                      const int* __restrict__ seq_first_row, const int* __restrict__ seq_start,
+                      const int* __restrict__ seq_count, float* __restrict__ o_raw, int heads, int dim, int vdim, int vp) {
+    extern __shared__ __align__(16) float read_smem[];
+    __shared__ float pw[kChunkTokens + 1];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int h = blockIdx.y, v0 = blockIdx.z * BV;
+    const RetChunk ch = ret_chunk(chunks, seq_first_row, seq_start, seq_count, blockIdx.x);
+    decay_powers(decay[h], pw);
+    const size_t unit = (size_t)blockIdx.x * heads + h;
+    const float* q = packed + unit * packed_floats(dim, vp);
+    unsigned long long acc[8][BV / 32];
+    chunk_read_tile<BV>(q, q + (size_t)kChunkTokens * dim, ch.start > 0 ? chunk_state + unit * dim * vp : nullptr,
+                        q + (size_t)3 * kChunkTokens * dim, dim, vp, v0, ch.count, read_smem, acc,
+                        [&](int i, int j, float x) { return j <= i ? x * pw[i - j] : 0.f; },
+                        [&](int i) { return pw[i + 1]; });
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const bool whole = (vdim & 3) == 0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int t = ty * 8 + r;
+        if (t >= ch.count) continue;
+        float* row = o_raw + ((size_t)(ch.first + t) * heads + h) * vdim;
+#pragma unroll
+        for (int c = 0; c < BV / 64; ++c) {
+            const int j = v0 + c * 64 + tx * 4;
+            const float2 a = halves(acc[r][2 * c]), b = halves(acc[r][2 * c + 1]);
+            if (whole) {
+                if (j < vdim) store4(row + j, make_float4(a.x, a.y, b.x, b.y));
             } else {
-                qs[i * ld + j + half] = pre(qh[j + half], act);
-            }
-        }
-        __syncthreads();
-        const int i0 = warp * 4;
-        if (i0 < cnt) {
-            float inter[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-            for (int d = 0; d < dim; d += 4) {
-                float s0 = Ss[d * 32 + lane], s1 = Ss[(d + 1) * 32 + lane];
-                float s2 = Ss[(d + 2) * 32 + lane], s3 = Ss[(d + 3) * 32 + lane];
+                const float x[4] = {a.x, a.y, b.x, b.y};
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    float4 x = *reinterpret_cast<const float4*>(qs + (i0 + r) * ld + d);
-                    inter[r] = fmaf(x.x, s0, fmaf(x.y, s1, fmaf(x.z, s2, fmaf(x.w, s3, inter[r]))));
-                }
+                for (int e = 0; e < 4; ++e)
+                    if (j + e < vdim) row[j + e] = x[e];
             }
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-                if (live && i0 + r < cnt) {
-                    float* o = o_raw + ((size_t)(first + t0 + i0 + r) * heads + h) * vdim + col;
-                    *o = fmaf(pw[t0 + i0 + r + 1], inter[r], *o);
-                }
         }
     }
+}
+
+template <typename T>
+static int launch_chunks(const T* qkvg, const float* freq, const float* decay, float* state, const int* seq_slots,
+                         const int* seq_first_row, const int* seq_start, const int* seq_count, const int* chunks,
+                         int n_chunks, const int* seq_first_chunk, float* packed, float* chunk_state, float* o_raw,
+                         int n_seqs, int heads, int dim, int vdim, int rot_dims, int act, float k_scale,
+                         cudaStream_t stream) {
+    const int vp = (vdim + 3) & ~3, bv = vp > 64 ? 128 : 64;
+    const int pack_smem = 2 * kChunkTokens * (dim + 1) * 4, update_smem = kChunkTokens * (64 + bv) * 4;
+    const int read_smem = (bv == 128 ? chunk_read_floats<128>() : chunk_read_floats<64>()) * 4;
+    auto update = bv == 128 ? retention_update_kernel<128> : retention_update_kernel<64>;
+    auto read = bv == 128 ? retention_read_kernel<128> : retention_read_kernel<64>;
+    cudaError_t e = cudaFuncSetAttribute(retention_pack_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, pack_smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(update, cudaFuncAttributeMaxDynamicSharedMemorySize, update_smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(read, cudaFuncAttributeMaxDynamicSharedMemorySize, read_smem);
+    const int v_tiles = (vp + bv - 1) / bv;
+    if (e == cudaSuccess)
+        e = launch_dependent(retention_pack_kernel<T>, dim3(n_chunks, heads), 256, pack_smem, stream, qkvg, freq, decay,
+                             chunks, seq_first_row, seq_start, seq_count, packed, heads, dim, vdim, vp, rot_dims, act, k_scale);
+    if (e == cudaSuccess)
+        e = launch_dependent(update, dim3(n_chunks, heads, (dim + 63) / 64 * v_tiles), 128, update_smem, stream,
+                             (const float*)packed, chunk_state, heads, dim, vp);
+    if (e == cudaSuccess)
+        e = launch_dependent(retention_carry_kernel, dim3(n_seqs, heads, (dim * (vp / 4) + 127) / 128), 128, 0, stream,
+                             chunk_state, state, decay, seq_slots, seq_start, seq_count, seq_first_chunk, heads, dim, vdim, vp);
+    if (e == cudaSuccess)
+        e = launch_dependent(read, dim3(n_chunks, heads, v_tiles), 128, read_smem, stream, (const float*)packed,
+                             (const float*)chunk_state, decay, chunks, seq_first_row, seq_start, seq_count, o_raw, heads,
+                             dim, vdim, vp);
+    return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 
 // out[n, h, :] = o[n, h, :] / sqrt(mean(o[n, h, :]^2) + eps) * silu(g[n, h, :]); a warp
@@ -463,70 +425,30 @@ template <typename T>
 static int launch_retention(const void* qkvg, const float* freq, const float* decay, float* state,
                             const int* token_pos, const int* token_seq, const int* seq_slots,
                             const int* seq_first_row, const int* seq_start, const int* seq_count,
-                            const int* segments, int n_segments, const int* seq_first_segment, int seg_len,
-                            float* seg_state, float* o_raw, void* out, int n_tokens, int n_units, int heads, int dim,
+                            const int* chunks, int n_chunks, const int* seq_first_chunk, float* packed,
+                            float* chunk_state, float* o_raw, void* out, int n_tokens, int n_units, int heads, int dim,
                             int vdim, int rot_dims, float eps, int act, float k_scale, const float* norm_w,
                             int gate_kind, cudaStream_t stream) {
     dim3 grid(n_units, heads, (vdim + 31) / 32);
-    if (seq_first_row && (dim == 32 || dim == 64 || dim == 128 || dim == 256)) {
-        // a prompt step: chunks of tokens (other key sizes walk the tokens one by one below)
-        constexpr int C = kRetChunk;
-        size_t chunk_smem = (2 * (size_t)C * (dim + 4) + (size_t)dim * 32 + C * (C + 1) + C * 32 + C + 1) *
-                            sizeof(float);
-        size_t carry_smem = ((size_t)C * (dim + 4) + (size_t)dim * 32 + seg_len + 1) * sizeof(float);
-        dim3 chunk_grid(segments ? n_segments : n_units, heads, (vdim + 31) / 32);
-        cudaError_t e = cudaSuccess;
-#define NNIS_RET_CHUNK(DR4) \
-        do { \
-            auto kernel = retention_chunk_kernel<T, DR4>; \
-            if (chunk_smem > 48 * 1024) \
-                e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_smem); \
-            if (e == cudaSuccess) \
-                kernel<<<chunk_grid, 256, chunk_smem, stream>>>((const T*)qkvg, freq, decay, state, seq_slots, \
-                                                                seq_first_row, seq_start, seq_count, segments, \
-                                                                seg_len, seg_state, o_raw, heads, vdim, rot_dims, act, k_scale); \
-            if (e == cudaSuccess && segments) { \
-                retention_prefix_kernel<<<dim3(n_units, heads, (dim * vdim + 255) / 256), 256, 0, stream>>>( \
-                    seg_state, state, decay, seq_slots, seq_count, seq_first_segment, seg_len, heads, dim * vdim); \
-                auto carry = retention_carry_kernel<T, DR4>; \
-                if (carry_smem > 48 * 1024) \
-                    e = cudaFuncSetAttribute(carry, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)carry_smem); \
-                if (e == cudaSuccess) \
-                    carry<<<chunk_grid, 256, carry_smem, stream>>>((const T*)qkvg, freq, decay, seg_state, \
-                                                                   seq_first_row, seq_start, seq_count, segments, \
-                                                                   seg_len, o_raw, heads, vdim, rot_dims, act, k_scale); \
-            } \
-        } while (0)
-        if (dim == 32) NNIS_RET_CHUNK(1);
-        else if (dim == 64) NNIS_RET_CHUNK(2);
-        else if (dim == 128) NNIS_RET_CHUNK(4);
-        else NNIS_RET_CHUNK(8);
-#undef NNIS_RET_CHUNK
-        if (e != cudaSuccess) return (int)e;
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return (int)e;
-        if (norm_w) {
-            retention_gate_joined_kernel<T><<<(unsigned)n_tokens, 256, 0, stream>>>(
-                o_raw, (const T*)qkvg, norm_w, token_pos, (T*)out, heads, dim, vdim, eps, gate_kind);
-            NNIS_RETURN_LAUNCH();
-        }
-        long long gate_units = (long long)n_tokens * heads;
-        retention_gate_kernel<T><<<(unsigned)((gate_units + 7) / 8), 256, 0, stream>>>(
-            o_raw, (const T*)qkvg, token_pos, (T*)out, gate_units, heads, dim, vdim, eps, gate_kind);
-        NNIS_RETURN_LAUNCH();
-    }
-    size_t smem = (2 * (size_t)dim + 256) * sizeof(float);
     cudaError_t le = cudaSuccess;
+    if (chunks) {  // a prompt step, chunks of tokens side by side (other key sizes walk the tokens one by one below)
+        int rc = launch_chunks<T>((const T*)qkvg, freq, decay, state, seq_slots, seq_first_row, seq_start, seq_count,
+                                  chunks, n_chunks, seq_first_chunk, packed, chunk_state, o_raw, n_units, heads, dim,
+                                  vdim, rot_dims, act, k_scale, stream);
+        if (rc != NNIS_OK) return rc;
+    } else {
+        size_t smem = (2 * (size_t)dim + 256) * sizeof(float);
 #define NNIS_RET_CASE(R) \
-    le = launch_dependent(retention_scan_kernel<T, R>, grid, 256, smem, stream, (const T*)qkvg, freq, decay, state, \
-                          token_pos, token_seq, seq_slots, seq_first_row, seq_start, seq_count, o_raw, heads, dim, \
-                          vdim, rot_dims, act, k_scale)
-    if (dim <= 32) NNIS_RET_CASE(4);
-    else if (dim <= 64) NNIS_RET_CASE(8);
-    else if (dim <= 128) NNIS_RET_CASE(16);
-    else NNIS_RET_CASE(32);
+        le = launch_dependent(retention_scan_kernel<T, R>, grid, 256, smem, stream, (const T*)qkvg, freq, decay, state, \
+                              token_pos, token_seq, seq_slots, seq_first_row, seq_start, seq_count, o_raw, heads, dim, \
+                              vdim, rot_dims, act, k_scale)
+        if (dim <= 32) NNIS_RET_CASE(4);
+        else if (dim <= 64) NNIS_RET_CASE(8);
+        else if (dim <= 128) NNIS_RET_CASE(16);
+        else NNIS_RET_CASE(32);
 #undef NNIS_RET_CASE
-    if (le != cudaSuccess) return (int)le;
+        if (le != cudaSuccess) return (int)le;
+    }
     if (norm_w) {
         le = launch_dependent(retention_gate_joined_kernel<T>, (unsigned)n_tokens, 256, 0, stream,
                               (const float*)o_raw, (const T*)qkvg, norm_w, token_pos, (T*)out, heads, dim, vdim, eps,
@@ -547,17 +469,17 @@ using namespace nnis;
 // `seq_first_row` null: every row is a sequence of its own bringing one token
 // (`n_units` = n_tokens); else `n_units` sequences with their first row, first
 // position and token count.  `o_raw`: float32 scratch [n_tokens, heads * vdim].
-// `segments` (optional, prompt steps): int32 [n_segments, 2] = (sequence, first token of
-// the run among the sequence's tokens of this step), runs of `seg_len` tokens in the order
-// of the sequences, with `seq_first_segment` [n_units + 1] and `seg_state` float32
-// [n_segments, heads, dim, vdim]: the runs are worked side by side.
+// `chunks` (prompt steps, key sizes 32, 64, 128 and 256; without it the tokens are walked one by one): int32
+// [n_chunks, 2] = (sequence, first token of the chunk among the sequence's tokens of this step), 64 tokens each in the
+// order of the sequences, with `seq_first_chunk` [n_units + 1] and, vp = vdim rounded up to a multiple of four, float32
+// scratch `packed` [n_chunks, heads, 64 (3 dim + vp)] and `chunk_state` [n_chunks, heads, dim, vp].
 // `act` 1: q, k, v through silu; `k_scale`: the keys' multiplier; `norm_w` (float32 [heads * vdim]): one
 // norm over the joined heads with this weight instead of a norm per head; `gate_kind` 0 silu, 1 sigmoid.
 NNIS_API int nnis_retention(const void* qkvg, const float* freq, const float* decay, float* state,
                             const int* token_pos, const int* token_seq, const int* seq_slots,
                             const int* seq_first_row, const int* seq_start, const int* seq_count,
-                            const int* segments, int n_segments, const int* seq_first_segment, int seg_len,
-                            float* seg_state, float* o_raw, void* out, int n_tokens, int n_units, int heads, int dim,
+                            const int* chunks, int n_chunks, const int* seq_first_chunk, float* packed,
+                            float* chunk_state, float* o_raw, void* out, int n_tokens, int n_units, int heads, int dim,
                             int vdim, int rot_dims, float eps, int act, float k_scale, const float* norm_w,
                             int gate_kind, int dtype, cudaStream_t stream) {
     if (n_tokens <= 0 || n_units <= 0 || heads <= 0 || dim <= 0 || vdim <= 0 || rot_dims < 0 ||
@@ -565,20 +487,18 @@ NNIS_API int nnis_retention(const void* qkvg, const float* freq, const float* de
         !token_pos || !token_seq || !seq_slots || !o_raw || !out)
         return NNIS_ERR_ARGUMENT;
     if (seq_first_row && (!seq_start || !seq_count)) return NNIS_ERR_ARGUMENT;
-    // runs side by side: only for prompt steps of key sizes the chunk kernel takes
-    if (segments && (!seq_first_row || n_segments <= 0 || !seq_first_segment || !seg_state || seg_len <= 0 ||
-                     seg_len % 32 || seg_len > 4096 || !(dim == 32 || dim == 64 || dim == 128 || dim == 256)))
+    if (chunks && (!seq_first_row || n_chunks <= 0 || !seq_first_chunk || !packed || !chunk_state ||
+                   !(dim == 32 || dim == 64 || dim == 128 || dim == 256)))
         return NNIS_ERR_ARGUMENT;
+    if (chunks && ((uintptr_t)packed | (uintptr_t)chunk_state | (uintptr_t)o_raw) % 16) return NNIS_ERR_ALIGNMENT;
     if (dim > 256 || heads > 65535 || (vdim + 31) / 32 > 65535) return NNIS_ERR_UNSUPPORTED;
     if (dtype == NNIS_DTYPE_F32)
         return launch_retention<float>(qkvg, freq, decay, state, token_pos, token_seq, seq_slots,
-                                       seq_first_row, seq_start, seq_count, segments, n_segments,
-                                       seq_first_segment, seg_len, seg_state, o_raw, out, n_tokens,
-                                       n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, stream);
+                                       seq_first_row, seq_start, seq_count, chunks, n_chunks,
+                                       seq_first_chunk, packed, chunk_state, o_raw, out, n_tokens, n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, stream);
     if (dtype == NNIS_DTYPE_BF16)
         return launch_retention<bf16>(qkvg, freq, decay, state, token_pos, token_seq, seq_slots,
-                                      seq_first_row, seq_start, seq_count, segments, n_segments,
-                                      seq_first_segment, seg_len, seg_state, o_raw, out, n_tokens,
-                                      n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, stream);
+                                      seq_first_row, seq_start, seq_count, chunks, n_chunks,
+                                      seq_first_chunk, packed, chunk_state, o_raw, out, n_tokens, n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, stream);
     return NNIS_ERR_UNSUPPORTED;
 }

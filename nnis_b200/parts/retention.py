@@ -11,11 +11,10 @@ the residual stream.  S [heads, dim, vdim] is float32, starts at zero and is the
 layer's whole memory of a sequence: it lives in the cache's state area, one per
 slot, so a later chunk or a single token goes on from what the tokens before left.
 
-Single tokens update the state in registers.  Prompts go 32 tokens at a time (the
-recurrence written as three small products per chunk, all float32); a long prompt is
-cut into runs of 256 tokens that start from zero side by side, after which the states
-between the runs are put together in order and every token receives what the tokens
-before its run contribute.
+Single tokens update the state in registers.  Prompts go 64 tokens at a time (the
+recurrence written as three products per chunk, all float32): what every chunk adds to
+the state, all chunks side by side; the state before each chunk, in order; the outputs,
+all chunks side by side again.
 
 Variants, each a parameter: ``activation`` "silu" passes q, k and v through silu before the
 recurrence (lightning attention's form); ``key_scale`` replaces dim^-1/2 (1.0: no scale);
@@ -105,16 +104,14 @@ class Retention(Part):
         return 2.0 * sum(counts) * (W * 2 * H * (self.dim + self.vdim) + H * self.vdim * W
                                     + 2 * H * self.dim * self.vdim)
 
-    SEGMENTS, FIRST_SEGMENT = "retention/segments", "retention/first_segment"
+    CHUNKS, FIRST_CHUNK = "retention/chunks", "retention/first_chunk"
 
     def step_tables(self, counts, starts, have=()):
-        """Prompt steps with a sequence longer than a run: the runs of every sequence, worked
-        side by side (the same list for every retention layer of the model)."""
-        seg = ops.RETENTION_SEGMENT
-        if not ops.retention_takes_segments(self.dim) or max(counts) <= seg or self.SEGMENTS in have:
+        """The chunks of every sequence of a prompt step (the same list for every retention layer of the model)."""
+        if not ops.retention_takes_chunks(self.dim) or self.CHUNKS in have:
             return {}
-        segments, first = ops.retention_segments(counts, seg)
-        return {self.SEGMENTS: segments, self.FIRST_SEGMENT: first}
+        chunks, first = ops.scan_segments(counts, ops.RETENTION_CHUNK)
+        return {self.CHUNKS: chunks, self.FIRST_CHUNK: first}
 
     def forward(self, x: torch.Tensor, ctx, residual: torch.Tensor, cache: StateView) -> None:
         n = residual.shape[0]
@@ -123,14 +120,17 @@ class Retention(Part):
         linear(x, self.w_in, None, qkvg, STORE, decode=ctx.decode)
         o_raw = ws.get("retention_o", (n, H * self.vdim), torch.float32)
         gated = ws.get("retention_gated", (n, H * self.vdim), self.dtype)
-        segments = ctx.tables.get(self.SEGMENTS) if ops.retention_takes_segments(self.dim) else None
-        seg_state = ws.get("retention_runs", (segments.shape[0], H, self.dim, self.vdim), torch.float32) \
-            if segments is not None else None
+        chunks = ctx.tables.get(self.CHUNKS) if ops.retention_takes_chunks(self.dim) else None
+        packed = chunk_state = None
+        if chunks is not None:
+            sizes = ops.retention_scratch(chunks.shape[0], H, self.dim, self.vdim)
+            packed = ws.get("retention_packed", (sizes[0],), torch.float32)
+            chunk_state = ws.get("retention_chunk_state", (sizes[1],), torch.float32)
         ops.retention(qkvg, self.position.frequencies(), self._decay, cache.state, ctx.token_pos,
                       ctx.token_seq, ctx.seq_slots, ctx.seq_first_row, ctx.seq_start, ctx.seq_count,
                       o_raw, gated, H, self.dim, self.vdim, self.position.dims, self.eps,
-                      segments=segments, seq_first_segment=ctx.tables.get(self.FIRST_SEGMENT),
-                      seg_state=seg_state, seg_len=ops.RETENTION_SEGMENT,
+                      chunks=chunks, seq_first_chunk=ctx.tables.get(self.FIRST_CHUNK), packed=packed,
+                      chunk_state=chunk_state,
                       activation=self.activation == "silu",
                       key_scale=None if self.key_scale is None else float(self.key_scale),
                       norm_weight=self.norm_weight, gate=self.gate)

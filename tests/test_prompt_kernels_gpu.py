@@ -150,3 +150,60 @@ def test_cached_latent_rows_one_after_another(rank, rot):
         rows = min(64, lengths[s] - 64 * p)
         want[64 * b:64 * b + rows, :rank + rot] = cache[int(table[s, p]), 0, :rows]
     assert torch.equal(torch.cat([c, r], 1).cpu(), want)
+
+
+@pytest.mark.parametrize("dim,vdim", [(32, 1), (64, 30), (128, 256), (256, 200), (128, 64)])
+@pytest.mark.parametrize("dtype,act", [("float32", True), ("bfloat16", False)])
+def test_retention_of_prompts_in_chunks(dim, vdim, dtype, act):
+    """Sequences of one token, a chunk, a chunk and one, several; fresh ones and ones with a state; a token whose values
+    are infinite is not felt before it."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim + vdim)
+    H, new, starts, rot = 2, [1, 64, 65, 200, 130], [0, 7, 0, 64, 0], dim // 2
+    n, decay = sum(new), torch.tensor([0.97, 0.3])
+    rows = torch.randn(n, 2 * H * (dim + vdim), generator=g).to(getattr(torch, dtype))
+    last = n - 20  # in the last sequence's last chunk but one
+    rows[last, 2 * H * dim:2 * H * dim + H * vdim] = math.inf if not act else 1.0
+    freq = 100.0 ** (-torch.arange(rot // 2, dtype=torch.float32) / rot)
+    state = torch.randn(9, H, dim, vdim, generator=g)
+    slots = [3, 0, 8, 5, 1]
+    for s, st in zip(slots, starts):
+        if st == 0:
+            state[s] = 0.0
+    chunks, first = o.scan_segments(new, o.RETENTION_CHUNK)
+    sizes = o.retention_scratch(len(chunks), H, dim, vdim)
+    o_raw = torch.full((n, H * vdim), 5.0, device=DEV)
+    out = torch.empty(n, H * vdim, dtype=rows.dtype, device=DEV)
+    got_state = state.to(DEV)
+    pos = [st + t for st, c in zip(starts, new) for t in range(c)]
+    seq = [i for i, c in enumerate(new) for _ in range(c)]
+    o.retention(rows.to(DEV), freq.to(DEV), decay.to(DEV), got_state, i32(pos), i32(seq), i32(slots),
+                i32([sum(new[:i]) for i in range(len(new))]), i32(starts), i32(new), o_raw, out, H, dim, vdim, rot, 1e-5,
+                chunks=torch.from_numpy(chunks).to(DEV), seq_first_chunk=torch.from_numpy(first).to(DEV),
+                packed=torch.full((sizes[0],), math.nan, device=DEV),
+                chunk_state=torch.full((sizes[1],), math.nan, device=DEV), activation=act)
+    x = rows.double()
+    x = x * torch.sigmoid(x) if act else x
+    q, k = (x[:, i * H * dim:(i + 1) * H * dim].reshape(n, H, dim).clone() for i in (0, 1))
+    v = x[:, 2 * H * dim:2 * H * dim + H * vdim].reshape(n, H, vdim)
+    ang = torch.tensor(pos, dtype=torch.float32)[:, None] * freq[None, :]
+    c, s = torch.cos(ang.double())[:, None], torch.sin(ang.double())[:, None]
+    half = rot // 2
+    for y in (q, k):
+        a, b = y[..., :half].clone(), y[..., half:rot].clone()
+        y[..., :half], y[..., half:rot] = a * c - b * s, b * c + a * s
+    k = k * dim ** -0.5
+    want, row = torch.empty(n, H, vdim, dtype=torch.float64), 0
+    for i, cnt in enumerate(new):
+        S = state[slots[i]].double()
+        for _ in range(cnt):
+            S = decay.double()[:, None, None] * S + k[row][:, :, None] * v[row][:, None, :]
+            want[row] = torch.einsum("hdv,hd->hv", S, q[row])
+            row += 1
+        if torch.isfinite(S).all():
+            err = (got_state[slots[i]].cpu().double() - S).abs().max() / S.abs().max()
+            assert err < 2e-6, (i, float(err))
+    fine = n if act else last
+    err = (o_raw.cpu().double()[:fine] - want.reshape(n, -1)[:fine]).abs().max() / want[:fine].abs().max()
+    assert err < 2e-6, float(err)  # sums of at most 64 + dim products of order one and a rounding per chunk: a few ulps
+    assert act or not torch.isfinite(o_raw[last]).any()
