@@ -539,6 +539,21 @@ NNIS_API int nnis_delta_prep(const float* a, const float* conv_w, float* tail, c
     return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 
+// The convolutions' state moved on alone, after nnis_delta_prompt has read it.
+NNIS_API int nnis_delta_conv_tail(const float* a, float* tail, const int* token_pos, const int* token_seq,
+                                  const int* seq_slots, const int* seq_first_row, const int* seq_count, int n_units,
+                                  int H, int G, int dim, int vdim, int taps, cudaStream_t stream) {
+    if (n_units <= 0 || H <= 0 || G <= 0 || dim <= 0 || vdim <= 0 || taps < 1 || !a || !tail || !token_pos ||
+        !token_seq || !seq_slots || (seq_first_row && !seq_count))
+        return NNIS_ERR_ARGUMENT;
+    if (taps == 1) return NNIS_OK;
+    const int conv_cols = 2 * G * dim + H * vdim;
+    cudaError_t e = launch_dependent(delta_conv_tail_kernel, dim3(n_units, (conv_cols + 255) / 256), 256, 0, stream, a,
+                                     tail, token_pos, token_seq, seq_slots, seq_first_row, seq_count, conv_cols,
+                                     conv_cols + H * vdim + 2 * H, taps);
+    return e == cudaSuccess ? NNIS_OK : (int)e;
+}
+
 namespace nnis {
 
 template <int KL, int SKL, int SKS, int SNC>

@@ -2082,6 +2082,53 @@ def delta_scan(qkv: torch.Tensor, beta_g: torch.Tensor, state: torch.Tensor, tok
            "delta_scan", 3 if segments is not None else 1)
 
 
+DELTA_CHUNK = 64       # tokens of a chunk of delta_prompt
+DELTA_CHUNK_MIN = 64   # prompts whose longest sequence has more tokens run in chunks
+
+
+def delta_takes_chunks(dim: int, vdim: int) -> bool:
+    """Key and value sizes of which a prompt's chunks are worked side by side."""
+    return dim in (64, 128) and vdim <= 512
+
+
+def delta_prompt(a: torch.Tensor, conv_w: torch.Tensor, tail: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
+                 state: torch.Tensor, token_pos: torch.Tensor, token_seq: torch.Tensor, seq_slots: torch.Tensor,
+                 seq_first_row: torch.Tensor, seq_count: torch.Tensor, chunks: torch.Tensor,
+                 seq_first_chunk: torch.Tensor, buffer, o_raw: torch.Tensor, heads: int, kv_heads: int, dim: int,
+                 vdim: int, unit_eps: float, q_scale: float) -> None:
+    """What ``delta_prep`` and ``delta_scan`` do for a prompt step, from the projection's rows to o_raw [n, heads *
+    vdim], the sequences' states and the convolutions' tails, a chunk of DELTA_CHUNK tokens at a time (``chunks``,
+    ``seq_first_chunk`` of ``scan_segments``).  ``buffer(name, shape, dtype)`` hands out scratch."""
+    _seq_tables(token_pos, token_seq, seq_slots, seq_first_row, seq_count)
+    _cuda(a, conv_w, tail, a_log, dt_bias, state, chunks, seq_first_chunk, o_raw)
+    n, channels, taps = a.shape[0], 2 * kv_heads * dim + heads * vdim, conv_w.shape[1]
+    _need(delta_takes_chunks(dim, vdim) and seq_first_row is not None, "delta_prompt: a prompt step of sizes it takes")
+    _need(a.dtype == torch.float32 and a.shape[1] == channels + heads * vdim + 2 * heads,
+          "delta_prompt: float32 rows [q | k | v | gate | b | a]")
+    _need(conv_w.dtype == tail.dtype == torch.float32 and conv_w.shape[0] == channels and conv_w.is_contiguous()
+          and tail.dim() == 3 and tuple(tail.shape[1:]) == (max(taps - 1, 1), channels),
+          "delta_prompt: float32 conv_w [channels, taps], tail [slots, taps - 1, channels]")
+    _need(a_log.dtype == dt_bias.dtype == state.dtype == o_raw.dtype == torch.float32
+          and a_log.numel() == dt_bias.numel() == heads and tuple(state.shape[1:]) == (heads, dim, vdim)
+          and o_raw.numel() >= n * heads * vdim, "delta_prompt: float32 a_log, dt_bias [heads], state, o_raw")
+    seqs, c = seq_first_row.numel(), chunks.shape[0]
+    _need(chunks.dtype == seq_first_chunk.dtype == torch.int32 and chunks.dim() == 2 and chunks.shape[1] == 2
+          and seq_first_chunk.numel() == seqs + 1, "delta_prompt: chunks int32 [n, 2], seq_first_chunk [sequences + 1]")
+    vp, f = -(-vdim // 4) * 4, torch.float32
+    scratch = [buffer("delta_chunk_qk", (c, kv_heads, 3 * DELTA_CHUNK * dim), f),
+               buffer("delta_chunk_u", (c, heads, DELTA_CHUNK, vp), f), buffer("delta_chunk_w", (c, heads, dim, DELTA_CHUNK), f),
+               buffer("delta_chunk_state", (c, heads, dim, vp), f), buffer("delta_chunk_beta", (c, heads, DELTA_CHUNK), f),
+               buffer("delta_chunk_logs", (c, heads, DELTA_CHUNK), torch.float64)]
+    _check(_lib().nnis_delta_prompt(_ptr(a), _ptr(conv_w), _ptr(tail), _ptr(a_log), _ptr(dt_bias), _ptr(state),
+                                    _ptr(seq_slots), _ptr(seq_first_row), _ptr(seq_count), _ptr(chunks), c,
+                                    _ptr(seq_first_chunk), *(_ptr(t) for t in scratch), _ptr(o_raw), seqs, heads, kv_heads,
+                                    dim, vdim, taps, ctypes.c_float(unit_eps), ctypes.c_float(q_scale), _stream()),
+           "delta_prompt", 4)
+    _check(_lib().nnis_delta_conv_tail(_ptr(a), _ptr(tail), _ptr(token_pos), _ptr(token_seq), _ptr(seq_slots),
+                                       _ptr(seq_first_row), _ptr(seq_count), seqs, heads, kv_heads, dim, vdim, taps,
+                                       _stream()), "delta_conv_tail", 1 if taps > 1 else 0)
+
+
 DELTA_SEGMENT = int(os.environ.get("NNIS_DELTA_SEGMENT", "128"))  # tokens of a run of the delta rule; 0: no runs
 
 

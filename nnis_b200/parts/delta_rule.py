@@ -106,10 +106,17 @@ class GatedDeltaRule(Part):
                                     + 3 * H * self.dim * self.vdim)
 
     SEGMENTS, FIRST_SEGMENT = "delta/segments", "delta/first_segment"
+    CHUNKS, FIRST_CHUNK = "delta/chunks", "delta/first_chunk"
 
     def step_tables(self, counts, starts, have=()):
-        """Prompt steps with a sequence longer than two runs: the runs of every sequence, worked side
-        by side (the same list for every delta rule layer of the model)."""
+        """Prompt steps with a sequence longer than a chunk: the chunks of every sequence (the same list for every delta
+        rule layer of the model that takes them).  Sizes that do not run in chunks, and a sequence longer than two
+        runs: the runs of every sequence, worked side by side."""
+        if ops.delta_takes_chunks(self.dim, self.vdim):
+            if max(counts) <= ops.DELTA_CHUNK_MIN or self.CHUNKS in have:
+                return {}
+            chunks, first = ops.scan_segments(counts, ops.DELTA_CHUNK)
+            return {self.CHUNKS: chunks, self.FIRST_CHUNK: first}
         seg = ops.DELTA_SEGMENT
         if seg <= 0 or max(counts) <= 2 * seg or self.SEGMENTS in have:
             return {}
@@ -121,12 +128,27 @@ class GatedDeltaRule(Part):
         H, G, ws = self.heads, self.kv_heads, ctx.workspace
         rows = ws.get("delta_in", (n, self.w_in.shape[0]), torch.float32)
         linear(x, self.w_in, None, rows, STORE_F32, decode=ctx.decode)
+        o_raw = ws.get("delta_o", (n, H * self.vdim), torch.float32)
+        chunks = ctx.tables.get(self.CHUNKS) if not ctx.decode and ops.delta_takes_chunks(self.dim, self.vdim) else None
+        if chunks is not None:
+            ops.delta_prompt(rows, self.conv, cache.extra[0], self.a_log, self.dt_bias, cache.state, ctx.token_pos,
+                             ctx.token_seq, ctx.seq_slots, ctx.seq_first_row, ctx.seq_count, chunks,
+                             ctx.tables[self.FIRST_CHUNK], ws.get, o_raw, H, G, self.dim, self.vdim, self.unit_eps,
+                             self.dim ** -0.5)
+        else:
+            self._walk(ctx, rows, cache, o_raw, n)
+        gated = ws.get("delta_gated", (n, H * self.vdim), self.dtype)
+        ops.delta_finish(o_raw, rows, self.channels, self.norm, ctx.token_pos, gated, H, self.vdim, self.eps)
+        linear(gated, self.w_o, None, residual, ADD_F32, ws, decode=ctx.decode)
+
+    def _walk(self, ctx, rows, cache, o_raw, n: int) -> None:
+        """The recurrence token by token, long prompts in runs."""
+        H, G, ws = self.heads, self.kv_heads, ctx.workspace
         qkv = ws.get("delta_qkv", (n, self.channels), torch.float32)
         beta_g = ws.get("delta_beta_g", (n, 2 * H), torch.float32)
         ops.delta_prep(rows, self.conv, cache.extra[0], self.a_log, self.dt_bias, ctx.token_pos, ctx.token_seq,
                        ctx.seq_slots, ctx.seq_first_row, ctx.seq_count, qkv, beta_g, H, G, self.dim, self.vdim,
                        self.unit_eps, self.dim ** -0.5)
-        o_raw = ws.get("delta_o", (n, H * self.vdim), torch.float32)
         segments = ctx.tables.get(self.SEGMENTS) if not ctx.decode else None
         runs = segments.shape[0] if segments is not None else 0
         ops.delta_scan(qkv, beta_g, cache.state, ctx.token_pos, ctx.token_seq, ctx.seq_slots, ctx.seq_first_row,
@@ -135,9 +157,6 @@ class GatedDeltaRule(Part):
                        seg_state=ws.get("delta_run_state", (runs, H, self.dim, self.vdim), torch.float32) if runs else None,
                        seg_trans=ws.get("delta_run_trans", (runs, H, self.dim, self.dim), torch.float32) if runs else None,
                        q_run=ws.get("delta_run_q", (n, H, self.dim), torch.float32) if runs else None)
-        gated = ws.get("delta_gated", (n, H * self.vdim), self.dtype)
-        ops.delta_finish(o_raw, rows, self.channels, self.norm, ctx.token_pos, gated, H, self.vdim, self.eps)
-        linear(gated, self.w_o, None, residual, ADD_F32, ws, decode=ctx.decode)
 
 
 MIXERS.register("gated_delta_rule", GatedDeltaRule)

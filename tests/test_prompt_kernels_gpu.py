@@ -207,3 +207,53 @@ def test_retention_of_prompts_in_chunks(dim, vdim, dtype, act):
     err = (o_raw.cpu().double()[:fine] - want.reshape(n, -1)[:fine]).abs().max() / want[:fine].abs().max()
     assert err < 2e-6, float(err)  # sums of at most 64 + dim products of order one and a rounding per chunk: a few ulps
     assert act or not torch.isfinite(o_raw[last]).any()
+
+
+@pytest.mark.parametrize("dim,vdim,taps", [(64, 30, 4), (128, 128, 4), (64, 200, 1), (128, 64, 3)])
+@pytest.mark.parametrize("slow", [True, False])
+def test_delta_rule_of_prompts_in_chunks(dim, vdim, taps, slow):
+    """Against the walk token by token and the recurrence in 64 bits: sequences of one token, a chunk, a chunk and one,
+    several, that go on from states and convolution inputs; decays near one, and fast ones among which some are zero."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim + vdim + taps)
+    H, G, new = 4, 2, [1, 64, 65, 200, 130]
+    n, channels = sum(new), 2 * G * dim + H * vdim
+    rows = torch.randn(n, channels + H * vdim + 2 * H, generator=g)
+    if not slow:
+        rows[70:90, -1] = 1e4  # the last head's decay is zero there
+    conv = torch.randn(channels, taps, generator=g).to(DEV)
+    a_log = (torch.empty(H).uniform_(-7.0, -4.0, generator=g) if slow else torch.empty(H).uniform_(-1.0, 1.0, generator=g)).to(DEV)
+    bias = torch.empty(H).uniform_(-1.0, 1.0, generator=g).to(DEV)
+    begin = torch.randn(9, H, dim, vdim, generator=g) * 0.3
+    tails = torch.randn(9, max(taps - 1, 1), channels, generator=g)
+    slots, first, count = i32([3, 0, 8, 5, 1]), i32([sum(new[:i]) for i in range(len(new))]), i32(new)
+    pos, seq = i32([t + 9 for c in new for t in range(c)]), i32([i for i, c in enumerate(new) for _ in range(c)])
+    rd = rows.to(DEV)
+    qkv, beta_g = torch.empty(n, channels, device=DEV), torch.empty(n, 2 * H, device=DEV)
+    state, tail, walked = begin.to(DEV), tails.to(DEV), torch.empty(n, H * vdim, device=DEV)
+    o.delta_prep(rd, conv, tail, a_log, bias, pos, seq, slots, first, count, qkv, beta_g, H, G, dim, vdim, 1e-6, dim ** -0.5)
+    o.delta_scan(qkv, beta_g, state, pos, seq, slots, first, count, walked, H, G, dim, vdim)
+    chunks, first_chunk = o.scan_segments(new, o.DELTA_CHUNK)
+    state2, tail2, got = begin.to(DEV), tails.to(DEV), torch.full((n, H * vdim), math.nan, device=DEV)
+    o.delta_prompt(rd, conv, tail2, a_log, bias, state2, pos, seq, slots, first, count, torch.from_numpy(chunks).to(DEV),
+                   torch.from_numpy(first_chunk).to(DEV),
+                   lambda name, shape, dtype: torch.full(shape, math.nan, dtype=dtype, device=DEV), got, H, G, dim, vdim,
+                   1e-6, dim ** -0.5)
+    assert torch.equal(tail, tail2)
+    x, bg = qkv.double().cpu(), beta_g.double().cpu()
+    q, k = (x[:, i * G * dim:(i + 1) * G * dim].view(n, G, dim).repeat_interleave(H // G, 1) for i in (0, 1))
+    v, want, row = x[:, 2 * G * dim:].view(n, H, vdim), torch.empty(n, H, vdim, dtype=torch.float64), 0
+    finals = begin.double().clone()
+    for i, c in enumerate(new):
+        S = begin[int(slots[i])].double()
+        for _ in range(c):
+            S = bg[row, H:, None, None] * S
+            u = bg[row, :H, None] * (v[row] - torch.einsum("hdv,hd->hv", S, k[row]))
+            S = S + k[row][:, :, None] * u[:, None, :]
+            want[row] = torch.einsum("hdv,hd->hv", S, q[row])
+            row += 1
+        finals[int(slots[i])] = S
+    # (a few hundred float32 roundings of values of order one, on either way: 1e-5 of the largest is some 80 ulps)
+    for y, s in ((walked, state), (got, state2)):
+        assert (y.cpu().double() - want.reshape(n, -1)).abs().max() < 1e-5 * want.abs().max()
+        assert (s.cpu().double() - finals).abs().max() < 1e-5 * finals.abs().max()
