@@ -17,7 +17,7 @@
 // keep): a token costs 2.2 dim vdim + 64 (dim + vdim) multiply-adds or so instead of 2.3 times three dim vdim, all but the chain side
 // by side, and a thread's 8 x 8 outputs share what is read.
 // Two prompts of 2,048 and 555 tokens, 32 heads over 16 key heads of 128 x 128, on a B200: prep 201, walk 707, prefix 270
-// and apply 235 us before; now pack 79, solve 148, chain 331 and read 132.
+// and apply 235 us before; now pack 79, solve 148, chain 256 and read 132.
 #include "async_copy.cuh"
 #include "common.cuh"
 #include "linear_chunks.cuh"
@@ -272,12 +272,29 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, fl
     float* us = u0s + kDC * CW;         // [64][32]: U times e^(c - c_j)
     float* ss = us + kDC * CW;          // [DIM][32]
     float* red = ss + DIM * CW;         // [8][64][32] or [SPLIT][DIM][32]
-    __shared__ float left[kDC];
-    __shared__ float whole;
+    __shared__ float left[2][kDC], whole[2];
+    __shared__ int mine;
     pdl_wait();
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int seq = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * CW, g = h / (H / G);
+    const int h = blockIdx.y, col0 = blockIdx.x * CW, g = h / (H / G), n_seqs = gridDim.z;
+    // The longest sequences first: CTAs start in the order of their numbers, one to an SM, and a walk is serial (a prompt
+    // of 2,048 tokens beside one of 555 in the order of the batch: 331 us, so 256).
+    if (n_seqs <= 64) {
+        if (tid < n_seqs) {
+            const int n = seq_first_chunk[tid + 1] - seq_first_chunk[tid];
+            int rank = 0;
+            for (int s = 0; s < n_seqs; ++s) {
+                const int m = seq_first_chunk[s + 1] - seq_first_chunk[s];
+                rank += m > n || (m == n && s < tid);
+            }
+            if (rank == (int)blockIdx.z) mine = tid;
+        }
+    } else if (tid == 0) {
+        mine = blockIdx.z;
+    }
+    __syncthreads();
+    const int seq = mine;
     const int c0 = seq_first_chunk[seq], c1 = seq_first_chunk[seq + 1];
     if (c1 <= c0) return;
     float* slot = state + ((size_t)seq_slots[seq] * H + h) * DIM * vdim;
@@ -305,13 +322,14 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, fl
     };
     bring_w(c0);
     bring_k(c0);
+    if (tid < kDC) {
+        const double* lg = logs + ((size_t)c0 * H + h) * kDC;
+        left[0][tid] = expf((float)(lg[kDC - 1] - lg[tid]));
+        if (tid == 0) whole[0] = expf((float)lg[kDC - 1]);
+    }
     for (int c = c0; c < c1; ++c) {
         const size_t unit = (size_t)c * H + h;
-        if (tid < kDC) {
-            const double end = logs[unit * kDC + kDC - 1];
-            left[tid] = expf((float)(end - logs[unit * kDC + tid]));
-            if (tid == 0) whole = expf((float)end);
-        }
+        const int now = (c - c0) & 1;
         copy_wait<1>();   // W and U0 (K may still be on its way)
         __syncthreads();  // ... and the state
         for (int it = tid; it < DIM * CW / 4; it += 256) {  // the state before the chunk
@@ -357,12 +375,18 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, fl
             }
             const int t = it >> 3, j = col0 + (it & 7) * 4;
             if (j < vp) store4(u + unit * kDC * vp + (size_t)t * vp + j, x);
-            const float f = left[t];
+            const float f = left[now][t];
             store4(us + it * 4, make_float4(x.x * f, x.y * f, x.z * f, x.w * f));
         }
         copy_wait<0>();   // K
         __syncthreads();
         bring_w(c + 1);   // (W and U0 are done with)
+        double log_end = 0.0, log_own = 0.0;  // the next chunk's, on their way under the product
+        if (tid < kDC && c + 1 < c1) {
+            const double* lg = logs + (unit + H) * kDC;
+            log_end = lg[kDC - 1];
+            log_own = lg[tid];
+        }
         {   // K^T U: a split takes KT tokens; 8 rows and 8 columns of the state a thread
             constexpr int TPS = 256 / SPLIT;  // threads of a split: DIM / 8 x 4
             const int split = tid / TPS, t = tid % TPS, tx = t & 3, ty = t >> 2;
@@ -393,9 +417,13 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, fl
                 *reinterpret_cast<ulonglong2*>(to + 16 + tx * 4) = make_ulonglong2(acc[i][2], acc[i][3]);
             }
         }
+        if (tid < kDC) {
+            left[now ^ 1][tid] = expf((float)(log_end - log_own));
+            if (tid == 0) whole[now ^ 1] = expf((float)log_end);
+        }
         __syncthreads();
         bring_k(c + 1);
-        const float keep = whole;
+        const float keep = whole[now];
         for (int it = tid; it < DIM * CW / 4; it += 256) {
             const float4 s = load4(ss + it * 4);
             float4 x = make_float4(s.x * keep, s.y * keep, s.z * keep, s.w * keep);
@@ -406,7 +434,7 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, fl
             }
             store4(ss + it * 4, x);
         }
-        __syncthreads();  // the sums, `left` and `whole` are read
+        __syncthreads();  // the sums are read
     }
     copy_wait<0>();
     for (int it = tid; it < DIM * CW; it += 256) {
@@ -484,7 +512,7 @@ NNIS_API int nnis_delta_prompt(const float* a, const float* conv_w, const float*
         !conv_w || !tail || !a_log || !dt_bias || !state || !seq_slots || !seq_first_row || !seq_count || !chunks ||
         !seq_first_chunk || !qk || !u || !w || !before || !beta || !logs || !o_raw)
         return NNIS_ERR_ARGUMENT;
-    if ((dim != 64 && dim != 128) || vdim > 512 || taps > 64 || 2 * G + H + 1 > 65535) return NNIS_ERR_UNSUPPORTED;
+    if ((dim != 64 && dim != 128) || vdim > 512 || taps > 64 || 2 * G + H + 1 > 65535 || n_seqs > 65535) return NNIS_ERR_UNSUPPORTED;
     if (((uintptr_t)conv_w | (uintptr_t)qk | (uintptr_t)u | (uintptr_t)w | (uintptr_t)before | (uintptr_t)o_raw) % 16)
         return NNIS_ERR_ALIGNMENT;
     const int vp = (vdim + 3) & ~3, bv = vp > 64 ? 128 : 64, width = dim > vdim ? dim : vdim;
@@ -508,7 +536,7 @@ NNIS_API int nnis_delta_prompt(const float* a, const float* conv_w, const float*
         e = launch_dependent(solve, dim3(n_chunks, H), 128, solve_smem, stream, (const float*)qk, (const float*)u,
                              (const float*)beta, (const double*)logs, w, u, H, G, vp);
     if (e == cudaSuccess)
-        e = launch_dependent(chain, dim3(n_seqs, H, (vp + 31) / 32), 256, chain_smem, stream, (const float*)qk,
+        e = launch_dependent(chain, dim3((vp + 31) / 32, H, n_seqs), 256, chain_smem, stream, (const float*)qk,
                              (const float*)w, u, (const double*)logs, before, state, seq_slots, seq_count, seq_first_chunk,
                              H, G, vdim, vp);
     if (e == cudaSuccess)
