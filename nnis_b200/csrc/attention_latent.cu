@@ -84,6 +84,63 @@ latent_prep_kernel(const float* __restrict__ a, const float* __restrict__ wq,
     }
 }
 
+// The same for ranks of multiples of four, up to 1,024 and 512, with rows on 16-byte borders: both norms' rows are asked
+// for at once and their sums meet at one barrier.
+template <typename T>
+__global__ void __launch_bounds__(128)
+latent_prep_quads_kernel(const float* __restrict__ a, const float* __restrict__ wq,
+                         const float* __restrict__ wkv, const float* __restrict__ freq,
+                         const int* __restrict__ token_pos, const int* __restrict__ token_seq,
+                         const int* __restrict__ page_table, int table_cols, T* __restrict__ cq,
+                         T* __restrict__ cache, int q_rank, int kv_rank, int rot, int rot_dims,
+                         int page_size, float eps, int neighbours) {
+    __shared__ float sums[2][4];
+    const int tid = threadIdx.x, n = blockIdx.x, q4 = q_rank >> 2, c4 = kv_rank >> 2;
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 g0 = tid < q4 ? load4(wq + 4 * tid) : none, g1 = tid + 128 < q4 ? load4(wq + 4 * (tid + 128)) : none;
+    const float4 gc = tid < c4 ? load4(wkv + 4 * tid) : none;  // (the weights depend on no kernel)
+    pdl_wait();
+    pdl_launch_dependents();
+    const int pos = token_pos[n];
+    if (pos < 0) return;  // a padding row
+    const int page = page_table[(size_t)token_seq[n] * table_cols + pos / page_size];
+    const float* row = a + (size_t)n * (q_rank + kv_rank + rot);
+    const float* c = row + q_rank;
+    const float4 x0 = tid < q4 ? load4(row + 4 * tid) : none, x1 = tid + 128 < q4 ? load4(row + 4 * (tid + 128)) : none;
+    const float4 xc = tid < c4 ? load4(c + 4 * tid) : none;
+    auto squares = [](float4 v) { return fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))); };
+    const float sq = warp_sum(squares(x0) + squares(x1)), sc = warp_sum(squares(xc));
+    if ((tid & 31) == 0) {
+        sums[0][tid >> 5] = sq;
+        sums[1][tid >> 5] = sc;
+    }
+    __syncthreads();
+    const float s = 1.0f / sqrtf((sums[0][0] + sums[0][1] + sums[0][2] + sums[0][3]) / (float)q_rank + eps);
+    const float z = 1.0f / sqrtf((sums[1][0] + sums[1][1] + sums[1][2] + sums[1][3]) / (float)kv_rank + eps);
+    T* q_out = cq + (size_t)n * q_rank;
+    T* dst = cache + ((size_t)page * page_size + pos % page_size) * (size_t)(kv_rank + rot);
+    auto scaled = [](float4 v, float f, float4 g) {
+        return make_float4((v.x * f) * g.x, (v.y * f) * g.y, (v.z * f) * g.z, (v.w * f) * g.w);
+    };
+    if (tid < q4) store4(q_out + 4 * tid, scaled(x0, s, g0));
+    if (tid + 128 < q4) store4(q_out + 4 * (tid + 128), scaled(x1, s, g1));
+    if (tid < c4) store4(dst + 4 * tid, scaled(xc, z, gc));
+    const float* kr = c + kv_rank;
+    const int half = rot_dims >> 1;
+    for (int j = tid; j < rot - half; j += 128) {
+        if (j < half) {
+            const float ang = (float)pos * freq[j];
+            const float cs = cosf(ang), sn = sinf(ang);
+            const int i0 = neighbours ? 2 * j : j, i1 = neighbours ? 2 * j + 1 : j + half;
+            const float u = kr[i0], v = kr[i1];
+            dst[kv_rank + i0] = from_float<T>(u * cs - v * sn);
+            dst[kv_rank + i1] = from_float<T>(v * cs + u * sn);
+        } else {
+            dst[kv_rank + j + half] = from_float<T>(kr[j + half]);
+        }
+    }
+}
+
 // The cached rows of whole sequences, page by page, into two buffers whose rows follow one another: the latents
 // [R, kv_rank], and the rotated part padded to 64 values [R, 64].  A CTA per page: `blocks` = (sequence, page); rows
 // past the sequence's last position are zero.  Bound by latency: 4 MB at 3,359 rows of 576 values take 10 us.
@@ -302,13 +359,15 @@ NNIS_API int nnis_latent_prep(const float* a, const float* wq, const float* wkv,
         rot_dims > rot || page_size <= 0 || table_cols <= 0 || !(eps > 0.f) || !a || !wq || !wkv ||
         !freq || !cq || !cache)
         return NNIS_ERR_ARGUMENT;
+    const bool quads = q_rank % 4 == 0 && q_rank <= 1024 && kv_rank % 4 == 0 && kv_rank <= 512 && rot % 4 == 0 &&
+                       ((uintptr_t)a | (uintptr_t)wq | (uintptr_t)wkv | (uintptr_t)cq | (uintptr_t)cache) % 16 == 0;
     cudaError_t e;
     if (dtype == NNIS_DTYPE_F32)
-        e = launch_dependent(latent_prep_kernel<float>, n_tokens, 128, 0, stream, a, wq, wkv, freq, token_pos,
+        e = launch_dependent(quads ? latent_prep_quads_kernel<float> : latent_prep_kernel<float>, n_tokens, 128, 0, stream, a, wq, wkv, freq, token_pos,
                              token_seq, page_table, table_cols, (float*)cq, (float*)cache, q_rank, kv_rank, rot,
                              rot_dims, page_size, eps, neighbours);
     else if (dtype == NNIS_DTYPE_BF16)
-        e = launch_dependent(latent_prep_kernel<bf16>, n_tokens, 128, 0, stream, a, wq, wkv, freq, token_pos,
+        e = launch_dependent(quads ? latent_prep_quads_kernel<bf16> : latent_prep_kernel<bf16>, n_tokens, 128, 0, stream, a, wq, wkv, freq, token_pos,
                              token_seq, page_table, table_cols, (bf16*)cq, (bf16*)cache, q_rank, kv_rank, rot,
                              rot_dims, page_size, eps, neighbours);
     else

@@ -32,6 +32,7 @@
 // A row whose position is -1 (padding) is skipped everywhere.
 #include "async_copy.cuh"
 #include "common.cuh"
+#include "row_quads.cuh"
 
 namespace nnis {
 
@@ -504,6 +505,37 @@ delta_finish_kernel(const float* __restrict__ o_raw, const float* __restrict__ g
     }
 }
 
+// The same for heads of a multiple of four values, at most 128 Q, with rows on 16-byte borders.
+template <typename T, int Q>
+__global__ void __launch_bounds__(256)
+delta_finish_quads_kernel(const float* __restrict__ o_raw, const float* __restrict__ gate_rows, int gate_stride,
+                          int gate_off, const float* __restrict__ w, const int* __restrict__ token_pos,
+                          T* __restrict__ out, long long n_units, int heads, int vdim, float eps) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (unit >= n_units) return;
+    const int lane = threadIdx.x & 31, n4 = vdim >> 2;
+    const long long n = unit / heads;
+    T* dst = out + (size_t)unit * vdim;
+    if (token_pos[n] < 0) {
+        for (int i = lane; i < n4; i += 32) store4(dst + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
+        return;
+    }
+    const float* gate = gate_rows + (size_t)n * gate_stride + gate_off + (size_t)(unit - n * heads) * vdim;
+    finish_head<T, Q>(o_raw + (size_t)unit * vdim, dst, n4, eps, lane, [&](int i) {
+        const float4 z = load4(gate + 4 * i), g = load4(w + 4 * i);
+        return make_float4(g.x * (z.x / (1.0f + expf(-z.x))), g.y * (z.y / (1.0f + expf(-z.y))),
+                           g.z * (z.z / (1.0f + expf(-z.z))), g.w * (z.w / (1.0f + expf(-z.w))));
+    });
+}
+
+template <typename T>
+static auto delta_finish_of(int vdim, bool quads) {
+    return !quads ? delta_finish_kernel<T> : vdim <= 128 ? delta_finish_quads_kernel<T, 1>
+           : vdim <= 256 ? delta_finish_quads_kernel<T, 2> : delta_finish_quads_kernel<T, 4>;
+}
+
 }  // namespace nnis
 
 using namespace nnis;
@@ -632,12 +664,14 @@ NNIS_API int nnis_delta_finish(const float* o_raw, const float* gate_rows, int g
     if (n_tokens <= 0 || heads <= 0 || vdim <= 0 || !(eps > 0.f) || !o_raw || !gate_rows || !w || !token_pos || !out)
         return NNIS_ERR_ARGUMENT;
     const long long units = (long long)n_tokens * heads;
+    const bool quads = vdim % 4 == 0 && vdim <= 512 && gate_stride % 4 == 0 && gate_off % 4 == 0 &&
+                       ((uintptr_t)o_raw | (uintptr_t)gate_rows | (uintptr_t)w | (uintptr_t)out) % 16 == 0;
     cudaError_t e;
     if (dtype == NNIS_DTYPE_F32)
-        e = launch_dependent(delta_finish_kernel<float>, (unsigned)((units + 7) / 8), 256, 0, stream, o_raw, gate_rows,
+        e = launch_dependent(delta_finish_of<float>(vdim, quads), (unsigned)((units + 7) / 8), 256, 0, stream, o_raw, gate_rows,
                              gate_stride, gate_off, w, token_pos, (float*)out, units, heads, vdim, eps);
     else if (dtype == NNIS_DTYPE_BF16)
-        e = launch_dependent(delta_finish_kernel<bf16>, (unsigned)((units + 7) / 8), 256, 0, stream, o_raw, gate_rows,
+        e = launch_dependent(delta_finish_of<bf16>(vdim, quads), (unsigned)((units + 7) / 8), 256, 0, stream, o_raw, gate_rows,
                              gate_stride, gate_off, w, token_pos, (bf16*)out, units, heads, vdim, eps);
     else
         return NNIS_ERR_UNSUPPORTED;

@@ -5,6 +5,7 @@
 // activation are computed in float32 and rounded once on the store.
 #include "async_copy.cuh"
 #include "common.cuh"
+#include "row_quads.cuh"
 
 #include <stdlib.h>
 #include <string.h>
@@ -39,6 +40,23 @@ __global__ void embed_kernel(const T* __restrict__ table, const int* __restrict_
     for (int i = threadIdx.x; i < width; i += blockDim.x) out[i] = bad ? 0.f : to_float(row[i]) * scale;
 }
 
+// The same, four neighbours a load (rows of a multiple of four values).
+template <typename T>
+__global__ void __launch_bounds__(256)
+embed_quads_kernel(const T* __restrict__ table, const int* __restrict__ tokens, float* __restrict__ hidden, int n_quads,
+                   int vocab, int* __restrict__ status, float scale) {
+    const int n = blockIdx.x, token = tokens[n];
+    const bool bad = token < 0 || token >= vocab;
+    if (bad && threadIdx.x == 0) atomicExch(status, 1);
+    const T* row = table + (size_t)(bad ? 0 : token) * n_quads * 4;
+    float* out = hidden + (size_t)n * n_quads * 4;
+    for (int i = threadIdx.x; i < n_quads; i += 256) {
+        const float4 v = load4(row + 4 * i);
+        store4(out + 4 * i, bad ? make_float4(0.f, 0.f, 0.f, 0.f)
+                                : make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale));
+    }
+}
+
 // ---------------------------------------------------------------------------
 // y = (x * 1/sqrt(mean(x^2) + eps)) * w, one block per output row; `rows`
 // (optional) picks the input row of each output row.
@@ -70,6 +88,41 @@ __global__ void rmsnorm_kernel(const float* __restrict__ x, const int* __restric
     float s = scale_s;
     T* out = y + (size_t)r * width;
     for (int i = threadIdx.x; i < width; i += blockDim.x) out[i] = from_float<T>((in[i] * s) * w[i]);
+}
+
+// The same for rows of a multiple of four values, at most 1,024 Q: a CTA of 256 threads a row, the row and the weights in
+// registers.  1,850 rows of 2,048: 10.5 -> 5.2 us on a B200 (23 MB, 4.4 TB/s).
+template <typename T, int Q>
+__global__ void __launch_bounds__(256)
+rmsnorm_quads_kernel(const float* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ w,
+                     T* __restrict__ y, int width, float eps) {
+    __shared__ float partial[8];
+    const int tid = threadIdx.x, n4 = width >> 2, r = blockIdx.x;
+    float4 g[Q], v[Q];
+#pragma unroll
+    for (int j = 0; j < Q; ++j) g[j] = tid + 256 * j < n4 ? load4(w + 4 * (tid + 256 * j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    pdl_wait();  // (the weights depend on no kernel)
+    pdl_launch_dependents();
+    const float* in = x + (size_t)(rows ? rows[r] : r) * width;
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < Q; ++j) {
+        v[j] = tid + 256 * j < n4 ? load4(in + 4 * (tid + 256 * j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        ss = fmaf(v[j].x, v[j].x, fmaf(v[j].y, v[j].y, fmaf(v[j].z, v[j].z, fmaf(v[j].w, v[j].w, ss))));
+    }
+    ss = warp_sum(ss);
+    if ((tid & 31) == 0) partial[tid >> 5] = ss;
+    __syncthreads();
+    float total = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) total += partial[k];
+    const float s = 1.0f / sqrtf(total * (1.0f / (float)width) + eps);
+    T* out = y + (size_t)r * width;
+#pragma unroll
+    for (int j = 0; j < Q; ++j)
+        if (tid + 256 * j < n4)
+            store4(out + 4 * (tid + 256 * j), make_float4((v[j].x * s) * g[j].x, (v[j].y * s) * g[j].y,
+                                                          (v[j].z * s) * g[j].z, (v[j].w * s) * g[j].w));
 }
 
 // The same for many rows of moderate width (a multiple of 4, at most 1,024): a
@@ -226,6 +279,47 @@ group_rmsnorm_kernel(const float* x, const int* __restrict__ rows,
     for (int i = lane; i < gw; i += 32) out[i] = from_float<T>((in[i] * s) * wg[i]);
 }
 
+// The same for groups of a multiple of four values, at most 128 Q: the run and its weights in registers.
+template <typename T, int Q>
+__global__ void __launch_bounds__(256)
+group_rmsnorm_quads_kernel(const float* x, const int* __restrict__ rows, const float* __restrict__ w, T* y,
+                           long long n_units, int width, int groups, float eps) {
+    const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (unit >= n_units) {
+        pdl_wait();
+        pdl_launch_dependents();
+        return;
+    }
+    const int lane = threadIdx.x & 31, gw = width / groups;
+    const long long r = unit / groups;
+    const int g = (int)(unit - r * groups);
+    RowQuads<Q> weight, run;
+    weight.load(w + (size_t)g * gw, gw >> 2, lane);  // (depend on no kernel)
+    pdl_wait();
+    pdl_launch_dependents();
+    run.load(x + (size_t)(rows ? rows[r] : r) * width + (size_t)g * gw, gw >> 2, lane);
+    const float s = 1.0f / sqrtf(warp_sum(run.squares()) / (float)gw + eps);
+    T* out = y + (size_t)r * width + (size_t)g * gw;
+#pragma unroll
+    for (int j = 0; j < Q; ++j)
+        if (lane + 32 * j < gw >> 2)
+            store4(out + 4 * (lane + 32 * j),
+                   make_float4((run.v[j].x * s) * weight.v[j].x, (run.v[j].y * s) * weight.v[j].y,
+                               (run.v[j].z * s) * weight.v[j].z, (run.v[j].w * s) * weight.v[j].w));
+}
+
+template <typename T>
+static cudaError_t launch_group_rmsnorm(const float* x, const int* rows, const float* w, T* y, long long units, int width,
+                                        int groups, float eps, cudaStream_t stream) {
+    const unsigned blocks = (unsigned)((units + 7) / 8);
+    const int gw = width / groups;
+    auto kernel = group_rmsnorm_kernel<T>;
+    if (gw % 4 == 0 && gw <= 1024 && ((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) % 16 == 0)
+        kernel = gw <= 128 ? group_rmsnorm_quads_kernel<T, 1> : gw <= 256 ? group_rmsnorm_quads_kernel<T, 2>
+                 : gw <= 512 ? group_rmsnorm_quads_kernel<T, 4> : group_rmsnorm_quads_kernel<T, 8>;
+    return launch_dependent(kernel, blocks, 256, 0, stream, x, rows, w, y, units, width, groups, eps);
+}
+
 // ---------------------------------------------------------------------------
 // a += b, float32, elementwise: where two branches of a layer that ran side by side meet
 // in the residual stream.
@@ -318,7 +412,14 @@ NNIS_API int nnis_embed(const void* table, int dtype, const int* tokens, float* 
                         int n_tokens, int width, int vocab, int* status, float scale, cudaStream_t stream) {
     if (n_tokens <= 0 || width <= 0 || vocab <= 0 || !status) return NNIS_ERR_ARGUMENT;
     int threads = width >= 256 ? 256 : 64;
-    if (dtype == NNIS_DTYPE_F32)
+    const bool quads = width % 4 == 0 && ((uintptr_t)table | (uintptr_t)hidden) % 16 == 0;
+    if (quads && dtype == NNIS_DTYPE_F32)
+        embed_quads_kernel<float><<<n_tokens, 256, 0, stream>>>((const float*)table, tokens, hidden, width / 4, vocab,
+                                                                status, scale);
+    else if (quads && dtype == NNIS_DTYPE_BF16)
+        embed_quads_kernel<bf16><<<n_tokens, 256, 0, stream>>>((const bf16*)table, tokens, hidden, width / 4, vocab,
+                                                               status, scale);
+    else if (dtype == NNIS_DTYPE_F32)
         embed_kernel<float><<<n_tokens, threads, 0, stream>>>((const float*)table, tokens, hidden,
                                                               n_tokens, width, vocab, status, scale);
     else if (dtype == NNIS_DTYPE_BF16)
@@ -329,17 +430,23 @@ NNIS_API int nnis_embed(const void* table, int dtype, const int* tokens, float* 
     NNIS_RETURN_LAUNCH();
 }
 
+template <typename T>
+static auto rmsnorm_of(int width) {
+    return width <= 1024 ? rmsnorm_quads_kernel<T, 1> : width <= 2048 ? rmsnorm_quads_kernel<T, 2>
+           : width <= 4096 ? rmsnorm_quads_kernel<T, 4> : rmsnorm_quads_kernel<T, 8>;
+}
+
 // `pdl`: launch as a programmatic dependent of the kernel before it on the stream
 // (the kernel waits for that kernel's results itself).
 NNIS_API int nnis_rmsnorm(const float* x, const int* rows, const float* w, void* y, int out_dtype,
                           int n_rows, int width, float eps, int pdl, cudaStream_t stream) {
     if (n_rows <= 0 || width <= 0 || !(eps > 0.f)) return NNIS_ERR_ARGUMENT;
     // many rows of moderate width on 16-byte boundaries: a warp per row
-    const bool by_rows = n_rows >= 64 && width % 4 == 0 && width <= 1024 &&
-                         ((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) % 16 == 0;
+    const bool quads = width % 4 == 0 && width <= 8192 && ((uintptr_t)x | (uintptr_t)w | (uintptr_t)y) % 16 == 0;
+    const bool by_rows = n_rows >= 64 && quads && width <= 1024;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(by_rows ? (n_rows + 7) / 8 : n_rows);
-    cfg.blockDim = dim3(by_rows ? 256 : (width >= 1024 ? 256 : (width >= 256 ? 128 : 32)));
+    cfg.blockDim = dim3(quads ? 256 : (width >= 1024 ? 256 : (width >= 256 ? 128 : 32)));
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -349,10 +456,10 @@ NNIS_API int nnis_rmsnorm(const float* x, const int* rows, const float* w, void*
     cudaError_t e;
     if (out_dtype == NNIS_DTYPE_F32)
         e = by_rows ? cudaLaunchKernelEx(&cfg, rmsnorm_rows_kernel<float>, x, rows, w, (float*)y, n_rows, width, eps, trace_slot("rmsnorm rows"))
-                    : cudaLaunchKernelEx(&cfg, rmsnorm_kernel<float>, x, rows, w, (float*)y, width, eps);
+                    : cudaLaunchKernelEx(&cfg, quads ? rmsnorm_of<float>(width) : rmsnorm_kernel<float>, x, rows, w, (float*)y, width, eps);
     else if (out_dtype == NNIS_DTYPE_BF16)
         e = by_rows ? cudaLaunchKernelEx(&cfg, rmsnorm_rows_kernel<bf16>, x, rows, w, (bf16*)y, n_rows, width, eps, trace_slot("rmsnorm rows"))
-                    : cudaLaunchKernelEx(&cfg, rmsnorm_kernel<bf16>, x, rows, w, (bf16*)y, width, eps);
+                    : cudaLaunchKernelEx(&cfg, quads ? rmsnorm_of<bf16>(width) : rmsnorm_kernel<bf16>, x, rows, w, (bf16*)y, width, eps);
     else
         return NNIS_ERR_UNSUPPORTED;
     return e == cudaSuccess ? NNIS_OK : (int)e;
@@ -416,14 +523,11 @@ NNIS_API int nnis_group_rmsnorm(const float* x, const int* rows, const float* w,
     if (n_rows <= 0 || width <= 0 || groups <= 0 || width % groups || !(eps > 0.f))
         return NNIS_ERR_ARGUMENT;
     long long units = (long long)n_rows * groups;
-    unsigned blocks = (unsigned)((units + 7) / 8);
     cudaError_t e;
     if (out_dtype == NNIS_DTYPE_F32)
-        e = launch_dependent(group_rmsnorm_kernel<float>, blocks, 256, 0, stream, x, rows, w, (float*)y, units,
-                             width, groups, eps);
+        e = launch_group_rmsnorm(x, rows, w, (float*)y, units, width, groups, eps, stream);
     else if (out_dtype == NNIS_DTYPE_BF16)
-        e = launch_dependent(group_rmsnorm_kernel<bf16>, blocks, 256, 0, stream, x, rows, w, (bf16*)y, units,
-                             width, groups, eps);
+        e = launch_group_rmsnorm(x, rows, w, (bf16*)y, units, width, groups, eps, stream);
     else
         return NNIS_ERR_UNSUPPORTED;
     return e == cudaSuccess ? NNIS_OK : (int)e;

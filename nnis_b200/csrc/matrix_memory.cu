@@ -30,6 +30,7 @@
 // A row whose position is -1 (padding) is skipped.
 #include "async_copy.cuh"
 #include "common.cuh"
+#include "row_quads.cuh"
 
 namespace nnis {
 
@@ -531,6 +532,33 @@ memory_out_kernel(const float* __restrict__ a, int a_cols, const double* __restr
     }
 }
 
+// The finishing kernel for heads of a multiple of four values, at most 128 Q, with rows on 16-byte borders.
+template <typename T, int Q>
+__global__ void __launch_bounds__(256)
+memory_finish_quads_kernel(const float* __restrict__ o_raw, const float* __restrict__ a, int a_cols, int gate_off,
+                           const float* __restrict__ w, const int* __restrict__ token_pos, T* __restrict__ out,
+                           long long n_units, int H, int vdim, float eps) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (unit >= n_units) return;
+    const int lane = threadIdx.x & 31, n4 = vdim >> 2;
+    const long long n = unit / H;
+    const int h = (int)(unit - n * H);
+    T* dst = out + (size_t)unit * vdim;
+    if (token_pos[n] < 0) {
+        for (int i = lane; i < n4; i += 32) store4(dst + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
+        return;
+    }
+    const float* g = a + (size_t)n * a_cols + gate_off + (size_t)h * vdim;
+    const float* wh = w + (size_t)h * vdim;
+    finish_head<T, Q>(o_raw + (size_t)unit * vdim, dst, n4, eps, lane, [&](int i) {
+        const float4 z = load4(g + 4 * i), m = load4(wh + 4 * i);
+        return make_float4(m.x * (1.0f / (1.0f + expf(-z.x))), m.y * (1.0f / (1.0f + expf(-z.y))),
+                           m.z * (1.0f / (1.0f + expf(-z.z))), m.w * (1.0f / (1.0f + expf(-z.w))));
+    });
+}
+
 // A warp per (token, head).
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -595,6 +623,12 @@ static cudaError_t launch_memory_prompt(const float* a, int a_cols, float* state
                                                               chunks, seq_first_row, seq_start, seq_count, o_raw, H,
                                                               dim, vdim, q_scale, floor_add);
     return cudaGetLastError();
+}
+
+template <typename T>
+static auto memory_finish_of(int vdim, bool quads) {
+    return !quads ? memory_finish_kernel<T> : vdim <= 128 ? memory_finish_quads_kernel<T, 1>
+           : vdim <= 256 ? memory_finish_quads_kernel<T, 2> : memory_finish_quads_kernel<T, 4>;
 }
 
 }  // namespace nnis
@@ -666,12 +700,14 @@ NNIS_API int nnis_memory_finish(const float* o_raw, const float* a, int a_cols, 
         return NNIS_ERR_ARGUMENT;
     const long long units = (long long)n_tokens * H;
     const unsigned blocks = (unsigned)((units + 7) / 8);
+    const bool quads = vdim % 4 == 0 && vdim <= 512 && a_cols % 4 == 0 && gate_off % 4 == 0 &&
+                       ((uintptr_t)o_raw | (uintptr_t)a | (uintptr_t)w | (uintptr_t)out) % 16 == 0;
     cudaError_t e;
     if (dtype == NNIS_DTYPE_F32)
-        e = launch_dependent(memory_finish_kernel<float>, blocks, 256, 0, stream, o_raw, a, a_cols, gate_off, w,
+        e = launch_dependent(memory_finish_of<float>(vdim, quads), blocks, 256, 0, stream, o_raw, a, a_cols, gate_off, w,
                              token_pos, (float*)out, units, H, vdim, eps);
     else if (dtype == NNIS_DTYPE_BF16)
-        e = launch_dependent(memory_finish_kernel<bf16>, blocks, 256, 0, stream, o_raw, a, a_cols, gate_off, w,
+        e = launch_dependent(memory_finish_of<bf16>(vdim, quads), blocks, 256, 0, stream, o_raw, a, a_cols, gate_off, w,
                              token_pos, (bf16*)out, units, H, vdim, eps);
     else
         return NNIS_ERR_UNSUPPORTED;

@@ -20,6 +20,7 @@
 #include "async_copy.cuh"
 #include "common.cuh"
 #include "linear_chunks.cuh"
+#include "row_quads.cuh"
 
 namespace nnis {
 
@@ -386,6 +387,41 @@ retention_gate_kernel(const float* __restrict__ o_raw, const T* __restrict__ qkv
     }
 }
 
+// The same for heads of a multiple of four values, at most 128 Q, with rows on 16-byte borders.
+template <typename T, int Q>
+__global__ void __launch_bounds__(256)
+retention_gate_quads_kernel(const float* __restrict__ o_raw, const T* __restrict__ qkvg,
+                            const int* __restrict__ token_pos, T* __restrict__ out, long long n_units,
+                            int heads, int dim, int vdim, float eps, int gate_kind) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (unit >= n_units) return;
+    const int lane = threadIdx.x & 31, n4 = vdim >> 2;
+    const long long n = unit / heads;
+    T* dst = out + (size_t)unit * vdim;
+    if (token_pos[n] < 0) {
+        for (int i = lane; i < n4; i += 32) store4(dst + 4 * i, make_float4(0.f, 0.f, 0.f, 0.f));
+        return;
+    }
+    const T* gate = qkvg + (size_t)n * ((size_t)2 * heads * (dim + vdim)) + (size_t)2 * heads * dim +
+                    (size_t)heads * vdim + (size_t)(unit - n * heads) * vdim;
+    finish_head<T, Q>(o_raw + (size_t)unit * vdim, dst, n4, eps, lane, [&](int i) {
+        const float4 z = load4(gate + 4 * i);
+        const float4 s = make_float4(1.0f / (1.0f + expf(-z.x)), 1.0f / (1.0f + expf(-z.y)), 1.0f / (1.0f + expf(-z.z)),
+                                     1.0f / (1.0f + expf(-z.w)));
+        return gate_kind ? s : make_float4(z.x * s.x, z.y * s.y, z.z * s.z, z.w * s.w);
+    });
+}
+
+template <typename T>
+static auto retention_gate_of(const float* o_raw, const T* qkvg, const T* out, int heads, int dim, int vdim) {
+    const bool quads = vdim % 4 == 0 && vdim <= 512 && (2 * heads * dim) % 4 == 0 &&
+                       ((uintptr_t)o_raw | (uintptr_t)qkvg | (uintptr_t)out) % 16 == 0;
+    return !quads ? retention_gate_kernel<T> : vdim <= 128 ? retention_gate_quads_kernel<T, 1>
+           : vdim <= 256 ? retention_gate_quads_kernel<T, 2> : retention_gate_quads_kernel<T, 4>;
+}
+
 // The same with ONE norm over the joined heads of a token and a weight per value:
 // out[n, :] = o[n, :] / sqrt(mean(o[n, :]^2) + eps) * w * gate(g[n, :]); a CTA per token
 template <typename T>
@@ -456,7 +492,7 @@ static int launch_retention(const void* qkvg, const float* freq, const float* de
         return le == cudaSuccess ? NNIS_OK : (int)le;
     }
     long long units = (long long)n_tokens * heads;
-    le = launch_dependent(retention_gate_kernel<T>, (unsigned)((units + 7) / 8), 256, 0, stream,
+    le = launch_dependent(retention_gate_of<T>(o_raw, (const T*)qkvg, (const T*)out, heads, dim, vdim), (unsigned)((units + 7) / 8), 256, 0, stream,
                           (const float*)o_raw, (const T*)qkvg, token_pos, (T*)out, units, heads, dim, vdim, eps,
                           gate_kind);
     return le == cudaSuccess ? NNIS_OK : (int)le;

@@ -257,3 +257,44 @@ def test_delta_rule_of_prompts_in_chunks(dim, vdim, taps, slow):
     for y, s in ((walked, state), (got, state2)):
         assert (y.cpu().double() - want.reshape(n, -1)).abs().max() < 1e-5 * want.abs().max()
         assert (s.cpu().double() - finals).abs().max() < 1e-5 * finals.abs().max()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width,groups", [(4, 1), (1028, 1), (2048, 4), (4096, 1), (8192, 2), (8196, 3), (516, 129), (30, 5)])
+@pytest.mark.parametrize("n", [1, 70])
+def test_norms_and_gather_of_rows(dtype, width, groups, n):
+    """Rows that are held whole in registers, in one, two, four and eight pieces, and rows that are not."""
+    o, dt = ops(), getattr(torch, dtype)
+    g = torch.Generator().manual_seed(width + n)
+    x, w = torch.randn(n + 3, width, generator=g), torch.randn(width, generator=g)
+    rows = torch.randperm(n + 3, generator=g)[:n].to(torch.int32)
+    pick = x[rows.long()].double()
+    out = torch.empty(n, width, dtype=dt, device=DEV)
+    o.rmsnorm(x.to(DEV), w.to(DEV), 1e-5, out, rows.to(DEV))
+    close(out, pick / torch.sqrt((pick * pick).mean(-1, keepdim=True) + 1e-5) * w.double(), dtype, "norm")
+    o.group_rmsnorm(x.to(DEV), w.to(DEV), 1e-5, groups, out, rows.to(DEV))
+    y = pick.view(n, groups, -1)
+    close(out, (y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5)).view(n, width) * w.double(), dtype, "groups")
+    table, hidden = x.to(dt), torch.empty(n, width, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    o.embed(table.to(DEV), rows.to(DEV), hidden, status)
+    assert torch.equal(hidden.cpu(), table[rows.long()].float()) and int(status) == 0
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H,vdim", [(2, 4), (4, 128), (2, 132), (2, 256), (2, 512), (2, 516), (3, 30)])
+def test_heads_normed_and_gated(dtype, H, vdim):
+    o, dt = ops(), getattr(torch, dtype)
+    g = torch.Generator().manual_seed(H * vdim)
+    n, off = 9, 8
+    raw, rows = torch.randn(n, H * vdim, generator=g), torch.randn(n, off + H * vdim + 4, generator=g)
+    pos = i32([0, 1, -1, 3, 4, 5, 6, 7, 8])
+    z, y = rows[:, off:off + H * vdim].double().view(n, H, vdim), raw.double().view(n, H, vdim)
+    y = y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-5)
+    live = (pos.cpu() >= 0).double()[:, None]
+    for w, finish, f in ((torch.randn(vdim, generator=g), o.delta_finish, z * torch.sigmoid(z)),
+                         (torch.randn(H * vdim, generator=g), o.memory_finish, torch.sigmoid(z))):
+        out = torch.full((n, H * vdim), 5.0, dtype=dt, device=DEV)
+        args = (raw.to(DEV), rows.to(DEV), off, w.to(DEV), pos, out, H, vdim, 1e-5)
+        finish(*args)
+        close(out, (y * w.double().view(-1, vdim) * f).view(n, -1) * live, dtype, finish.__name__)
