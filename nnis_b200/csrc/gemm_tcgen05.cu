@@ -18,6 +18,20 @@
 // Rows and columns beyond M, N and K are zero-filled by TMA on the way in and
 // clipped on the way out, so any M and N and any K that is a multiple of 8 work.
 //
+// PAIR: two CTAs of a cluster work a tile of 256 rows x 256 rows of W: each loads its 128 rows of A and half of the rows of
+// W, and one thread of the first CTA issues cta_group::2 products that read both halves.  A CTA of its own with a tile of
+// 128 x 128 asks L2 for 128 bytes a cycle of products, more than an SM is given (the large products stood at 600 to 1,000
+// TFLOP/s); this one asks for 64.  4,096 x 4,096 x 4,096: 132 -> 99 us (1,391 TFLOP/s); 3,359 x 2,048 x 6,144: 93 -> 68 us.
+//   - The bytes of both CTAs' loads count on the first CTA's barrier and its loaders announce them for both.  (An arrival
+//     of the second CTA for every stage, with a release to the cluster, took 2,048 x 2,048 x 2,048 from 22 to 35 us.)
+//   - Each epilogue warp sends its own 32 rows out, a box of 4 KB as soon as it is written: 3,359 x 2,048 x 2,048 in
+//     28.3 us (bfloat16) and 30.4 us (float32), against 30.6 and 31.9 with all boxes of a warp at the end, and 29.8 and
+//     34.0 with half as many warps.
+//   - Two CTAs share an SM, three stages each, while there are more than SMs; six stages otherwise.
+//   - The gated product takes 64 gate rows and the matching 64 up rows in each CTA: one product of 256 columns makes both.
+//   - One pair of CTAs per pair of SMs that walked over the tiles with two accumulators was slower: its epilogue hid under
+//     the products, but whole tiles a pair left SMs idle at the end (3,359 x 2,048 x 6,144: 82 us).
+//
 // Every wait is bounded: a wait that runs out sets a status word and an abort
 // flag that the other roles see; all warps still meet at the end, and tensor
 // memory is always freed.
@@ -75,17 +89,18 @@ struct GemmArgs {
 };
 
 // Two CTAs share an SM when their stages leave room for it.
-__host__ __device__ constexpr int gemm_ctas_per_sm(int bn, int stages, int mode, int ksub) {
-    return stages * ksub * (kBM + (mode == GEMM_GATED ? 2 : 1) * bn) * kBK * 2 <= 110 * 1024 ? 2 : 1;
+__host__ __device__ constexpr int gemm_ctas_per_sm(int bn, int stages, int mode, int ksub, bool pair = false) {
+    return stages * ksub * (kBM + (mode == GEMM_GATED ? 2 : 1) * (pair ? bn / 2 : bn)) * kBK * 2 <= 110 * 1024 ? 2 : 1;
 }
 // A warp that is alone on its scheduler runs every instruction at full latency, so
 // a CTA that has its SM alone brings eight epilogue warps, two per quarter of the
 // rows, each taking every other chunk of 32 columns; with two CTAs per SM the four
 // epilogue warps of each leave the registers for both.  The wide gate/up tile (192 + 192
 // columns, two special-function instructions a value) brings sixteen: its epilogue went
-// from 4.0 to 2.4 us of arithmetic at 2,048 rows.
-__host__ __device__ constexpr int gemm_threads(int bn, int stages, int mode, int ksub) {
-    return gemm_ctas_per_sm(bn, stages, mode, ksub) == 1 ? (bn == 192 ? 576 : 320) : 192;
+// from 4.0 to 2.4 us of arithmetic at 2,048 rows; so do pairs' tiles of 256 columns.
+__host__ __device__ constexpr int gemm_threads(int bn, int stages, int mode, int ksub, bool pair = false) {
+    return gemm_ctas_per_sm(bn, stages, mode, ksub, pair) == 1 ? (bn >= 192 && mode != GEMM_QKV ? 576 : 320)
+           : pair && mode != GEMM_QKV ? 320 : 192;
 }
 
 // MODE GEMM_GATED: W holds gate rows then up rows ([2 I, K]); the CTA multiplies
@@ -94,8 +109,8 @@ __host__ __device__ constexpr int gemm_threads(int bn, int stages, int mode, int
 // (BN = 128: two heads of 64 or one of 128).
 // SPLIT: K cut among the CTAs of a tile (GemmArgs::k_splits), a build of its own so that
 // the others carry none of it.
-template <int BN, int STAGES, int MODE, int KSUB, bool SPLIT = false>
-__global__ void __launch_bounds__(gemm_threads(BN, STAGES, MODE, KSUB), gemm_ctas_per_sm(BN, STAGES, MODE, KSUB))
+template <int BN, int STAGES, int MODE, int KSUB, bool SPLIT = false, bool PAIR = false>
+__global__ void __launch_bounds__(gemm_threads(BN, STAGES, MODE, KSUB, PAIR), gemm_ctas_per_sm(BN, STAGES, MODE, KSUB, PAIR))
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                const __grid_constant__ CUtensorMap map_out, GemmArgs g) {
     trace_mark(g.trace, 0);
@@ -104,9 +119,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     unsigned char* base = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     constexpr int NB = MODE == GEMM_GATED ? 2 : 1;  // B tiles (and accumulators) per stage
-    constexpr int kEpiWarps = gemm_threads(BN, STAGES, MODE, KSUB) / 32 - 2;
+    constexpr int kEpiWarps = gemm_threads(BN, STAGES, MODE, KSUB, PAIR) / 32 - 2;
     constexpr int kColStep = 32 * (kEpiWarps / 4);  // columns between two chunks of one warp
-    constexpr uint32_t kBytesA = kBM * kBK * 2, kBytesB = BN * kBK * 2;
+    constexpr int BL = PAIR ? BN / 2 : BN;          // columns of W (its rows) that this CTA loads
+    constexpr uint32_t kBytesA = kBM * kBK * 2, kBytesB = BL * kBK * 2;
     // tensor memory comes in powers of two of columns
     constexpr uint32_t kTmemCols = NB * BN <= 64 ? 64 : NB * BN <= 128 ? 128 : NB * BN <= 256 ? 256 : 512;
     // a stage holds KSUB slices of 64 columns of K: [KSUB] A tiles, then [KSUB][NB] W tiles
@@ -119,10 +135,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __shared__ volatile int abort_flag;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.y * kBM, n0 = blockIdx.x * BN;
-    const int expert = g.tile_expert ? g.tile_expert[blockIdx.y] : 0;
+    const int m0 = (PAIR ? blockIdx.x : blockIdx.y) * kBM, n0 = (PAIR ? blockIdx.y : blockIdx.x) * BN;
+    const int expert = !PAIR && g.tile_expert ? g.tile_expert[blockIdx.y] : 0;
     if (expert < 0) return;  // a tile of rows past the last group: nothing is allocated or awaited yet
-    const int w_row0 = expert * g.expert_rows + n0;  // this tile's first row of W
+    const uint32_t rank = PAIR ? cluster_rank() : 0;
+    const int w_row0 = expert * g.expert_rows + n0 + (int)rank * BL;  // the first row of W that this CTA loads
     const int k_slices = (g.K + kBK - 1) / kBK;
     const int k_blocks_all = (k_slices + KSUB - 1) / KSUB;
     // this CTA's run of k-blocks (all of them without a split of K)
@@ -138,7 +155,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            mbar_init(&full_bar[s], 2);   // the two loaders
+            mbar_init(&full_bar[s], 2);   // the two loaders (of a pair: the first CTA's)
             mbar_init(&empty_bar[s], 1);
         }
         mbar_init(&acc_bar, 1);
@@ -148,9 +165,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         abort_flag = 0;
         mbar_fence_init();
     }
-    if (warp == 1) tmem_alloc(&tmem_base_s, kTmemCols);
+    if (warp == 1) {
+        if constexpr (PAIR) pair_tmem_alloc(&tmem_base_s, kTmemCols);
+        else tmem_alloc(&tmem_base_s, kTmemCols);
+    }
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_meet();  // the other CTA's barriers exist, and its tensor memory
     tc_fence_after();
     const uint32_t tmem_acc = tmem_base_s;
 
@@ -160,6 +181,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     // have arrived and all bytes are there.
     auto load_stage = [&](bool loads_a, int kb) {
         const int s = kb % STAGES;
+        // The bytes of a pair count on the first CTA's barrier, whose loaders announce them for both CTAs.  (The second
+        // CTA's may land ahead of that: the phase still lacks the announcing arrival and stays open.)
+        if constexpr (PAIR) {
+            const uint32_t bar = leader_addr(&full_bar[s]);
+            if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * (loads_a ? kStageA : kStageB));
+#pragma unroll
+            for (int h = 0; h < KSUB; ++h) {
+                const int k0 = (kb * KSUB + h) * kBK;
+                if (loads_a) {
+                    pair_load_2d(tile_a + (size_t)s * kStageA + (size_t)h * kBytesA, &map_a, k0, m0, bar);
+                } else {
+                    unsigned char* b_dst = tile_b + (size_t)s * kStageB + (size_t)h * NB * kBytesB;
+                    pair_load_2d(b_dst, &map_w, k0, w_row0, bar);
+                    if (NB == 2) pair_load_2d(b_dst + kBytesB, &map_w, k0, inter + w_row0, bar);
+                }
+            }
+            return;
+        }
         // (slices beyond K arrive as zeros and are not multiplied)
         mbar_expect_tx(&full_bar[s], loads_a ? kStageA : kStageB);
 #pragma unroll
@@ -201,8 +240,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (warp == 0) {
         // nothing more: the loader of A waits for the end with its warp
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = instr_desc(kBM, BN);
+        if (lane == 0 && rank == 0) {
+            // (a pair's gate and up rows lie one after the other in either CTA: one product of 2 BN columns)
+            constexpr uint32_t idesc = instr_desc(PAIR ? 2 * kBM : kBM, PAIR ? NB * BN : BN);
+            auto mma = [](uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+                if constexpr (PAIR) pair_mma(d, a, b, idesc, acc);
+                else tc_mma(d, a, b, idesc, acc);
+            };
+            auto commit = [](uint64_t* bar) {
+                if constexpr (PAIR) pair_commit(bar);
+                else tc_commit(bar);
+            };
             const uint64_t desc_a0 = smem_desc_k128(smem_addr(tile_a));
             const uint64_t desc_b0 = smem_desc_k128(smem_addr(tile_b));
             bool ok = true;
@@ -225,17 +273,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
                     for (int k = 0; k < kBK / kUmmaK; ++k) {
                         // 16 columns of K further along the swizzled row: 32 bytes
-                        tc_mma(tmem_acc, desc_advance(da, k * kUmmaK * 2), desc_advance(db, k * kUmmaK * 2),
-                               idesc, (kb | h | k) != 0);
-                        if (NB == 2)
-                            tc_mma(tmem_acc + BN, desc_advance(da, k * kUmmaK * 2),
-                                   desc_advance(db, kBytesB + k * kUmmaK * 2), idesc, (kb | h | k) != 0);
+                        mma(tmem_acc, desc_advance(da, k * kUmmaK * 2), desc_advance(db, k * kUmmaK * 2), (kb | h | k) != 0);
+                        if (NB == 2 && !PAIR)
+                            mma(tmem_acc + BN, desc_advance(da, k * kUmmaK * 2),
+                                desc_advance(db, kBytesB + k * kUmmaK * 2), (kb | h | k) != 0);
                     }
                 }
-                tc_commit(&empty_bar[s]);  // the stage is free once these MMAs have read it
+                commit(&empty_bar[s]);  // the stage is free once these MMAs have read it
             }
-            if (!ok) abort_flag = 1;
-            tc_commit(&acc_bar);  // arrives when all MMAs above are complete (also after an abort)
+            if (!ok) {
+                abort_flag = 1;
+                if constexpr (PAIR) follower_set(&abort_flag, 1);
+            }
+            commit(&acc_bar);  // arrives when all MMAs above are complete (also after an abort)
         }
     } else {
         // epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. + 31 = tile rows
@@ -366,7 +416,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             constexpr bool split = SPLIT && MODE == GEMM_ADD_F32;
             const size_t tile_id = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
             float* tile_sums = g.split_scratch + (tile_id * (size_t)g.k_splits * kBM + row) * BN;
-            bool finishes = true;
+            bool finishes = !PAIR || m0 < g.M;  // (a pair's second CTA may have no rows)
             if constexpr (split) {
                 float* mine = tile_sums + (size_t)blockIdx.z * kBM * BN;
 #pragma unroll 1
@@ -403,8 +453,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 if (!mbar_wait(&split_done, 0)) abort_flag = 1;
                 finishes = split_last != 0 && !abort_flag;
             }
+            // The warps of a pair's CTA send their own 32 rows out in boxes of 4 KB; a box of 64 bfloat16 columns takes
+            // two chunks of one warp.
+            constexpr int kGroups = kEpiWarps / 4, kPerBox = PAIR && kOut16 ? 2 : 1;
+            constexpr int kBoxes = BN / kBoxCols / kGroups, kFit = STAGES * (int)(kStageA + kStageB) / (kEpiWarps * 4096);
+            constexpr int kSlots = !PAIR ? 1 : kBoxes < kFit ? kBoxes : kFit;
+            static_assert(!PAIR || kFit >= 1, "a box of every warp fits the ring");
+            const int group = (warp - 2) >> 2;
+            unsigned char* own_boxes = base + (size_t)(warp - 2) * (kSlots * 4096);
 #pragma unroll 1
-            for (int c0 = c_first; c0 < BN && finishes; c0 += kColStep) {
+            for (int c0 = PAIR ? group * 32 * kPerBox : c_first, i = 0; c0 < BN && finishes; ++i,
+                     c0 = PAIR ? (i / kPerBox * kGroups + group) * 32 * kPerBox + i % kPerBox * 32 : c0 + kColStep) {
+                const int box_i = i / kPerBox;
+                if (PAIR && g.out_by_tma && box_i >= kSlots && i % kPerBox == 0) {
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(kSlots - 1) : "memory");
+                    __syncwarp();
+                }
                 uint32_t v[32], u[32];
                 if constexpr (split) {
                     // the splits' sums of this row: all asked for at once (one trip to L2),
@@ -433,8 +497,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                         v[j * 4 + 3] = __float_as_uint(sum.w);
                     }
                 } else {
-                    tmem_load32_issue(lane_base + (uint32_t)c0, v);
-                    if constexpr (MODE == GEMM_GATED) tmem_load32_issue(lane_base + (uint32_t)(BN + c0), u);
+                    // (a pair's accumulator: gate then up of the first CTA's half of the columns, then of the second's)
+                    const int acc = PAIR && MODE == GEMM_GATED ? c0 / BL * BN + c0 % BL : c0;
+                    tmem_load32_issue(lane_base + (uint32_t)acc, v);
+                    if constexpr (MODE == GEMM_GATED) tmem_load32_issue(lane_base + (uint32_t)(BL + acc), u);
                     tmem_load_wait();
                 }
                 const int nb = n0 + c0;
@@ -485,7 +551,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                 }
                 if (g.out_by_tma) {
-                    unsigned char* box = stage_row + (size_t)(c0 / kBoxCols) * (kBM * 128);
+                    unsigned char* box = PAIR ? own_boxes + (box_i % kSlots) * 4096 + lane * 128
+                                              : stage_row + (size_t)(c0 / kBoxCols) * (kBM * 128);
                     if (kOut16) {
                         const int u0 = (c0 % 64) / 8;
 #pragma unroll
@@ -505,6 +572,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                             *reinterpret_cast<float4*>(box + ((j ^ (row & 7)) << 4)) =
                                 make_float4(f[j * 4], f[j * 4 + 1], f[j * 4 + 2], f[j * 4 + 3]);
                     }
+                    if (PAIR && i % kPerBox == kPerBox - 1) {
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        __syncwarp();
+                        const int col = n0 + c0 / kBoxCols * kBoxCols, m_first = m0 + quarter * 32;
+                        if (lane == 0) {
+                            const unsigned char* src = own_boxes + (box_i % kSlots) * 4096;
+                            if (col < out_cols && m_first < g.M) {
+                                if (MODE == GEMM_ADD_F32) tma_add_2d(&map_out, col, m_first, src);
+                                else tma_store_2d(&map_out, col, m_first, src);
+                            }
+                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                        }
+                    }
                 } else if (m < g.M) {
                     const size_t off = (size_t)m * out_cols + nb;
 #pragma unroll
@@ -520,7 +600,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     }
                 }
             }
-            if (g.out_by_tma && finishes) {
+            if (PAIR) {
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            } else if (g.out_by_tma && finishes) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&staged_bar);  // every epilogue warp
@@ -540,36 +622,75 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     tc_fence_before();
     __syncthreads();
+    if constexpr (PAIR) cluster_meet();  // neither CTA's memory or barriers are used by the other any more
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_acc, kTmemCols);
+        if constexpr (PAIR) pair_tmem_dealloc(tmem_acc, kTmemCols);
+        else tmem_dealloc(tmem_acc, kTmemCols);
     }
+    if constexpr (PAIR) cluster_meet();
     if (threadIdx.x == 0 && abort_flag && g.status) atomicExch(g.status, 3);
     trace_mark(g.trace, 1);
 }
 
-template <int BN, int STAGES, int MODE, int KSUB, bool SPLIT = false>
+template <int BN, int STAGES, int MODE, int KSUB, bool SPLIT = false, bool PAIR = false>
 static int launch_gemm_tc(const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap& mo,
                           const GemmArgs& g, bool pdl,
                           cudaStream_t stream) {
     constexpr int NB = MODE == GEMM_GATED ? 2 : 1;
-    size_t smem = (size_t)STAGES * KSUB * (kBM + NB * BN) * kBK * 2 + 1024;
-    auto kernel = gemm_tc_kernel<BN, STAGES, MODE, KSUB, SPLIT>;
+    size_t smem = (size_t)STAGES * KSUB * (kBM + NB * (PAIR ? BN / 2 : BN)) * kBK * 2 + 1024;
+    static_assert(STAGES * KSUB * (kBM + NB * (PAIR ? BN / 2 : BN)) * kBK * 2 + 1024 <= 227 * 1024, "one CTA's shared memory");
+    auto kernel = gemm_tc_kernel<BN, STAGES, MODE, KSUB, SPLIT, PAIR>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     int n_cols = MODE == GEMM_GATED ? g.N / 2 : g.N;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((n_cols + BN - 1) / BN, (g.M + kBM - 1) / kBM, g.k_splits);
-    cfg.blockDim = dim3(gemm_threads(BN, STAGES, MODE, KSUB));
+    const int m_tiles = (g.M + kBM - 1) / kBM;
+    const int n_tiles = (n_cols + BN - 1) / BN;
+    cfg.gridDim = PAIR ? dim3((m_tiles + 1) / 2 * 2, n_tiles) : dim3(n_tiles, m_tiles, g.k_splits);
+    cfg.blockDim = dim3(gemm_threads(BN, STAGES, MODE, KSUB, PAIR));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int attrs = 0;
+    if (PAIR) {
+        attr[attrs].id = cudaLaunchAttributeClusterDimension;
+        attr[attrs].val.clusterDim.x = 2;
+        attr[attrs].val.clusterDim.y = 1;
+        attr[attrs++].val.clusterDim.z = 1;
+    }
+    if (pdl) {
+        attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = attrs;
     e = cudaLaunchKernelEx(&cfg, kernel, ma, mw, mo, g);
     return e == cudaSuccess ? NNIS_OK : (int)e;
+}
+
+static long pair_ctas(long m_tiles, long cols, int bn) { return (m_tiles + 1) / 2 * 2 * ((cols + bn - 1) / bn); }
+
+// Which products run on pairs of CTAs: those whose tiles of 128 x 256 (gated: 128 x 128 of the output) occupy three fifths
+// of the SMs, with a K that carries the cluster's start (it does not begin under the kernel before it).  Both sides
+// measured, us alone -> in pairs, weights from memory:
+//   storing 512 x 6,144 x 2,048 (96 CTAs) 20.4 -> 18.4; 3,359 x 1,024 x 2,048 (112) 20.2 -> 18.5; 1,024 x 4,096 x 1,024
+//   (128) 13.0 -> 13.3; 2,048 x 3,072 x 576 (192) 17.1 -> 13.1; 3,359 x 2,048 x 2,048 (224) 37.4 -> 28.3, x 6,144
+//   93 -> 68; 4,096 x 4,096 x 4,096 132 -> 99; fewer: 2,048 x 1,024 x 2,048 (64) 15.2 -> 17.3, 300 x 4,096 x 4,096 (64)
+//   27.8 -> 29.1, 640 x 3,072 x 512 (72) 6.9 -> 9.1.
+static bool gemm_pairs(long m_tiles, long cols, int K, int sms) {
+    const long ctas = pair_ctas(m_tiles, cols, 256);
+    return (cols + 255) / 256 <= 65535 && 5 * ctas >= 3 * sms && K >= (ctas > sms ? 512 : 2048);
+}
+// The gated product (`cols` columns of the output) also stays with single CTAs where tiles of 192 + 192 columns take one
+// CTA per SM and pairs would take two:
+//   512 x 3,072 x 2,048 (96 CTAs) 25.0 -> 21.6; 1,024 x 2,048 x 1,024 (128) 17.1 -> 15.3; 2,048 x 1,152 x 2,048 (144)
+//   25.9 -> 22.2; 3,359 x 1,024 x 2,048 (224) 48.7 -> 29.8; 3,359 x 6,144 x 2,048 (1,344) 166 -> 147; 2,048 x 1,280 x 2,048
+//   (160, or 112 wide ones) 26.1 -> 29.5; 2,048 x 1,536 x 576 (192, or 128 wide ones) 13.5 -> 15.1.
+static bool gemm_pairs_gated(long m_tiles, long cols, int K, int sms) {
+    const long ctas = pair_ctas(m_tiles, cols, 128);
+    return (cols + 127) / 128 <= 65535 && 5 * ctas >= 3 * sms && K >= 1024 &&
+           (ctas <= sms || m_tiles * ((cols + 191) / 192) > sms);
 }
 
 // Into how many runs of k-blocks the adding product cuts K: more than one where 64-column
@@ -652,6 +773,9 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* C,
 #define NNIS_GEMM_TC128(BN, MODE, CTAS) \
     return (CTAS) <= sms ? launch_gemm_tc<BN, 3, MODE, 2>(ma, mw, mo, g, pdl != 0, stream) \
                          : launch_gemm_tc<BN, 3, MODE, 1>(ma, mw, mo, g, pdl != 0, stream)
+#define NNIS_GEMM_PAIR(BN, MODE, CTAS) \
+    return (CTAS) <= sms ? launch_gemm_tc<BN, 6, MODE, 1, false, true>(ma, mw, mo, g, pdl != 0, stream) \
+                         : launch_gemm_tc<BN, 3, MODE, 1, false, true>(ma, mw, mo, g, pdl != 0, stream)
     if (mode == GEMM_QKV) {
         if ((d != 64 && d != 128) || N != (nq + 2 * nkv) * d || !token_pos) return NNIS_ERR_UNSUPPORTED;
         if (nkv > 0 && (!token_seq || !page_table || !k_cache || !v_cache || page_size <= 0))
@@ -659,6 +783,7 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* C,
         if (!make_map(&ma, A, M, K, kBM) || !make_map(&mw, W, N, K, 128)) return NNIS_ERR_UNSUPPORTED;
         mo = ma;  // not used: this epilogue scatters rows into the cache
         g.out_by_tma = 0;
+        if (gemm_pairs(m_tiles, N, K, sms)) { NNIS_GEMM_PAIR(256, GEMM_QKV, pair_ctas(m_tiles, N, 256)); }
         NNIS_GEMM_TC128(128, GEMM_QKV, m_tiles * ((N + 127) / 128));
     }
     if (mode == GEMM_GATED) {
@@ -670,19 +795,29 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* C,
         // a decode step of many sequences, three times as many narrow tiles pull the weights
         // from memory faster: 1.7B shape at 64 rows 28 -> 18 us)
         const bool fat = N / 2 > 128 && 2 * m_tiles * ((N / 2 + 191) / 192) >= sms;
-        if (!make_map(&ma, A, M, K, kBM) || !make_map(&mw, W, N, K, fat ? 192 : 64)) return NNIS_ERR_UNSUPPORTED;
-        g.out_by_tma = (N / 2) % 8 == 0 && make_map(&mo, C, M, N / 2, kBM);
+        const bool pairs = gemm_pairs_gated(m_tiles, N / 2, K, sms);
+        if (!make_map(&ma, A, M, K, kBM) || !make_map(&mw, W, N, K, fat && !pairs ? 192 : 64)) return NNIS_ERR_UNSUPPORTED;
+        g.out_by_tma = (N / 2) % 8 == 0 && make_map(&mo, C, M, N / 2, pairs ? 32 : kBM);
         if (!g.out_by_tma) mo = ma;
+        if (pairs) { NNIS_GEMM_PAIR(128, GEMM_GATED, pair_ctas(m_tiles, N / 2, 128)); }
         if (fat) return launch_gemm_tc<192, 3, GEMM_GATED, 1>(ma, mw, mo, g, pdl != 0, stream);
         NNIS_GEMM_TC128(64, GEMM_GATED, m_tiles * ((N / 2 + 63) / 64));
     }
     long tiles128 = (long)((N + 127) / 128) * m_tiles;
     bool wide = tiles128 >= sms;
-    if (!make_map(&ma, A, M, K, kBM) || !make_map(&mw, W, N, K, wide ? 128 : 64))
+    const bool pairs = gemm_pairs(m_tiles, N, K, sms);
+    if (!make_map(&ma, A, M, K, kBM) || !make_map(&mw, W, N, K, wide || pairs ? 128 : 64))
         return NNIS_ERR_UNSUPPORTED;
-    g.out_by_tma = mode == GEMM_STORE ? (N % 8 == 0 && make_map(&mo, C, M, N, kBM))
-                                      : (N % 4 == 0 && make_map(&mo, C, M, N, kBM, 0, 4));
+    const int out_rows = pairs ? 32 : kBM;
+    g.out_by_tma = mode == GEMM_STORE ? (N % 8 == 0 && make_map(&mo, C, M, N, out_rows))
+                                      : (N % 4 == 0 && make_map(&mo, C, M, N, out_rows, 0, 4));
     if (!g.out_by_tma) mo = ma;
+    if (pairs) {
+        const long ctas = pair_ctas(m_tiles, N, 256);
+        if (mode == GEMM_STORE) { NNIS_GEMM_PAIR(256, GEMM_STORE, ctas); }
+        if (mode == GEMM_STORE_F32) { NNIS_GEMM_PAIR(256, GEMM_STORE_F32, ctas); }
+        NNIS_GEMM_PAIR(256, GEMM_ADD_F32, ctas);
+    }
 #define NNIS_GEMM_TC(MODE) \
     if (wide) NNIS_GEMM_TC128(128, MODE, tiles128); \
     NNIS_GEMM_TC64(MODE, m_tiles * ((N + 63) / 64))
@@ -696,6 +831,7 @@ static int gemm_tc_run(const void* A, const void* W, const float* bias, void* C,
         return launch_gemm_tc<64, 2, GEMM_ADD_F32, 4, true>(ma, mw, mo, g, pdl != 0, stream);
     }
     NNIS_GEMM_TC(GEMM_ADD_F32);
+#undef NNIS_GEMM_PAIR
 #undef NNIS_GEMM_TC64
 #undef NNIS_GEMM_TC128
 #undef NNIS_GEMM_TC

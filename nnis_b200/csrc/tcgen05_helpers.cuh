@@ -99,6 +99,64 @@ __device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&v)[32]) {
     tmem_load_wait();
 }
 
+// ---- a pair of CTAs (a cluster of two) that works one tile of 256 rows --------------------------------------------
+// Each CTA keeps 128 rows of A and half of B's rows in its own shared memory, at the same offsets; one thread of the
+// first CTA issues the products for both, and either CTA's tensor memory receives its own 128 rows.
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// Both CTAs; every thread of each calls it.
+__device__ __forceinline__ void cluster_meet() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of the first CTA's copy of a shared variable.
+__device__ __forceinline__ uint32_t leader_addr(const void* p) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(smem_addr(p)));
+    return r;
+}
+// Sets the second CTA's copy of a shared int; the first CTA calls it.
+__device__ __forceinline__ void follower_set(volatile int* p, int value) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 1;" : "=r"(r) : "r"(smem_addr((const void*)p)));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(r), "r"(value) : "memory");
+}
+// A tile load into this CTA's shared memory whose bytes count on the first CTA's barrier.
+__device__ __forceinline__ void pair_load_2d(void* dst_smem, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(smem_addr(dst_smem)), "l"(map), "r"(c0), "r"(c1), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void pair_tmem_alloc(uint32_t* dst_smem, uint32_t columns) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(dst_smem)), "r"(columns)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pair_tmem_dealloc(uint32_t addr, uint32_t columns) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(columns) : "memory");
+}
+__device__ __forceinline__ void pair_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                         uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// One arrival on both CTAs' copies of the barrier when the products issued so far are complete.
+__device__ __forceinline__ void pair_commit(uint64_t* bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+            smem_addr(bar)), "h"((uint16_t)3)
+        : "memory");
+}
+
 // Shared memory matrix descriptor of a K-major tile whose rows are 128 bytes
 // (64 bfloat16) and 128-byte swizzled: 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc_k128(uint32_t smem_byte_addr) {

@@ -298,3 +298,63 @@ def test_heads_normed_and_gated(dtype, H, vdim):
         args = (raw.to(DEV), rows.to(DEV), off, w.to(DEV), pos, out, H, vdim, 1e-5)
         finish(*args)
         close(out, (y * w.double().view(-1, vdim) * f).view(n, -1) * live, dtype, finish.__name__)
+
+
+# 14 tiles of rows by 8 of 256 columns (an SM for each CTA); 19 by 10 (two on an SM, the last pair's second CTA without
+# rows); rows of the output off 16-byte boundaries; tails of K
+@pytest.mark.parametrize("m,n,k", [(1700, 1928, 2056), (2400, 2312, 520), (2300, 2306, 584), (2560, 4096, 1024)])
+def test_products_on_pairs_of_ctas(m, n, k):
+    """Storing, adding and gated products large enough for pairs of CTAs against 64 bits.  A float32 sum of k products,
+    however it is grouped, is within k 2^-23 of the sum of their sizes (2^-23: sums that are cut, not rounded)."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(m + n + k)
+    a = torch.randn(m, k, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(n, k, generator=g, device=DEV) / math.sqrt(k)).bfloat16()
+    bias = torch.randn(n, generator=g, device=DEV)
+    want = a.double() @ w.double().t() + bias.double()
+    bound = k * 2.0 ** -23 * (a.double().abs() @ w.double().abs().t() + bias.double().abs()) + 1e-12
+    out = torch.full((m, n), 7.0, device=DEV)
+    o.gemm_tc(a, w, bias, out, o.STORE_F32)
+    assert bool(((out.double() - want).abs() <= bound).all())
+    base = torch.randn(m, n, generator=g, device=DEV)
+    acc = base.clone()
+    o.gemm_tc(a, w, bias, acc, o.ADD_F32)
+    total = base.double() + want
+    assert bool(((acc.double() - total).abs() <= bound + 2.0 ** -23 * total.abs()).all())
+    half = torch.full((m, n), 7.0, dtype=torch.bfloat16, device=DEV)
+    o.gemm_tc(a, w, bias, half, o.STORE)
+    assert bool(((half.double() - want).abs() <= bound + 2.0 ** -8 * want.abs()).all())
+    gated = torch.full((m, n // 2), 7.0, dtype=torch.bfloat16, device=DEV)
+    o.gemm_tc(a, w, bias, gated, o.GEMM_GATED)
+    close(gated, P.swiglu(want[:, :n // 2], want[:, n // 2:]), "bfloat16", "gated product of pairs")
+    o.check_status(DEV)
+
+
+@pytest.mark.parametrize("nq,nkv,d,m,k", [(16, 4, 128, 1100, 2048), (35, 3, 64, 2500, 576)])
+def test_qkv_products_on_pairs_of_ctas(nq, nkv, d, m, k):
+    """Heads rotated and stored from tiles of 256 columns: the same bits as the tiles of 128 that fewer rows take."""
+    o = ops()
+    g = torch.Generator(device=DEV).manual_seed(nq + m)
+    n, page = (nq + 2 * nkv) * d, 64
+    w = (torch.randn(n, k, generator=g, device=DEV) / math.sqrt(k)).bfloat16()
+    bias = torch.randn(n, generator=g, device=DEV)
+    x = torch.randn(m, k, generator=g, device=DEV).bfloat16()
+    cos, sin = (t.float().to(DEV) for t in P.rope_tables(m, d, 10000.0))
+    pos = torch.arange(m, dtype=torch.int32, device=DEV)
+    pos[m - 1] = -1  # a padding row
+    pages = -(-m // page)
+    table = torch.randperm(pages, generator=g, device=DEV).int().view(1, -1)
+
+    def product(rows):
+        q = torch.full((m, nq * d), 9.0, dtype=torch.bfloat16, device=DEV)
+        kc, vc = (torch.zeros(pages, nkv, page, d, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        for r in range(0, m, rows):
+            e = min(r + rows, m)
+            o.gemm_tc(x[r:e], w, bias, q[r:e], o.GEMM_QKV, token_pos=pos[r:e], token_seq=torch.zeros_like(pos[r:e]),
+                      page_table=table, cos=cos, sin=sin, k_cache=kc, v_cache=vc, heads=nq, kv_heads=nkv, head_dim=d,
+                      page_size=page)
+        return q, kc, vc
+
+    for whole, parts in zip(product(m), product(128)):
+        assert torch.equal(whole, parts)
+    o.check_status(DEV)
