@@ -100,8 +100,9 @@ class EngineBackend:
 
     def decode_logits(self, slot: int, token: int, again: bool) -> torch.Tensor:
         """Logits [vocab] of one sequence's next token.  A step of the SmolLM2-135M shape is 154 launches, 4.0 ms from
-        Python one by one and 0.5 ms as a replay; to capture one takes some 10 ms, so the first token that a session
-        decodes (``again`` False) captures nothing, and replays only where the graph is there already."""
+        Python one by one and 0.5 ms as a replay; to capture one takes some 10 ms, as long as three of them, so the first
+        tokens that a session decodes (``again`` False) capture nothing, and replay only where the graph is there
+        already."""
         engine = self.engine
         if self.decode_greedy is None or not (
                 again or self._decoder_key(1, engine.cache.length(slot) + 1, True) in self._decoders):
@@ -278,11 +279,13 @@ class LLM:
 class InferenceSession:
     """One sequence on one slot; logits come back to the host as float32."""
 
+    EAGER_TOKENS = 8  # that a session decodes before its step is captured
+
     def __init__(self, llm: LLM):
         self.llm = llm
         self.engine = llm.engine
         self.slot = self.engine.acquire_slot()
-        self._decoded = False  # whether this session has decoded a token
+        self._decoded = 0  # tokens that this session has decoded one by one
 
     def position(self) -> int:
         return self.engine.cache.length(self.slot)
@@ -323,8 +326,8 @@ class InferenceSession:
         return logits[0].cpu().numpy()
 
     def decode_one(self, token: int) -> np.ndarray:
-        logits = self.llm.backend.decode_logits(self.slot, int(token), self._decoded)
-        self._decoded = True
+        logits = self.llm.backend.decode_logits(self.slot, int(token), self._decoded >= self.EAGER_TOKENS)
+        self._decoded += 1
         return logits.cpu().numpy()
 
     def generate(self, input_ids: Sequence[int], generation: GenerationConfig,
