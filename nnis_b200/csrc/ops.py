@@ -1378,6 +1378,10 @@ def retention(qkvg: torch.Tensor, freq: torch.Tensor, decay: torch.Tensor, state
 
 
 RETENTION_CHUNK = 64  # tokens of a chunk
+# Prompts whose longest sequence has more tokens run in chunks, the others walk.  Whole prompts of one layer with experts, 16
+# heads of 64 / 128, us walked and in chunks: 32 tokens 366 / 385 and 410 / 422, 64 tokens 379 / 399 and 413 / 430, 100 tokens
+# 389 / 439 and 415 / 438, 128 tokens 403 / 501 and 415 / 438, 256 tokens 623 / 727 and 222 / 322.
+RETENTION_CHUNK_MIN = 96
 
 
 def retention_takes_chunks(dim: int) -> bool:
@@ -2083,7 +2087,10 @@ def delta_scan(qkv: torch.Tensor, beta_g: torch.Tensor, state: torch.Tensor, tok
 
 
 DELTA_CHUNK = 64       # tokens of a chunk of delta_prompt
-DELTA_CHUNK_MIN = 64   # prompts whose longest sequence has more tokens run in chunks
+# Prompts whose longest sequence has more tokens run in chunks.  Whole prompts of one layer of 16 heads of 64 / 128, us walked
+# and in chunks: 192 tokens 361 / 413 and 399 / 405, 256 tokens 276 / 348 and 183 / 257, 4 x 128 tokens 278 / 382 and
+# 301 / 402, 3 x 300 tokens 391 / 576 and 291 / 485.
+DELTA_CHUNK_MIN = 192
 
 
 def delta_takes_chunks(dim: int, vdim: int) -> bool:

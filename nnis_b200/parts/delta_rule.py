@@ -109,7 +109,7 @@ class GatedDeltaRule(Part):
     CHUNKS, FIRST_CHUNK = "delta/chunks", "delta/first_chunk"
 
     def step_tables(self, counts, starts, have=()):
-        """Prompt steps with a sequence longer than a chunk: the chunks of every sequence (the same list for every delta
+        """Prompt steps with a sequence long enough: the chunks of every sequence (the same list for every delta
         rule layer of the model that takes them).  Sizes that do not run in chunks, and a sequence longer than two
         runs: the runs of every sequence, worked side by side."""
         if ops.delta_takes_chunks(self.dim, self.vdim):

@@ -184,15 +184,18 @@ class LatentAttention(Part):
         """Whether a prompt step multiplies the latents out.  The operations of either way, those of the way through
         the latent's space four times: its kernels (mma.sync) run at 145 to 200 TFLOP/s, the tcgen05 ones at 600 to 800.
         A portion of a few tokens after a long past keeps the latent's space (every position of the past would be
-        multiplied out for them), and so does a step whose keys and values would take over half a gigabyte."""
+        multiplied out for them), and so does a step whose keys and values would take over half a gigabyte, and one that
+        would not save 4 G multiply-adds by that count, which is what the launches more cost (one layer of 16 heads, us in
+        the latent's space and multiplied out: heads of 128, 192 tokens 385 and 411, 300 189 and 182, 512 214 and 196, 8 x 64
+        260 and 249; heads of 32 + 64, 384 tokens 177 and 186, 512 189 and 195, 768 214 and 208, 4 x 128 213 and 218)."""
         if not self._expandable():
             return False
         rows = sum(-(-(int(c) + int(st)) // PAGE_SIZE) * PAGE_SIZE for c, st in zip(counts, starts))
         pairs = sum(int(c) * int(st) + int(c) * (int(c) + 1) // 2 for c, st in zip(counts, starts))
         up = self.kv_rank * (self.dim + self.vdim)
-        return (rows * self.heads * (self.dim + self.vdim) * 2 <= 1 << 29
-                and rows * up + pairs * (self.dim + self.rot + self.vdim)
-                <= 4 * (sum(int(c) for c in counts) * up + pairs * (2 * self.kv_rank + self.rot)))
+        saved = (4 * (sum(int(c) for c in counts) * up + pairs * (2 * self.kv_rank + self.rot))
+                 - rows * up - pairs * (self.dim + self.rot + self.vdim))
+        return rows * self.heads * (self.dim + self.vdim) * 2 <= 1 << 29 and self.heads * saved >= 1 << 32
 
     def step_tables(self, counts, starts, have=()):
         """The tiles of the tensor-core kernel for a prompt step: 64 or 128 stacked (token,

@@ -107,8 +107,9 @@ class Retention(Part):
     CHUNKS, FIRST_CHUNK = "retention/chunks", "retention/first_chunk"
 
     def step_tables(self, counts, starts, have=()):
-        """The chunks of every sequence of a prompt step (the same list for every retention layer of the model)."""
-        if not ops.retention_takes_chunks(self.dim) or self.CHUNKS in have:
+        """Prompt steps with a sequence longer than a few tokens: the chunks of every sequence (the same list for every
+        retention layer of the model)."""
+        if not ops.retention_takes_chunks(self.dim) or max(counts) <= ops.RETENTION_CHUNK_MIN or self.CHUNKS in have:
             return {}
         chunks, first = ops.scan_segments(counts, ops.RETENTION_CHUNK)
         return {self.CHUNKS: chunks, self.FIRST_CHUNK: first}
