@@ -138,7 +138,10 @@ class DecoderModel:
         if self._keeps_embedding:
             kept = ctx.workspace.get("embedding_output", (ctx.n_tokens, self.spec.hidden_size), torch.float32)
             ops.copy_async(kept, hidden)
-        ctx.hidden_copy = ctx.normed_rows = None  # (a context may run more than one step: nothing of the last one counts)
+        # (a context may run more than one step, a recorded one twice: nothing of the last one counts, and each asks for
+        # the same buffers)
+        ctx.hidden_copy = ctx.normed_rows = None
+        ctx.copy_turn = 0
         schedule = self.spec.schedule
         for i, entry in enumerate(schedule):
             if entry.enter is not None and (entry.enter.embedding or entry.enter.tensor is not None):

@@ -251,3 +251,26 @@ def test_a_layer_without_feed_forward_tolerates_a_stored_second_norm(tmp_path):
     save_file(w, path)
     with pytest.raises(WeightError, match="unexpected"):
         check_weights(d, wanted)
+
+
+def test_a_step_run_a_second_time_asks_for_the_same_buffers(monkeypatch):
+    """A step that is recorded as a graph is run twice over one context, the second time with its workspace frozen; one
+    layer without a feed-forward takes its two stream buffers in turn an odd number of times."""
+    from nnis_b200.config import config_from_dict
+    from nnis_b200.csrc import ops
+    from nnis_b200.engine.context import StepContext
+    from nnis_b200.engine.model import DecoderModel
+    from nnis_b200.engine.workspace import Workspace
+    from tazadra_models import ONLY_MAMBA
+    cpu = torch.device("cpu")
+    model = DecoderModel(config_from_dict(ONLY_MAMBA).to_spec(), torch.bfloat16, cpu)
+    for name in ("norm_scale_add", "cast_rows"):
+        monkeypatch.setattr(ops, name, lambda *args, **kwargs: None)
+    model.embedding.forward = model.blocks[0].mixer.forward = lambda *args: None
+    model._views = [None]
+    one = torch.zeros(1, dtype=torch.int32)
+    ctx = StepContext(n_tokens=1, n_seqs=1, tokens=one, token_pos=one, token_seq=one, seq_slots=one, page_tables=[],
+                      workspace=Workspace(cpu), decode=True, max_context=1)
+    model._run_blocks(ctx)
+    ctx.workspace.frozen = True
+    model._run_blocks(ctx)
