@@ -74,7 +74,8 @@ delta_pack_kernel(const float* __restrict__ a, const float* __restrict__ conv_w,
                     bt[e] = 1.0f / (1.0f + expf(-g[h]));
                     const float x = g[H + h] + dt_bias[h];
                     const float decay = expf(-expf(a_log[h]) * (x > 20.f ? x : log1pf(expf(x))));
-                    lg[e] = fmax(log((double)decay), kDeltaLeastLog);
+                    const double l = log((double)decay);
+                    lg[e] = l < kDeltaLeastLog ? kDeltaLeastLog : l;  // (a decay that is no number stays one)
                 }
             }
             double sum = lg[0] + lg[1];
@@ -83,10 +84,12 @@ delta_pack_kernel(const float* __restrict__ a, const float* __restrict__ conv_w,
                 const double x = __shfl_up_sync(0xffffffffu, sum, o);
                 if (lane >= o) sum += x;
             }
+            double before = __shfl_up_sync(0xffffffffu, sum, 1);
+            if (lane == 0) before = 0.0;
             const size_t at = ((size_t)blockIdx.x * H + h) * kDC + 2 * lane;
             beta[at] = bt[0];
             beta[at + 1] = bt[1];
-            logs[at] = sum - lg[1];
+            logs[at] = before + lg[0];
             logs[at + 1] = sum;
         }
         return;

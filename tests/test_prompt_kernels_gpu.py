@@ -259,6 +259,36 @@ def test_delta_rule_of_prompts_in_chunks(dim, vdim, taps, slow):
         assert (s.cpu().double() - finals).abs().max() < 1e-5 * finals.abs().max()
 
 
+@pytest.mark.parametrize("column", [-1, -3])  # the last head's decay gate, and its strength of writing
+def test_a_gate_of_the_delta_rule_that_is_no_number(column):
+    """It is seen from its token on, as in the walk, and not before it."""
+    o = ops()
+    g = torch.Generator().manual_seed(7)
+    H, G, dim, vdim, taps, n, at = 2, 1, 64, 32, 4, 200, 71
+    channels = 2 * G * dim + H * vdim
+    rows = torch.randn(n, channels + H * vdim + 2 * H, generator=g)
+    rows[at, column] = math.nan
+    conv, tails = torch.randn(channels, taps, generator=g).to(DEV), torch.zeros(1, taps - 1, channels, device=DEV)
+    a_log, bias, rd = torch.full((H,), -2.0, device=DEV), torch.zeros(H, device=DEV), rows.to(DEV)
+    slots, first, count, pos, seq = i32([0]), i32([0]), i32([n]), i32(list(range(n))), i32([0] * n)
+    qkv, beta_g = torch.empty(n, channels, device=DEV), torch.empty(n, 2 * H, device=DEV)
+    state, walked = torch.zeros(1, H, dim, vdim, device=DEV), torch.empty(n, H * vdim, device=DEV)
+    o.delta_prep(rd, conv, tails.clone(), a_log, bias, pos, seq, slots, first, count, qkv, beta_g, H, G, dim, vdim, 1e-6, 1.0)
+    o.delta_scan(qkv, beta_g, state, pos, seq, slots, first, count, walked, H, G, dim, vdim)
+    chunks, first_chunk = o.scan_segments([n], o.DELTA_CHUNK)
+    state2, got = torch.zeros(1, H, dim, vdim, device=DEV), torch.full((n, H * vdim), 7.0, device=DEV)
+    o.delta_prompt(rd, conv, tails.clone(), a_log, bias, state2, pos, seq, slots, first, count,
+                   torch.from_numpy(chunks).to(DEV), torch.from_numpy(first_chunk).to(DEV),
+                   lambda name, shape, dtype: torch.full(shape, math.nan, dtype=dtype, device=DEV), got, H, G, dim, vdim,
+                   1e-6, 1.0)
+    bad = torch.zeros(n, H, vdim, dtype=torch.bool)
+    bad[at:, -1] = True
+    for y, s in ((walked, state), (got, state2)):
+        assert torch.equal(torch.isnan(y.cpu()).view(n, H, vdim), bad)
+        assert torch.equal(torch.isnan(s.cpu())[0].flatten(1).all(1), bad[-1, :, 0]) and not torch.isnan(s[0, ~bad[-1, :, 0]]).any()
+    assert (walked - got)[~bad.view(n, -1)].abs().max() < 1e-5 * walked[~bad.view(n, -1)].abs().max()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("width,groups", [(4, 1), (1028, 1), (2048, 4), (4096, 1), (8192, 2), (8196, 3), (516, 129), (30, 5)])
 @pytest.mark.parametrize("n", [1, 70])
