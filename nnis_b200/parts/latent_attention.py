@@ -175,10 +175,12 @@ class LatentAttention(Part):
     def _expandable(self) -> bool:
         """Whether the tcgen05 kernel takes this layer's sizes and options."""
         return (self.dtype == torch.bfloat16 and self.q_rank > 0 and not self.window and not self.has_gate
-                and not self.has_sink and ops.attention_wide_tc_takes_expanded(self.dim, self.rot, self.vdim, self.kv_rank))
+                and not self.has_sink and self.scale > 0.0 and ops.attention_wide_tc_takes_expanded(self.dim, self.rot, self.vdim, self.kv_rank))
 
     def _expand_name(self) -> str:
         return f"latent_wide/{self.heads}x{self.dim}+{self.rot}+{self.vdim}/rank{self.kv_rank}"
+
+    EXPAND_SAVES = 1 << 32  # multiply-adds
 
     def _expands(self, counts, starts) -> bool:
         """Whether a prompt step multiplies the latents out.  The operations of either way, those of the way through
@@ -195,7 +197,12 @@ class LatentAttention(Part):
         up = self.kv_rank * (self.dim + self.vdim)
         saved = (4 * (sum(int(c) for c in counts) * up + pairs * (2 * self.kv_rank + self.rot))
                  - rows * up - pairs * (self.dim + self.rot + self.vdim))
-        return rows * self.heads * (self.dim + self.vdim) * 2 <= 1 << 29 and self.heads * saved >= 1 << 32
+        return rows * self.heads * (self.dim + self.vdim) * 2 <= 1 << 29 and self.heads * saved >= self.EXPAND_SAVES
+
+    def _takes_expanded(self, ctx) -> bool:
+        """Whether this step runs with the latents multiplied out: a layer that can asked for the tables, which another
+        layer of the same sizes, with a window say, finds there too."""
+        return self.w_kv is not None and not ctx.decode and self._expand_name() + "/units" in ctx.tables
 
     def step_tables(self, counts, starts, have=()):
         """The tiles of the tensor-core kernel for a prompt step: 64 or 128 stacked (token,
@@ -234,7 +241,7 @@ class LatentAttention(Part):
         freq = self.position.frequencies()
         down = ws.get("latent_down", (n, self.w_down.shape[0]), torch.float32)
         linear(x, self.w_down, None, down, STORE_F32, decode=ctx.decode)
-        if not ctx.decode and self._expand_name() + "/units" in ctx.tables:
+        if self._takes_expanded(ctx):
             self._forward_expanded(ctx, down, freq, table, residual, cache)
             return
         q_lat = ws.get("latent_q_abs", (n, H * self.row), self.dtype)

@@ -407,3 +407,36 @@ def test_replay_program_runs_a_model_folder(models, tmp_path):
     want = plain_logits(models, "odd", "float32", toks)
     check_logits(read_step(out, 0, cfg["vocab"]), torch.stack([want[0], want[29], want[6]]), "float32", "program")
     check_logits(read_step(out, 1, cfg["vocab"]), torch.stack([want[30], want[7]]), "float32", "program")
+
+
+def test_prompts_whose_latents_are_multiplied_out(tmp_path, monkeypatch):
+    """Both sizes of heads that the tensor-core kernel takes, in a model: whole prompts, later portions of them (keys and
+    values of the past multiplied out too), single tokens after them, and a shape that recurs, recorded and replayed."""
+    from nafezen_models import config, dense, latent, layer
+    from nnis_b200.engine import Engine, SequenceStep
+    from nnis_b200.parts.latent_attention import LatentAttention
+    cfg = config(150, 96, 1, 1e-5, [layer("latent_attention", latent(2, 128, 64, 128, 48, 64), None),
+                                    layer("latent_attention", latent(3, 64, 32, 64, 40, 72), dense(40))])
+    d = make_model(str(tmp_path), cfg, seed=81)
+    w = load_weights(d, True)
+    engine = Engine.from_dir(d, dtype="bfloat16", max_tokens=64 * 64)
+    monkeypatch.setattr(LatentAttention, "EXPAND_SAVES", 0)
+    calls, real = [], LatentAttention._forward_expanded
+    monkeypatch.setattr(LatentAttention, "_forward_expanded", lambda self, *a: (calls.append(1), real(self, *a))[1])
+    rng = random.Random(6)
+    for round_ in range(4):
+        seqs = [random_tokens(rng, 303, cfg["vocab"]), random_tokens(rng, 121, cfg["vocab"])]
+        want = [P.forward(cfg, w, t, emulate_bf16=True) for t in seqs]
+        slots, at = [engine.acquire_slot() for _ in seqs], [0, 0]
+        for counts in ([200, 70], [100, 50], [1, 1], [2, 0]):
+            batch = [SequenceStep(s, t[a:a + c], list(range(c))) for s, t, a, c in zip(slots, seqs, at, counts) if c]
+            rows = torch.cat([x[a:a + c] for x, a, c in zip(want, at, counts)])
+            before = len(calls)
+            check_logits(engine.step(batch).cpu().numpy(), rows, "bfloat16", f"round {round_}, {counts}")
+            if round_ == 0 and max(counts) > 2:
+                assert len(calls) == before + 2, counts
+            at = [a + c for a, c in zip(at, counts)]
+        for s in slots:
+            engine.release_slot(s)
+    assert len(engine._step_graphs) == 1
+    engine.check_status()

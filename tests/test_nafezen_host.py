@@ -190,3 +190,44 @@ def test_cache_groups_without_values_and_state_areas():
     assert b == a and float(cache.view(1).state[b].abs().max()) == 0.0  # a slot used again starts at zero
     cache.release(b)
     cache.check()
+
+
+def _latent_part(heads=16, dim=128, rot=64, vdim=128, q_rank=96, kv_rank=512, dtype=torch.bfloat16, **more):
+    from nnis_b200.config.spec import PartSpec
+    from nnis_b200.parts import MIXERS
+    names = {k: k for k in ("dq", "dq_norm", "uq", "q", "dkv", "dkv_norm", "uk", "uv", "o", "gate", "sink")}
+    return MIXERS.build("latent_attention", {
+        "hidden_size": 64, "heads": heads, "dim": dim, "rot_dim": rot, "vdim": vdim, "q_rank": q_rank, "kv_rank": kv_rank,
+        "scale": 0.1, "eps": 1e-5, "position": PartSpec("rope_frequencies", {"dims": rot, "base": 1e4}), "leaf": "",
+        "names": names, **more}, "l0", dtype, torch.device("cpu"))
+
+
+def test_which_prompts_multiply_the_latents_out(monkeypatch):
+    part = _latent_part()
+    assert part._expands([2048, 1311], [0, 0])
+    assert not part._expands([64], [0])              # too little to save
+    assert not part._expands([8], [8000])            # a long past for few tokens
+    assert not part._expands([1] * 300, [4000] * 300)
+    # half a gigabyte of keys and values: 65,536 positions of 16 heads of 128 + 128
+    assert part._expands([65536], [0]) and not part._expands([65537], [0])
+    for other in (_latent_part(window=100), _latent_part(q_rank=0, gate="head"), _latent_part(sink=True), _latent_part(q_rank=0),
+                  _latent_part(dim=64), _latent_part(dtype=torch.float32), _latent_part(scale=-0.1)):
+        assert not other._expands([2048, 1311], [0, 0])
+    monkeypatch.setattr(type(part), "EXPAND_SAVES", 0)
+    assert part._expands([70], [0])
+
+
+def test_a_layer_that_cannot_multiply_out_keeps_its_way_beside_one_that_does(monkeypatch):
+    """The tables of a step are shared by name: a layer of the same sizes with a window finds them too."""
+    from types import SimpleNamespace
+    from nnis_b200.csrc import ops
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    one, other = _latent_part(), _latent_part(window=100)
+    one.w_kv = torch.zeros(1)
+    tables = one.step_tables([2048], [0])
+    assert one._expand_name() == other._expand_name() and one._expand_name() + "/units" in tables
+    for decode in (False, True):
+        ctx = SimpleNamespace(decode=decode, tables=tables)
+        assert one._takes_expanded(ctx) == (not decode) and not other._takes_expanded(ctx)
+    assert not one._takes_expanded(SimpleNamespace(decode=False, tables={}))
+    assert not any(k.startswith("latent_wide") for k in other.step_tables([2048], [0], tuple(tables)))
