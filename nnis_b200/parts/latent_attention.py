@@ -145,6 +145,8 @@ class LatentAttention(Part):
         self.w_o = tensors[self._name("o")]
 
     def parameter_bytes(self) -> int:
+        """What a step of single tokens reads.  (A layer that may multiply its latents out holds W_uk a second time, heads x
+        dim x kv_rank values beside these, which such prompts alone read.)"""
         return sum(t.numel() * t.element_size() for t in
                    (self.w_down, self.w_uq, self.w_ukt, self.w_uv, self.w_o, self.norm_q, self.norm_kv)
                    if t is not None)
@@ -160,10 +162,14 @@ class LatentAttention(Part):
         H, W = self.heads, self.hidden
         tokens = sum(counts)
         into_q = W * self.q_rank + self.q_rank * self.q_cols if self.q_rank else W * (self.q_cols + self.gate_cols)
-        per_token = into_q + W * self.row + H * self.dim * self.kv_rank + H * self.vdim * self.kv_rank + H * self.vdim * W
+        per_token = into_q + W * self.row + H * self.vdim * W
+        up = H * (self.dim + self.vdim) * self.kv_rank  # into the latent's space and out of it, or a position multiplied out
         keys = sum(sum(min(st + q + 1, self.window) for q in range(c)) if self.window
                    else c * st + c * (c + 1) // 2 for c, st in zip(counts, starts))
-        return 2.0 * tokens * per_token + 2.0 * H * (self.row + self.kv_rank) * keys
+        if self._expands(counts, starts):
+            positions = sum(c + st for c, st in zip(counts, starts))
+            return 2.0 * (tokens * per_token + positions * up + H * (self.dim + self.rot + self.vdim) * keys)
+        return 2.0 * (tokens * (per_token + up) + H * (self.row + self.kv_rank) * keys)
 
     # -- work lists ---------------------------------------------------------
     def _tiles_name(self) -> str:

@@ -231,3 +231,15 @@ def test_a_layer_that_cannot_multiply_out_keeps_its_way_beside_one_that_does(mon
         assert one._takes_expanded(ctx) == (not decode) and not other._takes_expanded(ctx)
     assert not one._takes_expanded(SimpleNamespace(decode=False, tables={}))
     assert not any(k.startswith("latent_wide") for k in other.step_tables([2048], [0], tuple(tables)))
+
+
+def test_operations_of_a_latent_layer_are_those_of_the_way_it_takes():
+    part = _latent_part()                          # 16 heads of 128 + 64 and 128, ranks 96 and 512, width 64
+    shared = 64 * 96 + 96 * 16 * 192 + 64 * 576 + 16 * 128 * 64
+    up, pairs = 16 * 256 * 512, 2048 * 2049 // 2
+    assert part.step_flops([2048], [0]) == 2.0 * (2048 * (shared + up) + 16 * (128 + 64 + 128) * pairs)
+    assert part.step_flops([2000], [48]) == 2.0 * (2000 * shared + 2048 * up
+                                                   + 16 * (128 + 64 + 128) * (2000 * 48 + 2000 * 2001 // 2))
+    assert part.step_flops([1], [2047]) == 2.0 * (shared + up + 16 * (576 + 512) * 2048)
+    windowed = _latent_part(window=100)
+    assert windowed.step_flops([2048], [0]) == 2.0 * (2048 * (shared + up) + 16 * (576 + 512) * (100 * 101 // 2 + 1948 * 100))
