@@ -75,7 +75,15 @@ class EngineBackend:
         if not single or self.decode_greedy is None or len(batch) > self.max_rows:
             self._picked = None
             return self.engine.step_in_portions(batch, self.max_step_tokens)
-        dec = self._graph_step([s.slot for s in batch], [s.tokens[0] for s in batch], need_logits)
+        vocab = self.engine.spec.vocab_size
+        slots, tokens = [], []
+        for s in batch:
+            token = int(s.tokens[0])
+            if not 0 <= token < vocab:
+                raise StepError(f"slot {s.slot}: token {s.tokens[0]} is outside the vocabulary")
+            slots.append(s.slot)
+            tokens.append(token)
+        dec = self._replay(slots, tokens, need_logits)
         n = len(batch)
         views = self._views.get((id(dec), n))
         if views is None:  # (slicing a tensor costs microseconds: once per decoder and row count)
@@ -83,17 +91,14 @@ class EngineBackend:
         self._picked = views[0]
         return views[1] if need_logits else None
 
-    def _graph_step(self, slots: List[int], tokens: Sequence[int], need_logits: bool) -> GraphDecoder:
+    def _replay(self, slots: List[int], tokens: List[int], need_logits: bool) -> GraphDecoder:
         """One token per slot as a replay of the captured step; its inputs go up in one copy."""
-        cache, vocab = self.engine.cache, self.engine.spec.vocab_size
-        for slot, token in zip(slots, tokens):
-            if not 0 <= int(token) < vocab:
-                raise StepError(f"slot {slot}: token {token} is outside the vocabulary")
+        cache = self.engine.cache
         positions = [cache.length(s) for s in slots]
         new_lengths = [p + 1 for p in positions]
         cache.reserve(slots, new_lengths)
         dec = self._decoder(len(slots), max(new_lengths), need_logits)
-        self.h2d_bytes += dec.upload([int(t) for t in tokens], positions, slots)
+        self.h2d_bytes += dec.upload(tokens, positions, slots)
         dec.launch()
         cache.commit(slots, new_lengths)
         return dec
@@ -107,7 +112,9 @@ class EngineBackend:
         if self.decode_greedy is None or not (
                 again or self._decoder_key(1, engine.cache.length(slot) + 1, True) in self._decoders):
             return engine.step([SequenceStep(slot, [token], [0])])[0]
-        return self._graph_step([slot], [token], True).logits[0]
+        if not 0 <= token < engine.spec.vocab_size:
+            raise StepError(f"slot {slot}: token {token} is outside the vocabulary")
+        return self._replay([slot], [token], True).logits[0]
 
     def greedy(self, logits: Optional[torch.Tensor]) -> List[int]:
         if self._picked is not None:  # the graph has picked already
