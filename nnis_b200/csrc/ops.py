@@ -1340,7 +1340,7 @@ def retention(qkvg: torch.Tensor, freq: torch.Tensor, decay: torch.Tensor, state
     joined heads, times this weight, instead of a norm per head; ``gate``: "silu" or "sigmoid".
     Without ``seq_first_row`` every row is one token of a sequence of its own.  With ``chunks`` (``scan_segments`` of
     RETENTION_CHUNK tokens) and the scratch that ``retention_scratch`` names a prompt step's chunks are worked side by
-    side (``retention_takes_chunks``)."""
+    side (``retention_takes_chunks``); without them in order."""
     _cuda(qkvg, freq, decay, state, token_pos, token_seq, seq_slots, seq_first_row, seq_start, seq_count,
           o_raw, out, chunks, seq_first_chunk, packed, chunk_state, norm_weight)
     _need(gate in ("silu", "sigmoid"), "retention: the gate is silu or sigmoid")
@@ -1378,15 +1378,28 @@ def retention(qkvg: torch.Tensor, freq: torch.Tensor, decay: torch.Tensor, state
 
 
 RETENTION_CHUNK = 64  # tokens of a chunk
-# Prompts whose longest sequence has more tokens run in chunks, the others walk.  Whole prompts of one layer with experts, 16
-# heads of 64 / 128, us walked and in chunks: 32 tokens 366 / 385 and 410 / 422, 64 tokens 379 / 399 and 413 / 430, 100 tokens
-# 389 / 439 and 415 / 438, 128 tokens 403 / 501 and 415 / 438, 256 tokens 623 / 727 and 222 / 322.
-RETENTION_CHUNK_MIN = 96
+# Prompt steps of fewer tokens are worked in order (0: all are).
+RETENTION_SEGMENT = int(os.environ.get("NNIS_RETENTION_SEGMENT", "256"))
 
 
 def retention_takes_chunks(dim: int) -> bool:
-    """Whether prompts of this key size are worked a chunk of tokens at a time, chunks side by side."""
-    return dim in (32, 64, 128, 256)
+    """Whether prompts of this key size can be worked with their chunks of tokens side by side."""
+    return RETENTION_SEGMENT > 0 and RETENTION_SEGMENT % 32 == 0 and dim in (32, 64, 128, 256)
+
+
+def retention_side_by_side(counts, heads: int, dim: int, vdim: int, sms: int) -> bool:
+    """Whether a prompt step's chunks of 64 tokens are worked side by side (four kernels and two tables) or its chunks of 32
+    in order by one kernel, whose CTAs (a sequence, a head, 32 columns) run together up to four on an SM (two with keys
+    of 256) and take about 17 us a chunk of 32; the four kernels take as long as four such chunks, and 30 to 50 us more
+    where they are launched one by one, as steps of fewer than 256 tokens always are.  Whole prompts of one layer with
+    experts, 4 / 8 heads of 128 x 256, us in order and side by side, launched one by one: 90 tokens 373 / 396 and
+    423 / 442, 150 tokens 376 / 398 and 420 / 444, 255 tokens 387 / 409 and 427 / 452; replayed: 4 x 90 tokens 234 / 335
+    and 261 / 357, 4 x 128 tokens 267 / 385 and 271 / 388, 2 x 200 tokens 287 / 389 and 250 / 352, 300 tokens 323 / 434 and
+    236 / 331, 16 x 100 tokens 514 / 787 and 540 / 653."""
+    if not retention_takes_chunks(dim) or sum(counts) < RETENTION_SEGMENT:
+        return False
+    waves = -(-len(counts) * heads * -(-vdim // 32) // ((2 if dim == 256 else 4) * sms))
+    return waves * -(-max(counts) // 32) > 4
 
 
 def retention_scratch(n_chunks: int, heads: int, dim: int, vdim: int):

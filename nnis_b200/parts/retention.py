@@ -11,10 +11,10 @@ the residual stream.  S [heads, dim, vdim] is float32, starts at zero and is the
 layer's whole memory of a sequence: it lives in the cache's state area, one per
 slot, so a later chunk or a single token goes on from what the tokens before left.
 
-Single tokens update the state in registers.  Prompts go 64 tokens at a time (the
-recurrence written as three products per chunk, all float32): what every chunk adds to
-the state, all chunks side by side; the state before each chunk, in order; the outputs,
-all chunks side by side again.
+Single tokens update the state in registers.  Short prompts go 32 tokens at a time in
+order (the recurrence written as three products per chunk, all float32), long ones 64 at a
+time: what every chunk adds to the state, all chunks side by side; the state before each
+chunk, in order; the outputs, all chunks side by side again.
 
 Variants, each a parameter: ``activation`` "silu" passes q, k and v through silu before the
 recurrence (lightning attention's form); ``key_scale`` replaces dim^-1/2 (1.0: no scale);
@@ -107,9 +107,10 @@ class Retention(Part):
     CHUNKS, FIRST_CHUNK = "retention/chunks", "retention/first_chunk"
 
     def step_tables(self, counts, starts, have=()):
-        """Prompt steps with a sequence longer than a few tokens: the chunks of every sequence (the same list for every
-        retention layer of the model)."""
-        if not ops.retention_takes_chunks(self.dim) or max(counts) <= ops.RETENTION_CHUNK_MIN or self.CHUNKS in have:
+        """Prompt steps that are long enough: the chunks of every sequence (the same list for every retention layer of
+        the model)."""
+        if self.CHUNKS in have or not ops.retention_takes_chunks(self.dim) or not ops.retention_side_by_side(
+                counts, self.heads, self.dim, self.vdim, ops.sm_count(self.device)):
             return {}
         chunks, first = ops.scan_segments(counts, ops.RETENTION_CHUNK)
         return {self.CHUNKS: chunks, self.FIRST_CHUNK: first}

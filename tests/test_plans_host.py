@@ -258,3 +258,14 @@ def test_which_kernel_takes_the_projections_of_a_decode_step():
     assert o.gemv_kind(8, 576, 576, o.EPI_STORE, shared_norm=True) == 0
     # the adding tensor-core product cuts a long K among CTAs only where tiles are few
     assert o.gemm_tc_splits(64, 2048, 8192)[0] == 4 and o.gemm_tc_splits(2048, 576, 1536)[0] == 1
+
+
+def test_which_retention_prompts_work_their_chunks_side_by_side(monkeypatch):
+    from nnis_b200.csrc import ops as o
+    side = lambda counts, heads=8, dim=128, vdim=256: o.retention_side_by_side(counts, heads, dim, vdim, 148)
+    assert side([300]) and side([200, 200]) and side([2048]) and side([100] * 16) and not side([100] * 16, heads=4)
+    assert not side([150]) and not side([255]) and not side([90] * 4) and not side([128] * 4) and not side([60] * 4)
+    assert not side([2048], dim=48)
+    for off in (0, 100):  # (no multiple of 32)
+        monkeypatch.setattr(o, "RETENTION_SEGMENT", off)
+        assert not side([2048]) and not o.retention_takes_chunks(128)

@@ -154,7 +154,8 @@ def test_cached_latent_rows_one_after_another(rank, rot):
 
 @pytest.mark.parametrize("dim,vdim", [(32, 1), (64, 30), (128, 256), (256, 200), (128, 64)])
 @pytest.mark.parametrize("dtype,act", [("float32", True), ("bfloat16", False)])
-def test_retention_of_prompts_in_chunks(dim, vdim, dtype, act):
+@pytest.mark.parametrize("in_order", [False, True])
+def test_retention_of_prompts_in_chunks(dim, vdim, dtype, act, in_order):
     """Sequences of one token, a chunk, a chunk and one, several; fresh ones and ones with a state; a token whose values
     are infinite is not felt before it."""
     o = ops()
@@ -177,11 +178,12 @@ def test_retention_of_prompts_in_chunks(dim, vdim, dtype, act):
     got_state = state.to(DEV)
     pos = [st + t for st, c in zip(starts, new) for t in range(c)]
     seq = [i for i, c in enumerate(new) for _ in range(c)]
+    side_by_side = {} if in_order else dict(
+        chunks=torch.from_numpy(chunks).to(DEV), seq_first_chunk=torch.from_numpy(first).to(DEV),
+        packed=torch.full((sizes[0],), math.nan, device=DEV), chunk_state=torch.full((sizes[1],), math.nan, device=DEV))
     o.retention(rows.to(DEV), freq.to(DEV), decay.to(DEV), got_state, i32(pos), i32(seq), i32(slots),
                 i32([sum(new[:i]) for i in range(len(new))]), i32(starts), i32(new), o_raw, out, H, dim, vdim, rot, 1e-5,
-                chunks=torch.from_numpy(chunks).to(DEV), seq_first_chunk=torch.from_numpy(first).to(DEV),
-                packed=torch.full((sizes[0],), math.nan, device=DEV),
-                chunk_state=torch.full((sizes[1],), math.nan, device=DEV), activation=act)
+                activation=act, **side_by_side)
     x = rows.double()
     x = x * torch.sigmoid(x) if act else x
     q, k = (x[:, i * H * dim:(i + 1) * H * dim].reshape(n, H, dim).clone() for i in (0, 1))
