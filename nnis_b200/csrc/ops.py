@@ -1346,9 +1346,10 @@ def retention(qkvg: torch.Tensor, freq: torch.Tensor, decay: torch.Tensor, state
     _need(gate in ("silu", "sigmoid"), "retention: the gate is silu or sigmoid")
     _need(norm_weight is None or (norm_weight.dtype == torch.float32 and norm_weight.numel() == heads * vdim),
           "retention: norm_weight float32 [heads * vdim]")
-    n_chunks = 0
+    n_chunks = wave = 0
     if chunks is not None:
         n_chunks = chunks.shape[0]
+        wave = retention_wave(n_chunks, heads, dim, vdim)
         sizes = retention_scratch(n_chunks, heads, dim, vdim)
         _need(retention_takes_chunks(dim) and seq_first_row is not None and seq_first_chunk is not None
               and packed is not None and packed.dtype == torch.float32 and packed.numel() >= sizes[0]
@@ -1369,12 +1370,12 @@ def retention(qkvg: torch.Tensor, freq: torch.Tensor, decay: torch.Tensor, state
     units = seq_first_row.numel() if seq_first_row is not None else n
     _check(_lib().nnis_retention(_ptr(qkvg), _ptr(freq), _ptr(decay), _ptr(state), _ptr(token_pos),
                                  _ptr(token_seq), _ptr(seq_slots), _ptr(seq_first_row), _ptr(seq_start),
-                                 _ptr(seq_count), _ptr(chunks), n_chunks, _ptr(seq_first_chunk), _ptr(packed),
+                                 _ptr(seq_count), _ptr(chunks), n_chunks, _ptr(seq_first_chunk), wave, _ptr(packed),
                                  _ptr(chunk_state), _ptr(o_raw), _ptr(out), n, units, heads, dim, vdim,
                                  rot_dims, ctypes.c_float(eps), 1 if activation else 0,
                                  ctypes.c_float(dim ** -0.5 if key_scale is None else key_scale),
                                  _ptr(norm_weight), 1 if gate == "sigmoid" else 0, code_of(out.dtype), _stream()),
-           "retention", 5 if chunks is not None else 2)
+           "retention", 4 * -(-n_chunks // wave) + 1 if chunks is not None else 2)
 
 
 RETENTION_CHUNK = 64  # tokens of a chunk
@@ -1402,10 +1403,19 @@ def retention_side_by_side(counts, heads: int, dim: int, vdim: int, sms: int) ->
     return waves * -(-max(counts) // 32) > 4
 
 
+RETENTION_SCRATCH = 1 << 27  # bytes; 8 heads of 128 x 256 fill it with 3,584 tokens
+
+
+def retention_wave(n_chunks: int, heads: int, dim: int, vdim: int) -> int:
+    """How many of a prompt step's chunks are worked at a time: all of them as long as the scratch holds them."""
+    vp = -(-vdim // 4) * 4
+    return max(1, min(n_chunks, RETENTION_SCRATCH // (4 * heads * (RETENTION_CHUNK * (3 * dim + vp) + dim * vp))))
+
+
 def retention_scratch(n_chunks: int, heads: int, dim: int, vdim: int):
     """Float32 values of ``packed`` and ``chunk_state`` for a prompt step of ``n_chunks`` chunks."""
-    vp = -(-vdim // 4) * 4
-    return n_chunks * heads * RETENTION_CHUNK * (3 * dim + vp), n_chunks * heads * dim * vp
+    vp, n = -(-vdim // 4) * 4, retention_wave(n_chunks, heads, dim, vdim)
+    return n * heads * RETENTION_CHUNK * (3 * dim + vp), n * heads * dim * vp
 
 
 def moe_route(h: torch.Tensor, w_router: torch.Tensor, b_router: Optional[torch.Tensor],

@@ -281,7 +281,9 @@ retention_in_order_kernel(const T* __restrict__ qkvg, const float* __restrict__ 
 // Longer prompts: the same a chunk of 64 tokens at a time, chunks side by side, all in float32 on the CUDA cores.  Four kernels: `pack` turns q, k and v of every (chunk, head) into the layouts that
 // the products read (rotated once, not once per tile of columns); `update` makes what every chunk adds to the state, all
 // chunks side by side; `carry` walks a sequence's chunks in order and leaves the state before each of them, and the
-// slot's state; `read` makes the outputs, all chunks side by side.  The products are linear_chunks.cuh's.
+// slot's state; `read` makes the outputs, all chunks side by side.  The products are linear_chunks.cuh's.  More chunks
+// than the scratch holds go through the four kernels in waves, the slot's state from one to the next (the same bits: the
+// state is float32 there too).
 // Before, chunks of 32 in runs of 256 tokens from zero, 32 columns a CTA with A made again for each, 2 x 2 entries of A
 // and 4 x 1 of the output a thread, took 495 us for 2,048 tokens and 8 heads of 128 x 256 on a B200 (chunk 351, prefix
 // 30, carry 114); now 143 (pack 39, update 25, carry 12, read 68: 22 TFLOP/s of multiply-adds).
@@ -388,12 +390,13 @@ retention_update_kernel(const float* __restrict__ packed, float* __restrict__ ch
 }
 
 // The state before every chunk in place of what the chunk adds, in order, a thread per four values of a row, eight
-// chunks fetched ahead; the state after the last goes to the slot (whose rows have vdim values and no alignment).
+// chunks fetched ahead; the state after the last goes to the slot (whose rows have vdim values and no alignment).  The
+// wave's chunks: `wave_n` from `wave0` on, the first of which chunk_state begins with.
 __global__ void __launch_bounds__(128)
 retention_carry_kernel(float* chunk_state, float* state, const float* __restrict__ decay,
                        const int* __restrict__ seq_slots, const int* __restrict__ seq_start,
-                       const int* __restrict__ seq_count, const int* __restrict__ seq_first_chunk, int heads, int dim,
-                       int vdim, int vp) {
+                       const int* __restrict__ seq_count, const int* __restrict__ seq_first_chunk, int wave0, int wave_n,
+                       int heads, int dim, int vdim, int vp) {
     constexpr int AHEAD = 8;
     pdl_wait();
     pdl_launch_dependents();
@@ -401,16 +404,17 @@ retention_carry_kernel(float* chunk_state, float* state, const float* __restrict
     const int e = blockIdx.z * 128 + threadIdx.x;
     if (e >= dim * quads) return;
     const int d = e / quads, j = (e - d * quads) * 4;
-    const int c0 = seq_first_chunk[seq], c1 = seq_first_chunk[seq + 1], count = seq_count[seq];
+    const int begin = seq_first_chunk[seq], end = seq_first_chunk[seq + 1], count = seq_count[seq];
+    const int c0 = max(begin, wave0), c1 = min(end, wave0 + wave_n);
     if (c1 <= c0) return;
     const float g = decay[h];
     float g_chunk = 1.f, g_last = 1.f;  // as decay_powers makes them
-    const int last = count - (c1 - c0 - 1) * kChunkTokens;
+    const int last = count - (end - begin - 1) * kChunkTokens;
     for (int n = 0; n < kChunkTokens; ++n) {
         g_chunk *= g;
         if (n < last) g_last *= g;
     }
-    float* own = chunk_state + ((size_t)c0 * heads + h) * dim * vp + (size_t)d * vp + j;
+    float* own = chunk_state + ((size_t)(c0 - wave0) * heads + h) * dim * vp + (size_t)d * vp + j;
     const size_t step = (size_t)heads * dim * vp;
     float* slot = state + ((size_t)seq_slots[seq] * heads + h) * dim * vdim + (size_t)d * vdim + j;
     float run[4];
@@ -425,7 +429,7 @@ retention_carry_kernel(float* chunk_state, float* state, const float* __restrict
         for (int k = 0; k < AHEAD; ++k) {
             if (c + k >= c1) break;
             store4(own + (size_t)(c - c0 + k) * step, make_float4(run[0], run[1], run[2], run[3]));
-            const float f = c + k == c1 - 1 ? g_last : g_chunk;
+            const float f = c + k == end - 1 ? g_last : g_chunk;
             run[0] = fmaf(f, run[0], add[k].x);
             run[1] = fmaf(f, run[1], add[k].y);
             run[2] = fmaf(f, run[2], add[k].z);
@@ -483,7 +487,7 @@ retention_read_kernel(const float* __restrict__ packed, const float* __restrict_
 template <typename T>
 static int launch_chunks(const T* qkvg, const float* freq, const float* decay, float* state, const int* seq_slots,
                          const int* seq_first_row, const int* seq_start, const int* seq_count, const int* chunks,
-                         int n_chunks, const int* seq_first_chunk, float* packed, float* chunk_state, float* o_raw,
+                         int n_chunks, const int* seq_first_chunk, int wave, float* packed, float* chunk_state, float* o_raw,
                          int n_seqs, int heads, int dim, int vdim, int rot_dims, int act, float k_scale,
                          cudaStream_t stream) {
     const int vp = (vdim + 3) & ~3, bv = vp > 64 ? 128 : 64;
@@ -495,19 +499,23 @@ static int launch_chunks(const T* qkvg, const float* freq, const float* decay, f
     if (e == cudaSuccess) e = cudaFuncSetAttribute(update, cudaFuncAttributeMaxDynamicSharedMemorySize, update_smem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(read, cudaFuncAttributeMaxDynamicSharedMemorySize, read_smem);
     const int v_tiles = (vp + bv - 1) / bv;
-    if (e == cudaSuccess)
-        e = launch_dependent(retention_pack_kernel<T>, dim3(n_chunks, heads), 256, pack_smem, stream, qkvg, freq, decay,
-                             chunks, seq_first_row, seq_start, seq_count, packed, heads, dim, vdim, vp, rot_dims, act, k_scale);
-    if (e == cudaSuccess)
-        e = launch_dependent(update, dim3(n_chunks, heads, (dim + 63) / 64 * v_tiles), 128, update_smem, stream,
-                             (const float*)packed, chunk_state, heads, dim, vp);
-    if (e == cudaSuccess)
-        e = launch_dependent(retention_carry_kernel, dim3(n_seqs, heads, (dim * (vp / 4) + 127) / 128), 128, 0, stream,
-                             chunk_state, state, decay, seq_slots, seq_start, seq_count, seq_first_chunk, heads, dim, vdim, vp);
-    if (e == cudaSuccess)
-        e = launch_dependent(read, dim3(n_chunks, heads, v_tiles), 128, read_smem, stream, (const float*)packed,
-                             (const float*)chunk_state, decay, chunks, seq_first_row, seq_start, seq_count, o_raw, heads,
-                             dim, vdim, vp);
+    for (int c0 = 0; c0 < n_chunks && e == cudaSuccess; c0 += wave) {
+        const int n = n_chunks - c0 < wave ? n_chunks - c0 : wave;
+        const int* own = chunks + 2 * c0;
+        e = launch_dependent(retention_pack_kernel<T>, dim3(n, heads), 256, pack_smem, stream, qkvg, freq, decay, own,
+                             seq_first_row, seq_start, seq_count, packed, heads, dim, vdim, vp, rot_dims, act, k_scale);
+        if (e == cudaSuccess)
+            e = launch_dependent(update, dim3(n, heads, (dim + 63) / 64 * v_tiles), 128, update_smem, stream,
+                                 (const float*)packed, chunk_state, heads, dim, vp);
+        if (e == cudaSuccess)
+            e = launch_dependent(retention_carry_kernel, dim3(n_seqs, heads, (dim * (vp / 4) + 127) / 128), 128, 0, stream,
+                                 chunk_state, state, decay, seq_slots, seq_start, seq_count, seq_first_chunk, c0, n, heads,
+                                 dim, vdim, vp);
+        if (e == cudaSuccess)
+            e = launch_dependent(read, dim3(n, heads, v_tiles), 128, read_smem, stream, (const float*)packed,
+                                 (const float*)chunk_state, decay, own, seq_first_row, seq_start, seq_count, o_raw, heads,
+                                 dim, vdim, vp);
+    }
     return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 
@@ -618,7 +626,7 @@ template <typename T>
 static int launch_retention(const void* qkvg, const float* freq, const float* decay, float* state,
                             const int* token_pos, const int* token_seq, const int* seq_slots,
                             const int* seq_first_row, const int* seq_start, const int* seq_count,
-                            const int* chunks, int n_chunks, const int* seq_first_chunk, float* packed,
+                            const int* chunks, int n_chunks, const int* seq_first_chunk, int wave, float* packed,
                             float* chunk_state, float* o_raw, void* out, int n_tokens, int n_units, int heads, int dim,
                             int vdim, int rot_dims, float eps, int act, float k_scale, const float* norm_w,
                             int gate_kind, cudaStream_t stream) {
@@ -626,7 +634,7 @@ static int launch_retention(const void* qkvg, const float* freq, const float* de
     cudaError_t le = cudaSuccess;
     if (chunks) {  // a prompt step, chunks of tokens side by side
         int rc = launch_chunks<T>((const T*)qkvg, freq, decay, state, seq_slots, seq_first_row, seq_start, seq_count,
-                                  chunks, n_chunks, seq_first_chunk, packed, chunk_state, o_raw, n_units, heads, dim,
+                                  chunks, n_chunks, seq_first_chunk, wave, packed, chunk_state, o_raw, n_units, heads, dim,
                                   vdim, rot_dims, act, k_scale, stream);
         if (rc != NNIS_OK) return rc;
     } else if (seq_first_row && (dim == 32 || dim == 64 || dim == 128 || dim == 256)) {
@@ -676,13 +684,14 @@ using namespace nnis;
 // `chunks` (prompt steps, key sizes 32, 64, 128 and 256; without it the tokens are worked in order): int32
 // [n_chunks, 2] = (sequence, first token of the chunk among the sequence's tokens of this step), 64 tokens each in the
 // order of the sequences, with `seq_first_chunk` [n_units + 1] and, vp = vdim rounded up to a multiple of four, float32
-// scratch `packed` [n_chunks, heads, 64 (3 dim + vp)] and `chunk_state` [n_chunks, heads, dim, vp].
+// scratch `packed` [wave, heads, 64 (3 dim + vp)] and `chunk_state` [wave, heads, dim, vp] (of n_chunks, if these are
+// fewer): `wave` chunks are worked at a time.
 // `act` 1: q, k, v through silu; `k_scale`: the keys' multiplier; `norm_w` (float32 [heads * vdim]): one
 // norm over the joined heads with this weight instead of a norm per head; `gate_kind` 0 silu, 1 sigmoid.
 NNIS_API int nnis_retention(const void* qkvg, const float* freq, const float* decay, float* state,
                             const int* token_pos, const int* token_seq, const int* seq_slots,
                             const int* seq_first_row, const int* seq_start, const int* seq_count,
-                            const int* chunks, int n_chunks, const int* seq_first_chunk, float* packed,
+                            const int* chunks, int n_chunks, const int* seq_first_chunk, int wave, float* packed,
                             float* chunk_state, float* o_raw, void* out, int n_tokens, int n_units, int heads, int dim,
                             int vdim, int rot_dims, float eps, int act, float k_scale, const float* norm_w,
                             int gate_kind, int dtype, cudaStream_t stream) {
@@ -691,7 +700,7 @@ NNIS_API int nnis_retention(const void* qkvg, const float* freq, const float* de
         !token_pos || !token_seq || !seq_slots || !o_raw || !out)
         return NNIS_ERR_ARGUMENT;
     if (seq_first_row && (!seq_start || !seq_count)) return NNIS_ERR_ARGUMENT;
-    if (chunks && (!seq_first_row || n_chunks <= 0 || !seq_first_chunk || !packed || !chunk_state ||
+    if (chunks && (!seq_first_row || n_chunks <= 0 || wave <= 0 || !seq_first_chunk || !packed || !chunk_state ||
                    !(dim == 32 || dim == 64 || dim == 128 || dim == 256)))
         return NNIS_ERR_ARGUMENT;
     if (chunks && ((uintptr_t)packed | (uintptr_t)chunk_state | (uintptr_t)o_raw) % 16) return NNIS_ERR_ALIGNMENT;
@@ -699,10 +708,10 @@ NNIS_API int nnis_retention(const void* qkvg, const float* freq, const float* de
     if (dtype == NNIS_DTYPE_F32)
         return launch_retention<float>(qkvg, freq, decay, state, token_pos, token_seq, seq_slots,
                                        seq_first_row, seq_start, seq_count, chunks, n_chunks,
-                                       seq_first_chunk, packed, chunk_state, o_raw, out, n_tokens, n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, stream);
+                                       seq_first_chunk, wave, packed, chunk_state, o_raw, out, n_tokens, n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, stream);
     if (dtype == NNIS_DTYPE_BF16)
         return launch_retention<bf16>(qkvg, freq, decay, state, token_pos, token_seq, seq_slots,
                                       seq_first_row, seq_start, seq_count, chunks, n_chunks,
-                                      seq_first_chunk, packed, chunk_state, o_raw, out, n_tokens, n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, stream);
+                                      seq_first_chunk, wave, packed, chunk_state, o_raw, out, n_tokens, n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, stream);
     return NNIS_ERR_UNSUPPORTED;
 }

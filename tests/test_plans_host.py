@@ -269,3 +269,15 @@ def test_which_retention_prompts_work_their_chunks_side_by_side(monkeypatch):
     for off in (0, 100):  # (no multiple of 32)
         monkeypatch.setattr(o, "RETENTION_SEGMENT", off)
         assert not side([2048]) and not o.retention_takes_chunks(128)
+
+
+def test_chunks_of_recurrent_layers_keep_their_scratch_within_its_bound():
+    """As many chunks at a time as the scratch holds, one at least; all of them as long as they fit."""
+    from nnis_b200.csrc import ops as o
+    assert o.retention_wave(32, 8, 128, 256) == 32   # 2,048 tokens
+    for chunks in (1, 56, 57, 256, 4096):
+        a, b = o.retention_scratch(chunks, 8, 128, 256)
+        wave = o.retention_wave(chunks, 8, 128, 256)
+        assert 1 <= wave <= chunks and (a, b) == (wave * 8 * 64 * (3 * 128 + 256), wave * 8 * 128 * 256)
+        assert 4 * (a + b) <= o.RETENTION_SCRATCH
+    assert o.retention_wave(9, 4096, 256, 1024) == 1  # (more than the bound for a single one)
