@@ -10,6 +10,8 @@
 //   delta_chain   a CTA per (sequence, head, 32 columns) walks the chunks: U = U0 - W S, S <- e^c S + K^T (e^(c - c_j) U);
 //                 it leaves U and the state before every chunk;
 //   delta_read    a CTA per (chunk, head, columns), all side by side: the outputs (linear_chunks.cuh).
+// More chunks than the scratch holds go through the four kernels in waves, the slot's state from one to the next (the same
+// bits: the state is float32 there too).
 // Everything is float32 with fmaf on the CUDA cores; c is double (differences of sums of up to 64 logs keep float32's
 // digits), a decay of zero counts as e^-200, which is zero in float32 and leaves the tokens after it exact.
 //
@@ -265,7 +267,8 @@ template <int DIM>
 __global__ void __launch_bounds__(256)
 delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, float* u, const double* __restrict__ logs,
                    float* __restrict__ before, float* __restrict__ state, const int* __restrict__ seq_slots,
-                   const int* __restrict__ seq_count, const int* __restrict__ seq_first_chunk, int H, int G, int vdim, int vp) {
+                   const int* __restrict__ seq_count, const int* __restrict__ seq_first_chunk, int wave0, int wave_n, int H,
+                   int G, int vdim, int vp) {
     constexpr int CW = 32, KW = DIM / 8;             // the state's rows per warp in the first product
     constexpr int SPLIT = DIM == 128 ? 4 : 8, KT = kDC / SPLIT;  // the tokens per split in the second
     extern __shared__ __align__(16) float chain_smem[];
@@ -298,7 +301,8 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, fl
     }
     __syncthreads();
     const int seq = mine;
-    const int c0 = seq_first_chunk[seq], c1 = seq_first_chunk[seq + 1];
+    // (the sequence's chunks among the wave's, numbered as the scratch is)
+    const int c0 = max(seq_first_chunk[seq], wave0) - wave0, c1 = min(seq_first_chunk[seq + 1], wave0 + wave_n) - wave0;
     if (c1 <= c0) return;
     float* slot = state + ((size_t)seq_slots[seq] * H + h) * DIM * vdim;
     for (int it = tid; it < DIM * CW; it += 256) {
@@ -501,17 +505,17 @@ static cudaError_t most_shared(K kernel, int bytes) {
 
 // a, conv_w, tail, a_log, dt_bias as for nnis_delta_prep (the tail is read; nnis_delta_conv_tail moves it on); dim 64 or
 // 128; chunks int32 [n_chunks, 2] = (sequence, first token of the chunk among the step's), 64 tokens each, with
-// seq_first_chunk [n_seqs + 1].  Float32 scratch, vp = vdim rounded up to a multiple of four: qk [n_chunks, G, 192 dim],
-// u [n_chunks, H, 64, vp], w [n_chunks, H, dim, 64], before [n_chunks, H, dim, vp], beta [n_chunks, H, 64]; double logs
-// [n_chunks, H, 64].  o_raw float32 [n, H vdim].
+// seq_first_chunk [n_seqs + 1].  Float32 scratch, vp = vdim rounded up to a multiple of four: qk [wave, G, 192 dim],
+// u [wave, H, 64, vp], w [wave, H, dim, 64], before [wave, H, dim, vp], beta [wave, H, 64]; double logs [wave, H, 64]
+// (of n_chunks, if these are fewer): `wave` chunks are worked at a time.  o_raw float32 [n, H vdim].
 NNIS_API int nnis_delta_prompt(const float* a, const float* conv_w, const float* tail, const float* a_log,
                                const float* dt_bias, float* state, const int* seq_slots, const int* seq_first_row,
-                               const int* seq_count, const int* chunks, int n_chunks, const int* seq_first_chunk,
+                               const int* seq_count, const int* chunks, int n_chunks, const int* seq_first_chunk, int wave,
                                float* qk, float* u, float* w, float* before, float* beta, double* logs, float* o_raw,
                                int n_seqs, int H, int G, int dim, int vdim, int taps, float unit_eps, float q_scale,
                                cudaStream_t stream) {
     using namespace nnis;
-    if (n_seqs <= 0 || n_chunks <= 0 || H <= 0 || G <= 0 || H % G || vdim <= 0 || taps < 1 || !(unit_eps > 0.f) || !a ||
+    if (n_seqs <= 0 || n_chunks <= 0 || wave <= 0 || H <= 0 || G <= 0 || H % G || vdim <= 0 || taps < 1 || !(unit_eps > 0.f) || !a ||
         !conv_w || !tail || !a_log || !dt_bias || !state || !seq_slots || !seq_first_row || !seq_count || !chunks ||
         !seq_first_chunk || !qk || !u || !w || !before || !beta || !logs || !o_raw)
         return NNIS_ERR_ARGUMENT;
@@ -530,21 +534,24 @@ NNIS_API int nnis_delta_prompt(const float* a, const float* conv_w, const float*
     if (e == cudaSuccess) e = most_shared(solve, solve_smem);
     if (e == cudaSuccess) e = most_shared(chain, chain_smem);
     if (e == cudaSuccess) e = most_shared(read, read_smem);
-    if (e == cudaSuccess)
-        e = launch_dependent(pack, dim3(n_chunks, 2 * G + H + 1), 256, pack_smem, stream, a, conv_w, tail, a_log, dt_bias,
-                             chunks, seq_slots, seq_first_row, seq_count, qk, u, beta, logs, H, G, dim, vdim, vp, taps,
-                             unit_eps, q_scale);
-    // (values become U0 in place: a CTA of the solve reads a column of its own values before it writes it)
-    if (e == cudaSuccess)
-        e = launch_dependent(solve, dim3(n_chunks, H), 128, solve_smem, stream, (const float*)qk, (const float*)u,
-                             (const float*)beta, (const double*)logs, w, u, H, G, vp);
-    if (e == cudaSuccess)
-        e = launch_dependent(chain, dim3((vp + 31) / 32, H, n_seqs), 256, chain_smem, stream, (const float*)qk,
-                             (const float*)w, u, (const double*)logs, before, state, seq_slots, seq_count, seq_first_chunk,
-                             H, G, vdim, vp);
-    if (e == cudaSuccess)
-        e = launch_dependent(read, dim3(n_chunks, H, (vp + bv - 1) / bv), 128, read_smem, stream, (const float*)qk,
-                             (const float*)u, (const double*)logs, (const float*)before, chunks, seq_first_row, seq_count,
-                             o_raw, H, G, dim, vdim, vp);
+    for (int c0 = 0; c0 < n_chunks && e == cudaSuccess; c0 += wave) {
+        const int n = n_chunks - c0 < wave ? n_chunks - c0 : wave;
+        const int* own = chunks + 2 * c0;
+        e = launch_dependent(pack, dim3(n, 2 * G + H + 1), 256, pack_smem, stream, a, conv_w, tail, a_log, dt_bias, own,
+                             seq_slots, seq_first_row, seq_count, qk, u, beta, logs, H, G, dim, vdim, vp, taps, unit_eps,
+                             q_scale);
+        // (values become U0 in place: a CTA of the solve reads a column of its own values before it writes it)
+        if (e == cudaSuccess)
+            e = launch_dependent(solve, dim3(n, H), 128, solve_smem, stream, (const float*)qk, (const float*)u,
+                                 (const float*)beta, (const double*)logs, w, u, H, G, vp);
+        if (e == cudaSuccess)
+            e = launch_dependent(chain, dim3((vp + 31) / 32, H, n_seqs), 256, chain_smem, stream, (const float*)qk,
+                                 (const float*)w, u, (const double*)logs, before, state, seq_slots, seq_count,
+                                 seq_first_chunk, c0, n, H, G, vdim, vp);
+        if (e == cudaSuccess)
+            e = launch_dependent(read, dim3(n, H, (vp + bv - 1) / bv), 128, read_smem, stream, (const float*)qk,
+                                 (const float*)u, (const double*)logs, (const float*)before, own, seq_first_row, seq_count,
+                                 o_raw, H, G, dim, vdim, vp);
+    }
     return e == cudaSuccess ? NNIS_OK : (int)e;
 }

@@ -2116,6 +2116,16 @@ DELTA_CHUNK = 64       # tokens of a chunk of delta_prompt
 DELTA_CHUNK_MIN = 192
 
 
+DELTA_SCRATCH = 1 << 29  # bytes; 32 heads over 16 of 128 x 128 fill it with 5,800 tokens
+
+
+def delta_wave(n_chunks: int, heads: int, kv_heads: int, dim: int, vdim: int) -> int:
+    """How many of a prompt step's chunks are worked at a time: all of them as long as the scratch holds them."""
+    vp = -(-vdim // 4) * 4
+    floats = 3 * kv_heads * DELTA_CHUNK * dim + heads * (DELTA_CHUNK * (vp + dim + 3) + dim * vp)
+    return max(1, min(n_chunks, DELTA_SCRATCH // (4 * floats)))
+
+
 def delta_takes_chunks(dim: int, vdim: int) -> bool:
     """Key and value sizes of which a prompt's chunks are worked side by side."""
     return dim in (64, 128) and vdim <= 512
@@ -2145,15 +2155,16 @@ def delta_prompt(a: torch.Tensor, conv_w: torch.Tensor, tail: torch.Tensor, a_lo
     _need(chunks.dtype == seq_first_chunk.dtype == torch.int32 and chunks.dim() == 2 and chunks.shape[1] == 2
           and seq_first_chunk.numel() == seqs + 1, "delta_prompt: chunks int32 [n, 2], seq_first_chunk [sequences + 1]")
     vp, f = -(-vdim // 4) * 4, torch.float32
-    scratch = [buffer("delta_chunk_qk", (c, kv_heads, 3 * DELTA_CHUNK * dim), f),
-               buffer("delta_chunk_u", (c, heads, DELTA_CHUNK, vp), f), buffer("delta_chunk_w", (c, heads, dim, DELTA_CHUNK), f),
-               buffer("delta_chunk_state", (c, heads, dim, vp), f), buffer("delta_chunk_beta", (c, heads, DELTA_CHUNK), f),
-               buffer("delta_chunk_logs", (c, heads, DELTA_CHUNK), torch.float64)]
+    wave = delta_wave(c, heads, kv_heads, dim, vdim)
+    scratch = [buffer("delta_chunk_qk", (wave, kv_heads, 3 * DELTA_CHUNK * dim), f),
+               buffer("delta_chunk_u", (wave, heads, DELTA_CHUNK, vp), f), buffer("delta_chunk_w", (wave, heads, dim, DELTA_CHUNK), f),
+               buffer("delta_chunk_state", (wave, heads, dim, vp), f), buffer("delta_chunk_beta", (wave, heads, DELTA_CHUNK), f),
+               buffer("delta_chunk_logs", (wave, heads, DELTA_CHUNK), torch.float64)]
     _check(_lib().nnis_delta_prompt(_ptr(a), _ptr(conv_w), _ptr(tail), _ptr(a_log), _ptr(dt_bias), _ptr(state),
                                     _ptr(seq_slots), _ptr(seq_first_row), _ptr(seq_count), _ptr(chunks), c,
-                                    _ptr(seq_first_chunk), *(_ptr(t) for t in scratch), _ptr(o_raw), seqs, heads, kv_heads,
+                                    _ptr(seq_first_chunk), wave, *(_ptr(t) for t in scratch), _ptr(o_raw), seqs, heads, kv_heads,
                                     dim, vdim, taps, ctypes.c_float(unit_eps), ctypes.c_float(q_scale), _stream()),
-           "delta_prompt", 4)
+           "delta_prompt", 4 * -(-c // wave))
     _check(_lib().nnis_delta_conv_tail(_ptr(a), _ptr(tail), _ptr(token_pos), _ptr(token_seq), _ptr(seq_slots),
                                        _ptr(seq_first_row), _ptr(seq_count), seqs, heads, kv_heads, dim, vdim, taps,
                                        _stream()), "delta_conv_tail", 1 if taps > 1 else 0)

@@ -281,3 +281,11 @@ def test_chunks_of_recurrent_layers_keep_their_scratch_within_its_bound():
         assert 1 <= wave <= chunks and (a, b) == (wave * 8 * 64 * (3 * 128 + 256), wave * 8 * 128 * 256)
         assert 4 * (a + b) <= o.RETENTION_SCRATCH
     assert o.retention_wave(9, 4096, 256, 1024) == 1  # (more than the bound for a single one)
+
+
+def test_chunks_of_the_delta_rule_keep_their_scratch_within_its_bound():
+    from nnis_b200.csrc import ops as o
+    assert o.delta_wave(52, 32, 16, 128, 128) == 52   # 3,300 tokens
+    wave = o.delta_wave(4096, 32, 16, 128, 128)
+    assert 4 * wave * (3 * 16 * 64 * 128 + 32 * (64 * (128 + 128 + 3) + 128 * 128)) <= o.DELTA_SCRATCH < 1 << 30 and wave > 52
+    assert o.delta_wave(9, 4096, 4096, 128, 512) >= 1

@@ -289,6 +289,32 @@ def test_delta_rule_of_prompts_in_chunks(dim, vdim, taps, slow):
         assert (s.cpu().double() - finals).abs().max() < 1e-5 * finals.abs().max()
 
 
+@pytest.mark.parametrize("wave", [1, 3, 4])
+def test_delta_rule_chunks_in_waves(wave, monkeypatch):
+    """More chunks than the scratch holds: the same bits, whether a wave ends inside a sequence or with it."""
+    o = ops()
+    g = torch.Generator().manual_seed(wave)
+    H, G, dim, vdim, taps, new = 2, 1, 64, 40, 4, [130, 64, 1, 300]
+    n, channels = sum(new), 2 * G * dim + H * vdim
+    rows = torch.randn(n, channels + H * vdim + 2 * H, generator=g).to(DEV)
+    conv, a_log, bias = torch.randn(channels, taps, generator=g).to(DEV), torch.full((H,), -2.0, device=DEV), torch.zeros(H, device=DEV)
+    begin, tails = torch.randn(4, H, dim, vdim, generator=g) * 0.3, torch.randn(4, taps - 1, channels, generator=g)
+    chunks, first = (torch.from_numpy(t).to(DEV) for t in o.scan_segments(new, o.DELTA_CHUNK))
+    tables = [i32(x) for x in ([t + 9 for c in new for t in range(c)], [i for i, c in enumerate(new) for _ in range(c)],
+                               [0, 1, 2, 3], [sum(new[:i]) for i in range(len(new))], new)]
+    got = []
+    for scratch in (o.DELTA_SCRATCH, 4 * wave * (3 * G * 64 * dim + H * (64 * (vdim + dim + 3) + dim * vdim))):
+        monkeypatch.setattr(o, "DELTA_SCRATCH", scratch)
+        assert o.delta_wave(len(chunks), H, G, dim, vdim) == (len(chunks) if not got else wave)
+        state, tail, o_raw = begin.to(DEV), tails.to(DEV), torch.full((n, H * vdim), 5.0, device=DEV)
+        o.delta_prompt(rows, conv, tail, a_log, bias, state, *tables, chunks, first,
+                       lambda name, shape, dtype: torch.full(shape, math.nan, dtype=dtype, device=DEV), o_raw, H, G, dim,
+                       vdim, 1e-6, 1.0)
+        got.append((o_raw, state, tail))
+    for one, other in zip(*got):
+        assert torch.equal(one, other)
+
+
 @pytest.mark.parametrize("column", [-1, -3])  # the last head's decay gate, and its strength of writing
 def test_a_gate_of_the_delta_rule_that_is_no_number(column):
     """It is seen from its token on, as in the walk, and not before it."""
