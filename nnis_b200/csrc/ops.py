@@ -2170,7 +2170,7 @@ def delta_prompt(a: torch.Tensor, conv_w: torch.Tensor, tail: torch.Tensor, a_lo
                                        _stream()), "delta_conv_tail", 1 if taps > 1 else 0)
 
 
-DELTA_SEGMENT = int(os.environ.get("NNIS_DELTA_SEGMENT", "128"))  # tokens of a run of the delta rule; 0: no runs
+DELTA_SEGMENT = int(os.environ.get("NNIS_DELTA_SEGMENT", "128"))  # tokens of a run of the delta rule; 0: neither runs nor chunks, all walk
 
 
 def delta_finish(o_raw: torch.Tensor, gate_rows: torch.Tensor, gate_off: int, weight: torch.Tensor,

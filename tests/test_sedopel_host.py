@@ -317,3 +317,20 @@ def test_plain_forward_runs_every_configuration_and_prefixes_agree(tmp_path):
         part = P.forward(read_config(d), w, toks[:17])
         assert torch.isfinite(whole).all() and torch.allclose(whole[:17], part, atol=1e-9), name
     assert ODD["width"] % 8 and MIXED["layers"][0]["type"] == "delta"
+
+
+def test_prompts_of_the_delta_rule_that_run_in_chunks(monkeypatch):
+    """Long ones, of the sizes that the kernel takes, unless the switch keeps every prompt in the walk."""
+    from nnis_b200.config import config_from_dict
+    from nnis_b200.csrc import ops
+    from nnis_b200.parts import MIXERS
+    mixer = {"heads": 2, "kv_heads": 1, "dim": 64, "vdim": 32, "conv": 4}
+    spec = config_from_dict({"architecture": "Sedopel", "vocab": 64, "width": 64, "norm": {"eps": 1e-6},
+                             "layers": [{"type": "delta", "mixer": mixer, "mlp": None}]}).to_spec()
+    params = spec.layers[0].part("mixer")
+    part = MIXERS.build(params.kind, params.params, "l0", torch.float32, torch.device("cpu"))
+    tables = part.step_tables([300, 5], [0, 0])
+    assert sorted(tables) == [part.CHUNKS, part.FIRST_CHUNK] and tables[part.CHUNKS].shape == (6, 2)
+    assert part.step_tables([ops.DELTA_CHUNK_MIN], [0]) == {} and part.step_tables([300], [0], tuple(tables)) == {}
+    monkeypatch.setattr(ops, "DELTA_SEGMENT", 0)
+    assert part.step_tables([3000], [0]) == {}
