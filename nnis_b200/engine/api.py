@@ -12,6 +12,7 @@ used here in process.
 """
 from __future__ import annotations
 
+import warnings
 from typing import Callable, List, Optional, Sequence, Union
 
 import numpy as np
@@ -42,6 +43,7 @@ class EngineBackend:
         # picks one step late.  False: every step's tokens come from the host.
         self.pipeline = pipeline
         self._decoders = {}
+        self._uncaptured = set()  # keys of decoders whose capture has failed for a session
         self._views = {}
         self._pinned = None
         self._picked = None
@@ -109,12 +111,26 @@ class EngineBackend:
         tokens that a session decodes (``again`` False) capture nothing, and replay only where the graph is there
         already."""
         engine = self.engine
-        if self.decode_greedy is None or not (
-                again or self._decoder_key(1, engine.cache.length(slot) + 1, True) in self._decoders):
-            return engine.step([SequenceStep(slot, [token], [0])])[0]
-        if not 0 <= token < engine.spec.vocab_size:
-            raise StepError(f"slot {slot}: token {token} is outside the vocabulary")
+        key = self._decoder_key(1, engine.cache.length(slot) + 1, True)
+        if self.decode_greedy is None or key in self._uncaptured or not (again or key in self._decoders) \
+                or not 0 <= token < engine.spec.vocab_size or not self._captured(key):
+            return engine.step([SequenceStep(slot, [token], [0])])[0]  # (which says what is wrong with a token)
         return self._replay([slot], [token], True).logits[0]
+
+    def _captured(self, key) -> bool:
+        """Whether the decoder of this key has its graph, captured now if need be.  Where that fails (no memory for its
+        buffers, say) it is not tried again."""
+        try:
+            if key not in self._decoders:
+                self._decoders[key] = GraphDecoder(self.engine, *key)
+            self._decoders[key].capture()
+        except RuntimeError as error:
+            self._decoders.pop(key, None)
+            self._uncaptured.add(key)
+            warnings.warn(f"a decode step of up to {key[1]} positions could not be captured and is launched kernel by "
+                          f"kernel: {error}", RuntimeWarning)
+            return False
+        return True
 
     def greedy(self, logits: Optional[torch.Tensor]) -> List[int]:
         if self._picked is not None:  # the graph has picked already

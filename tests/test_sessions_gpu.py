@@ -40,3 +40,34 @@ def test_a_model_with_one_sublayer(dtype, tmp_path):
         got = engine.step([SequenceStep(slot, tokens, [0, 150, 299])]).cpu().numpy()
         engine.release_slot(slot)
         check_logits(got, want[[0, 150, 299]], dtype, "prompt")
+
+
+def design(name, kind, folder, dtype="float32"):
+    """(model folder, vocabulary, plain logits of a token list) of one of a design's test models."""
+    import importlib
+    models, P = importlib.import_module(f"{name}_models"), importlib.import_module(f"plain_{name}")
+    cfg = models.CONFIGS[kind]
+    d = models.make_model(str(folder), cfg, seed=71)
+    w, bf = models.load_weights(d, dtype == "bfloat16"), dtype == "bfloat16"
+    if name in ("selovik", "setenex", "zadurax"):
+        return d, cfg["vocab"], lambda tokens: P.forward(tokens, w, cfg, emulate_bf16=bf)
+    return d, cfg["vocab"], lambda tokens: P.forward(cfg, w, tokens, emulate_bf16=bf)
+
+
+def test_a_step_that_cannot_be_captured_runs_as_before(tmp_path, monkeypatch):
+    """A recording that fails (no memory for the graph, say) leaves the session with steps launched one by one."""
+    from nnis_b200 import LLM
+    from nnis_b200.engine.decode import GraphDecoder
+    d, vocab, plain = design("nafezen", "mixed", tmp_path)
+    llm = LLM(d, dtype="float32", max_tokens=64 * 32, max_batch=2)
+    tokens, calls = random_tokens(random.Random(5), 40, vocab), []
+
+    def fails(self):
+        calls.append(1)
+        raise RuntimeError("planted")
+
+    monkeypatch.setattr(GraphDecoder, "capture", fails)
+    with pytest.warns(RuntimeWarning, match="planted"):
+        rows = session_rows(llm, tokens, 9)
+    check_logits(rows, plain(tokens)[8:], "float32", "session")
+    assert len(calls) == 1  # (not tried again for every token)
