@@ -106,9 +106,9 @@ class EngineBackend:
         return dec
 
     def decode_logits(self, slot: int, token: int, again: bool) -> torch.Tensor:
-        """Logits [vocab] of one sequence's next token.  A step of the SmolLM2-135M shape is 154 launches, 4.0 ms from
-        Python one by one and 0.5 ms as a replay; to capture one takes some 10 ms, as long as three of them, so the first
-        tokens that a session decodes (``again`` False) capture nothing, and replay only where the graph is there
+        """Logits [vocab] of one sequence's next token.  A step of the SmolLM2-135M shape is 154 launches, 4.1 ms from
+        Python one by one and 0.47 ms as a replay; to capture one takes 15 to 29 ms, what four to eight replays save, so the
+        first tokens that a session decodes (``again`` False) capture nothing, and replay only where the graph is there
         already."""
         engine = self.engine
         key = self._decoder_key(1, engine.cache.length(slot) + 1, True)
@@ -302,7 +302,7 @@ class LLM:
 class InferenceSession:
     """One sequence on one slot; logits come back to the host as float32."""
 
-    EAGER_TOKENS = 8  # that a session decodes before its step is captured
+    EAGER_TOKENS = 5  # that a session decodes before its step is captured (see ``EngineBackend.decode_logits``)
 
     def __init__(self, llm: LLM):
         self.llm = llm

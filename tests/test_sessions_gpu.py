@@ -71,3 +71,24 @@ def test_a_step_that_cannot_be_captured_runs_as_before(tmp_path, monkeypatch):
         rows = session_rows(llm, tokens, 9)
     check_logits(rows, plain(tokens)[8:], "float32", "session")
     assert len(calls) == 1  # (not tried again for every token)
+
+
+def test_a_session_captures_its_step_once_that_pays(tmp_path):
+    """The first five tokens are launched one by one; another session takes the graph that is there from its first on."""
+    from nnis_b200 import LLM
+    d, vocab, plain = design("tazadra", "wkv", tmp_path)
+    llm = LLM(d, dtype="float32", max_tokens=64 * 32, max_batch=2)
+    session, graphs = llm.new_session(), []
+    tokens = random_tokens(random.Random(2), 20, vocab)
+    rows = [session.prefill(tokens[:9])]
+    for t in tokens[9:]:
+        rows.append(session.decode_one(t))
+        graphs.append(sum(d.graph is not None for d in llm.backend._decoders.values()))
+    assert graphs == [0] * 5 + [1] * 6
+    check_logits(np.stack(rows), plain(tokens)[8:], "float32", "session")
+    other = llm.new_session()
+    other.prefill(tokens[:9])
+    replayed = []
+    llm.backend._decoders[next(iter(llm.backend._decoders))].launch = lambda: replayed.append(1)
+    other.decode_one(tokens[9])
+    assert replayed == [1]
