@@ -703,6 +703,29 @@ def attention_tile_f32_takes(head_dim: int, page_size: int, q_stride: int) -> bo
     return 0 < head_dim <= 128 and head_dim % 4 == 0 and page_size == 64 and q_stride % 4 == 0
 
 
+def attention_tile_f32_pays(counts, starts, window: int, heads: int) -> bool:
+    """Whether the tiles of a float32 prompt step take no longer than a warp for every query (attention_generic.cu).  A
+    tile multiplies a page of keys with 64 queries however many it has, as long as 500 keys take the other kernel, whose
+    longest query is a chain: where its warps do not fill the device it takes as long as that (a key of it like three pages
+    and heads of the tiles together).  Pages and heads of the tiles against the sum of the two; a chain of under 128 keys
+    is over before a tile has begun.  9 heads of 64 / 16 heads of 128 on a B200, us by warps and by tiles: 64 sequences
+    with one token more after 500 93 / 249 and 191 / 749, with 8 209 / 753 and 191 / 755, with 64 1,621 / 5,294 and
+    253 / 850; 8 with one more after 2,000 343 / 728 and 120 / 415; one with 8 more after 64 19.0 / 28.8 and 20.6 / 27.3;
+    64 of 8 tokens 11.6 / 22.7 and 27.3 / 76; 500 tokens beside 15 with one more after 2,000 414 / 1,200 and 262 / 895."""
+    pages = keys = longest = 0
+    for c, st in zip(counts, starts):
+        c, st = int(c), int(st)
+        for q0 in range(0, c, 64):
+            first, last = st + q0, st + min(q0 + 64, c) - 1
+            lo = max(0, first - window + 1) if window > 0 else 0
+            pages += last // 64 - lo // 64 + 1
+            whole = 0 if window <= 0 else max(0, last - max(first, window - 1) + 1)  # queries that see `window` keys
+            short = last - first + 1 - whole
+            keys += whole * window + short * (2 * first + short + 1) // 2
+        longest = max(longest, min(st + c, window) if window > 0 else st + c)
+    return pages * heads <= (3 * longest if longest >= 128 else 0) + keys * heads // 500
+
+
 def attention_tile_f32_splits(n_tiles: int, heads: int, max_context: int, device=None) -> int:
     """Slices of a tile's key range: enough CTAs for two per SM, at least four pages a slice."""
     want = -(-2 * sm_count(device) // max(1, n_tiles * heads))

@@ -115,13 +115,15 @@ class Attention(Part):
         tcgen05 kernels (head sizes 64 and 128), shared by all layers with this window
         and number of heads, where they pay; else the 64-query tiles of the
         mma.sync kernel (head sizes 64 and 128), the same for every layer.  In float32
-        the same 64-query tiles, the ones with the most keys first."""
+        64-query tiles, the ones with the most keys first, where they pay."""
         if self.dtype != torch.bfloat16:
-            if not self._tile_f32(self.heads * self.head_dim) or self.TILES_64 in have:
+            name = self._tile_f32_name()
+            if name in have or not self._tile_f32(self.heads * self.head_dim) \
+                    or not ops.attention_tile_f32_pays(counts, starts, self.window, self.heads):
                 return {}
             tiles = sorted(((i, q0) for i, c in enumerate(counts) for q0 in range(0, int(c), 64)),
                            key=lambda t: -(starts[t[0]] + t[1]))
-            return {self.TILES_64: np.asarray(tiles, dtype=np.int32).reshape(-1, 2)}
+            return {name: np.asarray(tiles, dtype=np.int32).reshape(-1, 2)}
         name = self._tc_plan_name()
         if ops.attention_prefill_tc_takes(self.head_dim, PAGE_SIZE, self.heads * self.head_dim) \
                 and ops.prefill_tc_pays(counts, starts, self.window):
@@ -140,8 +142,11 @@ class Attention(Part):
             return {self.TILES_64: np.asarray(tiles, dtype=np.int32).reshape(-1, 2)}
         return {}
 
+    def _tile_f32_name(self) -> str:
+        return f"prefill_f32/window{self.window}/heads{self.heads}"
+
     def _tile_f32(self, q_stride: int) -> bool:
-        """A float32 prompt step's attention runs as tiles of 64 queries."""
+        """The kernel with tiles of 64 queries takes a float32 prompt step."""
         return self.dtype == torch.float32 and ops.attention_tile_f32_takes(self.head_dim, PAGE_SIZE, q_stride)
 
     # -- run --------------------------------------------------------------
@@ -292,8 +297,8 @@ class Attention(Part):
             ops.attention_prefill_mma(q_buf, q_stride, cache.k, cache.v, ctx.tables[self.TILES_64],
                                       ctx.seq_first_row, ctx.seq_start, ctx.seq_count, table, attn,
                                       nq, nkv, d, self.window, self.scale)
-        elif not ctx.decode and self.TILES_64 in ctx.tables and self._tile_f32(q_stride):
-            tiles = ctx.tables[self.TILES_64]
+        elif not ctx.decode and self._tile_f32_name() in ctx.tables and self._tile_f32(q_stride):
+            tiles = ctx.tables[self._tile_f32_name()]
             splits = ops.attention_tile_f32_splits(tiles.shape[0], nq, ctx.max_context, self.device)
             partial = ws.get("attn_partial", (n * nq * splits * (d + 2),), torch.float32) if splits > 1 else None
             ops.attention_tile_f32(q_buf, q_stride, cache.k, cache.v, tiles, ctx.seq_first_row, ctx.seq_start,

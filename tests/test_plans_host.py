@@ -289,3 +289,22 @@ def test_chunks_of_the_delta_rule_keep_their_scratch_within_its_bound():
     wave = o.delta_wave(4096, 32, 16, 128, 128)
     assert 4 * wave * (3 * 16 * 64 * 128 + 32 * (64 * (128 + 128 + 3) + 128 * 128)) <= o.DELTA_SCRATCH < 1 << 30 and wave > 52
     assert o.delta_wave(9, 4096, 4096, 128, 512) >= 1
+
+
+def test_float32_prompts_take_tiles_where_these_pay():
+    """Enough queries to a tile, or a long chain of keys on an empty device; the counts behind the rule are those of the
+    tiles and of the keys that the queries see."""
+    from nnis_b200.csrc import ops as o
+    pays = o.attention_tile_f32_pays
+    assert pays([509, 131, 384], [0, 0, 0], 0, 9) and pays([64], [0], 0, 9) and pays([1] * 8, [2000] * 8, 0, 9)
+    assert not pays([1] * 64, [500] * 64, 0, 9) and not pays([8], [64], 0, 9) and not pays([8] * 64, [0] * 64, 0, 9)
+    assert pays([500] + [1] * 15, [0] + [2000] * 15, 0, 16) and not pays([4] * 64, [2000] * 64, 0, 16)
+    # a window of 50 keys: the far past counts for nothing
+    assert pays([64] * 64, [4000] * 64, 50, 9) == pays([64] * 64, [64 * 50] * 64, 50, 9)
+    assert not pays([1, 1, 2], [4000, 3000, 2000], 50, 9) and pays([1, 1, 2], [4000, 3000, 2000], 0, 9)
+    for window in (0, 1, 7, 64, 100):  # where the first part is nothing: pages x heads against keys x heads / 500
+        for c, st in ((1, 0), (20, 3), (64, 0), (65, 40), (100, 20)):
+            keys = sum(min(st + q + 1, window or 10 ** 9) for q in range(c))
+            tiles = [(st + q0, st + min(q0 + 64, c) - 1) for q0 in range(0, c, 64)]
+            pages = sum(b // 64 - (max(0, a - window + 1) if window else 0) // 64 + 1 for a, b in tiles)
+            assert pays([c], [st], window, 1000) == (pages * 1000 <= keys * 2)
