@@ -2133,10 +2133,12 @@ def delta_scan(qkv: torch.Tensor, beta_g: torch.Tensor, state: torch.Tensor, tok
 
 
 DELTA_CHUNK = 64       # tokens of a chunk of delta_prompt
-# Prompts whose longest sequence has more tokens run in chunks.  Whole prompts of one layer of 16 heads of 64 / 128, us walked
-# and in chunks: 192 tokens 361 / 413 and 399 / 405, 256 tokens 276 / 348 and 183 / 257, 4 x 128 tokens 278 / 382 and
-# 301 / 402, 3 x 300 tokens 391 / 576 and 291 / 485.
-DELTA_CHUNK_MIN = 192
+# Steps whose longest sequence has more tokens run in chunks, if they have DELTA_STEP_MIN tokens together: shorter steps are
+# launched one by one, where the three launches and two tables more cost 40 us.  Whole prompts of one layer, 16 heads
+# with keys of 64 / 32 with keys of 128, values of 128, us walked (beyond 256 tokens in runs) and in chunks: 200 tokens 351 / 354 and
+# 391 / 394, 255 tokens 355 / 371 and 387 / 396, replayed 256 tokens 276 / 364 and 175 / 254, 2 x 200 tokens 274 / 418 and
+# 225 / 346, 3 x 300 tokens 370 / 775 and 286 / 485; 4 x 128 tokens 278 / 382 and 301 / 402.
+DELTA_CHUNK_MIN, DELTA_STEP_MIN = 192, 256
 
 
 DELTA_SCRATCH = 1 << 29  # bytes; 32 heads over 16 of 128 x 128 fill it with 5,800 tokens

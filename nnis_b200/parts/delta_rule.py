@@ -113,7 +113,8 @@ class GatedDeltaRule(Part):
         rule layer of the model that takes them).  Sizes that do not run in chunks, and a sequence longer than two
         runs: the runs of every sequence, worked side by side."""
         if ops.delta_takes_chunks(self.dim, self.vdim):
-            if ops.DELTA_SEGMENT <= 0 or max(counts) <= ops.DELTA_CHUNK_MIN or self.CHUNKS in have:
+            if ops.DELTA_SEGMENT <= 0 or max(counts) <= ops.DELTA_CHUNK_MIN or sum(counts) < ops.DELTA_STEP_MIN \
+                    or self.CHUNKS in have:
                 return {}
             chunks, first = ops.scan_segments(counts, ops.DELTA_CHUNK)
             return {self.CHUNKS: chunks, self.FIRST_CHUNK: first}

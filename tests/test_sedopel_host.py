@@ -332,5 +332,7 @@ def test_prompts_of_the_delta_rule_that_run_in_chunks(monkeypatch):
     tables = part.step_tables([300, 5], [0, 0])
     assert sorted(tables) == [part.CHUNKS, part.FIRST_CHUNK] and tables[part.CHUNKS].shape == (6, 2)
     assert part.step_tables([ops.DELTA_CHUNK_MIN], [0]) == {} and part.step_tables([300], [0], tuple(tables)) == {}
+    assert part.step_tables([255], [0]) == {} and len(part.step_tables([255, 1], [0, 0])) == 2
+    assert part.step_tables([192] * 4, [0] * 4) == {}
     monkeypatch.setattr(ops, "DELTA_SEGMENT", 0)
     assert part.step_tables([3000], [0]) == {}
