@@ -19,14 +19,19 @@
 // more than 8 (a factor 256, harmless in float32 and bfloat16); then the warp waits for the products so far and
 // multiplies its rows of O.  Sum and output are relative to the same maximum, so the result is the exact softmax.
 //
+// A weight of zero does not take an infinity or a NaN out of a product, and a page holds tokens that a query of its tile
+// does not see: later ones, ones that its window has passed, slots that nobody has filled.  So a row whose sum of weights
+// is a number but whose output is not is made again by its thread, from what it sees alone (wide_redo_row).  (Taking such
+// values out of V before the product, in warp 2 or in warp 0, took 4,096 tokens from 128 to 131 and 155 us.)
+//
 // Why two tiles: shared memory (Q 96 KB of 208 at 192 key values) leaves one CTA to an SM, and one tile's softmax
 // would leave the tensor cores idle while it works on a page (about 1,000 cycles, the products of a page 640 to 830);
 // with two, one tile's products run under the other's softmax, and a page fetched serves both.  The host pairs a
 // prompt's first tile with its last, the second with the last but one: every pair has the same number of pages.
 // What bounds it: the softmax warps' special functions and instructions, two warps to a scheduler, and with few tiles
 // the longest CTA.  On a B200, 16 heads of 128 over 4 (paged), before (attention_prefill_mma.cu) and now: one prompt
-// of 512 tokens 67 -> 18 us, 2,048 169 -> 40, 4,096 408 -> 128 (540 TFLOP/s), eight of 300 81 -> 21.  Expanded, keys
-// of 192: 2,048 and 1,311 tokens 74 us, where attention in the latent's space (attention_latent_mma.cu) took 711.
+// of 512 tokens 67 -> 15 us, 2,048 169 -> 38, 4,096 408 -> 126 (549 TFLOP/s), eight of 300 81 -> 20.  Expanded, keys
+// of 192: 2,048 and 1,311 tokens 71 us, where attention in the latent's space (attention_latent_mma.cu) took 711.
 // With K and V in one ring of pages the same took 86: a page's K waited for the V before it to be done with.
 // Every wait is bounded; a wait that runs out raises an abort flag that every role sees, all warps still meet at the
 // end and tensor memory is freed.
@@ -104,6 +109,10 @@ __device__ __forceinline__ void wide_tmem_load16(uint32_t taddr, uint32_t (&v)[1
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void wide_add_zeros(uint32_t& sum, uint32_t two) {  // sum += 0 * two
+    asm("fma.rn.bf16x2 %0, %1, %2, %0;" : "+r"(sum) : "r"(two), "r"(0u));
+}
+
 struct WideArgs {
     const int* units;          // [n, 4]: sequence, first query of the first tile, of the second (-1: none), unused
     const int* seq_first_row;
@@ -116,7 +125,61 @@ struct WideArgs {
     int nq, nkv, q_head, k_head, v_off, window;
     float scale;
     int* status;
+    // the operands as they lie in memory, for a row that is made again: rows of q, of plain keys, of the shared part and of
+    // values, and the elements between these
+    const bf16 *q, *k, *r, *v;
+    int q_row, kv_row;
 };
+
+// A row of the output again, keys one by one: columns that hold no number although every value seen is one.  A column with
+// an infinity or a NaN among the values seen has what their sum is (weights are positive).  m, l: the row's maximum in use
+// (scaled, log2 units) and its sum against it.  Slow, and no row of a model whose values are numbers comes here.
+template <int KC, int KLAST, int DV, bool PAGED>
+__device__ __noinline__ void wide_redo_row(const WideArgs& p, int seq, int hq, int token, int pos, float m, float l) {
+    constexpr int SHARED = PAGED ? 0 : KLAST * 16, OWN = (KC - 1) * 64 + KLAST * 16 - SHARED;  // key values of the head, of all heads
+    const int hk = hq / (p.nq / p.nkv), lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+    const bf16* q = p.q + (size_t)token * p.q_row + (size_t)hq * p.q_head;
+    bf16* out = p.out + ((size_t)token * p.nq + hq) * DV;
+    auto row_of = [&](int key) {
+        return PAGED ? ((size_t)p.page_table[(size_t)seq * p.table_cols + key / kWidePage] * p.nkv + hk) * kWidePage + key % kWidePage
+                     : (size_t)p.key_base[seq] + key;
+    };
+    const size_t k_off = PAGED ? 0 : (size_t)hq * p.k_head, v_off = p.v_off + (PAGED ? 0 : (size_t)hq * DV);
+    for (int c0 = 0; c0 < DV; c0 += 8) {
+        uint32_t wrong = 0, nan = 0, up = 0, down = 0;  // a bit a column
+        for (int e = 0; e < 8; ++e) wrong |= isfinite(to_float(out[c0 + e])) ? 0u : 1u << e;
+        for (int key = pos; key >= lo && (wrong & ~nan); --key) {
+            const bf16* v = p.v + row_of(key) * p.kv_row + v_off + c0;
+            for (int e = 0; e < 8; ++e) {
+                const float x = to_float(v[e]);
+                if (isfinite(x)) continue;
+                if (x > 0.f) up |= 1u << e;
+                else if (x < 0.f) down |= 1u << e;
+                else nan |= 1u << e;
+            }
+        }
+        nan |= up & down;
+        for (int e = 0; e < 8; ++e)
+            if (wrong >> e & 1u && (nan | up | down) >> e & 1u)
+                out[c0 + e] = from_float<bf16>(nan >> e & 1u ? __int_as_float(0x7fffffff) : up >> e & 1u ? INFINITY : -INFINITY);
+        wrong &= ~(nan | up | down);
+        if (!wrong) continue;
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (int key = lo; key <= pos; ++key) {
+            const size_t row = row_of(key);
+            const bf16* k = p.k + row * p.kv_row + k_off;
+            float score = 0.f;
+            for (int i = 0; i < OWN; ++i) score = fmaf(to_float(q[i]), to_float(k[i]), score);
+            for (int i = 0; i < SHARED; ++i) score = fmaf(to_float(q[OWN + i]), to_float(p.r[row * 64 + i]), score);
+            const float w = to_float(from_float<bf16>(wide_ex2(fmaf(score, p.scale * 1.4426950408889634f, -m))));
+            const bf16* v = p.v + row * p.kv_row + v_off + c0;
+            for (int e = 0; e < 8; ++e)
+                if (wrong >> e & 1u) acc[e] = fmaf(w, to_float(v[e]), acc[e]);
+        }
+        for (int e = 0; e < 8; ++e)
+            if (wrong >> e & 1u) out[c0 + e] = from_float<bf16>(acc[e] / l);
+    }
+}
 
 // KC: chunks of 64 key values, the last one of which has 16 KLAST; DV: values; PAGED: which form of the keys (with
 // expanded keys the last chunk is the shared part).
@@ -124,7 +187,7 @@ template <int KC, int KLAST, int DV, bool PAGED, int STAGES>
 __global__ void __launch_bounds__(kWideThreads, 1)
 attn_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_v,
-                    const WideArgs p) {
+                    const __grid_constant__ WideArgs p) {
     constexpr int VC = DV / 64;
     constexpr uint32_t kStageK = KC * kWideK, kStageV = VC * kWideK, kTileQ = KC * kWideQ;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -414,6 +477,7 @@ attn_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         } else if (pages > 0) {
             tc_fence_after();
             const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+            uint32_t zero[4] = {0u, 0u, 0u, 0u};  // two bfloat16 each: no numbers once an output is none
             bf16* dst = p.out + (size_t)(row_base + (t ? q0[1] : q0[0]) + row) * p.nq * DV + (size_t)hq * DV;
 #pragma unroll 1
             for (int h = 0; h < DV / 32; ++h) {
@@ -428,12 +492,15 @@ attn_wide_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                             const __nv_bfloat162 pk = __floats2bfloat162_rn(__uint_as_float(ov[c + 2 * e]) * inv,
                                                                             __uint_as_float(ov[c + 2 * e + 1]) * inv);
                             w[e] = *reinterpret_cast<const uint32_t*>(&pk);
+                            wide_add_zeros(zero[e], w[e]);
                         }
                         *reinterpret_cast<uint4*>(dst + h * 32 + c) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
                 }
             }
             tc_fence_before();
+            if (((zero[0] | zero[1] | zero[2] | zero[3]) & 0x7fff7fffu) && isfinite(l_run))
+                wide_redo_row<KC, KLAST, DV, PAGED>(p, seq, hq, row_base + (t ? q0[1] : q0[0]) + row, pos, m_run, l_run);
         }
     }
     tc_fence_before();
@@ -489,7 +556,8 @@ NNIS_API int nnis_attention_wide_tc(const void* q, int q_stride, int n_tokens, c
         !make_map(&mv, v_cache, cache_rows, d, kWidePage))
         return NNIS_ERR_UNSUPPORTED;
     const WideArgs args = {units, seq_first_row, seq_start, seq_count, page_table, nullptr, table_cols, (bf16*)out,
-                           nq, nkv, d, d, 0, window, scale, status};
+                           nq, nkv, d, d, 0, window, scale, status, (const bf16*)q, (const bf16*)k_cache, nullptr,
+                           (const bf16*)v_cache, q_stride, d};
     return launch_wide<2, 4, 128, true, 3>(mq, mk, mk, mv, args, n_units, pdl, stream);
 }
 
@@ -513,7 +581,8 @@ NNIS_API int nnis_attention_wide_tc_expanded(const void* q, int n_tokens, const 
         !make_map(&mk, kv, n_rows, heads * (dim + vdim), kWidePage) || !make_map(&mr, kr, n_rows, 64, kWidePage))
         return NNIS_ERR_UNSUPPORTED;
     const WideArgs args = {units, seq_first_row, seq_start, seq_count, nullptr, key_base, 0, (bf16*)out,
-                           heads, heads, dim + rot, dim, heads * dim, window, scale, status};
+                           heads, heads, dim + rot, dim, heads * dim, window, scale, status, (const bf16*)q,
+                           (const bf16*)kv, (const bf16*)kr, (const bf16*)kv, heads * (dim + rot), heads * (dim + vdim)};
     return large ? launch_wide<3, 4, 128, false, 2>(mq, mk, mr, mk, args, n_units, pdl, stream)
                  : launch_wide<2, 2, 64, false, 4>(mq, mk, mr, mk, args, n_units, pdl, stream);
 }

@@ -81,7 +81,7 @@ def test_wide_prompt_attention_on_tcgen05(nq, nkv, window, pad, sms):
     o = ops()
     d, lengths, new = 128, [70, 1, 200, 64, 333, 129, 1500], [70, 1, 5, 64, 200, 65, 1500]
     case = PagedCase(lengths, new, nq, nkv, d, "bfloat16", seed=5 * nq + window)
-    kc, vc = stored(case, torch.bfloat16, 50.0)
+    kc, vc = stored(case, torch.bfloat16, math.nan)
     q = case.packed()[2]
     n, stride = q.shape[0], nq * d + pad
     qd = torch.full((n, stride), 3.0, dtype=torch.bfloat16, device=DEV)
@@ -131,6 +131,88 @@ def test_wide_prompt_attention_over_expanded_latents(dim, rot, heads, sms, sharp
         hidden = torch.arange(L)[None, :] > torch.arange(L - new[s], L)[:, None]
         want = torch.einsum("hts,shd->thd", torch.softmax(scores.masked_fill(hidden, -math.inf), -1), v)
         close(out[r:r + new[s]], want.reshape(new[s], -1), "bfloat16", f"sequence {s}")
+        r += new[s]
+
+
+def spoilt(v, at):
+    """Values with infinities and NaN in two of their columns at the positions ``at``."""
+    v = v.clone()
+    for i, t in enumerate(at):
+        v[t, :, 5] = math.nan if i % 2 else math.inf
+        v[t, :, 50] = -math.inf if i % 2 else math.inf
+    return v
+
+
+def check_spoilt(got, fine, v, at, starts, window, what):
+    """``got`` is ``fine`` for the queries that see none of the positions ``at`` and in the columns where these are
+    numbers; a query that sees them has what their sum with a positive weight each is."""
+    for t in range(got.shape[0]):
+        seen = [a for a in at if a <= starts + t and (window == 0 or starts + t - a < window)]
+        want = fine[t] + sum((torch.where(torch.isfinite(v[a].double()), 0.0, v[a].double()) for a in seen), torch.zeros(()))
+        same = torch.isfinite(want)
+        close(got[t][same], want[same], "bfloat16", f"{what}, query {t}")
+        assert torch.equal(torch.nan_to_num(got[t][~same].double(), 7.0), torch.nan_to_num(want[~same], 7.0)), (what, t)
+
+
+@pytest.mark.parametrize("window", [0, 70])
+@pytest.mark.parametrize("sms", [1000, 1])
+def test_wide_prompt_attention_and_values_that_are_no_numbers(window, sms):
+    """An infinity or a NaN among the values is not felt by a query that does not see its token: the ones before it in
+    its tile of 128, the ones whose window has passed it."""
+    o = ops()
+    d, nq, nkv = 128, 4, 2
+    lengths, new, at = [70, 300, 700], [70, 300, 500], [[69], [0, 64, 200, 299], [100, 230, 450, 451, 640]]
+    case = PagedCase(lengths, new, nq, nkv, d, "bfloat16", seed=window)
+    finite = case.v
+    case.v = [spoilt(v, a) for v, a in zip(finite, at)]
+    kc, vc = stored(case, torch.bfloat16, math.nan)
+    q = case.packed()[2]
+    n = q.shape[0]
+    first, start, count, starts = wide_inputs(new, lengths)
+    units = o.attention_wide_plan(new, starts, window, nq, sms)
+    out = torch.full((n, nq * d), 5.0, dtype=torch.bfloat16, device=DEV)
+    o.attention_wide_tc(q.reshape(n, -1).bfloat16().to(DEV), nq * d, kc, vc, torch.from_numpy(units).to(DEV), first, start,
+                        count, case.table.to(DEV), out, nq, nkv, d, window, 1.0 / math.sqrt(d))
+    o.check_status(DEV)
+    r = 0
+    for s, L in enumerate(lengths):
+        zeroed = torch.where(torch.isfinite(case.v[s]), case.v[s], torch.zeros(()))
+        fine = P.causal_attention(case.q[s], case.k[s], zeroed, window)[L - new[s]:]
+        check_spoilt(out[r:r + new[s]].cpu().view(new[s], nq, d), fine, case.v[s].repeat_interleave(nq // nkv, 1), at[s],
+                     L - new[s], window, f"sequence {s}")
+        r += new[s]
+
+
+@pytest.mark.parametrize("dim,rot", [(128, 64), (64, 32)])
+@pytest.mark.parametrize("sms", [1000, 1])
+def test_expanded_latents_and_values_that_are_no_numbers(dim, rot, sms):
+    o = ops()
+    g = torch.Generator().manual_seed(dim + sms)
+    heads, lengths, new, at = 2, [64, 333], [64, 200], [[63], [20, 140, 200, 201, 330]]
+    first, start, count, starts = wide_inputs(new, lengths)
+    base, rows, n = [0, 64], 64 + 384, sum(new)
+    q = torch.randn(n, heads, dim + rot, generator=g).bfloat16()
+    kv, kr = torch.randn(rows, heads * 2 * dim, generator=g).bfloat16(), torch.zeros(rows, 64)
+    kr[:, :rot] = torch.randn(rows, rot, generator=g)
+    kr, v = kr.bfloat16(), kv[:, heads * dim:].view(rows, heads, dim)
+    for s in range(2):
+        v[base[s]:base[s] + lengths[s]] = spoilt(v[base[s]:base[s] + lengths[s]], at[s])
+    v[base[1] + lengths[1]:] = math.nan  # (rows past the sequence's last position)
+    units = torch.from_numpy(o.attention_wide_plan(new, starts, 0, heads, sms)).to(DEV)
+    out = torch.full((n, heads * dim), 5.0, dtype=torch.bfloat16, device=DEV)
+    scale = (dim + rot) ** -0.5
+    o.attention_wide_tc_expanded(q.reshape(n, -1).to(DEV), kv.to(DEV), kr.to(DEV), units, i32(base), first, start, count,
+                                 out, heads, dim, rot, dim, 0, scale)
+    o.check_status(DEV)
+    r = 0
+    for s, L in enumerate(lengths):
+        part = slice(base[s], base[s] + L)
+        k = torch.cat([kv[part, :heads * dim].view(L, heads, dim), kr[part, None, :rot].expand(L, heads, rot)], -1).double()
+        zeroed = torch.where(torch.isfinite(v[part].double()), v[part].double(), 0.0)
+        scores = torch.einsum("thd,shd->hts", q[r:r + new[s]].double(), k) * scale
+        hidden = torch.arange(L)[None, :] > torch.arange(L - new[s], L)[:, None]
+        fine = torch.einsum("hts,shd->thd", torch.softmax(scores.masked_fill(hidden, -math.inf), -1), zeroed)
+        check_spoilt(out[r:r + new[s]].cpu().view(new[s], heads, dim), fine, v[part], at[s], L - new[s], 0, f"sequence {s}")
         r += new[s]
 
 
