@@ -93,13 +93,16 @@ class EngineBackend:
         self._picked = views[0]
         return views[1] if need_logits else None
 
-    def _replay(self, slots: List[int], tokens: List[int], need_logits: bool) -> GraphDecoder:
-        """One token per slot as a replay of the captured step; its inputs go up in one copy."""
+    def _replay(self, slots: List[int], tokens: List[int], need_logits: bool,
+                dec: Optional[GraphDecoder] = None) -> GraphDecoder:
+        """One token per slot as a replay of the captured step (``dec``: its decoder, where the caller has it); its inputs go
+        up in one copy."""
         cache = self.engine.cache
         positions = [cache.length(s) for s in slots]
         new_lengths = [p + 1 for p in positions]
         cache.reserve(slots, new_lengths)
-        dec = self._decoder(len(slots), max(new_lengths), need_logits)
+        if dec is None:
+            dec = self._decoder(len(slots), max(new_lengths), need_logits)
         self.h2d_bytes += dec.upload(tokens, positions, slots)
         dec.launch()
         cache.commit(slots, new_lengths)
@@ -112,14 +115,18 @@ class EngineBackend:
         already."""
         engine = self.engine
         key = self._decoder_key(1, engine.cache.length(slot) + 1, True)
-        if self.decode_greedy is None or key in self._uncaptured or not (again or key in self._decoders) \
-                or not 0 <= token < engine.spec.vocab_size or not self._captured(key):
+        dec = self._decoders.get(key)
+        if dec is None or dec.graph is None:
+            capture = again and self.decode_greedy is not None and key not in self._uncaptured \
+                and 0 <= token < engine.spec.vocab_size
+            dec = self._captured(key) if capture else None
+        if dec is None or not 0 <= token < engine.spec.vocab_size:
             return engine.step([SequenceStep(slot, [token], [0])])[0]  # (which says what is wrong with a token)
-        return self._replay([slot], [token], True).logits[0]
+        return self._replay([slot], [token], True, dec).logits[0]
 
-    def _captured(self, key) -> bool:
-        """Whether the decoder of this key has its graph, captured now if need be.  Where that fails (no memory for its
-        buffers, say) it is not tried again."""
+    def _captured(self, key) -> Optional[GraphDecoder]:
+        """The decoder of this key with its graph, captured now.  Where that fails (no memory for its buffers, say) None,
+        and it is not tried again."""
         try:
             if key not in self._decoders:
                 self._decoders[key] = GraphDecoder(self.engine, *key)
@@ -129,8 +136,8 @@ class EngineBackend:
             self._uncaptured.add(key)
             warnings.warn(f"a decode step of up to {key[1]} positions could not be captured and is launched kernel by "
                           f"kernel: {error}", RuntimeWarning)
-            return False
-        return True
+            return None
+        return self._decoders[key]
 
     def greedy(self, logits: Optional[torch.Tensor]) -> List[int]:
         if self._picked is not None:  # the graph has picked already
