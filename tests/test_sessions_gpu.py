@@ -83,7 +83,7 @@ def test_a_session_captures_its_step_once_that_pays(tmp_path):
     rows = [session.prefill(tokens[:9])]
     for t in tokens[9:]:
         rows.append(session.decode_one(t))
-        graphs.append(sum(d.graph is not None for d in llm.backend._decoders.values()))
+        graphs.append(sum(dec.graph is not None for dec in llm.backend._decoders.values()))
     assert graphs == [0] * 5 + [1] * 6
     check_logits(np.stack(rows), plain(tokens)[8:], "float32", "session")
     other = llm.new_session()
@@ -92,3 +92,25 @@ def test_a_session_captures_its_step_once_that_pays(tmp_path):
     llm.backend._decoders[next(iter(llm.backend._decoders))].launch = lambda: replayed.append(1)
     other.decode_one(tokens[9])
     assert replayed == [1]
+
+
+@pytest.mark.parametrize("name", ["nafezen", "sedopel", "selovik", "setenex", "tazadra", "zadurax"])
+def test_long_sessions_of_every_design(name, tmp_path):
+    """Two sessions that take turns, over the context where the next larger graph takes over: the states, caches and
+    page tables that a replay reads are those of its own session."""
+    from nnis_b200 import LLM
+    d, vocab, plain = design(name, "mixed", tmp_path)
+    llm = LLM(d, dtype="float32", max_tokens=64 * 32, max_batch=2)
+    rng = random.Random(9)
+    a, b = random_tokens(rng, 275, vocab), random_tokens(rng, 60, vocab)
+    one, two = llm.new_session(), llm.new_session()
+    rows = {0: [one.prefill(a[:240])], 1: [two.prefill(b[:30])]}
+    for i in range(35):
+        rows[0].append(one.decode_one(a[240 + i]))
+        if i < 30:
+            rows[1].append(two.decode_one(b[30 + i]))
+    assert len(llm.backend._decoders) >= 2  # (contexts of up to 256 and of up to 512)
+    check_logits(np.stack(rows[0]), plain(a)[239:], "float32", f"{name}: long session")
+    check_logits(np.stack(rows[1]), plain(b)[29:], "float32", f"{name}: short session")
+    one.close()
+    two.close()
