@@ -301,8 +301,7 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, fl
     }
     __syncthreads();
     const int seq = mine;
-    // (the sequence's chunks among the wave's, numbered as the scratch is)
-    const int c0 = max(seq_first_chunk[seq], wave0) - wave0, c1 = min(seq_first_chunk[seq + 1], wave0 + wave_n) - wave0;
+    const int c0 = max(seq_first_chunk[seq], wave0), c1 = min(seq_first_chunk[seq + 1], wave0 + wave_n);  // among the wave's
     if (c1 <= c0) return;
     float* slot = state + ((size_t)seq_slots[seq] * H + h) * DIM * vdim;
     for (int it = tid; it < DIM * CW; it += 256) {
@@ -544,10 +543,13 @@ NNIS_API int nnis_delta_prompt(const float* a, const float* conv_w, const float*
         if (e == cudaSuccess)
             e = launch_dependent(solve, dim3(n, H), 128, solve_smem, stream, (const float*)qk, (const float*)u,
                                  (const float*)beta, (const double*)logs, w, u, H, G, vp);
+        // (the chain numbers the chunks of all waves, so its scratch begins where the first wave's would)
+        const size_t gone = (size_t)c0 * H;
         if (e == cudaSuccess)
-            e = launch_dependent(chain, dim3((vp + 31) / 32, H, n_seqs), 256, chain_smem, stream, (const float*)qk,
-                                 (const float*)w, u, (const double*)logs, before, state, seq_slots, seq_count,
-                                 seq_first_chunk, c0, n, H, G, vdim, vp);
+            e = launch_dependent(chain, dim3((vp + 31) / 32, H, n_seqs), 256, chain_smem, stream,
+                                 (const float*)(qk - (size_t)c0 * G * delta_qk_floats(dim)),
+                                 (const float*)(w - gone * dim * kDC), u - gone * kDC * vp, (const double*)(logs - gone * kDC),
+                                 before - gone * dim * vp, state, seq_slots, seq_count, seq_first_chunk, c0, n, H, G, vdim, vp);
         if (e == cudaSuccess)
             e = launch_dependent(read, dim3(n, H, (vp + bv - 1) / bv), 128, read_smem, stream, (const float*)qk,
                                  (const float*)u, (const double*)logs, (const float*)before, own, seq_first_row, seq_count,
