@@ -110,7 +110,7 @@ class EngineBackend:
 
     def decode_logits(self, slot: int, token: int, again: bool) -> torch.Tensor:
         """Logits [vocab] of one sequence's next token.  A step of the SmolLM2-135M shape is 154 launches, 4.1 ms from
-        Python one by one and 0.47 ms as a replay; to capture one takes 15 to 29 ms, what four to eight replays save, so the
+        Python one by one and 0.47 ms as a replay; to capture one takes 11 to 29 ms, what three to eight replays save, so the
         first tokens that a session decodes (``again`` False) capture nothing, and replay only where the graph is there
         already."""
         engine = self.engine
