@@ -1,0 +1,410 @@
+// float32 matrix product on the fifth-generation tensor cores: C[M, N] (op)= A[M, K] . W[N, K]^T + bias, every float32
+// value taken as the exact sum of three bfloat16 values.
+//
+// A float32 value x has 24 significant bits.  h = bfloat16(x), m = bfloat16(x - h) and l = bfloat16(x - h - m) hold them
+// all (both differences are exact), and bfloat16 has float32's range of exponents, so no scaling is needed.  Of the nine
+// products of two such sums the six largest are made (h h, h m, m h, m m, h l, l h); what is left out is 2^-27 of a
+// product and less, where float32 rounds every sum at 2^-24.  The tensor cores cut their running sum off instead of
+// rounding it, so no sum stays there for long: 64 columns of K at a time, the small products first, and then the 64
+// columns' sum is added in registers, by an ordinary float32 addition.  Against 64-bit sums this is closer than the
+// chains of float32 multiply-adds of gemm_simt.cu (figures at the bottom of this comment).
+//
+// A product that is no number (an infinity among the operands: its h is one and its m is none) is made again from the
+// operands by a chain of multiply-adds, so infinities come out as they do there.
+//
+// One CTA works a tile of 128 x BN (BN 64 or 128), KS CTAs of a cluster share the tile's K and add their sums through
+// distributed shared memory, in the order of their ranks (the same bits every time).  Roles:
+//   warp 0       allocates tensor memory; one lane issues tcgen05.mma (kind::f16, 128 x BN x 16), 24 for 64 columns of K,
+//                into one of two accumulators;
+//   warps 1-16   bring A and W, 32 bytes a load, one block of K ahead in registers, write the three parts of each value
+//                into swizzled shared memory (two blocks of K), then read the accumulator of the block before with
+//                tcgen05.ld and add it to their registers (a row and a quarter of the columns a thread); at the end they
+//                write the tile, through shared memory, so that whole lines leave.
+// Splitting on the way in keeps the weights once in memory, as the decode kernels read them.
+//
+// What bounds it: the products read A and W again for each pair of parts, 8 KB of shared memory every 64 cycles (BN = 128),
+// beside 96 KB of parts written for 64 columns of K: 2,750 cycles a block of K where the products alone would take 1,536;
+// the splitting itself (ALU) takes 2,300 under them.  Rows x N x K on a B200, cold L2, gemm_slab_kernel -> here:
+// 1,024 x 3,072 x 576 104 -> 47 us (2 waves of tiles), 1,024 x 576 x 1,536 82 -> 29, 1,024 x 576 x 576 35 -> 18,
+// 2,048 x 2,048 x 2,048 416 -> 123 (140 TFLOP/s of float32), 17 x 576 x 576 35 -> 14.  Distance from 64-bit sums (2-norm, K =
+// 576 / 1,536 / 5,632): 2.2e-7 / 3.5e-7 / 6.7e-7 there, 0.98e-7 / 1.1e-7 / 1.5e-7 here.
+// Level: eight warps that split and eight that add (158 us at 1,024 x 2,048 x 5,632 here, 180 there).
+// Every wait is bounded, as in gemm_tcgen05.cu.
+// NNIS: crates/nnis-kernels/src/gemm.rs:16-64 (tiled float32 product on CUDA cores).
+#include "fma_pairs.cuh"
+#include "tcgen05_helpers.cuh"
+
+namespace nnis {
+
+constexpr int kSplitM = 128, kSplitK = 64;
+constexpr int kSplitStages = 2;
+constexpr int kSplitAccs = 4;    // accumulators
+constexpr int kSplitWorkers = 16;  // warps
+constexpr int kSplitThreads = 32 * (1 + kSplitWorkers);
+constexpr uint32_t kSplitPartA = kSplitM * 128;  // one part of a block of A: 128 rows of 64 bfloat16
+
+__host__ __device__ constexpr uint32_t split_stage_bytes(int bn) { return 3u * (kSplitPartA + (uint32_t)bn * 128u); }
+
+struct SplitArgs {
+    const float* A;
+    const float* W;
+    const float* bias;
+    float* C;
+    int M, N, K, add;
+    int* status;
+};
+
+// Eight consecutive floats in one load, in pairs; the address is a multiple of 32 bytes.
+__device__ __forceinline__ void load8(const float* p, unsigned long long (&v)[4]) {
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
+}
+
+// A pair of values' next bfloat16 parts, packed; what is left of the values stays in x.
+__device__ __forceinline__ uint32_t next_part(unsigned long long& x) {
+    uint32_t p;
+    asm("{\n\t.reg .f32 a, b;\n\t.reg .b32 lo, hi;\n\t.reg .b64 h;\n\t"
+        "mov.b64 {a, b}, %1;\n\t"
+        "cvt.rn.bf16x2.f32 %0, b, a;\n\t"
+        "shl.b32 lo, %0, 16;\n\t"
+        "and.b32 hi, %0, 0xffff0000;\n\t"
+        "mov.b64 h, {lo, hi};\n\t"
+        "sub.rn.f32x2 %1, %1, h;\n\t}"
+        : "=r"(p), "+l"(x));
+    return p;
+}
+__device__ __forceinline__ uint32_t last_part(unsigned long long x) {
+    const float2 f = halves(x);
+    uint32_t p;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p) : "f"(f.y), "f"(f.x));
+    return p;
+}
+
+// The element (m, n) by a chain of float32 multiply-adds, for sums that are no numbers.
+__device__ __noinline__ float split_again(const float* a, const float* w, int K) {
+    float s = 0.f;
+    for (int k = 0; k < K; ++k) s = fmaf(a[k], w[k], s);
+    return s;
+}
+
+// Four floats at the same place of the shared memory of the cluster's CTA `rank`.
+__device__ __forceinline__ float4 peer_load4(const float* p, uint32_t rank) {
+    uint32_t at;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_addr(p)), "r"(rank));
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+
+template <int BN, int KS>
+__global__ void __launch_bounds__(kSplitThreads, 1)
+gemm_split_kernel(const SplitArgs g) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* base = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    constexpr uint32_t kPartW = BN * 128, kStage = split_stage_bytes(BN);
+    constexpr uint32_t kTmemCols = kSplitAccs * BN;
+    __shared__ __align__(8) uint64_t full_bar[kSplitStages], empty_bar[kSplitStages], acc_full[kSplitAccs], acc_empty[kSplitAccs];
+    __shared__ uint32_t tmem_base_s;
+    __shared__ volatile int abort_flag;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n0 = (blockIdx.x / KS) * BN, m0 = blockIdx.y * kSplitM;
+    const int rank = KS > 1 ? (int)cluster_rank() : 0;
+    const int blocks_all = (g.K + kSplitK - 1) / kSplitK;
+    // this CTA's run of blocks of K
+    const int per = (blocks_all + KS - 1) / KS;
+    const int first = min(blocks_all, rank * per), blocks = min(per, blocks_all - first);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kSplitStages; ++s) {
+            mbar_init(&full_bar[s], kSplitWorkers);
+            mbar_init(&empty_bar[s], 1);
+        }
+        for (int b = 0; b < kSplitAccs; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], kSplitWorkers);
+        }
+        abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (warp == 0) tmem_alloc(&tmem_base_s, kTmemCols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base_s;
+
+    constexpr int kCols = BN / 4;  // columns of the accumulator to a worker warp
+    unsigned long long acc[kCols / 2];  // pairs
+#pragma unroll
+    for (int i = 0; i < kCols / 2; ++i) acc[i] = 0ull;
+    if (warp == 0) {
+        pdl_wait();
+        pdl_launch_dependents();
+        if (lane == 0) {
+            constexpr uint32_t idesc = instr_desc(kSplitM, BN);
+            const uint64_t desc_a0 = smem_desc_k128(smem_addr(base));
+            const uint64_t desc_w0 = smem_desc_k128(smem_addr(base) + 3 * kSplitPartA);
+            for (int kb = 0; kb < blocks; ++kb) {
+                const int s = kb & 1, b = kb & 3;
+                if (!mbar_wait(&full_bar[s], (uint32_t)(kb >> 1) & 1u) ||
+                    (kb >= 4 && !mbar_wait(&acc_empty[b], (uint32_t)((kb >> 2) - 1) & 1u)) || abort_flag) {
+                    abort_flag = 1;
+                    break;
+                }
+                tc_fence_after();
+                const uint64_t da = desc_advance(desc_a0, (uint32_t)s * kStage);
+                const uint64_t dw = desc_advance(desc_w0, (uint32_t)s * kStage);
+                // parts of A and W, the smallest products first
+                constexpr int kPartsA[6] = {2, 0, 1, 1, 0, 0}, kPartsW[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+                for (int p = 0; p < 6; ++p)
+#pragma unroll
+                    for (int k = 0; k < kSplitK / 16; ++k)
+                        tc_mma(tmem + (uint32_t)b * BN, desc_advance(da, kPartsA[p] * kSplitPartA + k * 32),
+                               desc_advance(dw, kPartsW[p] * kPartW + k * 32), idesc, (p | k) != 0);
+                tc_commit(&empty_bar[s]);
+                tc_commit(&acc_full[b]);
+            }
+        }
+        __syncwarp();
+    } else {
+        // a warp splits four rows at a time, eight floats a lane: (128 + BN) / 64 such items a thread and block of K
+        const int worker = warp - 1, r4 = lane >> 3, unit = lane & 7;
+        constexpr int kItemsA = kSplitM / (4 * kSplitWorkers), kItems = kItemsA + BN / (4 * kSplitWorkers);
+        unsigned long long v[kItems][4];
+        const float* src[kItems];
+        uint32_t there = 0;  // bit i: the row of item i exists
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            const int row = ((i < kItemsA ? i : i - kItemsA) * kSplitWorkers + worker) * 4 + r4;
+            const int at = i < kItemsA ? m0 + row : n0 + row;
+            src[i] = (i < kItemsA ? g.A : g.W) + (size_t)at * g.K + first * kSplitK + unit * 8;
+            if (at < (i < kItemsA ? g.M : g.N)) there |= 1u << i;
+            v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0ull;  // (rows beyond M and N are never loaded and stay zero)
+        }
+        auto load = [&](int i, uint32_t wanted) {
+            if (wanted & (1u << i)) load8(src[i], v[i]);
+            src[i] += kSplitK;
+        };
+        int k_left = g.K - first * kSplitK - unit * 8;  // columns from this lane's of the next block on
+        // (a warp reads the 32 lanes of tensor memory that its number gives it)
+        const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(worker >> 2) * kCols;
+        auto add_block = [&](int kb) {
+            const int b = kb & 3;
+            bool ok = mbar_wait(&acc_full[b], (uint32_t)(kb >> 2) & 1u);
+            ok = __all_sync(0xffffffffu, ok) && !abort_flag;
+            if (!ok) return false;
+            tc_fence_after();
+#pragma unroll
+            for (int c = 0; c < kCols; c += 16) {
+                uint32_t x[16];
+                tmem_load16_issue(lanes + (uint32_t)(b * BN + c), x);
+                tmem_load_wait();
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    asm("{\n\t.reg .b64 p;\n\tmov.b64 p, {%1, %2};\n\tadd.rn.f32x2 %0, %0, p;\n\t}"
+                        : "+l"(acc[c / 2 + i]) : "r"(x[2 * i]), "r"(x[2 * i + 1]));
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[b]);
+            return true;
+        };
+        uint32_t wanted = blocks > 0 && k_left > 0 ? there : 0u;
+#pragma unroll
+        for (int i = kItemsA; i < kItems; ++i) load(i, wanted);  // (weights depend on no kernel)
+        pdl_wait();
+#pragma unroll
+        for (int i = 0; i < kItemsA; ++i) load(i, wanted);
+        bool ok = true;
+        // half of the warps add before they split a block and half after it: one's wait for tensor memory under the
+        // other's arithmetic
+        const bool early = (worker & 4) != 0;
+        for (int kb = 0; kb < blocks && ok; ++kb) {
+            const int s = kb & 1;
+            if (early && kb >= 2 && !(ok = add_block(kb - 2))) break;
+            ok = kb < 2 || mbar_wait(&empty_bar[s], (uint32_t)((kb >> 1) - 1) & 1u);
+            ok = __all_sync(0xffffffffu, ok) && !abort_flag;
+            if (!ok) break;
+            if (k_left <= 0) {  // columns beyond K
+#pragma unroll
+                for (int i = 0; i < kItems; ++i) v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0ull;
+            }
+            k_left -= kSplitK;
+            wanted = kb + 1 < blocks && k_left > 0 ? there : 0u;
+            unsigned char* stage = base + (size_t)s * kStage + r4 * 128;
+#pragma unroll
+            for (int i = 0; i < kItems; ++i) {
+                const bool is_a = i < kItemsA;
+                const int row4 = ((is_a ? i : i - kItemsA) * kSplitWorkers + worker) * 4;
+                unsigned char* dst = stage + (is_a ? 0 : 3 * kSplitPartA) + row4 * 128 + ((unit ^ ((row4 & 4) + r4)) << 4);
+                uint4 o;
+                o.x = next_part(v[i][0]);
+                o.y = next_part(v[i][1]);
+                o.z = next_part(v[i][2]);
+                o.w = next_part(v[i][3]);
+                *reinterpret_cast<uint4*>(dst) = o;
+                o.x = next_part(v[i][0]);
+                o.y = next_part(v[i][1]);
+                o.z = next_part(v[i][2]);
+                o.w = next_part(v[i][3]);
+                *reinterpret_cast<uint4*>(dst + (is_a ? kSplitPartA : kPartW)) = o;
+                o.x = last_part(v[i][0]);
+                o.y = last_part(v[i][1]);
+                o.z = last_part(v[i][2]);
+                o.w = last_part(v[i][3]);
+                *reinterpret_cast<uint4*>(dst + 2 * (is_a ? kSplitPartA : kPartW)) = o;
+                load(i, wanted);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full_bar[s]);
+            if (!early && kb >= 2) ok = add_block(kb - 2);
+        }
+        for (int kb = max(0, blocks - 2); kb < blocks && ok; ++kb) ok = add_block(kb);
+        if (!ok) abort_flag = 1;
+    }
+
+    // ---- the tile: through shared memory, its lines whole ------------------------------------------------------
+    // (all products have been read out: the stages are free)
+    constexpr int kRow = BN + 4;  // floats between rows: 16-byte stores of neighbouring rows meet no bank twice
+    float* sums = reinterpret_cast<float*>(base);
+    __syncthreads();
+    const int quarter = warp & 3, c0 = warp > 0 ? ((warp - 1) >> 2) * kCols : 0;
+    if (warp > 0) {
+        float* mine = sums + (quarter * 32 + lane) * kRow + c0;
+#pragma unroll
+        for (int i = 0; i < kCols; i += 4)
+            *reinterpret_cast<ulonglong2*>(mine + i) = make_ulonglong2(acc[i / 2], acc[i / 2 + 1]);
+    }
+    if constexpr (KS > 1) cluster_meet();
+    else __syncwarp();
+    if (warp > 0 && !abort_flag) {
+        constexpr int kLanes = kCols / 4;       // lanes to a row's columns of this warp, four floats each
+        constexpr int kRows = 32 / kLanes;      // rows a warp writes at a time
+        const bool by_four = (g.N & 3) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15) == 0;
+        const int n = n0 + c0 + (lane % kLanes) * 4;
+#pragma unroll 4
+        for (int r = 0; r < 32 / KS; r += kRows) {
+            const int row = quarter * 32 + rank * (32 / KS) + r + lane / kLanes, m = m0 + row;
+            const float* at = sums + row * kRow + c0 + (lane % kLanes) * 4;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (m >= g.M || n >= g.N) continue;
+            if constexpr (KS > 1) {
+#pragma unroll
+                for (int z = 0; z < KS; ++z) {
+                    const float4 x = peer_load4(at, (uint32_t)z);
+                    v = make_float4(v.x + x.x, v.y + x.y, v.z + x.z, v.w + x.w);
+                }
+            } else {
+                v = *reinterpret_cast<const float4*>(at);
+            }
+            float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (n + e >= g.N) continue;
+                if (!isfinite(f[e])) f[e] = split_again(g.A + (size_t)m * g.K, g.W + (size_t)(n + e) * g.K, g.K);
+                if (g.bias) f[e] += g.bias[n + e];
+            }
+            float* out = g.C + (size_t)m * g.N + n;
+            if (by_four) {
+                float4 o = make_float4(f[0], f[1], f[2], f[3]);
+                if (g.add) {
+                    const float4 c = load4(out);
+                    o = make_float4(c.x + o.x, c.y + o.y, c.z + o.z, c.w + o.w);
+                }
+                store4(out, o);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (n + e < g.N) out[e] = g.add ? out[e] + f[e] : f[e];
+            }
+        }
+    }
+    tc_fence_before();
+    if constexpr (KS > 1) cluster_meet();  // no CTA leaves while another reads its sums
+    __syncthreads();
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, kTmemCols);
+    }
+    if (threadIdx.x == 0 && abort_flag && g.status) atomicExch(g.status, 3);
+}
+
+template <int BN, int KS>
+static int launch_split(const SplitArgs& g, cudaStream_t stream) {
+    auto kernel = gemm_split_kernel<BN, KS>;
+    constexpr size_t sums = (size_t)kSplitM * (BN + 4) * 4, stages = kSplitStages * (size_t)split_stage_bytes(BN);
+    constexpr size_t smem = (sums > stages ? sums : stages) + 1024;
+    static_assert(smem <= 227 * 1024 - 1024, "one CTA's shared memory");
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((g.N + BN - 1) / BN * KS), (unsigned)((g.M + kSplitM - 1) / kSplitM));
+    cfg.blockDim = dim3(kSplitThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int attrs = 0;
+    if (KS > 1) {
+        attr[attrs].id = cudaLaunchAttributeClusterDimension;
+        attr[attrs].val.clusterDim.x = KS;
+        attr[attrs].val.clusterDim.y = 1;
+        attr[attrs++].val.clusterDim.z = 1;
+    }
+    if (dependent_launches()) {
+        attr[attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[attrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = attrs;
+    e = cudaLaunchKernelEx(&cfg, kernel, g);
+    return e == cudaSuccess ? NNIS_OK : (int)e;
+}
+
+// Width of the tiles and CTAs that share a tile's K: the least cycles by waves of CTAs, a wave's cost as measured (start and
+// end 6,000 cycles, a cluster's meeting 1,500; a block of K 1,600 and 1,250 at widths 128 and 64 relative to those).  us at widths
+// x CTAs 64x1, 64x2, 64x4, 128x1, 128x2, 128x4: 1,024 x 576 x 1,536 45, 31, 49, 51, 34, 39; 1,024 x 3,072 x 576 57, 80, 125, 47,
+// 51, 78; 2,048 x 2,048 x 2,048 207, 215, 287, 125, 139, 170; 256 x 2,048 x 2,048 55, 37, 43, 66, 41, 29.
+static void split_shape(int M, int N, int K, int sms, int* bn, int* ks) {
+    const long m_tiles = (M + kSplitM - 1) / kSplitM;
+    const int blocks = (K + kSplitK - 1) / kSplitK;
+    long best = -1;
+    const int widths[2] = {128, 64}, splits[3] = {1, 2, 4};
+    for (int w : widths)
+        for (int s : splits) {
+            if (s > 1 && blocks < 2 * s) continue;
+            const long ctas = m_tiles * ((N + w - 1) / w) * s;
+            const long waves = (ctas + sms - 1) / sms;
+            const long cost = waves * (6000 + (s > 1 ? 1500 : 0) + (long)((blocks + s - 1) / s) * (w == 128 ? 1600 : 1250));
+            if (best < 0 || cost < best) {
+                best = cost;
+                *bn = w;
+                *ks = s;
+            }
+        }
+}
+
+}  // namespace nnis
+
+// Modes: 1 store, 2 add into C.  `shape` 0: by the rule; else (BN / 64) * 10 + KS.  Refuses (NNIS_ERR_UNSUPPORTED) K not a multiple of
+// 8; A and W start on 32-byte boundaries.
+NNIS_API int nnis_gemm_split_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
+                                 int mode, int shape, int sm_count, int* status, cudaStream_t stream) {
+    using namespace nnis;
+    if (M <= 0 || N <= 0 || K <= 0 || !A || !W || !C || mode < 1 || mode > 2) return NNIS_ERR_ARGUMENT;
+    if (K % 8 || (M + kSplitM - 1) / kSplitM > 65535) return NNIS_ERR_UNSUPPORTED;
+    if (((uintptr_t)A | (uintptr_t)W) % 32 || (uintptr_t)C % 4) return NNIS_ERR_ALIGNMENT;
+    SplitArgs g{A, W, bias, C, M, N, K, mode == 2, status};
+    int bn = 128, ks = 1;
+    split_shape(M, N, K, sm_count > 0 ? sm_count : 148, &bn, &ks);
+    if (shape) { bn = shape / 10 * 64; ks = shape % 10; }
+    if (bn == 128 && ks == 1) return launch_split<128, 1>(g, stream);
+    if (bn == 128 && ks == 2) return launch_split<128, 2>(g, stream);
+    if (bn == 128 && ks == 4) return launch_split<128, 4>(g, stream);
+    if (bn == 64 && ks == 1) return launch_split<64, 1>(g, stream);
+    if (bn == 64 && ks == 2) return launch_split<64, 2>(g, stream);
+    if (bn == 64 && ks == 4) return launch_split<64, 4>(g, stream);
+    return NNIS_ERR_ARGUMENT;
+}

@@ -192,6 +192,29 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
                                  mode, _stream()), "gemm_simt")
 
 
+def gemm_split_f32_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether this float32 product runs on the tensor cores (``gemm_split_f32``): rows that start on 32-byte
+    boundaries, and more of them than a decode step's kernel takes at once (17 rows x 576 x 576: 35 us on the
+    CUDA cores, 14 here; 16 rows read the weights once in 9)."""
+    return a.shape[0] > 16 and a.shape[1] % 8 == 0 and (a.data_ptr() | w.data_ptr()) % 32 == 0
+
+
+def gemm_split_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, mode: int,
+                   shape: int = 0) -> None:
+    """out (op)= a . w^T + bias for float32 operands on the tensor cores, every value as the exact sum of
+    three bfloat16 values.  ``shape``: 0 by the kernel's rule, or (tile columns / 64) * 10 + CTAs that share K."""
+    _cuda(a, w, bias, out)
+    m, k = a.shape
+    n = w.shape[0]
+    _need(w.shape[1] == k and a.dtype == w.dtype == out.dtype == torch.float32, "gemm: float32 a [m, k], w [n, k]")
+    _need(tuple(out.shape) == (m, n), "gemm: out [m, n]")
+    if bias is not None:
+        _need(bias.dtype == torch.float32 and bias.numel() == n, "gemm: bias float32 [n]")
+    _check(_lib().nnis_gemm_split_f32(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, 2 if mode == ADD_F32 else 1,
+                                      shape, sm_count(a.device), _ptr(status_word(a.device)), _stream()),
+           "gemm_split_f32")
+
+
 def attention_generic(q: torch.Tensor, q_stride: int, k_cache: torch.Tensor, v_cache: torch.Tensor,
                       token_pos: torch.Tensor, token_seq: torch.Tensor, page_table: torch.Tensor,
                       out: torch.Tensor, heads: int, kv_heads: int, head_dim: int, window: int,

@@ -1,7 +1,8 @@
 """y (op)= x . W^T + b: picks the kernel for a dtype and a shape.
 
-float32 operands always run on the CUDA cores (no tensor-core mode exists that
-keeps 32-bit products).  bfloat16 operands take the tcgen05 kernel where its
+float32 operands of more than a decode step's rows run on the tensor cores as exact
+sums of three bfloat16 values each, the others on the CUDA cores; both keep 32-bit
+products.  bfloat16 operands take the tcgen05 kernel where its
 tile rules hold and the row count makes it worthwhile, else the CUDA-core
 kernel.  NNIS makes the same kind of choice per projection family with its
 projection plans (crates/nnis-model/src/projection_plan.rs:10-90).
@@ -35,5 +36,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], 
                 scratch = workspace.get("gemm_split_sums", (floats,), torch.float32)
                 tickets = workspace.zeros("gemm_split_tickets", (tiles,), torch.int32)
         ops.gemm_tc(x, weight, bias, out, mode, split_scratch=scratch, split_tickets=tickets)
+    elif x.dtype == torch.float32 and ops.gemm_split_f32_takes(x, weight):
+        ops.gemm_split_f32(x, weight, bias, out, mode)
     else:
         ops.gemm_simt(x, weight, bias, out, mode)
