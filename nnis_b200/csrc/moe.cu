@@ -42,6 +42,17 @@
 
 namespace nnis {
 
+// eight products of bfloat16 pairs added to `acc`, in order
+__device__ __forceinline__ float row_dot8(const uint4& x, const uint4& y, float acc) {
+    const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        acc = fmaf(__uint_as_float(xs[k] << 16), __uint_as_float(ys[k] << 16), acc);
+        acc = fmaf(__uint_as_float(xs[k] & 0xffff0000u), __uint_as_float(ys[k] & 0xffff0000u), acc);
+    }
+    return acc;
+}
+
 // sum over a warp's share of two rows' product: 16-byte loads where the rows are bfloat16,
 // a multiple of eight long and 16-byte aligned, else element by element
 template <typename T>
@@ -51,13 +62,7 @@ __device__ __forceinline__ float warp_row_dot(const T* __restrict__ a, const T* 
         const uint4* a4 = reinterpret_cast<const uint4*>(a);
         const uint4* b4 = reinterpret_cast<const uint4*>(b);
         for (int i = lane; i < len / 8; i += 32) {
-            uint4 x = a4[i], y = b4[i];
-            const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                acc = fmaf(__uint_as_float(xs[k] << 16), __uint_as_float(ys[k] << 16), acc);
-                acc = fmaf(__uint_as_float(xs[k] & 0xffff0000u), __uint_as_float(ys[k] & 0xffff0000u), acc);
-            }
+            acc = row_dot8(a4[i], b4[i], acc);
         }
     } else {
         for (int i = lane; i < len; i += 32) acc = fmaf(to_float(a[i]), to_float(b[i]), acc);
@@ -65,48 +70,85 @@ __device__ __forceinline__ float warp_row_dot(const T* __restrict__ a, const T* 
     return warp_sum(acc);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256)
+// A CTA of `blockDim.x` / 32 warps takes TOK tokens.  With one token a warp takes an output at a time, and the launch brings
+// 32 warps, so that one SM asks L2 for a matrix of 32 rows at once (8 tokens, 32 experts, width 2,048: 9.9 -> 5.3 us).  With eight tokens a warp takes EXP rows of the matrix and all tokens, so a piece of a row is fetched once
+// for eight tokens and a piece of a token once for EXP rows (2,048 tokens of that layer: @R2@: every token's CTA
+// fetched the whole matrix, half a gigabyte from L2).  A logit is the same chain of multiply-adds either way.  Then warp k
+// chooses for token k.
+template <typename T, int TOK, int EXP>
+__global__ void __launch_bounds__(TOK == 1 ? 1024 : 256)
 moe_route_kernel(const T* __restrict__ h, const float* __restrict__ wr, const float* __restrict__ br,
                  const int* __restrict__ token_pos, int* __restrict__ ids,
                  float* __restrict__ weights, int n_tokens, int width, int experts, int top,
                  int sigmoid_scores) {
-    extern __shared__ float z[];  // [experts]
+    extern __shared__ float z_all[];  // [TOK][experts]
     pdl_wait();
     pdl_launch_dependents();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int n0 = blockIdx.x * TOK;
+    const bool by_four = (width & 3) == 0;  // rows of the router and of x start on 16- and 8-byte borders
+    const T* x[TOK];
+#pragma unroll
+    for (int k = 0; k < TOK; ++k) x[k] = h + (size_t)min(n0 + k, n_tokens - 1) * width;
+    for (int e0 = warp * EXP; e0 < experts; e0 += warps * EXP) {
+        const float* w[EXP];
+        float acc[EXP][TOK];
+#pragma unroll
+        for (int e = 0; e < EXP; ++e) {
+            w[e] = wr + (size_t)min(e0 + e, experts - 1) * width;
+#pragma unroll
+            for (int k = 0; k < TOK; ++k) acc[e][k] = 0.f;
+        }
+        auto columns = [&](int i) {
+            float4 wv[EXP];
+#pragma unroll
+            for (int e = 0; e < EXP; ++e) wv[e] = load4(w[e] + i);
+#pragma unroll
+            for (int k = 0; k < TOK; ++k) {
+                const float4 xv = load4(x[k] + i);
+#pragma unroll
+                for (int e = 0; e < EXP; ++e) {
+                    acc[e][k] = fmaf(wv[e].x, xv.x, acc[e][k]);
+                    acc[e][k] = fmaf(wv[e].y, xv.y, acc[e][k]);
+                    acc[e][k] = fmaf(wv[e].z, xv.z, acc[e][k]);
+                    acc[e][k] = fmaf(wv[e].w, xv.w, acc[e][k]);
+                }
+            }
+        };
+        if (by_four && TOK == 1) {  // several loads in flight per lane: the dot products are latency, not arithmetic
+#pragma unroll 8
+            for (int i = lane * 4; i < width; i += 128) columns(i);
+        } else if (by_four) {
+#pragma unroll 2
+            for (int i = lane * 4; i < width; i += 128) columns(i);
+        } else {
+            for (int i = lane; i < width; i += 32)
+#pragma unroll
+                for (int e = 0; e < EXP; ++e)
+#pragma unroll
+                    for (int k = 0; k < TOK; ++k) acc[e][k] = fmaf(w[e][i], to_float(x[k][i]), acc[e][k]);
+        }
+#pragma unroll
+        for (int e = 0; e < EXP; ++e)
+#pragma unroll
+            for (int k = 0; k < TOK; ++k) {
+                const float sum = warp_sum(acc[e][k]);
+                if (lane == 0 && e0 + e < experts) z_all[k * experts + e0 + e] = sum + (br ? br[e0 + e] : 0.f);
+            }
+    }
+    __syncthreads();
+    const int n = n0 + warp;
+    if (warp >= TOK || n >= n_tokens) return;
+    float* z = z_all + warp * experts;
     int* id = ids + (size_t)n * top;
     float* wt = weights + (size_t)n * top;
     if (token_pos[n] < 0) {
-        for (int s = threadIdx.x; s < top; s += 256) {
+        for (int s = lane; s < top; s += 32) {
             id[s] = 0;
             wt[s] = 0.f;
         }
         return;
     }
-    const T* x = h + (size_t)n * width;
-    const bool by_four = (width & 3) == 0;  // rows of the router and of x start on 16- and 8-byte borders
-    for (int e = warp; e < experts; e += 8) {  // a warp per expert, eight at a time
-        const float* w = wr + (size_t)e * width;
-        float acc = 0.f;
-        if (by_four) {  // several loads in flight per lane: the dot products are latency, not arithmetic
-#pragma unroll 4
-            for (int i = lane * 4; i < width; i += 128) {
-                float4 wv = load4(w + i), xv = load4(x + i);
-                acc = fmaf(wv.x, xv.x, acc);
-                acc = fmaf(wv.y, xv.y, acc);
-                acc = fmaf(wv.z, xv.z, acc);
-                acc = fmaf(wv.w, xv.w, acc);
-            }
-        } else {
-            for (int i = lane; i < width; i += 32) acc = fmaf(w[i], to_float(x[i]), acc);
-        }
-        acc = warp_sum(acc);
-        if (lane == 0) z[e] = acc + (br ? br[e] : 0.f);
-    }
-    __syncthreads();
-    if (warp != 0) return;
     // the `top` largest, one after another; the lanes of one warp share the search
     float first = 0.f, total = 0.f;
     for (int s = 0; s < top; ++s) {
@@ -127,6 +169,10 @@ moe_route_kernel(const T* __restrict__ h, const float* __restrict__ wr, const fl
                 best = ob;
                 arg = oa;
             }
+        }
+        if (arg >= experts) {  // (no logit left that is a number: nothing to choose by, and the token's output shows it)
+            arg = s;
+            best = NAN;
         }
         if (s == 0) first = best;
         float p = sigmoid_scores ? 1.0f / (1.0f + expf(-best)) : expf(best - first);
@@ -417,18 +463,25 @@ NNIS_API int nnis_moe_route(const void* h, const float* wr, const float* br, con
     if (n_tokens <= 0 || width <= 0 || experts <= 0 || top <= 0 || top > experts || !h || !wr || !ids ||
         !weights || !token_pos)
         return NNIS_ERR_ARGUMENT;
-    size_t smem = (size_t)experts * sizeof(float);
-    if (smem > 48 * 1024) return NNIS_ERR_UNSUPPORTED;
-    unsigned blocks = (unsigned)n_tokens;
+    const size_t per = (size_t)experts * sizeof(float);
+    if (per > 48 * 1024) return NNIS_ERR_UNSUPPORTED;
+    // eight tokens a CTA take about 12 us whatever their number up to two CTAs an SM, single ones 15 at 512 tokens and
+    // 10 at 300 (32 experts, width 2,048; 64 experts, width 1,536: 17 against 22 and 16)
+    const bool several = n_tokens >= 512 && 8 * per <= 48 * 1024;
+    const unsigned blocks = several ? (unsigned)((n_tokens + 7) / 8) : (unsigned)n_tokens;
+    const unsigned threads = several || n_tokens > 2 * 148 ? 256 : 32 * (unsigned)(experts < 32 ? (experts < 8 ? 8 : experts) : 32);
+    const size_t smem = several ? 8 * per : per;
     cudaError_t e;
+#define NNIS_ROUTE(T, TOK, EXP) \
+    launch_dependent(moe_route_kernel<T, TOK, EXP>, blocks, threads, smem, stream, (const T*)h, wr, br, token_pos, \
+                     ids, weights, n_tokens, width, experts, top, sigmoid_scores)
     if (dtype == NNIS_DTYPE_F32)
-        e = launch_dependent(moe_route_kernel<float>, blocks, 256, smem, stream, (const float*)h, wr, br, token_pos,
-                             ids, weights, n_tokens, width, experts, top, sigmoid_scores);
+        e = several ? NNIS_ROUTE(float, 8, 4) : NNIS_ROUTE(float, 1, 1);
     else if (dtype == NNIS_DTYPE_BF16)
-        e = launch_dependent(moe_route_kernel<bf16>, blocks, 256, smem, stream, (const bf16*)h, wr, br, token_pos,
-                             ids, weights, n_tokens, width, experts, top, sigmoid_scores);
+        e = several ? NNIS_ROUTE(bf16, 8, 4) : NNIS_ROUTE(bf16, 1, 1);
     else
         return NNIS_ERR_UNSUPPORTED;
+#undef NNIS_ROUTE
     return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 
