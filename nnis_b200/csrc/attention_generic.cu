@@ -141,10 +141,9 @@ static int launch_attention(const void* q, int q_stride, const void* k_cache, co
     if (e != cudaSuccess) return (int)e;
     if (n_splits > 1) {
         size_t rows = (size_t)n_tokens * nq;
-        attn_merge_kernel<T><<<(unsigned)rows, 128, 0, stream>>>(partial, (T*)out, rows,
-                                                                             d, n_splits, nullptr);
+        e = launch_merge<T>(partial, (T*)out, rows, d, n_splits, nullptr, stream);
     }
-    NNIS_RETURN_LAUNCH();
+    return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 
 }  // namespace nnis
@@ -153,9 +152,9 @@ static int launch_attention(const void* q, int q_stride, const void* k_cache, co
 extern "C" int nnis_attention_merge_bf16(const float* partial, void* out, long long n_rows, int d,
                                          int n_splits, cudaStream_t stream) {
     if (n_splits > 64) return NNIS_ERR_UNSUPPORTED;
-    nnis::attn_merge_kernel<nnis::bf16><<<(unsigned)n_rows, 128, 0, stream>>>(
-        partial, (nnis::bf16*)out, (size_t)n_rows, d, n_splits, nullptr);
-    NNIS_RETURN_LAUNCH();
+    const cudaError_t e =
+        nnis::launch_merge<nnis::bf16>(partial, (nnis::bf16*)out, (size_t)n_rows, d, n_splits, nullptr, stream);
+    return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 
 // Scratch: `partial` needs n_tokens * nq * n_splits * (d + 2) floats when

@@ -340,10 +340,9 @@ static int launch_latent(const void* q, const void* cache, const int* token_pos,
     if (e != cudaSuccess) return (int)e;
     if (n_splits > 1) {
         size_t rows = (size_t)n_tokens * heads;
-        attn_merge_kernel<T><<<(unsigned)rows, 128, 0, stream>>>(partial, (T*)out, rows, dv,
-                                                                             n_splits, gate);
+        e = launch_merge<T>(partial, (T*)out, rows, dv, n_splits, gate, stream);
     }
-    NNIS_RETURN_LAUNCH();
+    return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 
 }  // namespace nnis

@@ -354,8 +354,7 @@ NNIS_API int nnis_attention_latent_mma(const void* q, const void* cache, const i
     if (e != cudaSuccess) return (int)e;
     if (n_splits > 1) {
         size_t rows = (size_t)n_tokens * heads;
-        e = launch_dependent(attn_merge_kernel<bf16>, (unsigned)rows, 128, 0, stream, (const float*)partial,
-                             (bf16*)out, rows, dv, n_splits, gate);
+        e = launch_merge<bf16>(partial, (bf16*)out, rows, dv, n_splits, gate, stream);
     }
     return e == cudaSuccess ? NNIS_OK : (int)e;
 }

@@ -226,6 +226,6 @@ NNIS_API int nnis_attention_tile_f32(const void* q, int q_stride, const void* k_
         seq_start, seq_count, page_table, table_cols, (float*)out, partial, nq, nkv, d, window, scale, n_splits, stream);
     if (rc != NNIS_OK || n_splits == 1) return rc;
     const size_t rows = (size_t)n_tokens * nq;
-    attn_merge_kernel<float><<<(unsigned)rows, 128, 0, stream>>>(partial, (float*)out, rows, d, n_splits, nullptr);
-    NNIS_RETURN_LAUNCH();
+    const cudaError_t e = launch_merge<float>(partial, (float*)out, rows, d, n_splits, nullptr, stream);
+    return e == cudaSuccess ? NNIS_OK : (int)e;
 }

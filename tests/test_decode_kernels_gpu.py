@@ -42,3 +42,34 @@ def test_router_of_few_and_of_many_tokens(n, width, experts, top, sigmoid):
                 assert ids[t].tolist().index(0) < ids[t].tolist().index(experts - 1)
             share = torch.sigmoid(got) if sigmoid else torch.softmax(got, 0)
             assert torch.allclose(weights[t], share, atol=1e-4)
+
+
+@pytest.mark.parametrize("dim,rot,heads", [(16, 4, 3), (48, 16, 2), (144, 8, 5), (504, 8, 2)])
+@pytest.mark.parametrize("splits", [2, 8, 9, 64])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_merge_of_slices(dim, rot, heads, splits, dtype):
+    """Attention in slices against the same in one: rows of one warp and of a CTA, slices that hold no key, rows that are
+    no multiple of four."""
+    o = ops()
+    dt = getattr(torch, dtype)
+    g = torch.Generator().manual_seed(dim + splits)
+    lengths = [1, 64, 65, 300]
+    n, row = len(lengths), dim + rot
+    cache = torch.randn(16, 1, 64, row, generator=g).to(dt).to(DEV)
+    table = torch.full((n, 5), -1, dtype=torch.int32)
+    table.view(-1)[[0, 5, 10, 11, 15, 16, 17, 18, 19]] = torch.arange(9, dtype=torch.int32) + 2
+    q = torch.randn(n, heads * row, generator=g).to(dt).to(DEV)
+    pos = torch.tensor([length - 1 for length in lengths], dtype=torch.int32, device=DEV)
+    seq, table = torch.arange(n, dtype=torch.int32, device=DEV), table.to(DEV)
+    whole, cut = (torch.full((n, heads * dim), 9.0, dtype=dt, device=DEV) for _ in range(2))
+    o.attention_latent(q, cache, pos, seq, table, whole, heads, dim, 0.2, 1, None)
+    partial = torch.full((n * heads * splits * (dim + 2),), math.nan, device=DEV)
+    o.attention_latent(q, cache, pos, seq, table, cut, heads, dim, 0.2, splits, partial)
+    # float32: sums in another order; bfloat16: one rounding of the output
+    assert torch.allclose(whole.float(), cut.float(), atol=2e-6 if dtype == "float32" else 2e-2)
+    if dtype == "float32":
+        for t, length in enumerate(lengths):
+            rows = torch.cat([cache[int(p), 0] for p in table[t].cpu() if p >= 0])[:length].double()
+            for h in range(heads):
+                s = torch.softmax(rows @ q[t, h * row:(h + 1) * row].double() * 0.2, 0)
+                assert torch.allclose(cut[t, h * dim:(h + 1) * dim].double(), s @ rows[:, :dim], atol=1e-5)
