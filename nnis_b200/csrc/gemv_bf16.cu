@@ -14,6 +14,8 @@ int gemv_launch_tiles4(const GemvArgs&, int, int, const GemvPlan&, bool, cudaStr
 // gemv_rowtile.cu: the kernel for more rows than one tile and few output features
 int gemv_rowtile_units(int M, int N, int K, int epilogue, int pro, int sm_count);
 int gemv_launch_rowtile(const GemvArgs&, int, int, int, bool, cudaStream_t);
+int gemv_rowtile_parts(int M, int N, int K, int sm_count, int* columns, int* units);
+int gemv_launch_rowtile_parts(const GemvArgs&, int, bool, cudaStream_t);
 
 // Shared memory of one CTA: x, the weight stages (eight rows of `kc` columns each),
 // the barriers, and with split K the warps' partial sums.
@@ -116,7 +118,28 @@ static int rowtile_slices(int M, int N, int K, int epilogue, int pro, int sm_cou
     return 0;
 }
 
+// Parts of K of the adding product where they run as one launch whose CTAs share a tile's K (0: not so), for products
+// that would else take several launches; the columns of a part and the units of a CTA.
+static int shared_parts(int M, int N, int K, int sm_count, int* columns, int* units) {
+    int unused;
+    GemvPlan p;
+    const int rows = rowtile_slices(M, N, K, EPI_ADD_F32, PRO_PLAIN, sm_count, &unused);
+    if ((rows > 0 ? rows : gemv_slices(M, N, K, sm_count, &p)) < 2) return 0;
+    return gemv_rowtile_parts(M, N, K, sm_count, columns, units);
+}
+
 }  // namespace nnis
+
+// Scratch of the adding product with a plain prologue for the launch whose CTAs share a tile's K: `*floats` float32 and
+// `*tiles` tickets (zero before the first launch; the kernel leaves them zero); 0 and the return value 0 where it takes none.
+NNIS_API int nnis_gemv_parts(int M, int N, int K, int sm_count, long long* floats, int* tiles) {
+    int columns = 0, units = 1;
+    const int parts = nnis::shared_parts(M, N, K, sm_count, &columns, &units);
+    const long groups = parts ? (long)((M + 15) / 16) * ((N / 8 + units - 1) / units) : 0;
+    if (floats) *floats = (long long)groups * units * parts * 128;
+    if (tiles) *tiles = (int)groups;
+    return parts;
+}
 
 // Whether nnis_gemv_bf16 takes a shape (1) or the caller must use the general
 // kernels (0): at most 64 rows, K a multiple of 16, N a multiple of 8, and x plus
@@ -180,6 +203,8 @@ NNIS_API int nnis_gemv_grid(int M, int N, int K, int sm_count) {
 // `emit_w` [N] in bfloat16 [M, N], and per row and eight columns the sum of the output's
 // squares [M, N / 8], for a product that follows with `ss_parts` [M, K / 8]: x is then such
 // an `emit_x`, and `eps` the norm's (the kernel over tiles of rows only).
+// `split_sums` (`split_floats` float32) and `split_tickets` (`split_tiles` counters), optional, of at least the sizes that
+// nnis_gemv_parts gives: the adding product of a long K then runs as one launch where it says so.
 // `act` (STORE, optional): 1 stores the square of relu of the sums, 2 gelu (erf), 3 gelu's tanh form; with
 // GATED the same functions of the gate's sums in place of silu.
 NNIS_API int nnis_gemv_bf16(const void* x, const float* hidden, const int* rows, const float* norm_w,
@@ -189,8 +214,9 @@ NNIS_API int nnis_gemv_bf16(const void* x, const float* hidden, const int* rows,
                             const float* sin_t, void* k_cache, void* v_cache, int nq, int nkv, int d,
                             int page_size, float* logits, float* best_val, int* best_idx,
                             unsigned* ticket, int* next_tokens, int* next_pos, void* emit_x,
-                            const float* emit_w, float* emit_ss, const float* ss_parts, int act, int* status,
-                            int sm_count, int pdl, cudaStream_t stream) {
+                            const float* emit_w, float* emit_ss, const float* ss_parts, int act,
+                            float* split_sums, long long split_floats, unsigned* split_tickets, int split_tiles,
+                            int* status, int sm_count, int pdl, cudaStream_t stream) {
     using namespace nnis;
     if (M <= 0 || N <= 0 || K <= 0 || !w || !out) return NNIS_ERR_ARGUMENT;
     if (act && ((epilogue != EPI_STORE && epilogue != EPI_GATED) || act < 1 || act > 3)) return NNIS_ERR_ARGUMENT;
@@ -233,6 +259,20 @@ NNIS_API int nnis_gemv_bf16(const void* x, const float* hidden, const int* rows,
     a.ss_parts = ss_parts; a.ss_units = K / 8; a.act = act;
     a.ldx = K; a.ldw = K; a.kc = plan.kc; a.out_is_hot = 0;
     a.release_early = (pdl & 2) && slices == 1 ? 1 : 0;
+    a.k_parts = 1; a.split_sums = nullptr; a.split_tickets = nullptr;
+    a.K = K;
+    if (may_slice && slices > 1 && split_sums && split_tickets && !(pdl & 4)) {
+        long long floats;
+        int tiles, units;
+        if ((a.k_parts = nnis_gemv_parts(M, N, K, sm_count, &floats, &tiles)) > 1 && floats <= split_floats &&
+            tiles <= split_tiles) {
+            shared_parts(M, N, K, sm_count, &a.kc, &units);
+            a.split_sums = split_sums; a.split_tickets = split_tickets; a.emit_x = (bf16*)emit_x;
+            a.trace = trace_slot("gemv rows add_f32 parts");
+            return gemv_launch_rowtile_parts(a, units, (pdl & 1) != 0, stream);
+        }
+        a.k_parts = 1;
+    }
     a.K = K / slices;
     static const char* const kNames[] = {"gemv store", "gemv store_f32", "gemv add_f32", "gemv gated",
                                          "gemv qkv", "gemv argmax"};

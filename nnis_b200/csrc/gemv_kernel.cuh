@@ -56,6 +56,11 @@ struct GemvArgs {
     int M, N, K;
     int ldx, ldw;           // elements between rows of x and of w (K unless a slice of K is taken)
     int kc;                 // columns of K per weight stage (K: a stage holds whole rows)
+    // ADD_F32 in gemv_rowtile.cu: `k_parts` > 1 CTAs share a tile's K, `kc` columns each (K is all of it); their sums go
+    // to `split_sums` and the CTA that takes a tile's last ticket adds them and runs the epilogue
+    int k_parts;
+    float* split_sums;
+    unsigned* split_tickets;
     int out_is_hot;         // ADD_F32: the kernel just before this one wrote `out` (a slice of K)
     int release_early;      // the kernel after this one may start at once (see below)
     int* status;            // set non-zero when a bounded wait runs out

@@ -40,6 +40,7 @@
 namespace nnis {
 
 constexpr int kRowtileWarps = 8;
+constexpr int kRowtileMaxParts = 8;
 // 16-column steps of one warp of x in registers: K <= 768, or K <= 1,536 (LONGK)
 __host__ __device__ constexpr int rowtile_direct_steps(bool longk) { return longk ? 12 : 6; }
 
@@ -64,7 +65,10 @@ __host__ __device__ constexpr int rowtile_w_stride(int K, int pro) {
     return pro == PRO_NORM ? K + 8 : K + ((16 - K % 64) + 64) % 64;
 }
 
-template <int EPI, int PRO, int NU, bool LONGK>
+// PARTS (the adding epilogue, x as it is): K is cut among the CTAs (bx, by, 0 .. k_parts - 1), so that all of a long K's
+// weights are asked for before the wait, by one launch.  Each CTA leaves its units' sums in scratch and takes a ticket; the
+// last one adds the parts in their order (the same bits every time) and runs the epilogue.
+template <int EPI, int PRO, int NU, bool LONGK, bool PARTS = false>
 __global__ void __maxnreg__(rowtile_registers(EPI, PRO, LONGK))
 gemv_rowtile_kernel(GemvArgs a) {
     constexpr int WARPS = kRowtileWarps;
@@ -77,7 +81,9 @@ gemv_rowtile_kernel(GemvArgs a) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     trace_mark(a.trace, 0);
     if (a.release_early) pdl_launch_dependents();
-    const int K = a.K, KP = K + 8, KPW = rowtile_w_stride(K, PRO);
+    const int k_first = PARTS ? (int)blockIdx.z * a.kc : 0;
+    const int K = PARTS ? min(a.kc, a.K - k_first) : a.K;  // columns of this CTA
+    const int KP = K + 8, KPW = rowtile_w_stride(PARTS ? a.kc : K, PRO);
     const int row0 = blockIdx.y * 16;
     const int n_units = a.N >> 3;
     const int unit0 = blockIdx.x * NU;
@@ -104,7 +110,7 @@ gemv_rowtile_kernel(GemvArgs a) {
         }
         __syncwarp();
         for (int r = lane; r < units_here * 8; r += 32)
-            bulk_load(ws + (size_t)r * KPW, a.w + (size_t)unit_row<EPI>(a, unit0 + (r >> 3), r & 7) * a.ldw,
+            bulk_load(ws + (size_t)r * KPW, a.w + (size_t)unit_row<EPI>(a, unit0 + (r >> 3), r & 7) * a.ldw + k_first,
                       (uint32_t)K * 2u, &wbar);
     }
     // ... the norm weights and what the epilogue needs.  This preamble has to fit under
@@ -154,7 +160,7 @@ gemv_rowtile_kernel(GemvArgs a) {
     if (kDirect) {
         // lane (g, t): rows g and g + 8, columns 4 t .. 4 t + 3 of each step of 16
         const int g = lane >> 2, t4 = (lane & 3) * 4;
-        const bf16* x0 = a.x + (size_t)(row0 + g) * a.ldx + k_begin + t4;
+        const bf16* x0 = a.x + (size_t)(row0 + g) * a.ldx + k_first + k_begin + t4;
         const bf16* x1 = x0 + (size_t)8 * a.ldx;
         const bool in_a = row0 + g < a.M, in_b = row0 + g + 8 < a.M;
 #pragma unroll
@@ -278,10 +284,15 @@ gemv_rowtile_kernel(GemvArgs a) {
     // (a wait that runs out is flagged; the CTA goes on through its barriers)
     const bool arrived = mbar_wait(&wbar, 0);
     float acc[NU][4];
+    // (PARTS: two chains of products, half as long each: the tensor cores cut their running sums off)
+    float acc_odd[PARTS ? NU : 1][4];
 #pragma unroll
     for (int u = 0; u < NU; ++u)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[u][e] = 0.f;
+        for (int e = 0; e < 4; ++e) {
+            acc[u][e] = 0.f;
+            if (PARTS) acc_odd[u][e] = 0.f;
+        }
     if (kDirect) {
         // the weights in the order of x: lane (g, t) takes columns 4 t .. 4 t + 3 of row g
         const bf16* b_ptr = ws + (size_t)(lane >> 2) * KPW + (lane & 3) * 4;
@@ -294,8 +305,14 @@ gemv_rowtile_kernel(GemvArgs a) {
                 for (int u = 0; u < NU; ++u)
                     bw[u] = *reinterpret_cast<const uint2*>(b_ptr + (size_t)u * 8 * KPW + k0);
 #pragma unroll
-                for (int u = 0; u < NU; ++u) mma_bf16(acc[u], ax[s], bw[u].x, bw[u].y);
+                for (int u = 0; u < NU; ++u) mma_bf16(PARTS && (s & 1) ? acc_odd[PARTS ? u : 0] : acc[u], ax[s], bw[u].x, bw[u].y);
             }
+        }
+        if constexpr (PARTS) {
+#pragma unroll
+            for (int u = 0; u < NU; ++u)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[u][e] += acc_odd[u][e];
         }
     } else {
         // lanes 0-7: weight rows at columns k0..k0+7, lanes 8-15: k0+8..k0+15
@@ -322,14 +339,50 @@ gemv_rowtile_kernel(GemvArgs a) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) red[((size_t)(warp * NU + u) * 4 + e) * 32 + lane] = acc[u][e];
     __syncthreads();
+    float sum[4];
     if (epi_warp) {
-        float sum[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             float v = red[((size_t)warp * 4 + e) * 32 + lane];
             for (int w = 1; w < WARPS; ++w) v += red[((size_t)(w * NU + warp) * 4 + e) * 32 + lane];
             sum[e] = v;
         }
+    }
+    bool finishes = epi_warp;
+    if constexpr (PARTS) {
+        __shared__ int last;
+        const unsigned tile = blockIdx.y * gridDim.x + blockIdx.x;
+        float* place = a.split_sums + ((size_t)tile * NU + warp) * a.k_parts * 128 + lane;
+        if (epi_warp) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) __stcg(place + (size_t)blockIdx.z * 128 + e * 32, sum[e]);
+        }
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned old;
+            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;"
+                         : "=r"(old) : "l"(a.split_tickets + tile) : "memory");
+            last = old == (unsigned)a.k_parts - 1u;
+            if (last) a.split_tickets[tile] = 0u;  // (every part has arrived)
+        }
+        __syncthreads();
+        finishes = epi_warp && last;
+        if (finishes) {
+            float part[kRowtileMaxParts][4];  // all asked for at once: one trip to L2
+#pragma unroll
+            for (int z = 0; z < kRowtileMaxParts; ++z)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) part[z][e] = z < a.k_parts ? __ldcg(place + z * 128 + e * 32) : 0.f;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                sum[e] = part[0][e];
+#pragma unroll
+                for (int z = 1; z < kRowtileMaxParts; ++z) sum[e] += part[z][e];
+            }
+        }
+    }
+    if (finishes) {
         if (kScaled) {  // (written before the two barriers above)
             const float s_lo = row_scale[lane >> 2], s_hi = row_scale[(lane >> 2) + 8];
             sum[0] *= s_lo;
@@ -385,16 +438,43 @@ int gemv_rowtile_units(int M, int N, int K, int epilogue, int pro, int sm_count)
     return 0;
 }
 
-template <int EPI, int PRO, int NU, bool LONGK>
+// How a long K of the adding product is cut: into how many parts (0: not cut here) of how many columns, and units per CTA.
+// The fewest parts that the registers of a warp's x allow, and as few units as leave the CTAs resident together (four where
+// none do: the CTAs that wait for room start with their weights' copies even so).  Against a launch per slice, M x N x K in us
+// one after another in a graph, slices -> one launch: 8 x 2,048 x 5,632 17.6 -> 6.4, 1 x 2,048 x 5,632 11.4 -> 5.5, 8 x 2,048 x
+// 8,192 16.2 -> 10.7, 32 x 2,048 x 5,632 37 -> 13.4, 64 x 2,048 x 8,192 90 -> 36, 8 x 1,536 x 4,224 8.2 -> 5.4, 8 x 2,048 x 2,048
+// 5.5 -> 4.8, 8 x 1,024 x 2,816 4.8 -> 4.4.
+int gemv_rowtile_parts(int M, int N, int K, int sm_count, int* columns, int* units) {
+    if (M <= 0 || M > 128 || K <= 0 || K % 16 || N <= 0 || N % 8) return 0;
+    const int sms = sm_count > 0 ? sm_count : 148, steps = K / 16, mtiles = (M + 15) / 16;
+    const int most = rowtile_direct_steps(true) * kRowtileWarps;  // steps of a CTA
+    const int parts = (steps + most - 1) / most;
+    if (parts < 2 || parts > kRowtileMaxParts) return 0;
+    const int kc = (steps + parts - 1) / parts * 16;
+    for (int nu = mtiles >= 2 ? 4 : N / 8 >= 64 ? 2 : 1; nu <= 4; nu *= 2) {
+        const size_t smem = rowtile_smem(M, nu, kc, PRO_PLAIN);
+        int fit = (int)((220 * 1024) / (smem + 1024));
+        const bool longk = kc > rowtile_direct_steps(false) * 16 * kRowtileWarps;
+        if (fit > rowtile_ctas_per_sm(EPI_ADD_F32, PRO_PLAIN, longk)) fit = rowtile_ctas_per_sm(EPI_ADD_F32, PRO_PLAIN, longk);
+        const long ctas = (long)mtiles * ((N / 8 + nu - 1) / nu) * ((K + kc - 1) / kc);
+        if (smem > 200 * 1024 || (nu < 4 && ctas > (long)sms * fit)) continue;
+        *columns = kc;
+        *units = nu;
+        return (K + kc - 1) / kc;
+    }
+    return 0;
+}
+
+template <int EPI, int PRO, int NU, bool LONGK, bool PARTS = false>
 static int launch_rowtile_final(const GemvArgs& a, bool pdl, cudaStream_t stream) {
-    auto kernel = gemv_rowtile_kernel<EPI, PRO, NU, LONGK>;
-    const size_t smem = rowtile_smem(a.M, NU, a.K, PRO);
+    auto kernel = gemv_rowtile_kernel<EPI, PRO, NU, LONGK, PARTS>;
+    const size_t smem = rowtile_smem(a.M, NU, PARTS ? a.kc : a.K, PRO);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(((a.N >> 3) + NU - 1) / NU, (a.M + 15) / 16);
+    cfg.gridDim = dim3(((a.N >> 3) + NU - 1) / NU, (a.M + 15) / 16, PARTS ? a.k_parts : 1);
     cfg.blockDim = dim3(kRowtileWarps * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -420,6 +500,19 @@ static int launch_rowtile_units(const GemvArgs& a, int nu, bool pdl, cudaStream_
         if (nu == 2) return launch_rowtile_final<EPI, PRO, 2, false>(a, pdl, stream);
         if (nu == 4) return launch_rowtile_final<EPI, PRO, 4, false>(a, pdl, stream);
     }
+    return NNIS_ERR_UNSUPPORTED;
+}
+
+// `a.k_parts`, `a.kc` and `nu` from gemv_rowtile_parts for the same sizes.
+int gemv_launch_rowtile_parts(const GemvArgs& a, int nu, bool pdl, cudaStream_t stream) {
+    const bool longk = a.kc > rowtile_direct_steps(false) * 16 * kRowtileWarps;
+#define NNIS_PARTS(NU) \
+    return longk ? launch_rowtile_final<EPI_ADD_F32, PRO_PLAIN, NU, true, true>(a, pdl, stream) \
+                 : launch_rowtile_final<EPI_ADD_F32, PRO_PLAIN, NU, false, true>(a, pdl, stream)
+    if (nu == 1) NNIS_PARTS(1);
+    if (nu == 2) NNIS_PARTS(2);
+    if (nu == 4) NNIS_PARTS(4);
+#undef NNIS_PARTS
     return NNIS_ERR_UNSUPPORTED;
 }
 

@@ -8,6 +8,7 @@ here computes; without the compiled library nothing works, on purpose.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional
 
@@ -367,6 +368,27 @@ def gemv_slices(m: int, n: int, k: int, device=None, rows_kernel: bool = True) -
     return int(_lib().nnis_gemv_slices(m, n, k, sms))
 
 
+@functools.lru_cache(maxsize=4096)
+def _gemv_parts(m: int, n: int, k: int, sms: int):
+    floats, tiles = ctypes.c_longlong(0), ctypes.c_int(0)
+    _lib().nnis_gemv_parts(m, n, k, sms, ctypes.byref(floats), ctypes.byref(tiles))
+    return floats.value, tiles.value
+
+
+def gemv_split_scratch(m: int, n: int, k: int, device=None):
+    """Float32 values and tickets for an ADD_F32 product of these sizes as one launch whose CTAs share K; zeros where
+    it takes one launch anyway, or slices."""
+    return _gemv_parts(m, n, k, sm_count(device) if device is not None else 148)
+
+
+def gemv_split(m: int, n: int, k: int, workspace) -> Optional[tuple]:
+    """``gemv_bf16``'s ``split`` for an ADD_F32 product of these sizes, from a step's workspace; None where it needs none."""
+    floats, tiles = gemv_split_scratch(m, n, k, workspace.device)
+    if not floats:
+        return None
+    return workspace.get("gemv_split_sums", (floats,), torch.float32), workspace.zeros("gemv_split_tickets", (tiles,), torch.int32)
+
+
 def gemv_bf16(w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, epilogue: int,
               x: Optional[torch.Tensor] = None, hidden: Optional[torch.Tensor] = None,
               norm_weight: Optional[torch.Tensor] = None, eps: float = 0.0,
@@ -379,7 +401,7 @@ def gemv_bf16(w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, 
               scratch: Optional[torch.Tensor] = None, next_tokens: Optional[torch.Tensor] = None,
               next_pos: Optional[torch.Tensor] = None, release_early: bool = False,
               rows_kernel: bool = True, emit: Optional[tuple] = None,
-              shares: Optional[torch.Tensor] = None, act: int = 0) -> None:
+              shares: Optional[torch.Tensor] = None, act: int = 0, split: Optional[tuple] = None) -> None:
     """A decode-step projection with its prologue and epilogue fused (at most 64
     rows).  The input is ``x`` (bfloat16 [m, k]) or ``hidden`` (float32 residual
     rows, normed with ``norm_weight``/``eps`` on the way in; ``rows`` picks them).
@@ -397,9 +419,10 @@ def gemv_bf16(w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, 
     columns' sum of squares to ``shares`` (float32 [m, n / 8]).  The projection after it
     takes ``x=x_next, shares=shares, eps=`` the norm's, and scales its sums by
     ``1 / sqrt(mean of squares + eps)`` (``gemv_shares_norm`` says whether it can).
-    ``act``: an activation of the sums (EPI_STORE) or of the gate's sums in silu's place (EPI_GATED)."""
+    ``act``: an activation of the sums (EPI_STORE) or of the gate's sums in silu's place (EPI_GATED).
+    ``split`` (EPI_ADD_F32): ``gemv_split``'s buffers, with which a long K runs as one launch."""
     _cuda(w, bias, out, x, hidden, norm_weight, rows, token_pos, token_seq, page_table, cos, sin,
-          k_cache, v_cache, logits, scratch, next_tokens, next_pos, shares, *(emit or ()))
+          k_cache, v_cache, logits, scratch, next_tokens, next_pos, shares, *(emit or ()), *(split or ()))
     n, k = w.shape
     _need(w.dtype == torch.bfloat16, "gemv: bfloat16 weights")
     if hidden is not None:
@@ -466,6 +489,10 @@ def gemv_bf16(w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, 
                   and next_tokens.numel() >= m and next_pos.numel() >= m, "gemv: decode state int32")
     else:
         raise KernelError(f"gemv: unknown epilogue {epilogue}")
+    sums, tickets = split or (None, None)
+    if split is not None:
+        _need(epilogue == EPI_ADD_F32 and sums.dtype == torch.float32 and tickets.dtype == torch.int32,
+              "gemv: split (float32 sums, int32 tickets) goes with the adding epilogue")
     cols = page_table.shape[1] if page_table is not None else 0
     best_val = best_idx = ticket = 0
     if epilogue == EPI_ARGMAX:
@@ -477,11 +504,12 @@ def gemv_bf16(w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, 
         _ptr(page_table), cols, _ptr(cos), _ptr(sin), _ptr(k_cache), _ptr(v_cache), heads, kv_heads,
         head_dim, page_size, _ptr(logits), ctypes.c_void_p(best_val), ctypes.c_void_p(best_idx),
         ctypes.c_void_p(ticket), _ptr(next_tokens), _ptr(next_pos), _ptr(emit_x), _ptr(emit_w),
-        _ptr(emit_ss), _ptr(shares), act, _ptr(status_word(w.device)),
-        sm_count(w.device),
+        _ptr(emit_ss), _ptr(shares), act, _ptr(sums), ctypes.c_longlong(sums.numel() if sums is not None else 0),
+        _ptr(tickets), tickets.numel() if tickets is not None else 0, _ptr(status_word(w.device)), sm_count(w.device),
         PDL | (2 if release_early and PDL and EARLY_RELEASE else 0) | (0 if rows_kernel else 4), _stream()),
         "gemv_bf16",
-        gemv_slices(m, n, k, w.device, rows_kernel) if epilogue == EPI_ADD_F32 and hidden is None else 1)
+        1 if split is not None or epilogue != EPI_ADD_F32 or hidden is not None
+        else gemv_slices(m, n, k, w.device, rows_kernel))
 
 
 def argmax_scratch_ints(m: int, n: int, k: int, device) -> int:

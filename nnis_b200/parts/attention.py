@@ -310,8 +310,8 @@ class Attention(Part):
             ops.attention_generic(q_buf, q_stride, cache.k, cache.v, ctx.token_pos, ctx.token_seq,
                                   table, attn, nq, nkv, d, self.window, self.scale, splits, partial)
         if self._fused_out(ctx, n):
-            ops.gemv_bf16(self.w_o, self.b_o, residual, ops.EPI_ADD_F32, x=attn,
-                          emit=begin_norm(ctx, n, self.hidden))
+            ops.gemv_bf16(self.w_o, self.b_o, residual, ops.EPI_ADD_F32, x=attn, emit=begin_norm(ctx, n, self.hidden),
+                          split=ops.gemv_split(n, *self.w_o.shape, ws))
         else:
             linear(attn, self.w_o, self.b_o, residual, ADD_F32, ws)
 

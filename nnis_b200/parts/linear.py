@@ -27,7 +27,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], 
     by bulk copies ahead of the wait for the kernel before) where that kernel takes the shape."""
     m, (n, k) = x.shape[0], weight.shape
     if decode and x.dtype == torch.bfloat16 and ops.gemv_pays(m, n, k, mode, x.device):
-        ops.gemv_bf16(weight, bias, out, mode, x=x)  # (STORE, STORE_F32, ADD_F32 are its epilogues' codes)
+        split = ops.gemv_split(m, n, k, workspace) if mode == ADD_F32 and workspace is not None else None
+        ops.gemv_bf16(weight, bias, out, mode, x=x, split=split)  # (STORE, STORE_F32, ADD_F32 are its epilogues' codes)
     elif x.dtype == torch.bfloat16 and ops.gemm_tc_takes(m, n, k):
         scratch = tickets = None
         if mode == ADD_F32 and workspace is not None and ops.GEMM_SPLIT_K:

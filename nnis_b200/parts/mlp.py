@@ -132,7 +132,7 @@ class GatedMLP(Part):
                 ops.glu_clamp(gate_up, act, self.limit, self.alpha)
         if self._fused_down(ctx, n):
             ops.gemv_bf16(self.w_down, self.b_down, residual, ops.EPI_ADD_F32, x=act,
-                          emit=begin_norm(ctx, n, self.hidden))
+                          emit=begin_norm(ctx, n, self.hidden), split=ops.gemv_split(n, self.hidden, self.inter, ws))
         else:
             linear(act, self.w_down, self.b_down, residual, ADD_F32, ws)
 

@@ -73,3 +73,41 @@ def test_merge_of_slices(dim, rot, heads, splits, dtype):
             for h in range(heads):
                 s = torch.softmax(rows @ q[t, h * row:(h + 1) * row].double() * 0.2, 0)
                 assert torch.allclose(cut[t, h * dim:(h + 1) * dim].double(), s @ rows[:, :dim], atol=1e-5)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 2048, 5632), (16, 520, 12288), (8, 2048, 5632), (20, 960, 2560), (33, 1024, 3200),
+                                   (64, 2048, 8192), (5, 40, 12288)])
+@pytest.mark.parametrize("emits", [False, True])
+def test_adding_projection_whose_ctas_share_a_long_k(m, n, k, emits):
+    """One launch in place of one per slice: parts of unequal length, units that fill no CTA, several tiles of rows, the
+    next norm's values, and the same bits every time."""
+    o = ops()
+    g = torch.Generator().manual_seed(m + n + k)
+    x = torch.randn(m, k, generator=g).bfloat16().to(DEV)
+    w = (torch.randn(n, k, generator=g) / math.sqrt(k)).bfloat16().to(DEV)
+    bias, old = torch.randn(n, generator=g).to(DEV), torch.randn(m, n, generator=g).to(DEV)
+    floats, tiles = o.gemv_split_scratch(m, n, k, DEV)
+    assert floats and tiles and o.gemv_slices(m, n, k, DEV) > 1
+    split = (torch.full((floats,), math.nan, device=DEV), torch.zeros(tiles, dtype=torch.int32, device=DEV))
+    want = old.double() + bias.double() + x.double() @ w.double().T
+    emit_w = torch.rand(n, generator=g).to(DEV) + 0.5
+    first = None
+    for _ in range(3):
+        emit = (torch.empty(m, n, dtype=torch.bfloat16, device=DEV), emit_w, torch.empty(m, n // 8, device=DEV)) if emits else None
+        out = old.clone()
+        o.gemv_bf16(w, bias, out, o.EPI_ADD_F32, x=x, emit=emit, split=split)
+        first = out if first is None else first
+        assert torch.equal(out, first) and int(split[1].abs().sum()) == 0
+    # (float32 sums of products of bfloat16 values, cut off at 2^-23 of a running sum by the tensor cores: 96 of them a chain)
+    assert float((out.double() - want).norm() / want.norm()) < 1e-6
+    if emits:
+        assert torch.equal(emit[0], (out * emit_w).bfloat16())
+        assert torch.allclose(emit[2].double(), out.double().view(m, n // 8, 8).square().sum(-1), rtol=1e-6)
+    cut = old.clone()
+    o.gemv_bf16(w, bias, cut, o.EPI_ADD_F32, x=x)  # without the buffers: slices, as before
+    assert torch.allclose(cut, out, atol=1e-5)
+    small = (split[0][:floats - 1], split[1])  # buffers too small for it: slices
+    again = old.clone()
+    o.gemv_bf16(w, bias, again, o.EPI_ADD_F32, x=x, split=small)
+    assert torch.equal(again, cut)
+    o.check_status(DEV)
