@@ -17,6 +17,10 @@ int gemv_launch_rowtile(const GemvArgs&, int, int, int, bool, cudaStream_t);
 int gemv_rowtile_parts(int M, int N, int K, int sm_count, int* columns, int* units);
 int gemv_launch_rowtile_parts(const GemvArgs&, int, bool, cudaStream_t);
 
+// gemv_stream.cu: many output features of one tile of rows, a unit at a time
+bool gemv_stream_takes(int M, int N, int K, int epilogue, int pro, int sm_count);
+int gemv_launch_stream(const GemvArgs&, int, int, bool, cudaStream_t);
+
 // Shared memory of one CTA: x, the weight stages (eight rows of `kc` columns each),
 // the barriers, and with split K the warps' partial sums.
 static size_t gemv_smem(int mtiles, int warps, int stages, int K, int kc, bool splitk) {
@@ -220,7 +224,7 @@ NNIS_API int nnis_gemv_bf16(const void* x, const float* hidden, const int* rows,
     using namespace nnis;
     if (M <= 0 || N <= 0 || K <= 0 || !w || !out) return NNIS_ERR_ARGUMENT;
     if (act && ((epilogue != EPI_STORE && epilogue != EPI_GATED) || act < 1 || act > 3)) return NNIS_ERR_ARGUMENT;
-    GemvPlan plan;
+    GemvPlan plan = {};
     plan.kc = K;
     int pro = hidden ? PRO_NORM : ss_parts ? PRO_SCALED : PRO_PLAIN;
     if (hidden && ss_parts) return NNIS_ERR_ARGUMENT;
@@ -272,6 +276,11 @@ NNIS_API int nnis_gemv_bf16(const void* x, const float* hidden, const int* rows,
             return gemv_launch_rowtile_parts(a, units, (pdl & 1) != 0, stream);
         }
         a.k_parts = 1;
+    }
+    if (rowtile_cuts == 0 && !plan.splitk && !(pdl & 4) && gemv_stream_takes(M, N, K, epilogue, pro, sm_count)) {
+        a.trace = trace_slot("gemv stream");
+        a.emit_x = nullptr;
+        return gemv_launch_stream(a, epilogue, sm_count, (pdl & 1) != 0, stream);
     }
     a.K = K / slices;
     static const char* const kNames[] = {"gemv store", "gemv store_f32", "gemv add_f32", "gemv gated",

@@ -111,3 +111,33 @@ def test_adding_projection_whose_ctas_share_a_long_k(m, n, k, emits):
     o.gemv_bf16(w, bias, again, o.EPI_ADD_F32, x=x, split=small)
     assert torch.equal(again, cut)
     o.check_status(DEV)
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("n,k", [(2368, 2048), (2376, 2048), (6144, 1552), (2400, 3072), (9600, 2064)])
+def test_projection_of_many_output_features(m, n, k):
+    """A unit at a time, K shared by the warps: shares of K of unequal length, units that fill no round of the CTAs, each
+    epilogue."""
+    o = ops()
+    g = torch.Generator().manual_seed(m + n + k)
+    x = torch.randn(m, k, generator=g).bfloat16().to(DEV)
+    w = (torch.randn(n, k, generator=g) / math.sqrt(k)).bfloat16().to(DEV)
+    bias = torch.randn(n, generator=g).to(DEV)
+    assert o.gemv_kind(m, n, k, o.EPI_STORE, DEV) == 1
+    z = x.double() @ w.double().T + bias.double()
+    out = torch.full((m, n), math.nan, device=DEV)
+    o.gemv_bf16(w, bias, out, o.EPI_STORE_F32, x=x)
+    assert float((out.double() - z).norm() / z.norm()) < 1e-6  # (float32 sums; their chains are 24 products of 16 values)
+    half = torch.full((m, n), math.nan, dtype=torch.bfloat16, device=DEV)
+    o.gemv_bf16(w, bias, half, o.EPI_STORE, x=x)
+    assert torch.equal(half, out.bfloat16())
+    o.gemv_bf16(w, bias, half, o.EPI_STORE, x=x, act=o.GEMM_ACT_RELU2)
+    assert torch.equal(half, torch.relu(out).square().bfloat16())
+    gated = torch.full((m, n // 2), math.nan, dtype=torch.bfloat16, device=DEV)
+    o.gemv_bf16(w, bias, gated, o.EPI_GATED, x=x)
+    want = torch.nn.functional.silu(z[:, :n // 2]) * z[:, n // 2:]
+    assert torch.allclose(gated.double(), want, rtol=2.0 ** -8, atol=1e-5)  # (one rounding to bfloat16)
+    old = torch.empty_like(out)
+    o.gemv_bf16(w, bias, old, o.EPI_STORE_F32, x=x, rows_kernel=False)
+    assert torch.allclose(old, out, atol=2e-5)
+    o.check_status(DEV)
