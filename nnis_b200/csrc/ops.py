@@ -1554,6 +1554,35 @@ def latent_tiles(counts, starts, heads: int, tile_rows: int):
     return np.asarray(tiles, dtype=np.int32).reshape(-1, 2)
 
 
+def attention_latent_decode_takes(heads: int, dk: int, dv: int, page_size: int) -> bool:
+    """Whether a step of single tokens has a kernel of its own at these sizes (bfloat16 only)."""
+    return bool(LATENT_MMA) and bool(_lib().nnis_attention_latent_decode_takes(heads, dk, dv, page_size))
+
+
+def attention_latent_decode(q: torch.Tensor, cache: torch.Tensor, token_pos: torch.Tensor, token_seq: torch.Tensor,
+                            page_table: torch.Tensor, out: torch.Tensor, heads: int, dv: int, scale: float,
+                            n_splits: int = 1, partial: Optional[torch.Tensor] = None, window: int = 0,
+                            gate: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None) -> None:
+    """``attention_latent`` of single tokens on the tensor cores (bfloat16): every row is one token of a sequence of
+    its own.  Rows of the cache below the step's newest are read ahead of the kernel before."""
+    _cuda(q, cache, token_pos, token_seq, page_table, out, partial, gate, sink)
+    n = out.shape[0]
+    _need(gate is None or (gate.dtype == torch.float32 and gate.numel() >= n * heads), "attention_latent_decode: gate")
+    _need(sink is None or (sink.dtype == torch.float32 and sink.numel() == heads), "attention_latent_decode: sink [heads]")
+    pages, one, page_size, dk = cache.shape
+    _need(q.dtype == cache.dtype == out.dtype == torch.bfloat16, "attention_latent_decode: bfloat16")
+    _need(one == 1 and q.shape[1] == heads * dk and out.shape[1] == heads * dv, "attention_latent_decode: shapes")
+    _need(attention_latent_decode_takes(heads, dk, dv, page_size), "attention_latent_decode: sizes not taken")
+    _need(pages * page_size < 2 ** 31, "attention_latent_decode: the cache has too many rows")
+    if n_splits > 1:
+        _need(partial is not None and partial.dtype == torch.float32
+              and partial.numel() >= n * heads * n_splits * (dv + 2), "attention_latent_decode: partial scratch")
+    _check(_lib().nnis_attention_latent_decode(
+        _ptr(q), _ptr(cache), _ptr(token_pos), _ptr(token_seq), _ptr(page_table), page_table.shape[1], _ptr(out),
+        _ptr(partial), n, heads, dk, dv, pages, page_size, ctypes.c_float(scale), n_splits, window, _ptr(gate), _ptr(sink),
+        _ptr(status_word(q.device)), _stream()), "attention_latent_decode", 2 if n_splits > 1 else 1)
+
+
 def attention_latent_mma(q: torch.Tensor, cache: torch.Tensor, tiles: Optional[torch.Tensor],
                          seq_first_row: Optional[torch.Tensor], seq_start: Optional[torch.Tensor],
                          seq_count: Optional[torch.Tensor], token_pos: torch.Tensor, token_seq: torch.Tensor,

@@ -178,6 +178,10 @@ class LatentAttention(Part):
     def _tensor_cores(self) -> bool:
         return self.dtype == torch.bfloat16 and ops.attention_latent_mma_takes(self.row, self.kv_rank, PAGE_SIZE)
 
+    def _single_tokens(self) -> bool:
+        """Whether steps of single tokens have the kernel whose warps share a page."""
+        return self.dtype == torch.bfloat16 and ops.attention_latent_decode_takes(self.heads, self.row, self.kv_rank, PAGE_SIZE)
+
     def _expandable(self) -> bool:
         """Whether the tcgen05 kernel takes this layer's sizes and options."""
         return (self.dtype == torch.bfloat16 and self.q_rank > 0 and not self.window and not self.has_gate
@@ -233,10 +237,13 @@ class LatentAttention(Part):
     def _decode_splits(self, ctx, n: int) -> int:
         """Slices of the key range in a step of single tokens: enough CTAs for two per SM,
         at least two pages a slice."""
-        ctas = n * -(-self.heads // ops.latent_tile_rows(self.kv_rank)) * -(-self.kv_rank // 512)
         keys = ctx.max_context if not self.window else min(ctx.max_context, self.window + PAGE_SIZE - 1)
         pages = max(1, -(-keys // PAGE_SIZE))
-        want = -(-2 * ops.sm_count(self.device) // max(1, ctas * max(1, ctx.share)))
+        if self._single_tokens():  # (one CTA an SM: they hold two pages of the widest rows)
+            want = ops.sm_count(self.device) // max(1, n * -(-self.heads // 16) * max(1, ctx.share))
+        else:
+            ctas = n * -(-self.heads // ops.latent_tile_rows(self.kv_rank)) * -(-self.kv_rank // 512)
+            want = -(-2 * ops.sm_count(self.device) // max(1, ctas * max(1, ctx.share)))
         return int(max(1, min(want, pages // 2, 64)))
 
     # -- run --------------------------------------------------------------
@@ -263,7 +270,13 @@ class LatentAttention(Part):
             ops.batched_linear(q, self.dim, self.w_ukt, q_lat, self.row)
         o_lat = ws.get("latent_o", (n, H * self.kv_rank), self.dtype)
         tiles = ctx.tables.get(self._tiles_name())
-        if self._tensor_cores() and (ctx.decode or tiles is not None):
+        if ctx.decode and self._single_tokens():
+            splits = self._decode_splits(ctx, n)
+            partial = ws.get("attn_partial", (n * H * splits * (self.kv_rank + 2),), torch.float32) \
+                if splits > 1 else None
+            ops.attention_latent_decode(q_lat, cache.k, ctx.token_pos, ctx.token_seq, table, o_lat, H, self.kv_rank,
+                                        self.scale, splits, partial, window=self.window, gate=gate, sink=self.sink)
+        elif self._tensor_cores() and (ctx.decode or tiles is not None):
             splits = self._decode_splits(ctx, n) if ctx.decode else 1
             partial = ws.get("attn_partial", (n * H * splits * (self.kv_rank + 2),), torch.float32) \
                 if splits > 1 else None

@@ -141,3 +141,56 @@ def test_projection_of_many_output_features(m, n, k):
     o.gemv_bf16(w, bias, old, o.EPI_STORE_F32, x=x, rows_kernel=False)
     assert torch.allclose(old, out, atol=2e-5)
     o.check_status(DEV)
+
+
+@pytest.mark.parametrize("heads", [1, 8, 16, 17, 32])
+@pytest.mark.parametrize("dk,dv", [(576, 512), (288, 256), (24, 16), (72, 64), (56, 48)])
+@pytest.mark.parametrize("window", [0, 1, 70])
+def test_latent_attention_of_single_tokens(heads, dk, dv, window):
+    """Against 64 bits: pages that are not full, a slot of a page that no token has filled or that the window hides (NaN
+    there), more pages than the ring holds, slices without a key, padding rows, gates and sinks."""
+    o = ops()
+    assert o.attention_latent_decode_takes(heads, dk, dv, 64) and not o.attention_latent_decode_takes(33, dk, dv, 64)
+    g = torch.Generator().manual_seed(heads + dk + window)
+    lengths = [1, 64, 65, 0, 130, 700]
+    n, cols = len(lengths), 11
+    cache = torch.full((40, 1, 64, dk), math.nan, dtype=torch.bfloat16)
+    table = torch.full((n, cols), -1, dtype=torch.int32)
+    kept, page = [], 3
+    for t, length in enumerate(lengths):
+        rows = torch.randn(length, dk, generator=g).bfloat16()
+        kept.append(rows.double())
+        for p in range(-(-length // 64)):
+            table[t, p] = page
+            part = rows[p * 64:(p + 1) * 64]
+            cache[page, 0, :len(part)] = part
+            page += 1
+        if window:  # (rows that the token does not see any more)
+            for i in range(0, max(0, length - window)):
+                cache[int(table[t, i // 64]), 0, i % 64] = math.nan
+    q = torch.randn(n, heads * dk, generator=g).bfloat16()
+    gate, sink = torch.rand(n, heads, generator=g), torch.randn(heads, generator=g)
+    pos = torch.tensor([length - 1 for length in lengths], dtype=torch.int32)
+    d = lambda t: t.to(DEV)
+    scale = dk ** -0.5
+    for splits in (1, 2, 7, 64):
+        for with_gate, with_sink in ((False, False), (True, True)):
+            out = torch.full((n, heads * dv), 9.0, dtype=torch.bfloat16, device=DEV)
+            partial = torch.full((n * heads * splits * (dv + 2),), math.nan, device=DEV) if splits > 1 else None
+            o.attention_latent_decode(d(q), d(cache), d(pos), torch.arange(n, dtype=torch.int32, device=DEV), d(table), out,
+                                      heads, dv, scale, splits, partial, window, d(gate) if with_gate else None,
+                                      d(sink) if with_sink else None)
+            got = out.cpu().double().view(n, heads, dv)
+            for t, length in enumerate(lengths):
+                if not length:
+                    continue
+                rows = kept[t][max(0, length - window) if window else 0:]
+                s = q[t].double().view(heads, dk) @ rows.T * scale
+                if with_sink:
+                    s = torch.cat([s, sink.double()[:, None]], 1)
+                p = torch.softmax(s, 1)[:, :rows.shape[0]]
+                want = p @ rows[:, :dv] * (gate[t].double()[:, None] if with_gate else 1.0)
+                # (weights and outputs rounded to bfloat16, half a unit in eight bits each: 2^-7 of sums of |p v| together)
+                bound = 2.0 ** -7 * (p @ rows[:, :dv].abs()) * (gate[t].double()[:, None] if with_gate else 1.0) + 1e-4
+                assert ((got[t] - want).abs() <= bound).all(), (t, splits)
+    o.check_status(DEV)
