@@ -194,3 +194,25 @@ def test_latent_attention_of_single_tokens(heads, dk, dv, window):
                 bound = 2.0 ** -7 * (p @ rows[:, :dv].abs()) * (gate[t].double()[:, None] if with_gate else 1.0) + 1e-4
                 assert ((got[t] - want).abs() <= bound).all(), (t, splits)
     o.check_status(DEV)
+
+
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("heads,n,k", [(3, 8, 32), (2, 40, 96), (5, 24, 160), (16, 512, 128), (4, 128, 512), (2, 16, 544), (3, 12, 64)])
+@pytest.mark.parametrize("gate", [False, True])
+def test_small_matrix_per_head_on_few_rows(m, heads, n, k, gate):
+    """Pieces of K that fill no round, columns that fill no CTA, sizes and strides that are left to the CUDA cores, rows
+    and outputs with values of others between them."""
+    o = ops()
+    g = torch.Generator().manual_seed(m + n + k)
+    for a_head, out_head in ((k, n), (k + 8, n + 8), (k + 4, n + 1)):
+        a = torch.randn(m, heads * a_head, generator=g).bfloat16()
+        w = (torch.randn(heads, n, k, generator=g) / math.sqrt(k)).bfloat16()
+        logits = torch.randn(m, heads * n + 3, generator=g) if gate else None
+        out = torch.full((m, heads * out_head), 7.0, dtype=torch.bfloat16, device=DEV)
+        o.batched_linear(a.to(DEV), a_head, w.to(DEV), out, out_head, gate=logits.to(DEV) if gate else None, gate_off=3 if gate else 0)
+        want = torch.einsum("mhk,hnk->mhn", a.view(m, heads, a_head)[..., :k].double(), w.double())
+        if gate:
+            want = want * torch.sigmoid(logits[:, 3:].double()).view(m, heads, n)
+        got = out.cpu().double().view(m, heads, out_head)
+        assert torch.allclose(got[..., :n], want, rtol=2.0 ** -8, atol=1e-5)  # (one rounding to bfloat16)
+        assert (got[..., n:] == 7.0).all()
