@@ -149,6 +149,7 @@ class CacheManager:
                 group_of[e] = (len(self.groups), j)
             self.groups.append(g)
         self._states: List[torch.Tensor] = []
+        self._slot_states: Dict[int, List[torch.Tensor]] = {}
         for i, r in enumerate(requests):
             if isinstance(r, KVRequest):
                 gi, j = group_of[i]
@@ -187,9 +188,16 @@ class CacheManager:
         self.owners[slot] += 1
         for g in self.groups:
             g.tables[slot] = []
-        for t in self._states:
-            t[slot].zero_()
+        if self._states:
+            torch._foreach_zero_(self._states_of(slot))
         return slot
+
+    def _states_of(self, slot: int) -> List[torch.Tensor]:
+        """The slot's part of every state (views, made once a slot: each costs the host as much as a launch)."""
+        views = self._slot_states.get(slot)
+        if views is None:
+            views = self._slot_states[slot] = [t[slot] for t in self._states]
+        return views
 
     def release(self, slot: int) -> None:
         if not self.slots.is_held(slot):
@@ -294,7 +302,7 @@ class CacheManager:
         if not self.slots.is_held(slot):
             raise SlotError(f"slot {slot} is not held")
         return CacheSnapshot(slot, self.owners[slot], self.lengths[slot],
-                             [t[slot].clone() for t in self._states])
+                             [t.clone() for t in self._states_of(slot)])
 
     def restore(self, snapshot: CacheSnapshot) -> None:
         """Back to the snapshot: later positions are forgotten, the state is what it
@@ -308,8 +316,8 @@ class CacheManager:
                             f"sequence only {self.lengths[slot]}")
         if snapshot.length < self.lengths[slot]:
             self._forget_from(slot, snapshot.length)
-        for t, kept in zip(self._states, snapshot.states):
-            t[slot].copy_(kept)
+        for t, kept in zip(self._states_of(slot), snapshot.states):
+            t.copy_(kept)
 
     def page_table(self, group: int, slot: int) -> List[int]:
         return self.groups[group].tables[slot]

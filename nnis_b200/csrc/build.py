@@ -155,3 +155,16 @@ def load() -> ctypes.CDLL:
             except OSError as e:
                 raise KernelBuildError(f"cannot load {path}: {e}") from None
         return _lib
+
+
+_py_lib: Optional[ctypes.PyDLL] = None
+
+
+def load_locked() -> ctypes.PyDLL:
+    """The same library for entry points that use the interpreter's objects: calls keep its lock."""
+    global _py_lib
+    load()
+    with _lock:
+        if _py_lib is None:
+            _py_lib = ctypes.PyDLL(library_path())
+        return _py_lib

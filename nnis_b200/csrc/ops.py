@@ -105,6 +105,16 @@ def copy_async(dst: torch.Tensor, src: torch.Tensor) -> None:
         raise KernelError(f"copy_async: CUDA error {code}")
 
 
+def list_to_ints(values: list, limit: int):
+    """A list of whole numbers from 0 to below ``limit`` as an int32 array; None where it holds anything else (the
+    caller then looks at it number by number)."""
+    import numpy as np
+    out = np.empty(len(values), dtype=np.int32)
+    code = _build.load_locked().nnis_list_to_ints(ctypes.py_object(values), ctypes.c_long(len(values)), ctypes.c_long(limit),
+                                                  ctypes.c_void_p(out.__array_interface__["data"][0]))
+    return out if code == 0 else None
+
+
 def stream_synchronize() -> None:
     """Wait for the current stream (what ``Stream.synchronize`` does, without the object)."""
     code = _lib().nnis_stream_synchronize(_stream())

@@ -163,8 +163,18 @@ class Engine:
             raise StepError("a step needs at least one sequence")
         vocab = self.spec.vocab_size
         slots = [s.slot for s in batch]
-        counts, starts, token_arrays = [], [], []
+        counts, starts, token_arrays, wants = [], [], [], []
         for s in batch:
+            # (lists, what most callers have, are read and checked by native code; whatever it does not take, and whatever
+            # is wrong, is looked at here)
+            tok = ops.list_to_ints(s.tokens, vocab) if type(s.tokens) is list and s.tokens else None
+            want = ops.list_to_ints(s.want, tok.size) if tok is not None and type(s.want) is list else None
+            if want is not None:
+                token_arrays.append(tok)
+                wants.append(want)
+                counts.append(tok.size)
+                starts.append(self.cache.length(s.slot))
+                continue
             tok = np.asarray(s.tokens, dtype=np.int64).reshape(-1)
             if tok.size == 0:
                 raise StepError(f"slot {s.slot}: a sequence in a step brings at least one token")
@@ -176,6 +186,7 @@ class Engine:
                     raise StepError(f"slot {s.slot}: wanted place {w} is outside its "
                                     f"{tok.size} tokens")
             token_arrays.append(tok.astype(np.int32))
+            wants.append(np.asarray([int(w) for w in s.want], dtype=np.int32))
             counts.append(int(tok.size))
             starts.append(self.cache.length(s.slot))
         new_lengths = [a + b for a, b in zip(starts, counts)]
@@ -186,7 +197,7 @@ class Engine:
         pos = np.concatenate([np.arange(a, e, dtype=np.int32) for a, e in zip(starts, new_lengths)])
         seq = np.repeat(np.arange(b, dtype=np.int32), counts)
         first_rows = np.concatenate([[0], np.cumsum(counts)[:-1]]).astype(np.int32)
-        want_rows = i32([first_rows[i] + int(w) for i, s in enumerate(batch) for w in s.want])
+        want_rows = np.concatenate([first_rows[i] + w for i, w in enumerate(wants)]).astype(np.int32, copy=False)
         parts = [np.concatenate(token_arrays), pos, seq, i32(slots), want_rows]
         cols = []
         for g in range(len(self.cache.groups)):
