@@ -36,17 +36,17 @@ attn_merge_kernel(const float* __restrict__ partial, T* __restrict__ out, size_t
             int s = lane + 32 * k;
             ms[k] = s < n_splits ? rec[(size_t)s * (d + 2)] : 0.f;
             ls[k] = s < n_splits ? rec[(size_t)s * (d + 2) + 1] : 0.f;
-            if (ls[k] > 0.f) m = fmaxf(m, ms[k]);
+            if (ls[k] != 0.f) m = fmaxf(m, ms[k]);
         }
         m = warp_max(m);
         float l = 0.f;
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            ms[k] = ls[k] > 0.f ? expf(ms[k] - m) : 0.f;
+            ms[k] = ls[k] != 0.f ? expf(ms[k] - m) : 0.f;
             l += ls[k] * ms[k];
         }
         l = warp_sum(l);
-        float inv = l > 0.f ? 1.0f / l : 0.f;
+        float inv = l != 0.f ? 1.0f / l : 0.f;  // (a sum that is no number stays one)
         if (row_gate) inv *= row_gate[row];
         share[lane] = ms[0] * inv;
         share[lane + 32] = ms[1] * inv;
@@ -65,12 +65,12 @@ attn_merge_kernel(const float* __restrict__ partial, T* __restrict__ out, size_t
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     w[k] = s0 + k < n_splits ? share[s0 + k] : 0.f;
-                    v[k] = w[k] > 0.f ? *reinterpret_cast<const float2*>(rec + (size_t)(s0 + k) * (d + 2) + 2 + i)
+                    v[k] = w[k] != 0.f ? *reinterpret_cast<const float2*>(rec + (size_t)(s0 + k) * (d + 2) + 2 + i)
                                        : make_float2(0.f, 0.f);
                 }
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
-                    if (w[k] > 0.f) {
+                    if (w[k] != 0.f) {
                         o.x = fmaf(w[k], v[k].x, o.x);
                         o.y = fmaf(w[k], v[k].y, o.y);
                     }
@@ -84,7 +84,7 @@ attn_merge_kernel(const float* __restrict__ partial, T* __restrict__ out, size_t
         float o = 0.f;
         for (int s = 0; s < n_splits; ++s) {
             float w = share[s];
-            if (w > 0.f) o = fmaf(w, rec[(size_t)s * (d + 2) + 2 + i], o);
+            if (w != 0.f) o = fmaf(w, rec[(size_t)s * (d + 2) + 2 + i], o);
         }
         out[row * d + i] = from_float<T>(o);
     }

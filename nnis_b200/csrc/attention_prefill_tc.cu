@@ -52,18 +52,6 @@ constexpr float kTcLog2e = 1.4426950408889634f;
 constexpr int kTcPartial = kTcD + 2;  // floats per row of a chunk's result: O, maximum, sum
 constexpr float kTcRaise = 8.0f;  // log2 of how far a page's maximum may exceed the one in use
 
-// V tile as loaded ([64 keys, 64 d], rows of 128 bytes, 128-byte swizzle) read as
-// the MN-major B operand of O += P . V: 8-key groups are 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_mn128(uint32_t smem_byte_addr) {
-    uint64_t desc = 0;
-    desc |= (uint64_t)((smem_byte_addr >> 4) & 0x3FFF);
-    desc |= (uint64_t)1 << 16;              // leading byte offset: one 64-wide chunk only, unused
-    desc |= (uint64_t)(1024 >> 4) << 32;    // stride byte offset between groups of 8 keys
-    desc |= (uint64_t)1 << 46;              // descriptor version of sm_100
-    desc |= (uint64_t)2 << 61;              // SWIZZLE_128B
-    return desc;
-}
-
 __device__ __forceinline__ float max3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));

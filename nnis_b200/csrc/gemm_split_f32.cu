@@ -31,7 +31,7 @@
 // Level: eight warps that split and eight that add (158 us at 1,024 x 2,048 x 5,632 here, 180 there).
 // Every wait is bounded, as in gemm_tcgen05.cu.
 // NNIS: crates/nnis-kernels/src/gemm.rs:16-64 (tiled float32 product on CUDA cores).
-#include "fma_pairs.cuh"
+#include "split_parts.cuh"
 #include "tcgen05_helpers.cuh"
 
 namespace nnis {
@@ -53,31 +53,6 @@ struct SplitArgs {
     int M, N, K, add;
     int* status;
 };
-
-// Eight consecutive floats in one load, in pairs; the address is a multiple of 32 bytes.
-__device__ __forceinline__ void load8(const float* p, unsigned long long (&v)[4]) {
-    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
-}
-
-// A pair of values' next bfloat16 parts, packed; what is left of the values stays in x.
-__device__ __forceinline__ uint32_t next_part(unsigned long long& x) {
-    uint32_t p;
-    asm("{\n\t.reg .f32 a, b;\n\t.reg .b32 lo, hi;\n\t.reg .b64 h;\n\t"
-        "mov.b64 {a, b}, %1;\n\t"
-        "cvt.rn.bf16x2.f32 %0, b, a;\n\t"
-        "shl.b32 lo, %0, 16;\n\t"
-        "and.b32 hi, %0, 0xffff0000;\n\t"
-        "mov.b64 h, {lo, hi};\n\t"
-        "sub.rn.f32x2 %1, %1, h;\n\t}"
-        : "=r"(p), "+l"(x));
-    return p;
-}
-__device__ __forceinline__ uint32_t last_part(unsigned long long x) {
-    const float2 f = halves(x);
-    uint32_t p;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p) : "f"(f.y), "f"(f.x));
-    return p;
-}
 
 // The element (m, n) by a chain of float32 multiply-adds, for sums that are no numbers.
 __device__ __noinline__ float split_again(const float* a, const float* w, int K) {
@@ -155,14 +130,12 @@ gemm_split_kernel(const SplitArgs g) {
                 tc_fence_after();
                 const uint64_t da = desc_advance(desc_a0, (uint32_t)s * kStage);
                 const uint64_t dw = desc_advance(desc_w0, (uint32_t)s * kStage);
-                // parts of A and W, the smallest products first
-                constexpr int kPartsA[6] = {2, 0, 1, 1, 0, 0}, kPartsW[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
-                for (int p = 0; p < 6; ++p)
+                for (int p = 0; p < kSplitProducts; ++p)
 #pragma unroll
                     for (int k = 0; k < kSplitK / 16; ++k)
-                        tc_mma(tmem + (uint32_t)b * BN, desc_advance(da, kPartsA[p] * kSplitPartA + k * 32),
-                               desc_advance(dw, kPartsW[p] * kPartW + k * 32), idesc, (p | k) != 0);
+                        tc_mma(tmem + (uint32_t)b * BN, desc_advance(da, split_part_a(p) * kSplitPartA + k * 32),
+                               desc_advance(dw, split_part_b(p) * kPartW + k * 32), idesc, (p | k) != 0);
                 tc_commit(&empty_bar[s]);
                 tc_commit(&acc_full[b]);
             }
@@ -239,22 +212,7 @@ gemm_split_kernel(const SplitArgs g) {
                 const bool is_a = i < kItemsA;
                 const int row4 = ((is_a ? i : i - kItemsA) * kSplitWorkers + worker) * 4;
                 unsigned char* dst = stage + (is_a ? 0 : 3 * kSplitPartA) + row4 * 128 + ((unit ^ ((row4 & 4) + r4)) << 4);
-                uint4 o;
-                o.x = next_part(v[i][0]);
-                o.y = next_part(v[i][1]);
-                o.z = next_part(v[i][2]);
-                o.w = next_part(v[i][3]);
-                *reinterpret_cast<uint4*>(dst) = o;
-                o.x = next_part(v[i][0]);
-                o.y = next_part(v[i][1]);
-                o.z = next_part(v[i][2]);
-                o.w = next_part(v[i][3]);
-                *reinterpret_cast<uint4*>(dst + (is_a ? kSplitPartA : kPartW)) = o;
-                o.x = last_part(v[i][0]);
-                o.y = last_part(v[i][1]);
-                o.z = last_part(v[i][2]);
-                o.w = last_part(v[i][3]);
-                *reinterpret_cast<uint4*>(dst + 2 * (is_a ? kSplitPartA : kPartW)) = o;
+                store_parts(dst, is_a ? kSplitPartA : kPartW, v[i]);
                 load(i, wanted);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

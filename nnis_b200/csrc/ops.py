@@ -828,6 +828,86 @@ WIDE_QUERY_TILE = 128  # queries per CTA of attention_prefill_tc
 TC_ATTENTION = 0 if os.environ.get("NNIS_TC_ATTENTION", "1") == "0" else 1
 
 
+def attention_split_f32_takes(head_dim: int, page_size: int, q_stride: int) -> bool:
+    """Whether a float32 prompt step's attention can run on the tensor cores (``attention_split_f32``)."""
+    return bool(TC_ATTENTION) and head_dim == 64 and page_size == 64 and q_stride % 8 == 0
+
+
+def _f32_warps_time(counts, starts, window: int, heads: int) -> float:
+    """Microseconds of attention_generic.cu on a float32 prompt step: its longest query is a chain, and where its warps fill the
+    device 11 keys a nanosecond are worked."""
+    keys = longest = 0
+    for c, st in zip(counts, starts):
+        c, st = int(c), int(st)
+        whole = 0 if window <= 0 else max(0, st + c - max(st, window - 1))  # queries that see `window` keys
+        keys += whole * window + (c - whole) * (2 * st + c - whole + 1) // 2
+        longest = max(longest, min(st + c, window) if window > 0 else st + c)
+    return 3.0 + max(0.165 * longest, 9.2e-5 * keys * heads)
+
+
+def attention_split_f32_plan(counts, starts, window: int, heads: int, sms: int):
+    """Work list of ``attention_split_f32`` (int32 [n, 4] = (sequence, first query of 128, slice, slices of the tile), most pages
+    first) and the most slices of a tile; None where a warp for every query (attention_generic.cu) is thought to be faster.
+
+    A unit takes as long as its pages and two more, 3.1 us each; with more units than SMs the last ones end half a unit late;
+    records of slices have to be put together.  9 heads of 64 on a B200, us by warps, by tiles of 64 queries on the CUDA cores
+    and here: prompts of 509, 131 and 384 tokens 221 / 55 / 23, 1,024 497 / 88 / 38, 3 x 1,024 1,307 / 227 / 79, 64 13.7 / 11.5 / 8.8,
+    17 after 500 90 / 46 / 11, 64 after 2,000 358 / 49 / 19, 10 x 100 60 / 25 / 13; 17 6.6 / 9.4 / 7.7, 64 x 8 7.9 / 24 / 35,
+    300 in a window of 30 12.5 / 20 / 14."""
+    import numpy as np
+    tiles = []  # (sequence, first query, pages)
+    for i, (c, st) in enumerate(zip(counts, starts)):
+        for q0 in range(0, int(c), 128):
+            first, last = int(st) + q0, int(st) + min(q0 + 128, int(c)) - 1
+            lo = max(0, first - window + 1) if window > 0 else 0
+            tiles.append((i, q0, last // 64 - lo // 64 + 1))
+    pages, most = sum(t[2] for t in tiles), max(t[2] for t in tiles)
+    best = None
+    for per in sorted({-(-most // s) for s in range(1, min(16, most) + 1)}):
+        units = sum(-(-t[2] // per) for t in tiles)
+        time = per + 2.0 if units * heads <= sms else max(per + 2.0, (pages + 2.0 * units) * heads / sms + (per + 2.0) / 2)
+        time += 1.6 if per < most else 0.0
+        if best is None or time < best[0]:
+            best = time, per
+    if 3.1 * best[0] > _f32_warps_time(counts, starts, window, heads):
+        return None
+    units = []
+    for i, q0, n in tiles:
+        slices = -(-n // best[1])
+        units += [(-(-n // slices), i, q0, z, slices) for z in range(slices)]
+    units.sort(key=lambda u: -u[0])
+    return np.asarray([u[1:] for u in units], dtype=np.int32), max(u[4] for u in units)
+
+
+def attention_split_f32(q: torch.Tensor, q_stride: int, k_cache: torch.Tensor, v_cache: torch.Tensor, units: torch.Tensor,
+                        seq_first_row: torch.Tensor, seq_start: torch.Tensor, seq_count: torch.Tensor,
+                        page_table: torch.Tensor, out: torch.Tensor, heads: int, kv_heads: int, head_dim: int, window: int,
+                        scale: float, n_splits: int = 1, partial: Optional[torch.Tensor] = None) -> None:
+    """``attention_tile_f32`` on the tensor cores: 128 queries a tile, operands as exact sums of three bfloat16
+    values.  ``units`` and ``n_splits``: ``attention_split_f32_plan``'s."""
+    _cuda(k_cache, v_cache, units, seq_first_row, seq_start, seq_count, page_table, out, partial)
+    _need(q.is_cuda and q.dtype == torch.float32 == k_cache.dtype == v_cache.dtype == out.dtype,
+          "attention_split_f32: float32 tensors")
+    pages, nkv, page_size, d = k_cache.shape
+    n = out.shape[0]
+    _need(nkv == kv_heads and d == head_dim, "cache shape differs from the heads given")
+    _need(attention_split_f32_takes(head_dim, page_size, q_stride), "attention_split_f32: sizes not taken")
+    _need(heads % kv_heads == 0, "attention: heads is not a multiple of kv_heads")
+    _need(pages * nkv * page_size < 2 ** 31, "attention: the cache has too many rows")
+    _need(out.shape[1] == heads * head_dim, "attention: out [n, heads * d]")
+    for t in (units, seq_first_row, seq_start, seq_count):
+        _need(t.dtype == torch.int32, "attention_split_f32: int32 tables")
+    _need(units.dim() == 2 and units.shape[1] == 4 and units.shape[0] > 0, "units: int32 [n_units, 4]")
+    if n_splits > 1:
+        _need(partial is not None and partial.dtype == torch.float32
+              and partial.numel() >= n * heads * n_splits * (head_dim + 2), "attention: partial scratch too small")
+    _check(_lib().nnis_attention_split_f32(
+        _ptr(q), q_stride, _ptr(k_cache), _ptr(v_cache), _ptr(units), units.shape[0], _ptr(seq_first_row), _ptr(seq_start),
+        _ptr(seq_count), _ptr(page_table), page_table.shape[1], _ptr(out), _ptr(partial), n, heads, kv_heads, head_dim,
+        page_size, window, ctypes.c_float(scale), n_splits, _ptr(status_word(out.device)), _stream()),
+        "attention_split_f32", 2 if n_splits > 1 else 1)
+
+
 def attention_prefill_tc_takes(head_dim: int, page_size: int, q_stride: int) -> bool:
     """Whether the tcgen05 prompt attention kernel runs these sizes."""
     return bool(TC_ATTENTION) and head_dim == 64 and page_size == 64 and q_stride % 8 == 0

@@ -178,6 +178,18 @@ __device__ __forceinline__ uint64_t smem_desc_k128(uint32_t smem_byte_addr) {
     return desc;
 }
 
+// An attention's V tile as it lies ([64 keys, 64 d], rows of 128 bytes, 128-byte swizzle) read as
+// the MN-major B operand of O += P . V: 8-key groups are 1024 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc_mn128(uint32_t smem_byte_addr) {
+    uint64_t desc = 0;
+    desc |= (uint64_t)((smem_byte_addr >> 4) & 0x3FFF);
+    desc |= (uint64_t)1 << 16;              // leading byte offset: one 64-wide chunk only, unused
+    desc |= (uint64_t)(1024 >> 4) << 32;    // stride byte offset between groups of 8 keys
+    desc |= (uint64_t)1 << 46;              // descriptor version of sm_100
+    desc |= (uint64_t)2 << 61;              // SWIZZLE_128B
+    return desc;
+}
+
 // The same tile `bytes` further on in shared memory (a multiple of 16 that does
 // not carry out of the 14 address bits).  The one thread that issues the products
 // runs alone, every dependent instruction at full latency: building a descriptor

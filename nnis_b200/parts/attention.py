@@ -115,8 +115,15 @@ class Attention(Part):
         tcgen05 kernels (head sizes 64 and 128), shared by all layers with this window
         and number of heads, where they pay; else the 64-query tiles of the
         mma.sync kernel (head sizes 64 and 128), the same for every layer.  In float32
-        64-query tiles, the ones with the most keys first, where they pay."""
+        the units of the tensor cores' kernel (head size 64), else 64-query tiles, the ones
+        with the most keys first, where they pay."""
         if self.dtype != torch.bfloat16:
+            name = self._split_f32_name()
+            if self._split_f32(self.heads * self.head_dim):  # (or a warp for every query)
+                plan = None if name + "/units" in have else ops.attention_split_f32_plan(
+                    counts, starts, self.window, self.heads, ops.sm_count(self.device))
+                return {} if plan is None else {
+                    name + "/units": plan[0], name + "/slices": np.asarray([plan[1]], dtype=np.int32)}
             name = self._tile_f32_name()
             if name in have or not self._tile_f32(self.heads * self.head_dim) \
                     or not ops.attention_tile_f32_pays(counts, starts, self.window, self.heads):
@@ -141,6 +148,13 @@ class Attention(Part):
             tiles = [(i, q0) for i, c in enumerate(counts) for q0 in range(0, int(c), 64)]
             return {self.TILES_64: np.asarray(tiles, dtype=np.int32).reshape(-1, 2)}
         return {}
+
+    def _split_f32_name(self) -> str:
+        return f"prefill_split_f32/window{self.window}/heads{self.heads}"
+
+    def _split_f32(self, q_stride: int) -> bool:
+        """The kernel on the tensor cores takes a float32 prompt step."""
+        return self.dtype == torch.float32 and ops.attention_split_f32_takes(self.head_dim, PAGE_SIZE, q_stride)
 
     def _tile_f32_name(self) -> str:
         return f"prefill_f32/window{self.window}/heads{self.heads}"
@@ -297,6 +311,13 @@ class Attention(Part):
             ops.attention_prefill_mma(q_buf, q_stride, cache.k, cache.v, ctx.tables[self.TILES_64],
                                       ctx.seq_first_row, ctx.seq_start, ctx.seq_count, table, attn,
                                       nq, nkv, d, self.window, self.scale)
+        elif not ctx.decode and self._split_f32_name() + "/units" in ctx.tables and self._split_f32(q_stride):
+            name = self._split_f32_name()
+            slices = int(ctx.host_tables[name + "/slices"][0])
+            partial = ws.get("attn_partial", (n * nq * slices * (d + 2),), torch.float32) if slices > 1 else None
+            ops.attention_split_f32(q_buf, q_stride, cache.k, cache.v, ctx.tables[name + "/units"], ctx.seq_first_row,
+                                    ctx.seq_start, ctx.seq_count, table, attn, nq, nkv, d, self.window, self.scale, slices,
+                                    partial)
         elif not ctx.decode and self._tile_f32_name() in ctx.tables and self._tile_f32(q_stride):
             tiles = ctx.tables[self._tile_f32_name()]
             splits = ops.attention_tile_f32_splits(tiles.shape[0], nq, ctx.max_context, self.device)

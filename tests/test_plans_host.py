@@ -308,3 +308,28 @@ def test_float32_prompts_take_tiles_where_these_pay():
             tiles = [(st + q0, st + min(q0 + 64, c) - 1) for q0 in range(0, c, 64)]
             pages = sum(b // 64 - (max(0, a - window + 1) if window else 0) // 64 + 1 for a, b in tiles)
             assert pays([c], [st], window, 1000) == (pages * 1000 <= keys * 2)
+
+
+def test_units_of_the_float32_prompt_attention_cover_every_tile_once():
+    import random
+    from nnis_b200.csrc import ops as o
+    rng = random.Random(5)
+    for _ in range(300):
+        n = rng.randint(1, 6)
+        counts, starts = [rng.choice((1, 17, 128, 129, 700)) for _ in range(n)], [rng.choice((0, 5, 64, 900)) for _ in range(n)]
+        window = rng.choice((0, 0, 1, 100))
+        plan = o.attention_split_f32_plan(counts, starts, window, rng.choice((1, 9, 32)), rng.choice((1, 40, 148)))
+        if plan is None:
+            continue
+        units, slices = plan
+        seen = {}
+        for i, q0, z, k in units.tolist():
+            first, last = starts[i] + q0, starts[i] + min(q0 + 128, counts[i]) - 1
+            pages = last // 64 - (max(0, first - window + 1) if window else 0) // 64 + 1
+            per = -(-pages // k)
+            assert 0 <= z < k <= slices and (z * per < pages)  # (no slice is empty)
+            seen.setdefault((i, q0), []).append((z, k))
+        assert set(seen) == {(i, q0) for i, c in enumerate(counts) for q0 in range(0, c, 128)}
+        for parts in seen.values():
+            assert sorted(z for z, _ in parts) == list(range(parts[0][1])) and len({k for _, k in parts}) == 1
+        assert max(k for _, _, _, k in units.tolist()) == slices

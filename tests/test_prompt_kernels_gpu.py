@@ -68,6 +68,65 @@ def test_float32_prompt_attention_in_tiles(nq, nkv, d, window, splits):
         r += new[s]
 
 
+@pytest.mark.parametrize("nq,nkv", [(3, 3), (6, 2), (4, 1)])
+@pytest.mark.parametrize("window", [0, 1, 70, 300])
+@pytest.mark.parametrize("sms", [1, 40, 1000])
+def test_float32_prompt_attention_on_tcgen05(nq, nkv, window, sms):
+    """Head size 64, whole prompts and later portions, as the plans for one, some and very many SMs cut them (whole tiles, slices
+    of unequal number); a slot that no token has filled holds NaN."""
+    o = ops()
+    d, lengths, new = 64, [70, 200, 64, 333, 129, 1000], [70, 5, 64, 200, 65, 1000]
+    case = PagedCase(lengths, new, nq, nkv, d, "float32", seed=5 * nq + window)
+    kc, vc = stored(case, torch.float32, math.nan)
+    q = case.packed()[2]
+    n, stride = q.shape[0], nq * d + 8
+    qd = torch.full((n, stride), 3.0, device=DEV)
+    qd[:, :nq * d] = q.reshape(n, -1).to(DEV)
+    first, start, count, starts = wide_inputs(new, lengths)
+    plan = o.attention_split_f32_plan(new, starts, window, nq, sms)
+    if plan is None:  # (a window of one key: the other kernel's; these units run all the same)
+        plan = torch.tensor([(i, q0, 0, 1) for i, c in enumerate(new) for q0 in range(0, c, 128)]).numpy(), 1
+    units, slices = plan
+    out = torch.full((n, nq * d), 5.0, device=DEV)
+    partial = torch.full((n * nq * slices * (d + 2),), math.nan, device=DEV) if slices > 1 else None
+    o.attention_split_f32(qd, stride, kc, vc, i32(units), first, start, count, case.table.to(DEV), out, nq, nkv, d, window,
+                          1.0 / math.sqrt(d), slices, partial)
+    o.check_status(DEV)
+    r = 0
+    for s, L in enumerate(lengths):
+        full = P.causal_attention(case.q[s], case.k[s], case.v[s], window)[L - new[s]:].reshape(new[s], -1).double()
+        got = out[r:r + new[s]].cpu().double()
+        # scores of order one within 2e-7 of themselves, sums of at most 1,000 weights: 1e-6 of the result's 2-norm
+        assert float((got - full).norm() / full.norm()) < 1e-6, s
+        r += new[s]
+
+
+def test_float32_prompt_attention_on_tcgen05_with_values_that_are_no_numbers():
+    """An infinity or NaN among values or keys is felt by the queries that see it, as the kernel with chains of multiply-adds
+    has it, and by no other."""
+    o = ops()
+    nq, nkv, d, L = 2, 1, 64, 300
+    case = PagedCase([L], [L], nq, nkv, d, "float32", seed=3)
+    case.v[0][100, 0, 5], case.v[0][200, 0, 40], case.k[0][250, 0, 7] = math.inf, math.nan, math.inf
+    kc, vc = stored(case, torch.float32, 0.0)
+    q = case.packed()[2].reshape(L, -1).contiguous().to(DEV)
+    first, start, count, starts = wide_inputs([L], [L])
+    seq, pos = torch.zeros(L, dtype=torch.int32, device=DEV), torch.arange(L, dtype=torch.int32, device=DEV)
+    want = torch.empty(L, nq * d, device=DEV)
+    o.attention_generic(q, nq * d, kc, vc, pos, seq, case.table.to(DEV), want, nq, nkv, d, 0, 0.125, 1, None)
+    assert torch.isnan(want[299]).any() and torch.isinf(want[150]).any() and torch.isfinite(want[:100]).all()
+    for units, slices in (([(0, 0, 0, 1), (0, 128, 0, 1), (0, 256, 0, 1)], 1),
+                          ([(0, 0, 0, 1), (0, 128, 0, 2), (0, 128, 1, 2), (0, 256, 0, 3), (0, 256, 1, 3), (0, 256, 2, 3)], 3)):
+        out = torch.full((L, nq * d), 5.0, device=DEV)
+        partial = torch.full((L * nq * slices * (d + 2),), math.nan, device=DEV) if slices > 1 else None
+        o.attention_split_f32(q, nq * d, kc, vc, i32(units), first, start, count, case.table.to(DEV), out, nq, nkv, d, 0, 0.125,
+                              slices, partial)
+        o.check_status(DEV)
+        assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isinf(out), torch.isinf(want))
+        fine = torch.isfinite(want)
+        assert torch.allclose(out[fine], want[fine], atol=5e-6)
+
+
 def wide_inputs(new, lengths):
     starts = [L - c for L, c in zip(lengths, new)]
     return i32([sum(new[:i]) for i in range(len(new))]), i32(starts), i32(new), starts
