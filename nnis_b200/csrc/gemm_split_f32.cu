@@ -14,10 +14,10 @@
 //
 // One CTA works a tile of 128 x BN (BN 64 or 128), KS CTAs of a cluster share the tile's K and add their sums through
 // distributed shared memory, in the order of their ranks (the same bits every time).  Roles:
-//   warp 0       allocates tensor memory; one lane issues tcgen05.mma (kind::f16, 128 x BN x 16), 24 for 64 columns of K,
-//                into one of two accumulators;
-//   warps 1-16   bring A and W, 32 bytes a load, one block of K ahead in registers, write the three parts of each value
-//                into swizzled shared memory (two blocks of K), then read the accumulator of the block before with
+//   warp 0       (BN = 64: two warps) allocates tensor memory; one lane issues tcgen05.mma (kind::f16, 128 x BN x 16), 24 for 64 columns of K,
+//                into one of four accumulators;
+//   16 others    bring A and W, 32 bytes a load, one block of K ahead in registers, write the three parts of each value
+//                into swizzled shared memory (two or three blocks of K), and read the accumulator of two blocks before with
 //                tcgen05.ld and add it to their registers (a row and a quarter of the columns a thread); at the end they
 //                write the tile, through shared memory, so that whole lines leave.
 // Splitting on the way in keeps the weights once in memory, as the decode kernels read them.
@@ -28,7 +28,9 @@
 // 1,024 x 3,072 x 576 104 -> 47 us (2 waves of tiles), 1,024 x 576 x 1,536 82 -> 29, 1,024 x 576 x 576 35 -> 18,
 // 2,048 x 2,048 x 2,048 416 -> 123 (140 TFLOP/s of float32), 17 x 576 x 576 35 -> 14.  Distance from 64-bit sums (2-norm, K =
 // 576 / 1,536 / 5,632): 2.2e-7 / 3.5e-7 / 6.7e-7 there, 0.98e-7 / 1.1e-7 / 1.5e-7 here.
-// Level: eight warps that split and eight that add (158 us at 1,024 x 2,048 x 5,632 here, 180 there).
+// The gated product also applies silu and multiplies: a pass of 7 us over 1,024 x 3,072 less.
+// Level: tiles of 256 x 128 worked by pairs of CTAs (cta_group::2, 192 instead of 256 rows split a block: 49 and 50 us at 1,024 x
+// 3,072 x 576, 160 and 162 at 1,024 x 2,048 x 5,632); eight warps that split and eight that add (158 us at 1,024 x 2,048 x 5,632 here, 180 there).
 // Every wait is bounded, as in gemm_tcgen05.cu.
 // NNIS: crates/nnis-kernels/src/gemm.rs:16-64 (tiled float32 product on CUDA cores).
 #include "split_parts.cuh"
@@ -37,20 +39,25 @@
 namespace nnis {
 
 constexpr int kSplitM = 128, kSplitK = 64;
-constexpr int kSplitStages = 2;
 constexpr int kSplitAccs = 4;    // accumulators
 constexpr int kSplitWorkers = 16;  // warps
-constexpr int kSplitThreads = 32 * (1 + kSplitWorkers);
 constexpr uint32_t kSplitPartA = kSplitM * 128;  // one part of a block of A: 128 rows of 64 bfloat16
 
+// blocks of K in shared memory: as many as fit
+__host__ __device__ constexpr int split_stages(int bn) { return bn == 64 ? 3 : 2; }
 __host__ __device__ constexpr uint32_t split_stage_bytes(int bn) { return 3u * (kSplitPartA + (uint32_t)bn * 128u); }
+// Warps that issue products, a block of K in turn: an issuing thread spends 62 cycles on a product and 950 on a block's
+// barriers, under which the tensor cores run dry where a product takes them no longer (BN = 64: 59 -> 55 us at 1,024 x 3,072 x
+// 576, 276 -> 246 at 1,024 x 2,048 x 5,632; BN = 128 49 and 49, 160 and 168).
+__host__ __device__ constexpr int split_issuers(int bn) { return bn == 64 ? 2 : 1; }
+__host__ __device__ constexpr int split_threads(int bn) { return 32 * (split_issuers(bn) + 16); }
 
 struct SplitArgs {
     const float* A;
     const float* W;
     const float* bias;
     float* C;
-    int M, N, K, add;
+    int M, N, K, mode;  // 1 store, 2 add, 3 gated: W holds gate rows, then up rows; C [M, N / 2] = silu(gate) up
     int* status;
 };
 
@@ -72,11 +79,12 @@ __device__ __forceinline__ float4 peer_load4(const float* p, uint32_t rank) {
 }
 
 template <int BN, int KS>
-__global__ void __launch_bounds__(kSplitThreads, 1)
+__global__ void __launch_bounds__(split_threads(BN), 1)
 gemm_split_kernel(const SplitArgs g) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    constexpr int kSplitStages = split_stages(BN), kSplitIssuers = split_issuers(BN);
     constexpr uint32_t kPartW = BN * 128, kStage = split_stage_bytes(BN);
     constexpr uint32_t kTmemCols = kSplitAccs * BN;
     __shared__ __align__(8) uint64_t full_bar[kSplitStages], empty_bar[kSplitStages], acc_full[kSplitAccs], acc_empty[kSplitAccs];
@@ -84,12 +92,19 @@ gemm_split_kernel(const SplitArgs g) {
     __shared__ volatile int abort_flag;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slice = KS > 1 ? (int)cluster_rank() : 0;
     const int n0 = (blockIdx.x / KS) * BN, m0 = blockIdx.y * kSplitM;
-    const int rank = KS > 1 ? (int)cluster_rank() : 0;
     const int blocks_all = (g.K + kSplitK - 1) / kSplitK;
-    // this CTA's run of blocks of K
+    // this slice's run of blocks of K
     const int per = (blocks_all + KS - 1) / KS;
-    const int first = min(blocks_all, rank * per), blocks = min(per, blocks_all - first);
+    const int first = min(blocks_all, slice * per), blocks = min(per, blocks_all - first);
+    const int inter = g.N >> 1;  // mode 3: columns of the output
+    // row of W of the tile's column c, or -1
+    auto w_row = [&](int c) {
+        if (g.mode != 3) return n0 + c < g.N ? n0 + c : -1;
+        const int n = n0 / 2 + c % (BN / 2);
+        return n < inter ? (c < BN / 2 ? n : inter + n) : -1;
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kSplitStages; ++s) {
@@ -113,16 +128,16 @@ gemm_split_kernel(const SplitArgs g) {
     unsigned long long acc[kCols / 2];  // pairs
 #pragma unroll
     for (int i = 0; i < kCols / 2; ++i) acc[i] = 0ull;
-    if (warp == 0) {
+    if (warp < kSplitIssuers) {
         pdl_wait();
         pdl_launch_dependents();
         if (lane == 0) {
             constexpr uint32_t idesc = instr_desc(kSplitM, BN);
             const uint64_t desc_a0 = smem_desc_k128(smem_addr(base));
             const uint64_t desc_w0 = smem_desc_k128(smem_addr(base) + 3 * kSplitPartA);
-            for (int kb = 0; kb < blocks; ++kb) {
-                const int s = kb & 1, b = kb & 3;
-                if (!mbar_wait(&full_bar[s], (uint32_t)(kb >> 1) & 1u) ||
+            for (int kb = warp; kb < blocks; kb += kSplitIssuers) {
+                const int s = kb % kSplitStages, b = kb & 3;
+                if (!mbar_wait(&full_bar[s], (uint32_t)(kb / kSplitStages) & 1u) ||
                     (kb >= 4 && !mbar_wait(&acc_empty[b], (uint32_t)((kb >> 2) - 1) & 1u)) || abort_flag) {
                     abort_flag = 1;
                     break;
@@ -143,7 +158,7 @@ gemm_split_kernel(const SplitArgs g) {
         __syncwarp();
     } else {
         // a warp splits four rows at a time, eight floats a lane: (128 + BN) / 64 such items a thread and block of K
-        const int worker = warp - 1, r4 = lane >> 3, unit = lane & 7;
+        const int worker = warp - kSplitIssuers, r4 = lane >> 3, unit = lane & 7;
         constexpr int kItemsA = kSplitM / (4 * kSplitWorkers), kItems = kItemsA + BN / (4 * kSplitWorkers);
         unsigned long long v[kItems][4];
         const float* src[kItems];
@@ -151,9 +166,9 @@ gemm_split_kernel(const SplitArgs g) {
 #pragma unroll
         for (int i = 0; i < kItems; ++i) {
             const int row = ((i < kItemsA ? i : i - kItemsA) * kSplitWorkers + worker) * 4 + r4;
-            const int at = i < kItemsA ? m0 + row : n0 + row;
-            src[i] = (i < kItemsA ? g.A : g.W) + (size_t)at * g.K + first * kSplitK + unit * 8;
-            if (at < (i < kItemsA ? g.M : g.N)) there |= 1u << i;
+            const int at = i < kItemsA ? (m0 + row < g.M ? m0 + row : -1) : w_row(row);
+            src[i] = (i < kItemsA ? g.A : g.W) + (at < 0 ? 0 : (size_t)at * g.K + first * kSplitK + unit * 8);
+            if (at >= 0) there |= 1u << i;
             v[i][0] = v[i][1] = v[i][2] = v[i][3] = 0ull;  // (rows beyond M and N are never loaded and stay zero)
         }
         auto load = [&](int i, uint32_t wanted) {
@@ -195,9 +210,9 @@ gemm_split_kernel(const SplitArgs g) {
         // other's arithmetic
         const bool early = (worker & 4) != 0;
         for (int kb = 0; kb < blocks && ok; ++kb) {
-            const int s = kb & 1;
+            const int s = kb % kSplitStages;
             if (early && kb >= 2 && !(ok = add_block(kb - 2))) break;
-            ok = kb < 2 || mbar_wait(&empty_bar[s], (uint32_t)((kb >> 1) - 1) & 1u);
+            ok = kb < kSplitStages || mbar_wait(&empty_bar[s], (uint32_t)(kb / kSplitStages - 1) & 1u);
             ok = __all_sync(0xffffffffu, ok) && !abort_flag;
             if (!ok) break;
             if (k_left <= 0) {  // columns beyond K
@@ -229,60 +244,79 @@ gemm_split_kernel(const SplitArgs g) {
     constexpr int kRow = BN + 4;  // floats between rows: 16-byte stores of neighbouring rows meet no bank twice
     float* sums = reinterpret_cast<float*>(base);
     __syncthreads();
-    const int quarter = warp & 3, c0 = warp > 0 ? ((warp - 1) >> 2) * kCols : 0;
-    if (warp > 0) {
+    const int quarter = warp & 3, c0 = warp >= kSplitIssuers ? ((warp - kSplitIssuers) >> 2) * kCols : 0;
+    if (warp >= kSplitIssuers) {
         float* mine = sums + (quarter * 32 + lane) * kRow + c0;
 #pragma unroll
         for (int i = 0; i < kCols; i += 4)
             *reinterpret_cast<ulonglong2*>(mine + i) = make_ulonglong2(acc[i / 2], acc[i / 2 + 1]);
     }
     if constexpr (KS > 1) cluster_meet();
-    else __syncwarp();
-    if (warp > 0 && !abort_flag) {
-        constexpr int kLanes = kCols / 4;       // lanes to a row's columns of this warp, four floats each
-        constexpr int kRows = 32 / kLanes;      // rows a warp writes at a time
-        const bool by_four = (g.N & 3) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15) == 0;
-        const int n = n0 + c0 + (lane % kLanes) * 4;
-#pragma unroll 4
-        for (int r = 0; r < 32 / KS; r += kRows) {
-            const int row = quarter * 32 + rank * (32 / KS) + r + lane / kLanes, m = m0 + row;
-            const float* at = sums + row * kRow + c0 + (lane % kLanes) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (m >= g.M || n >= g.N) continue;
+    else __syncthreads();
+    if (warp >= kSplitIssuers && !abort_flag) {
+        const bool gated = g.mode == 3;
+        // a warp's columns of the output, its lanes to a row, four floats each, and the rows it writes at a time
+        const int width = gated ? kCols / 2 : kCols, lanes = width / 4, rows_at = 32 / lanes;
+        const int out_cols = gated ? inter : g.N;
+        const bool by_four = (out_cols & 3) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 15) == 0;
+        const int c = ((warp - kSplitIssuers) >> 2) * width + (lane % lanes) * 4, n = (gated ? n0 / 2 : n0) + c;
+        constexpr int kSliceRows = (32 / KS + 7) / 8 * 8;  // of the warp's 32: each slice finishes its share
+        const int r_end = min(32, (slice + 1) * kSliceRows);
+        auto sum_of = [&](const float* at) {
+            float4 v = *reinterpret_cast<const float4*>(at);
             if constexpr (KS > 1) {
+                v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int z = 0; z < KS; ++z) {
                     const float4 x = peer_load4(at, (uint32_t)z);
                     v = make_float4(v.x + x.x, v.y + x.y, v.z + x.z, v.w + x.w);
                 }
-            } else {
-                v = *reinterpret_cast<const float4*>(at);
             }
-            float f[4] = {v.x, v.y, v.z, v.w};
+            return v;
+        };
+#pragma unroll 2
+        for (int r = slice * kSliceRows; r < r_end; r += rows_at) {
+            const int row = quarter * 32 + r + lane / lanes, m = m0 + row;
+            if (r + lane / lanes >= r_end || m >= g.M || n >= out_cols) continue;
+            const float* at = sums + row * kRow + c;
+            const float4 v = sum_of(at);
+            float f[4] = {v.x, v.y, v.z, v.w}, u[4] = {0.f, 0.f, 0.f, 0.f};
+            if (gated) {
+                const float4 w = sum_of(at + BN / 2);
+                u[0] = w.x;
+                u[1] = w.y;
+                u[2] = w.z;
+                u[3] = w.w;
+            }
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                if (n + e >= g.N) continue;
+                if (n + e >= out_cols) continue;
                 if (!isfinite(f[e])) f[e] = split_again(g.A + (size_t)m * g.K, g.W + (size_t)(n + e) * g.K, g.K);
                 if (g.bias) f[e] += g.bias[n + e];
+                if (gated) {
+                    if (!isfinite(u[e])) u[e] = split_again(g.A + (size_t)m * g.K, g.W + (size_t)(inter + n + e) * g.K, g.K);
+                    if (g.bias) u[e] += g.bias[inter + n + e];
+                    f[e] = f[e] / (1.0f + expf(-f[e])) * u[e];
+                }
             }
-            float* out = g.C + (size_t)m * g.N + n;
+            float* out = g.C + (size_t)m * out_cols + n;
             if (by_four) {
                 float4 o = make_float4(f[0], f[1], f[2], f[3]);
-                if (g.add) {
-                    const float4 c = load4(out);
-                    o = make_float4(c.x + o.x, c.y + o.y, c.z + o.z, c.w + o.w);
+                if (g.mode == 2) {
+                    const float4 old = load4(out);
+                    o = make_float4(old.x + o.x, old.y + o.y, old.z + o.z, old.w + o.w);
                 }
                 store4(out, o);
             } else {
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    if (n + e < g.N) out[e] = g.add ? out[e] + f[e] : f[e];
+                    if (n + e < out_cols) out[e] = g.mode == 2 ? out[e] + f[e] : f[e];
             }
         }
     }
     tc_fence_before();
-    if constexpr (KS > 1) cluster_meet();  // no CTA leaves while another reads its sums
     __syncthreads();
+    if constexpr (KS > 1) cluster_meet();  // no CTA leaves while another reads its sums
     if (warp == 0) {
         tc_fence_after();
         tmem_dealloc(tmem, kTmemCols);
@@ -293,14 +327,14 @@ gemm_split_kernel(const SplitArgs g) {
 template <int BN, int KS>
 static int launch_split(const SplitArgs& g, cudaStream_t stream) {
     auto kernel = gemm_split_kernel<BN, KS>;
-    constexpr size_t sums = (size_t)kSplitM * (BN + 4) * 4, stages = kSplitStages * (size_t)split_stage_bytes(BN);
+    constexpr size_t sums = (size_t)kSplitM * (BN + 4) * 4, stages = split_stages(BN) * (size_t)split_stage_bytes(BN);
     constexpr size_t smem = (sums > stages ? sums : stages) + 1024;
-    static_assert(smem <= 227 * 1024 - 1024, "one CTA's shared memory");
+    static_assert(smem <= 227 * 1024 - 2048, "one CTA's shared memory");
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)((g.N + BN - 1) / BN * KS), (unsigned)((g.M + kSplitM - 1) / kSplitM));
-    cfg.blockDim = dim3(kSplitThreads);
+    cfg.blockDim = dim3(split_threads(BN));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -325,44 +359,44 @@ static int launch_split(const SplitArgs& g, cudaStream_t stream) {
 // end 6,000 cycles, a cluster's meeting 1,500; a block of K 1,600 and 1,250 at widths 128 and 64 relative to those).  us at widths
 // x CTAs 64x1, 64x2, 64x4, 128x1, 128x2, 128x4: 1,024 x 576 x 1,536 45, 31, 49, 51, 34, 39; 1,024 x 3,072 x 576 57, 80, 125, 47,
 // 51, 78; 2,048 x 2,048 x 2,048 207, 215, 287, 125, 139, 170; 256 x 2,048 x 2,048 55, 37, 43, 66, 41, 29.
-static void split_shape(int M, int N, int K, int sms, int* bn, int* ks) {
+static int split_shape(int M, int N, int K, int sms) {
     const long m_tiles = (M + kSplitM - 1) / kSplitM;
     const int blocks = (K + kSplitK - 1) / kSplitK;
     long best = -1;
-    const int widths[2] = {128, 64}, splits[3] = {1, 2, 4};
-    for (int w : widths)
-        for (int s : splits) {
-            if (s > 1 && blocks < 2 * s) continue;
-            const long ctas = m_tiles * ((N + w - 1) / w) * s;
-            const long waves = (ctas + sms - 1) / sms;
-            const long cost = waves * (6000 + (s > 1 ? 1500 : 0) + (long)((blocks + s - 1) / s) * (w == 128 ? 1600 : 1250));
+    int shape = 21;
+    for (int bn = 128; bn >= 64; bn -= 64)
+        for (int ks = 1; ks <= 4; ks *= 2) {
+            if (ks > 1 && blocks < 2 * ks) continue;
+            const long ctas = m_tiles * ((N + bn - 1) / bn) * ks, waves = (ctas + sms - 1) / sms;
+            const long cost = waves * (6000 + (ks > 1 ? 1500 : 0) + (long)((blocks + ks - 1) / ks) * (bn == 128 ? 1600 : 1250));
             if (best < 0 || cost < best) {
                 best = cost;
-                *bn = w;
-                *ks = s;
+                shape = bn / 64 * 10 + ks;
             }
         }
+    return shape;
 }
 
 }  // namespace nnis
 
-// Modes: 1 store, 2 add into C.  `shape` 0: by the rule; else (BN / 64) * 10 + KS.  Refuses (NNIS_ERR_UNSUPPORTED) K not a multiple of
-// 8; A and W start on 32-byte boundaries.
+// Modes: 1 store, 2 add into C, 3 gated (W = [gate rows; up rows], C [M, N / 2] = silu(gate) up).  `shape` 0: by the rule; else
+// (BN / 64) * 10 + KS.  Refuses (NNIS_ERR_UNSUPPORTED) K not a multiple of 8; A and W start on 32-byte
+// boundaries.
 NNIS_API int nnis_gemm_split_f32(const float* A, const float* W, const float* bias, float* C, int M, int N, int K,
                                  int mode, int shape, int sm_count, int* status, cudaStream_t stream) {
     using namespace nnis;
-    if (M <= 0 || N <= 0 || K <= 0 || !A || !W || !C || mode < 1 || mode > 2) return NNIS_ERR_ARGUMENT;
-    if (K % 8 || (M + kSplitM - 1) / kSplitM > 65535) return NNIS_ERR_UNSUPPORTED;
+    if (M <= 0 || N <= 0 || K <= 0 || !A || !W || !C || mode < 1 || mode > 3) return NNIS_ERR_ARGUMENT;
+    if (K % 8 || (mode == 3 && N % 2) || (M + kSplitM - 1) / kSplitM > 65535) return NNIS_ERR_UNSUPPORTED;
     if (((uintptr_t)A | (uintptr_t)W) % 32 || (uintptr_t)C % 4) return NNIS_ERR_ALIGNMENT;
-    SplitArgs g{A, W, bias, C, M, N, K, mode == 2, status};
-    int bn = 128, ks = 1;
-    split_shape(M, N, K, sm_count > 0 ? sm_count : 148, &bn, &ks);
-    if (shape) { bn = shape / 10 * 64; ks = shape % 10; }
-    if (bn == 128 && ks == 1) return launch_split<128, 1>(g, stream);
-    if (bn == 128 && ks == 2) return launch_split<128, 2>(g, stream);
-    if (bn == 128 && ks == 4) return launch_split<128, 4>(g, stream);
-    if (bn == 64 && ks == 1) return launch_split<64, 1>(g, stream);
-    if (bn == 64 && ks == 2) return launch_split<64, 2>(g, stream);
-    if (bn == 64 && ks == 4) return launch_split<64, 4>(g, stream);
-    return NNIS_ERR_ARGUMENT;
+    SplitArgs g{A, W, bias, C, M, N, K, mode, status};
+    if (!shape) shape = split_shape(M, N, K, sm_count > 0 ? sm_count : 148);
+    switch (shape) {
+        case 21: return launch_split<128, 1>(g, stream);
+        case 22: return launch_split<128, 2>(g, stream);
+        case 24: return launch_split<128, 4>(g, stream);
+        case 11: return launch_split<64, 1>(g, stream);
+        case 12: return launch_split<64, 2>(g, stream);
+        case 14: return launch_split<64, 4>(g, stream);
+        default: return NNIS_ERR_ARGUMENT;
+    }
 }

@@ -213,16 +213,17 @@ def gemm_split_f32_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
 def gemm_split_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, mode: int,
                    shape: int = 0) -> None:
     """out (op)= a . w^T + bias for float32 operands on the tensor cores, every value as the exact sum of
-    three bfloat16 values.  ``shape``: 0 by the kernel's rule, or (tile columns / 64) * 10 + CTAs that share K."""
+    three bfloat16 values.  GEMM_GATED: w = [gate rows; up rows], out [m, n / 2] = silu(gate) * up.  ``shape``: 0 by
+    the kernel's rule, or (tile columns / 64) * 10 + CTAs that share K."""
     _cuda(a, w, bias, out)
     m, k = a.shape
     n = w.shape[0]
     _need(w.shape[1] == k and a.dtype == w.dtype == out.dtype == torch.float32, "gemm: float32 a [m, k], w [n, k]")
-    _need(tuple(out.shape) == (m, n), "gemm: out [m, n]")
+    _need(tuple(out.shape) == ((m, n // 2) if mode == GEMM_GATED else (m, n)) and (mode != GEMM_GATED or n % 2 == 0), "gemm: out [m, n]")
     if bias is not None:
         _need(bias.dtype == torch.float32 and bias.numel() == n, "gemm: bias float32 [n]")
-    _check(_lib().nnis_gemm_split_f32(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, 2 if mode == ADD_F32 else 1,
-                                      shape, sm_count(a.device), _ptr(status_word(a.device)), _stream()),
+    _check(_lib().nnis_gemm_split_f32(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k,
+                                      3 if mode == GEMM_GATED else 2 if mode == ADD_F32 else 1, shape, sm_count(a.device), _ptr(status_word(a.device)), _stream()),
            "gemm_split_f32")
 
 

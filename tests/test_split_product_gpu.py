@@ -43,6 +43,31 @@ def test_against_64_bits(m, n, k):
     o.check_status(DEV)
 
 
+@pytest.mark.parametrize("m", [17, 129, 300])
+@pytest.mark.parametrize("inter,k", [(1, 8), (64, 72), (65, 200), (130, 576)])
+def test_gated(m, inter, k):
+    """silu(gate) * up in the epilogue, against 64 bits; an infinity among the sums of either."""
+    o = ops()
+    g = torch.Generator().manual_seed(m + 10 * inter + 100 * k)
+    a, w = torch.randn(m, k, generator=g), torch.randn(2 * inter, k, generator=g) / math.sqrt(k)
+    bias = torch.randn(2 * inter, generator=g)
+    z = a.double() @ w.double().T + bias
+    want = torch.nn.functional.silu(z[:, :inter]) * z[:, inter:]
+    room = torch.empty(m * inter + 1, device=DEV)
+    for shape in SHAPES:
+        for at in (0, 1):
+            out = room[at:at + m * inter].view(m, inter).fill_(float("nan"))
+            o.gemm_split_f32(a.to(DEV), w.to(DEV), bias.to(DEV), out, o.GEMM_GATED, shape)
+            assert off(out, want) < 2 * BOUND, (shape, at)  # (two sums, and expf's few units)
+    a[3, 0] = math.inf
+    z = a.double() @ w.double().T + bias
+    want = torch.nn.functional.silu(z[:, :inter]) * z[:, inter:]
+    o.gemm_split_f32(a.to(DEV), w.to(DEV), bias.to(DEV), out, o.GEMM_GATED)
+    want[3][torch.isneginf(z[3, :inter])] = math.nan  # (g / (1 + exp(-g)) of minus infinity, as the kernel for rows has it)
+    assert torch.equal(torch.isnan(out.cpu()), torch.isnan(want)) and torch.equal(torch.isinf(out.cpu()), torch.isinf(want))
+    o.check_status(DEV)
+
+
 @pytest.mark.parametrize("k", [576, 1536, 4096])
 def test_no_further_from_64_bits_than_chains_of_multiply_adds(k):
     o = ops()
