@@ -24,11 +24,14 @@
 //   memory_out     the outputs, all chunks side by side:
 //                  O_t = exp(m_before - M_t) S_before^T q_t + sum_{s <= t} exp(u_s - M_t) (q_t . k_s) v_s,
 //                  the denominator the same with n and without v.
+//   memory_chunk_split, memory_out_split: the two contractions by pairs of chunks on the tensor cores (chunk_read_split.cuh),
+//                  for heads of 64 or 128 keys.
 //   memory_finish  every head's o divided by its root mean square, times a weight per value, times
 //                  sigmoid(g), rounded once to the operand dtype.
 //
 // A row whose position is -1 (padding) is skipped.
 #include "async_copy.cuh"
+#include "chunk_read_split.cuh"
 #include "common.cuh"
 #include "row_quads.cuh"
 
@@ -226,7 +229,8 @@ memory_gates_kernel(const float* __restrict__ a, int a_cols, const float* __rest
     }
 }
 
-// A CTA of 256 threads per (chunk, head, 64 rows of dim x BV columns of vdim): 4 columns and BV / 16 rows a thread.
+// For the other sizes.  A CTA of 256 threads per (chunk, head, 64 rows of dim x BV columns of vdim): 4 columns and BV / 16 rows
+// a thread.
 template <int BV>
 __global__ void __launch_bounds__(256)
 memory_chunk_kernel(const float* __restrict__ a, int a_cols, const double* __restrict__ u,
@@ -301,13 +305,83 @@ memory_chunk_kernel(const float* __restrict__ a, int a_cols, const double* __res
     }
 }
 
+// Two neighbouring chunks of a sequence: blockIdx.x counts them through the sequences (more CTAs than pairs: none left).
+struct MemPair {
+    int seq, chunk, begin, first, count;  // of the first: chunk, token of the sequence in this step, row; tokens of both
+};
+__device__ __forceinline__ MemPair mem_pair(const int* seq_first_chunk, int n_seqs, const int* seq_first_row,
+                                            const int* seq_count) {
+    MemPair p;
+    int at = blockIdx.x;
+    for (p.seq = 0; p.seq < n_seqs; ++p.seq) {
+        const int c0 = seq_first_chunk[p.seq], n = (seq_first_chunk[p.seq + 1] - c0 + 1) / 2;
+        if (at < n) {
+            p.chunk = c0 + 2 * at;
+            p.begin = 2 * kMemChunk * at;
+            p.first = seq_first_row[p.seq] + p.begin;
+            p.count = min(2 * kMemChunk, seq_count[p.seq] - p.begin);
+            return p;
+        }
+        at -= n;
+    }
+    p.seq = -1;
+    return p;
+}
+// The largest u of a pair, counted from its first chunk's start.
+__device__ __forceinline__ double mem_pair_top(const double* ends, size_t at, int H, bool both) {
+    return both ? fmax(ends[at * 2 + 1], ends[(at + H) * 2 + 1] - ends[at * 2]) : ends[at * 2 + 1];
+}
+
+// memory_chunk_kernel on the tensor cores, two chunks and up to 256 columns a CTA: what both add, at the first one's place.
+// 3,701 tokens, four heads of 128 x 256: 46 -> 17 us, and memory_carry, with half the sums to walk, 11.6 -> 6.5 us.
+__global__ void __launch_bounds__(kCrThreads, 1)
+memory_chunk_split_kernel(const float* __restrict__ a, int a_cols, const double* __restrict__ u,
+                          const double* __restrict__ ends, const int* __restrict__ seq_first_chunk, int n_seqs,
+                          const int* __restrict__ seq_first_row, const int* __restrict__ seq_count,
+                          float* __restrict__ chunk_state, float* __restrict__ chunk_norm, int H, int dim, int vdim,
+                          int* __restrict__ status) {
+    constexpr int C = kMemChunk;
+    extern __shared__ __align__(1024) unsigned char sum_smem[];
+    __shared__ ChunkReadShared sh;
+    __shared__ float weight[2 * C];
+    const int h = blockIdx.y, v0 = blockIdx.z * kCrTiles * kCrCols, tid = threadIdx.x;
+    const MemPair pair = mem_pair(seq_first_chunk, n_seqs, seq_first_row, seq_count);
+    if (pair.seq < 0) return;
+    const size_t at = (size_t)pair.chunk * H + h;
+    const float* rows = a + (size_t)pair.first * a_cols;
+    ChunkReadRows g;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        g.k[i] = rows + (size_t)i * C * a_cols + (size_t)(H + h) * dim;
+        g.v[i] = rows + (size_t)i * C * a_cols + (size_t)2 * H * dim + (size_t)h * vdim + v0;
+    }
+    g.k_stride = g.v_stride = a_cols;
+    g.count = pair.count;
+    g.dim = dim;
+    g.cols = min(kCrTiles * kCrCols, vdim - v0);
+    chunk_sum_split(
+        g, v0 == 0 ? chunk_norm + at * dim : nullptr, sh, sum_smem, status,
+        [&] {
+            if (tid < 2 * C) {
+                const bool both = pair.count > C;
+                const double start = both && tid >= C ? ends[at * 2] : 0.0;
+                weight[tid] = tid < pair.count ? expf((float)(u[(size_t)(pair.first + tid) * H + h] - start -
+                                                              mem_pair_top(ends, at, H, both)))
+                                               : 0.f;
+            }
+            __syncthreads();
+        },
+        [&](int t) { return weight[t]; },
+        [&](int d, int c, const float* x) { store8(chunk_state + (at * dim + d) * vdim + v0 + c, x); });
+}
+
 // The running maximum from chunk to chunk of a sequence, in order (a warp per (sequence, head)): `before` of every chunk
-// but the first, the factors of the state before a chunk and of the chunk's own sum (`factors` float [n_chunks, H, 2]), and
-// the maximum that the step leaves.
+// but the first, the factors of the state before a chunk and of its own sum, or that of the pair it begins (`factors` float
+// [n_chunks, H, 2]; by = 1, 2 chunks a sum), and the maximum that the step leaves.
 __global__ void __launch_bounds__(32)
 memory_chain_kernel(const double* __restrict__ ends, double* before, float* __restrict__ factors,
                     float* __restrict__ max_state, const int* __restrict__ seq_slots, const int* __restrict__ seq_start,
-                    const int* __restrict__ seq_count, const int* __restrict__ seq_first_chunk, int H) {
+                    const int* __restrict__ seq_count, const int* __restrict__ seq_first_chunk, int H, int by) {
     const int seq = blockIdx.x, h = blockIdx.y, lane = threadIdx.x;
     const int c0 = seq_first_chunk[seq], c1 = seq_first_chunk[seq + 1];
     if (c1 <= c0) return;
@@ -322,23 +396,23 @@ memory_chain_kernel(const double* __restrict__ ends, double* before, float* __re
             m = fmax(m, __shfl_sync(0xffffffffu, u_max, j)) + __shfl_sync(0xffffffffu, b_end, j);
         }
         if (in) {
-            const double M = fmax(mine, u_max);
+            const double top = mem_pair_top(ends, at, H, by == 2 && c + lane + 1 < c1), M = fmax(mine, top);
             before[at] = mine;
             factors[at * 2] = expf((float)(mine - M));
-            factors[at * 2 + 1] = expf((float)(u_max - M));
+            factors[at * 2 + 1] = expf((float)(top - M));
         }
     }
     if (lane == 0)
         max_state[((size_t)seq_slots[seq] * 2 + ((seq_start[seq] + seq_count[seq]) & 1)) * H + h] = (float)m;
 }
 
-// A thread per V elements of S, then of n (V = 4 where dim and dim * vdim are multiples of four).
+// A thread per V elements of S, then of n (V = 4 where dim and dim * vdim are multiples of four), `by` chunks a sum.
 template <int V>
 __global__ void __launch_bounds__(256)
 memory_carry_kernel(float* chunk_state, float* chunk_norm, float* state, float* norm_state,
                     const float* __restrict__ factors, const int* __restrict__ seq_slots,
                     const int* __restrict__ seq_start, const int* __restrict__ seq_count,
-                    const int* __restrict__ seq_first_chunk, int H, int dim, int vdim) {
+                    const int* __restrict__ seq_first_chunk, int H, int dim, int vdim, int by) {
     constexpr int AHEAD = 8;
     struct alignas(4 * V) Pack { float x[V]; };
     const int seq = blockIdx.x, h = blockIdx.y, per = dim * vdim;
@@ -354,16 +428,16 @@ memory_carry_kernel(float* chunk_state, float* chunk_norm, float* state, float* 
                        : state + ((size_t)slot * H + h) * per + e;
     float* to = is_n ? norm_state + ((size_t)slot * 2 + (end & 1)) * H * dim + (size_t)h * dim + (e - per) : from;
     Pack run = *reinterpret_cast<const Pack*>(from);
-    for (int c = c0; c < c1; c += AHEAD) {
+    for (int c = c0; c < c1; c += AHEAD * by) {
         Pack add[AHEAD];
 #pragma unroll
         for (int j = 0; j < AHEAD; ++j)
-            if (c + j < c1) add[j] = *reinterpret_cast<const Pack*>(own + (size_t)(c - c0 + j) * step);
+            if (c + j * by < c1) add[j] = *reinterpret_cast<const Pack*>(own + (size_t)(c - c0 + j * by) * step);
 #pragma unroll
         for (int j = 0; j < AHEAD; ++j) {
-            if (c + j >= c1) break;
-            const float2 f = *reinterpret_cast<const float2*>(factors + ((size_t)(c + j) * H + h) * 2);
-            *reinterpret_cast<Pack*>(own + (size_t)(c - c0 + j) * step) = run;
+            if (c + j * by >= c1) break;
+            const float2 f = *reinterpret_cast<const float2*>(factors + ((size_t)(c + j * by) * H + h) * 2);
+            *reinterpret_cast<Pack*>(own + (size_t)(c - c0 + j * by) * step) = run;
 #pragma unroll
             for (int v = 0; v < V; ++v) run.x[v] = fmaf(f.x, run.x[v], f.y * add[j].x[v]);
         }
@@ -371,7 +445,7 @@ memory_carry_kernel(float* chunk_state, float* chunk_norm, float* state, float* 
     *reinterpret_cast<Pack*>(to) = run;
 }
 
-// A CTA of 256 threads per (chunk, head, BV columns of vdim).  Scores: 4 x 4 a thread; outputs: 4 columns and
+// For the other sizes.  A CTA of 256 threads per (chunk, head, BV columns of vdim).  Scores: 4 x 4 a thread; outputs: 4 columns and
 // BV / 16 rows a thread.
 template <int BV>
 __global__ void __launch_bounds__(256, 3)
@@ -532,6 +606,73 @@ memory_out_kernel(const float* __restrict__ a, int a_cols, const double* __restr
     }
 }
 
+// The same on the tensor cores, two neighbouring chunks of a sequence and `cols` columns a CTA.  With B the sum of the first
+// chunk's log forget gates, a token of the second sees the first one's keys with exp(u_s + B - M_t) and the state before the
+// first chunk with exp(m + B - M_t).  3,701 tokens, four heads of 128 x 256: 103 -> 35 us.
+__global__ void __launch_bounds__(kCrThreads, 1)
+memory_out_split_kernel(const float* __restrict__ a, int a_cols, const double* __restrict__ b, const double* __restrict__ u,
+                        const double* __restrict__ top, const double* __restrict__ ends, const double* __restrict__ before,
+                        const float* __restrict__ chunk_state, const float* __restrict__ chunk_norm,
+                        const int* __restrict__ seq_first_chunk, int n_seqs, const int* __restrict__ seq_first_row,
+                        const int* __restrict__ seq_start, const int* __restrict__ seq_count, float* __restrict__ o_raw,
+                        int H, int dim, int vdim, int cols, float q_scale, float floor_add, int* __restrict__ status) {
+    constexpr int C = kMemChunk;
+    extern __shared__ __align__(1024) unsigned char out_smem[];
+    __shared__ ChunkReadShared sh;
+    __shared__ double us[2 * C], Mt[2 * C];
+    __shared__ float carry[2 * C], least[2 * C];
+    const int h = blockIdx.y, v0 = blockIdx.z * cols, tid = threadIdx.x;
+    const MemPair pair = mem_pair(seq_first_chunk, n_seqs, seq_first_row, seq_count);
+    if (pair.seq < 0) return;
+    const int c = pair.chunk, first = pair.first, count = pair.count;
+    const bool fresh = pair.begin == 0 && seq_start[pair.seq] == 0;  // nothing before these chunks
+    const float* rows = a + (size_t)first * a_cols;
+    ChunkReadRows g;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        g.q[i] = rows + (size_t)i * C * a_cols + (size_t)h * dim;
+        g.k[i] = g.q[i] + (size_t)H * dim;
+        g.v[i] = rows + (size_t)i * C * a_cols + (size_t)2 * H * dim + (size_t)h * vdim + v0;
+    }
+    g.q_stride = g.k_stride = g.v_stride = a_cols;
+    g.state = fresh ? nullptr : chunk_state + ((size_t)c * H + h) * dim * vdim + v0;
+    g.state_stride = vdim;
+    g.count = count;
+    g.dim = dim;
+    g.cols = min(cols, vdim - v0);
+    g.q_scale = q_scale;
+    double first_sum = 0.0;
+    chunk_read_split(
+        g, fresh ? nullptr : chunk_norm + ((size_t)c * H + h) * dim, sh, out_smem, status,
+        [&] {
+            if (count > C) first_sum = ends[((size_t)c * H + h) * 2];
+            if (tid < 2 * C) {
+                us[tid] = Mt[tid] = 0.0;
+                carry[tid] = least[tid] = 0.f;
+                if (tid < count) {
+                    const size_t at = (size_t)(first + tid) * H + h;
+                    const double M = fmax(before[(size_t)(c + tid / C) * H + h], top[at]);
+                    us[tid] = u[at];
+                    Mt[tid] = M;
+                    carry[tid] = expf((float)(before[(size_t)c * H + h] + (tid < C ? 0.0 : first_sum) - M));
+                    least[tid] = expf((float)(-(b[at] + M)));
+                }
+            }
+            __syncthreads();
+        },
+        [&](int i, int j, float x) {
+            return x * expf((float)(us[j] + (i >= C && j < C ? first_sum : 0.0) - Mt[i]));
+        },
+        [&](int i) { return carry[i]; },
+        [&](int i, int col, const float* x, float sum, float dot) {
+            const float inv = 1.0f / (fmaxf(fabsf(fmaf(carry[i], dot, sum)), least[i]) + floor_add);
+            float o[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[e] = x[e] * inv;
+            store8(o_raw + ((size_t)(first + i) * H + h) * vdim + v0 + col, o);
+        });
+}
+
 // The finishing kernel for heads of a multiple of four values, at most 128 Q, with rows on 16-byte borders.
 template <typename T, int Q>
 __global__ void __launch_bounds__(256)
@@ -592,24 +733,48 @@ static cudaError_t launch_memory_prompt(const float* a, int a_cols, float* state
                                         const int* seq_slots, const int* seq_first_row, const int* seq_start,
                                         const int* seq_count, double* gates, double* chunk_gates, int n_tokens,
                                         float* chunk_state, float* chunk_norm, float* o_raw, int H, int dim, int vdim,
-                                        float q_scale, float floor_add, cudaStream_t stream) {
+                                        float q_scale, float floor_add, int sms, int* status, cudaStream_t stream) {
     double *b = gates, *u = gates + (size_t)n_tokens * H, *top = gates + (size_t)2 * n_tokens * H;
     double *ends = chunk_gates, *before = chunk_gates + (size_t)2 * n_chunks * H;
     const int v_tiles = (vdim + BV - 1) / BV, d_tiles = (dim + 63) / 64;
-    memory_chunk_kernel<BV><<<dim3(n_chunks, H, v_tiles * d_tiles), 256, 0, stream>>>(
-        a, a_cols, u, ends, chunks, seq_first_row, seq_count, chunk_state, chunk_norm, H, dim, vdim);
+    // Pairs of chunks on the tensor cores: heads of 64 or 128, rows on 32-byte boundaries, whole groups of eight columns.
+    const bool split = (dim == 64 || dim == 128) && vdim % 8 == 0 && a_cols % 8 == 0 &&
+                       ((uintptr_t)a | (uintptr_t)chunk_state | (uintptr_t)o_raw) % 32 == 0;
+    const int by = split ? 2 : 1, most_pairs = (n_chunks + n_seqs) / 2;
+    if (split) {
+        cudaError_t e = cudaFuncSetAttribute(memory_chunk_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCrSmem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(memory_out_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCrSmem);
+        if (e != cudaSuccess) return e;
+        memory_chunk_split_kernel<<<dim3(most_pairs, H, (vdim + kCrTiles * kCrCols - 1) / (kCrTiles * kCrCols)), kCrThreads,
+                                    kCrSmem, stream>>>(a, a_cols, u, ends, seq_first_chunk, n_seqs, seq_first_row,
+                                                       seq_count, chunk_state, chunk_norm, H, dim, vdim, status);
+    } else {
+        memory_chunk_kernel<BV><<<dim3(n_chunks, H, v_tiles * d_tiles), 256, 0, stream>>>(
+            a, a_cols, u, ends, chunks, seq_first_row, seq_count, chunk_state, chunk_norm, H, dim, vdim);
+    }
     float* factors = reinterpret_cast<float*>(chunk_gates + (size_t)3 * n_chunks * H);
     memory_chain_kernel<<<dim3(n_seqs, H), 32, 0, stream>>>(ends, before, factors, max_state, seq_slots, seq_start,
-                                                            seq_count, seq_first_chunk, H);
+                                                            seq_count, seq_first_chunk, H, by);
     const int elems = dim * vdim + dim;
     if (dim % 4 == 0)
         memory_carry_kernel<4><<<dim3(n_seqs, H, (elems / 4 + 255) / 256), 256, 0, stream>>>(
             chunk_state, chunk_norm, state, norm_state, factors, seq_slots, seq_start, seq_count, seq_first_chunk, H, dim,
-            vdim);
+            vdim, by);
     else
         memory_carry_kernel<1><<<dim3(n_seqs, H, (elems + 255) / 256), 256, 0, stream>>>(
             chunk_state, chunk_norm, state, norm_state, factors, seq_slots, seq_start, seq_count, seq_first_chunk, H, dim,
-            vdim);
+            vdim, by);
+    if (split) {
+        // two tiles of 128 columns a CTA split 14 blocks where two CTAs split 20: the fewer blocks of all waves
+        const long long pairs = (long long)most_pairs * H;
+        const auto cost = [&](int cols, int split) { return (pairs * ((vdim + cols - 1) / cols) + sms - 1) / sms * split; };
+        const int cols = vdim > kCrCols && cost(2 * kCrCols, 14) < cost(kCrCols, 10) ? 2 * kCrCols : kCrCols;
+        memory_out_split_kernel<<<dim3(most_pairs, H, (vdim + cols - 1) / cols), kCrThreads, kCrSmem, stream>>>(
+            a, a_cols, b, u, top, ends, before, chunk_state, chunk_norm, seq_first_chunk, n_seqs, seq_first_row, seq_start,
+            seq_count, o_raw, H, dim, vdim, cols, q_scale, floor_add, status);
+        return cudaGetLastError();
+    }
     const size_t smem = (size_t)(2 * 32 * (kMemChunk + 4) + kMemChunk * (kMemChunk + 4) + 32 * BV) * sizeof(float);
     auto kernel = memory_out_kernel<BV>;
     if (smem > 48 * 1024) {
@@ -669,7 +834,8 @@ NNIS_API int nnis_memory_prompt(const float* a, int a_cols, const float* i_bias,
                                 const int* seq_first_chunk, int n_seqs, const int* seq_slots, const int* seq_first_row,
                                 const int* seq_start, const int* seq_count, double* gates, double* chunk_gates,
                                 float* chunk_state, float* chunk_norm, float* o_raw, int n_tokens, int H, int dim,
-                                int vdim, float cap, float q_scale, float floor_add, cudaStream_t stream) {
+                                int vdim, float cap, float q_scale, float floor_add, int sms, int* status,
+                                cudaStream_t stream) {
     if (!a || !i_bias || !f_bias || !state || !norm_state || !max_state || !chunks || !seq_first_chunk || !seq_slots ||
         !seq_first_row || !seq_start || !seq_count || !gates || !chunk_gates || !chunk_state || !chunk_norm || !o_raw ||
         n_tokens <= 0 || n_chunks <= 0 || n_seqs <= 0 || H <= 0 || dim <= 0 || vdim <= 0 || !(cap > 0.f) ||
@@ -677,6 +843,7 @@ NNIS_API int nnis_memory_prompt(const float* a, int a_cols, const float* i_bias,
         return NNIS_ERR_ARGUMENT;
     const long long tiles = (long long)((dim + 63) / 64) * ((vdim + 63) / 64);
     if (H > 65535 || tiles > 65535 || ((long long)dim * vdim + dim + 255) / 256 > 65535) return NNIS_ERR_UNSUPPORTED;
+    if (sms <= 0) return NNIS_ERR_ARGUMENT;
     double *b = gates, *u = gates + (size_t)n_tokens * H, *top = gates + (size_t)2 * n_tokens * H;
     double *ends = chunk_gates, *before = chunk_gates + (size_t)2 * n_chunks * H;
     memory_gates_kernel<<<dim3(n_chunks, (H + 7) / 8), 256, 0, stream>>>(
@@ -685,10 +852,10 @@ NNIS_API int nnis_memory_prompt(const float* a, int a_cols, const float* i_bias,
     cudaError_t e = vdim > 64
         ? launch_memory_prompt<128>(a, a_cols, state, norm_state, max_state, chunks, n_chunks, seq_first_chunk, n_seqs,
                                     seq_slots, seq_first_row, seq_start, seq_count, gates, chunk_gates, n_tokens,
-                                    chunk_state, chunk_norm, o_raw, H, dim, vdim, q_scale, floor_add, stream)
+                                    chunk_state, chunk_norm, o_raw, H, dim, vdim, q_scale, floor_add, sms, status, stream)
         : launch_memory_prompt<64>(a, a_cols, state, norm_state, max_state, chunks, n_chunks, seq_first_chunk, n_seqs,
                                    seq_slots, seq_first_row, seq_start, seq_count, gates, chunk_gates, n_tokens,
-                                   chunk_state, chunk_norm, o_raw, H, dim, vdim, q_scale, floor_add, stream);
+                                   chunk_state, chunk_norm, o_raw, H, dim, vdim, q_scale, floor_add, sms, status, stream);
     return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 

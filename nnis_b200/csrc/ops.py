@@ -2609,7 +2609,7 @@ def memory_prompt(a: torch.Tensor, i_bias: torch.Tensor, f_bias: torch.Tensor, s
                                      _ptr(seq_first_row), _ptr(seq_start), _ptr(seq_count), _ptr(gates),
                                      _ptr(chunk_gates), _ptr(chunk_state), _ptr(chunk_norm), _ptr(o_raw), n, heads, dim,
                                      vdim, ctypes.c_float(cap), ctypes.c_float(q_scale), ctypes.c_float(floor),
-                                     _stream()), "memory_prompt", 5)
+                                     sm_count(a.device), _ptr(status_word(a.device)), _stream()), "memory_prompt", 5)
 
 
 def memory_finish(o_raw: torch.Tensor, a: torch.Tensor, gate_off: int, weight: torch.Tensor, token_pos: torch.Tensor,

@@ -212,6 +212,31 @@ def test_the_memory_in_every_cut(H, d, dv, cap):
     assert (o == 77.0).all() and all(torch.equal(x, y) for x, y in zip(before, (run.state, run.n, run.m)))
 
 
+@pytest.mark.parametrize("H, d, dv, cap", [(2, 64, 8, 12.0), (3, 128, 120, 15.0), (1, 128, 264, 15.0), (2, 64, 384, 9.0), (5, 128, 256, 15.0)])
+def test_the_memory_in_every_cut_in_pairs_of_chunks(H, d, dv, cap):
+    """Heads of 64 and 128 keys go to the tensor cores by pairs of chunks: columns that fill no tile, one, two, more."""
+    test_the_memory_in_every_cut(H, d, dv, cap)
+
+
+@pytest.mark.parametrize("bad", [math.inf, math.nan])
+def test_values_that_are_no_numbers_stay_in_their_column(bad):
+    H, d, dv, T = 2, 128, 256, 150
+    g = torch.Generator().manual_seed(3)
+    rows = memory_rows(T, H, d, dv, 4, g)
+    want, = MemoryRun(H, d, dv, 15.0, pad=4, seed=d).step([(0, rows)])
+    rows[70, 2 * H * d + dv + 200] = bad  # token 70, second head, column 200
+    run = MemoryRun(H, d, dv, 15.0, pad=4, seed=d)
+    got, = run.step([(0, rows)])
+    got, want = got.view(T, H, dv), want.view(T, H, dv)
+    assert not got[70:, 1, 200].isfinite().any()
+    got[70:, 1, 200] = want[70:, 1, 200] = 0.0
+    # (the columns that share a thread with it are made again in another order: what one rounding of sums of this size moves)
+    assert torch.allclose(got, want, rtol=1e-4, atol=1e-4)
+    assert not run.state[0, 1, :, 200].isfinite().any() and run.state[0, 0].isfinite().all()
+    run.state[0, 1, :, 200] = 0.0
+    assert run.state.isfinite().all()
+
+
 @pytest.mark.parametrize("i_size, f_centre, f_size, cap", [(6.0, -8.0, 4.0, 14.0), (9.0, 0.0, 9.0, 14.0), (0.2, 9.0, 1.0, 14.0),
                                                            (3.0, 30.0, 5.0, 40.0), (8.0, -30.0, 40.0, 12.0), (5.0, 3.0, 3.0, 0.5)])
 def test_the_memory_under_extreme_gates(i_size, f_centre, f_size, cap):
