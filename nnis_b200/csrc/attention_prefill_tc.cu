@@ -24,6 +24,10 @@
 //            128-byte-swizzled K-major layout the second product reads.  The halves
 //            have accumulators O of their own (the second product's first two
 //            K steps go to one, the last two to the other) and are merged at the end.
+// What bounds it: a softmax warp's chain through a page (wait, scores, maximum, 32 exponentials, fence, arrival: about 1,600
+// cycles with two CTAs on the SM, where the special function units need 1,024), and close behind it the second issuer's.
+// Scores are scaled and summed two at a time, and a wait that ran out is seen by the waits alone, not by a flag read each page:
+// 2,048 tokens of 9 heads 26.1 -> 25.4 us, 4,096 tokens 70.4 -> 66.2, 8,192 tokens 197 -> 184.
 // S and P are double-buffered.  O stays in tensor memory for the whole tile: the
 // maximum that P is taken against is only raised when a page's maximum exceeds it
 // by more than 8 (a factor 256, harmless in float32 and bfloat16); then the warp
@@ -39,6 +43,7 @@
 // NNIS has a batched causal kernel on CUDA cores (crates/nnis-kernels/src/attention.rs:46-150).
 #include <float.h>
 
+#include "fma_pairs.cuh"
 #include "tcgen05_helpers.cuh"
 
 namespace nnis {
@@ -299,7 +304,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         bool ok = true;
         for (int i = 0; i < n_pages; ++i) {
             const int b = i & 1;
-            ok = warp_wait(&s_full[b], (uint32_t)(i >> 1) & 1u, lane) && !abort_flag;
+            ok = warp_wait(&s_full[b], (uint32_t)(i >> 1) & 1u, lane);
             if (!ok) break;
             tc_fence_after();
             uint32_t sv[32];
@@ -340,10 +345,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 l_run *= alpha;
                 m_run = m_new;
             }
-            const float neg_base = m_run == -INFINITY ? 0.f : -m_run;
+            const unsigned long long neg_base = both(m_run == -INFINITY ? 0.f : -m_run);
             // (the product that read this buffer of P two pages ago is over: s_full said so)
             unsigned char* p_row = p_s + (size_t)b * kBytesQ + (size_t)row * 128;
-            float ps[4] = {0.f, 0.f, 0.f, 0.f};
+            unsigned long long ps[2] = {0ull, 0ull};
             // P row: 8 chunks of 8 keys, four of them this thread's; chunk j lands at
             // 16-byte slot j ^ (row % 8)
 #pragma unroll
@@ -352,16 +357,18 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     int c = j * 8 + e * 2;
-                    float p0 = ex2(fmaf(__uint_as_float(sv[c]), sc, neg_base));
-                    float p1 = ex2(fmaf(__uint_as_float(sv[c + 1]), sc, neg_base));
-                    ps[e] += p0 + p1;
+                    unsigned long long at = neg_base;
+                    fma2(at, pair_of(__uint_as_float(sv[c]), __uint_as_float(sv[c + 1])), both(sc));
+                    const float p0 = ex2(halves(at).x), p1 = ex2(halves(at).y);
+                    ps[e & 1] = add2(ps[e & 1], pair_of(p0, p1));
                     __nv_bfloat162 pk = __floats2bfloat162_rn(p0, p1);
                     w[e] = *reinterpret_cast<uint32_t*>(&pk);
                 }
                 *reinterpret_cast<uint4*>(p_row + (((half * 4 + j) ^ (row & 7)) << 4)) =
                     make_uint4(w[0], w[1], w[2], w[3]);
             }
-            l_run += (ps[0] + ps[1]) + (ps[2] + ps[3]);
+            const float2 s0 = halves(ps[0]), s1 = halves(ps[1]);
+            l_run += (s0.x + s0.y) + (s1.x + s1.y);
             fence_async_smem();  // the tensor core reads P through the async proxy
             tc_fence_before();   // and a rescaled O through tensor memory
             __syncwarp();
@@ -440,22 +447,33 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 }
                 if (warp_wait(&last_known, 0, lane) && is_last_chunk && !abort_flag) {
                     __threadfence();
+                    // (all that a chunk holds of the row is asked for at once: each trip to L2 counts here, as the tile's
+                    // other chunks are over)
+                    const float* of = tile_partial + (size_t)kTcD * kTcRows;
                     float m_tile = -INFINITY;
-                    for (int c = 0; c < n_chunks; ++c)
-                        m_tile = fmaxf(m_tile, __ldcg(tile_partial + (size_t)c * per_chunk_floats + (size_t)kTcD * kTcRows));
+                    for (int c0 = 0; c0 < n_chunks; c0 += 4) {
+                        float mc[4];
+#pragma unroll
+                        for (int c = 0; c < 4; ++c)
+                            mc[c] = c0 + c < n_chunks ? __ldcg(of + (size_t)(c0 + c) * per_chunk_floats) : -INFINITY;
+                        m_tile = fmaxf(fmaxf(m_tile, fmaxf(mc[0], mc[1])), fmaxf(mc[2], mc[3]));
+                    }
                     float acc[32];
 #pragma unroll
                     for (int j = 0; j < 32; ++j) acc[j] = 0.f;
                     float l_tile = 0.f;
                     for (int c = 0; c < n_chunks; ++c) {
                         const float* src = tile_partial + (size_t)c * per_chunk_floats;
+                        float x[32];
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) x[j] = __ldcg(src + (size_t)(half * 32 + j) * kTcRows);
+                        const float lc = __ldcg(src + (size_t)(kTcD + 1) * kTcRows);
                         const float mc = __ldcg(src + (size_t)kTcD * kTcRows);
                         if (mc == -INFINITY) continue;  // no key of this chunk was visible to the row
                         const float wc = exp2f(mc - m_tile);
-                        l_tile = fmaf(wc, __ldcg(src + (size_t)(kTcD + 1) * kTcRows), l_tile);
+                        l_tile = fmaf(wc, lc, l_tile);
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            acc[j] = fmaf(wc, __ldcg(src + (size_t)(half * 32 + j) * kTcRows), acc[j]);
+                        for (int j = 0; j < 32; ++j) acc[j] = fmaf(wc, x[j], acc[j]);
                     }
                     const float inv = l_tile > 0.f ? 1.0f / l_tile : 0.f;
                     if (row < rows) {
