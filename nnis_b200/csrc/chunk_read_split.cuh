@@ -44,6 +44,47 @@ struct ChunkReadShared {
 
 __device__ __forceinline__ void chunk_workers_meet() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kCrWorkers) : "memory"); }
 
+// Two neighbouring chunks of a sequence: `at` counts such pairs through the sequences, whose first chunks `first` [n_seqs + 1]
+// names.  seq = -1: there are fewer.  Each warp looks through 32 sequences at a time.
+struct ChunkPair {
+    int seq, chunk;
+};
+__device__ __forceinline__ ChunkPair find_chunk_pair(const int* first, int n_seqs, int at) {
+    const int lane = threadIdx.x & 31;
+    for (int s0 = 0; s0 < n_seqs; s0 += 32) {
+        int c0 = 0, pairs = 0;
+        if (s0 + lane < n_seqs) {
+            c0 = first[s0 + lane];
+            pairs = (first[s0 + lane + 1] - c0 + 1) / 2;
+        }
+        int to = pairs;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, to, o);
+            if (lane >= o) to += x;
+        }
+        const unsigned past = __ballot_sync(0xffffffffu, at < to);
+        if (past) {
+            const int l = __ffs(past) - 1;
+            return {s0 + l, __shfl_sync(0xffffffffu, c0 + 2 * (at - (to - pairs)), l)};
+        }
+        at -= __shfl_sync(0xffffffffu, to, 31);
+    }
+    return {-1, 0};
+}
+__device__ __forceinline__ int chunk_pairs_before(const int* first, int seq) {
+    int n = 0;
+    for (int s = threadIdx.x & 31; s < seq; s += 32) n += (first[s + 1] - first[s] + 1) / 2;
+    return __reduce_add_sync(0xffffffffu, n);
+}
+
+// Columns of a CTA that reads: two tiles of 128 split 14 blocks of 128 x 64 where two CTAs split 20, and the fewer of all waves
+// of CTAs, one to an SM, is faster (four heads of 256 columns: 120 CTAs 35 us, 240 CTAs 42 us).
+inline int chunk_read_cols(long long pairs, int vdim, int sms) {
+    const auto cost = [&](int cols, int split) { return (pairs * ((vdim + cols - 1) / cols) + sms - 1) / sms * split; };
+    return vdim > kCrCols && cost(2 * kCrCols, 14) < cost(kCrCols, 10) ? 2 * kCrCols : kCrCols;
+}
+
 // B of 64 rows x 128 columns as it lies (rows of 128 bytes, two runs of 64 columns 8 KB apart), read MN-major.
 __device__ __forceinline__ uint64_t chunk_desc_mn(uint32_t smem_byte_addr) {
     uint64_t desc = smem_desc_mn128(smem_byte_addr);

@@ -305,26 +305,17 @@ memory_chunk_kernel(const float* __restrict__ a, int a_cols, const double* __res
     }
 }
 
-// Two neighbouring chunks of a sequence: blockIdx.x counts them through the sequences (more CTAs than pairs: none left).
 struct MemPair {
-    int seq, chunk, begin, first, count;  // of the first: chunk, token of the sequence in this step, row; tokens of both
+    int seq, chunk, begin, first, count;  // of the first chunk: token of the sequence in this step, row; tokens of both
 };
 __device__ __forceinline__ MemPair mem_pair(const int* seq_first_chunk, int n_seqs, const int* seq_first_row,
                                             const int* seq_count) {
-    MemPair p;
-    int at = blockIdx.x;
-    for (p.seq = 0; p.seq < n_seqs; ++p.seq) {
-        const int c0 = seq_first_chunk[p.seq], n = (seq_first_chunk[p.seq + 1] - c0 + 1) / 2;
-        if (at < n) {
-            p.chunk = c0 + 2 * at;
-            p.begin = 2 * kMemChunk * at;
-            p.first = seq_first_row[p.seq] + p.begin;
-            p.count = min(2 * kMemChunk, seq_count[p.seq] - p.begin);
-            return p;
-        }
-        at -= n;
-    }
-    p.seq = -1;
+    const ChunkPair at = find_chunk_pair(seq_first_chunk, n_seqs, blockIdx.x);
+    MemPair p = {at.seq, at.chunk, 0, 0, 0};
+    if (p.seq < 0) return p;
+    p.begin = (p.chunk - seq_first_chunk[p.seq]) * kMemChunk;
+    p.first = seq_first_row[p.seq] + p.begin;
+    p.count = min(2 * kMemChunk, seq_count[p.seq] - p.begin);
     return p;
 }
 // The largest u of a pair, counted from its first chunk's start.
@@ -766,10 +757,7 @@ static cudaError_t launch_memory_prompt(const float* a, int a_cols, float* state
             chunk_state, chunk_norm, state, norm_state, factors, seq_slots, seq_start, seq_count, seq_first_chunk, H, dim,
             vdim, by);
     if (split) {
-        // two tiles of 128 columns a CTA split 14 blocks where two CTAs split 20: the fewer blocks of all waves
-        const long long pairs = (long long)most_pairs * H;
-        const auto cost = [&](int cols, int split) { return (pairs * ((vdim + cols - 1) / cols) + sms - 1) / sms * split; };
-        const int cols = vdim > kCrCols && cost(2 * kCrCols, 14) < cost(kCrCols, 10) ? 2 * kCrCols : kCrCols;
+        const int cols = chunk_read_cols((long long)most_pairs * H, vdim, sms);
         memory_out_split_kernel<<<dim3(most_pairs, H, (vdim + cols - 1) / cols), kCrThreads, kCrSmem, stream>>>(
             a, a_cols, b, u, top, ends, before, chunk_state, chunk_norm, seq_first_chunk, n_seqs, seq_first_row, seq_start,
             seq_count, o_raw, H, dim, vdim, cols, q_scale, floor_add, status);

@@ -1539,7 +1539,8 @@ def retention(qkvg: torch.Tensor, freq: torch.Tensor, decay: torch.Tensor, state
                                  _ptr(chunk_state), _ptr(o_raw), _ptr(out), n, units, heads, dim, vdim,
                                  rot_dims, ctypes.c_float(eps), 1 if activation else 0,
                                  ctypes.c_float(dim ** -0.5 if key_scale is None else key_scale),
-                                 _ptr(norm_weight), 1 if gate == "sigmoid" else 0, code_of(out.dtype), _stream()),
+                                 _ptr(norm_weight), 1 if gate == "sigmoid" else 0, code_of(out.dtype),
+                                 sm_count(out.device), _ptr(status_word(out.device)), _stream()),
            "retention", 4 * -(-n_chunks // wave) + 1 if chunks is not None else 2)
 
 

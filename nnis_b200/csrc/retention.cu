@@ -21,6 +21,7 @@
 //
 // Packed input rows: [q (H dim) | k (H dim) | v (H vdim) | g (H vdim)].
 #include "async_copy.cuh"
+#include "chunk_read_split.cuh"
 #include "common.cuh"
 #include "linear_chunks.cuh"
 #include "row_quads.cuh"
@@ -278,7 +279,7 @@ retention_in_order_kernel(const T* __restrict__ qkvg, const float* __restrict__ 
         if (live) S[(size_t)d * vdim + col] = Ss[d * 32 + lane];
 }
 
-// Longer prompts: the same a chunk of 64 tokens at a time, chunks side by side, all in float32 on the CUDA cores.  Four kernels: `pack` turns q, k and v of every (chunk, head) into the layouts that
+// Longer prompts: the same a chunk of 64 tokens at a time, chunks side by side, all in float32.  Four kernels: `pack` turns q, k and v of every (chunk, head) into the layouts that
 // the products read (rotated once, not once per tile of columns); `update` makes what every chunk adds to the state, all
 // chunks side by side; `carry` walks a sequence's chunks in order and leaves the state before each of them, and the
 // slot's state; `read` makes the outputs, all chunks side by side.  The products are linear_chunks.cuh's.  More chunks
@@ -286,7 +287,8 @@ retention_in_order_kernel(const T* __restrict__ qkvg, const float* __restrict__ 
 // state is float32 there too).
 // Before, chunks of 32 in runs of 256 tokens from zero, 32 columns a CTA with A made again for each, 2 x 2 entries of A
 // and 4 x 1 of the output a thread, took 495 us for 2,048 tokens and 8 heads of 128 x 256 on a B200 (chunk 351, prefix
-// 30, carry 114); now 143 (pack 39, update 25, carry 12, read 68: 22 TFLOP/s of multiply-adds).
+// 30, carry 114); these kernels 143 (pack 37, update 25, carry 12, read 66: 22 TFLOP/s of multiply-adds on the CUDA cores).
+// Keys of 64 and 128 have `update` and `read` on the tensor cores, by pairs of chunks (below): 70.
 
 // A packed (chunk, head): queries [dim][64], keys [dim][64], keys times g^(C-1-j) [64][dim], values [64][vp].
 __host__ __device__ __forceinline__ size_t packed_floats(int dim, int vp) {
@@ -389,24 +391,35 @@ retention_update_kernel(const float* __restrict__ packed, float* __restrict__ ch
                           (int)(blockIdx.z / v_tiles) * 64, (int)(blockIdx.z % v_tiles) * BV, update_smem);
 }
 
+// The chunk at which the scratch of a wave of pairs begins.
+__device__ __forceinline__ int wave_chunk(const int* seq_first_chunk, int n_seqs, int pair0) {
+    return pair0 ? find_chunk_pair(seq_first_chunk, n_seqs, pair0).chunk : 0;
+}
+
 // The state before every chunk in place of what the chunk adds, in order, a thread per four values of a row, eight
 // chunks fetched ahead; the state after the last goes to the slot (whose rows have vdim values and no alignment).  The
-// wave's chunks: `wave_n` from `wave0` on, the first of which chunk_state begins with.
+// wave's chunks: `wave_n` from `wave0` on, the first of which chunk_state begins with; `by` = 2: pairs of chunks, each of which
+// has added as one.
 __global__ void __launch_bounds__(128)
 retention_carry_kernel(float* chunk_state, float* state, const float* __restrict__ decay,
                        const int* __restrict__ seq_slots, const int* __restrict__ seq_start,
                        const int* __restrict__ seq_count, const int* __restrict__ seq_first_chunk, int wave0, int wave_n,
-                       int heads, int dim, int vdim, int vp) {
+                       int heads, int dim, int vdim, int vp, int by) {
     constexpr int AHEAD = 8;
     pdl_wait();
     pdl_launch_dependents();
     const int seq = blockIdx.x, h = blockIdx.y, quads = vp >> 2;
     const int e = blockIdx.z * 128 + threadIdx.x;
-    if (e >= dim * quads) return;
     const int d = e / quads, j = (e - d * quads) * 4;
     const int begin = seq_first_chunk[seq], end = seq_first_chunk[seq + 1], count = seq_count[seq];
-    const int c0 = max(begin, wave0), c1 = min(end, wave0 + wave_n);
-    if (c1 <= c0) return;
+    int base = wave0, c0 = max(begin, wave0), c1 = min(end, wave0 + wave_n);
+    if (by == 2) {
+        const int pairs = chunk_pairs_before(seq_first_chunk, seq);
+        base = wave_chunk(seq_first_chunk, gridDim.x, wave0);
+        c0 = begin + 2 * max(wave0 - pairs, 0);
+        c1 = min(end, begin + 2 * max(wave0 + wave_n - pairs, 0));
+    }
+    if (c1 <= c0 || e >= dim * quads) return;
     const float g = decay[h];
     float g_chunk = 1.f, g_last = 1.f;  // as decay_powers makes them
     const int last = count - (end - begin - 1) * kChunkTokens;
@@ -414,22 +427,23 @@ retention_carry_kernel(float* chunk_state, float* state, const float* __restrict
         g_chunk *= g;
         if (n < last) g_last *= g;
     }
-    float* own = chunk_state + ((size_t)(c0 - wave0) * heads + h) * dim * vp + (size_t)d * vp + j;
+    float* own = chunk_state + ((size_t)(c0 - base) * heads + h) * dim * vp + (size_t)d * vp + j;
     const size_t step = (size_t)heads * dim * vp;
     float* slot = state + ((size_t)seq_slots[seq] * heads + h) * dim * vdim + (size_t)d * vdim + j;
     float run[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) run[v] = j + v < vdim ? slot[v] : 0.f;
-    for (int c = c0; c < c1; c += AHEAD) {
+    for (int c = c0; c < c1; c += AHEAD * by) {
         float4 add[AHEAD];
 #pragma unroll
         for (int k = 0; k < AHEAD; ++k)
-            if (c + k < c1) add[k] = load4(own + (size_t)(c - c0 + k) * step);
+            if (c + k * by < c1) add[k] = load4(own + (size_t)(c - c0 + k * by) * step);
 #pragma unroll
         for (int k = 0; k < AHEAD; ++k) {
-            if (c + k >= c1) break;
-            store4(own + (size_t)(c - c0 + k) * step, make_float4(run[0], run[1], run[2], run[3]));
-            const float f = c + k == end - 1 ? g_last : g_chunk;
+            const int at = c + k * by, past = min(at + by, c1);
+            if (at >= c1) break;
+            store4(own + (size_t)(at - c0) * step, make_float4(run[0], run[1], run[2], run[3]));
+            const float f = (past == end ? g_last : g_chunk) * (past - at == 2 ? g_chunk : 1.f);
             run[0] = fmaf(f, run[0], add[k].x);
             run[1] = fmaf(f, run[1], add[k].y);
             run[2] = fmaf(f, run[2], add[k].z);
@@ -484,12 +498,186 @@ retention_read_kernel(const float* __restrict__ packed, const float* __restrict_
     }
 }
 
+// Keys of 64 and 128, 64 values and more in whole groups of eight: `update` and `read` by pairs of chunks on the tensor cores
+// (with fewer values most of a tile of 128 columns would be padding).  A wave holds whole pairs, so that results have the same
+// bits however many fit it; its first chunk is the one at which the scratch begins.  A packed
+// (chunk, head) is then queries [64][dim], keys [64][dim] and values [64][vdim], rows of tokens that are not there left alone;
+// four CTAs a (chunk, head), 16 tokens each: 2,048 tokens, eight heads of 128 x 256, 37 -> 16 us (three layouts and powers of the
+// decay made by one thread before).
+template <typename T>
+__global__ void __launch_bounds__(256)
+retention_pack_rows_kernel(const T* __restrict__ qkvg, const float* __restrict__ freq, const int* __restrict__ chunks,
+                           const int* __restrict__ seq_first_row, const int* __restrict__ seq_start,
+                           const int* __restrict__ seq_count, float* __restrict__ packed, int heads, int dim, int vdim,
+                           int rot_dims, int act, float k_scale, const int* __restrict__ seq_first_chunk, int n_seqs,
+                           int pair0) {
+    pdl_wait();
+    pdl_launch_dependents();
+    constexpr int TOKENS = kChunkTokens / 4;
+    const int h = blockIdx.y, t0 = blockIdx.z * TOKENS, tid = threadIdx.x;
+    const ChunkPair pair = find_chunk_pair(seq_first_chunk, n_seqs, pair0 + (int)blockIdx.x / 2);
+    const int c = pair.chunk + (int)(blockIdx.x & 1);
+    if (pair.seq < 0 || c >= seq_first_chunk[pair.seq + 1]) return;
+    const size_t unit = (size_t)(c - wave_chunk(seq_first_chunk, n_seqs, pair0)) * heads + h;
+    const RetChunk ch = ret_chunk(chunks, seq_first_row, seq_start, seq_count, c);
+    const int there = min(TOKENS, ch.count - t0);
+    if (there <= 0) return;
+    const size_t row_len = (size_t)2 * heads * (dim + vdim);
+    const T* q = qkvg + (size_t)(ch.first + t0) * row_len + (size_t)h * dim;
+    const T* k = q + (size_t)heads * dim;
+    const T* v = qkvg + (size_t)(ch.first + t0) * row_len + (size_t)2 * heads * dim + (size_t)h * vdim;
+    float* qt = packed + unit * packed_floats(dim, vdim) + (size_t)t0 * dim;
+    float* kt = qt + (size_t)kChunkTokens * dim;
+    float* vt = qt + (size_t)2 * kChunkTokens * dim - (size_t)t0 * dim + (size_t)t0 * vdim;
+    const int half = rot_dims >> 1, rest = dim - rot_dims;
+    for (int it = tid; it < there * half; it += 256) {
+        const int t = it / half, j = it - t * half;
+        const T *qr = q + t * row_len + j, *kr = k + t * row_len + j;
+        const float q0 = pre(qr[0], act), q1 = pre(qr[half], act);
+        const float k0 = pre(kr[0], act) * k_scale, k1 = pre(kr[half], act) * k_scale;
+        const float ang = (float)(ch.start + t0 + t) * freq[j];
+        const float c = cosf(ang), sn = sinf(ang);
+        qt[t * dim + j] = q0 * c - q1 * sn;
+        qt[t * dim + j + half] = q1 * c + q0 * sn;
+        kt[t * dim + j] = k0 * c - k1 * sn;
+        kt[t * dim + j + half] = k1 * c + k0 * sn;
+    }
+    for (int it = tid; it < there * rest; it += 256) {
+        const int t = it / rest, j = rot_dims + it - t * rest;
+        qt[t * dim + j] = pre(q[t * row_len + j], act);
+        kt[t * dim + j] = pre(k[t * row_len + j], act) * k_scale;
+    }
+    const int quads = vdim >> 2;
+    for (int it = tid; it < there * quads; it += 256) {
+        const int t = it / quads, j = (it - t * quads) * 4;
+        float4 x = load4(v + t * row_len + j);
+        if (act) x = make_float4(pre(x.x, 1), pre(x.y, 1), pre(x.z, 1), pre(x.w, 1));
+        store4(vt + (size_t)t * vdim + j, x);
+    }
+}
+
+struct RetPair {
+    int seq, first, start, count;  // of the first chunk: row, position; tokens of both
+    ChunkReadRows rows;
+};
+__device__ __forceinline__ RetPair ret_pair(const float* packed, const int* seq_first_chunk, int n_seqs, int pair0, const int* seq_first_row,
+                                            const int* seq_start, const int* seq_count, int heads,
+                                            int dim, int vdim, int cols, size_t& unit) {
+    const ChunkPair at = find_chunk_pair(seq_first_chunk, n_seqs, pair0 + (int)blockIdx.x);
+    RetPair p;
+    p.seq = at.seq;
+    if (at.seq < 0) return p;
+    const int begin = (at.chunk - seq_first_chunk[at.seq]) * kChunkTokens, v0 = blockIdx.z * cols;
+    p.first = seq_first_row[at.seq] + begin;
+    p.start = seq_start[at.seq] + begin;
+    p.count = min(2 * kChunkTokens, seq_count[at.seq] - begin);
+    unit = (size_t)(at.chunk - wave_chunk(seq_first_chunk, n_seqs, pair0)) * heads + blockIdx.y;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        p.rows.q[i] = packed + (unit + (size_t)i * heads) * packed_floats(dim, vdim);
+        p.rows.k[i] = p.rows.q[i] + (size_t)kChunkTokens * dim;
+        p.rows.v[i] = p.rows.k[i] + (size_t)kChunkTokens * dim + v0;
+    }
+    p.rows.q_stride = p.rows.k_stride = dim;
+    p.rows.v_stride = p.rows.state_stride = vdim;
+    p.rows.state = nullptr;
+    p.rows.count = p.count;
+    p.rows.dim = dim;
+    p.rows.cols = min(cols, vdim - v0);
+    p.rows.q_scale = 1.f;
+    return p;
+}
+// g^0 .. g^128: the second chunk's as what a state that passes the first one's end is multiplied by
+__device__ __forceinline__ void decay_powers_of_pairs(float g, float* pw) {
+    decay_powers(g, pw);
+    if (threadIdx.x > 0 && threadIdx.x <= kChunkTokens) pw[kChunkTokens + threadIdx.x] = pw[kChunkTokens] * pw[threadIdx.x];
+    __syncthreads();
+}
+
+// 2,048 tokens, eight heads of 128 x 256: 25 -> 16 us, and retention_carry, with half the sums to walk, 12 -> 8 us.
+__global__ void __launch_bounds__(kCrThreads, 1)
+retention_update_split_kernel(const float* __restrict__ packed, float* __restrict__ chunk_state,
+                              const float* __restrict__ decay, const int* __restrict__ seq_first_chunk, int n_seqs,
+                              int pair0, const int* __restrict__ seq_first_row,
+                              const int* __restrict__ seq_start, const int* __restrict__ seq_count, int heads, int dim,
+                              int vdim, int* __restrict__ status) {
+    extern __shared__ __align__(1024) unsigned char sum_smem[];
+    __shared__ ChunkReadShared sh;
+    __shared__ float pw[2 * kChunkTokens + 1];
+    pdl_wait();
+    pdl_launch_dependents();
+    constexpr int COLS = kCrTiles * kCrCols;
+    size_t unit = 0;
+    const RetPair p = ret_pair(packed, seq_first_chunk, n_seqs, pair0, seq_first_row, seq_start, seq_count, heads, dim, vdim,
+                               COLS, unit);
+    if (p.seq < 0) return;
+    float* to = chunk_state + unit * dim * vdim + blockIdx.z * COLS;
+    chunk_sum_split(
+        p.rows, nullptr, sh, sum_smem, status, [&] { decay_powers_of_pairs(decay[blockIdx.y], pw); },
+        [&](int t) { return t < p.count ? pw[p.count - 1 - t] : 0.f; },
+        [&](int d, int c, const float* x) { store8(to + (size_t)d * vdim + c, x); });
+}
+
+// 2,048 tokens, eight heads of 128 x 256: 66 -> 30 us.
+__global__ void __launch_bounds__(kCrThreads, 1)
+retention_read_split_kernel(const float* __restrict__ packed, const float* __restrict__ chunk_state,
+                            const float* __restrict__ decay, const int* __restrict__ seq_first_chunk, int n_seqs, int pair0,
+                            const int* __restrict__ seq_first_row, const int* __restrict__ seq_start,
+                            const int* __restrict__ seq_count, float* __restrict__ o_raw, int heads, int dim, int vdim,
+                            int cols, int* __restrict__ status) {
+    extern __shared__ __align__(1024) unsigned char read_smem_split[];
+    __shared__ ChunkReadShared sh;
+    __shared__ float pw[2 * kChunkTokens + 1];
+    pdl_wait();
+    pdl_launch_dependents();
+    size_t unit = 0;
+    RetPair p = ret_pair(packed, seq_first_chunk, n_seqs, pair0, seq_first_row, seq_start, seq_count, heads, dim, vdim, cols,
+                         unit);
+    if (p.seq < 0) return;
+    const int h = blockIdx.y, v0 = blockIdx.z * cols;
+    if (p.start > 0) p.rows.state = chunk_state + unit * dim * vdim + v0;
+    chunk_read_split(
+        p.rows, nullptr, sh, read_smem_split, status, [&] { decay_powers_of_pairs(decay[h], pw); },
+        [&](int i, int j, float x) { return x * pw[i - j]; }, [&](int i) { return pw[i + 1]; },
+        [&](int i, int c, const float* x, float, float) {
+            store8(o_raw + ((size_t)(p.first + i) * heads + h) * vdim + v0 + c, x);
+        });
+}
+
 template <typename T>
 static int launch_chunks(const T* qkvg, const float* freq, const float* decay, float* state, const int* seq_slots,
                          const int* seq_first_row, const int* seq_start, const int* seq_count, const int* chunks,
                          int n_chunks, const int* seq_first_chunk, int wave, float* packed, float* chunk_state, float* o_raw,
-                         int n_seqs, int heads, int dim, int vdim, int rot_dims, int act, float k_scale,
+                         int n_seqs, int heads, int dim, int vdim, int rot_dims, int act, float k_scale, int sms, int* status,
                          cudaStream_t stream) {
+    // (rows of q, k and v in whole groups of eight on 16-byte borders, float32 rows on 32-byte borders)
+    if ((dim == 64 || dim == 128) && vdim >= 64 && vdim % 8 == 0 && (wave >= 2 || n_chunks == 1) && (uintptr_t)qkvg % 16 == 0 &&
+        ((uintptr_t)packed | (uintptr_t)chunk_state | (uintptr_t)o_raw) % 32 == 0) {
+        cudaError_t e = cudaFuncSetAttribute(retention_update_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCrSmem);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(retention_read_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCrSmem);
+        const int all = (n_chunks + n_seqs) / 2, most = kCrTiles * kCrCols;  // pairs: at most as many
+        const int held = n_chunks <= wave ? all : wave / 2;
+        for (int p0 = 0; p0 < all && e == cudaSuccess; p0 += held) {
+            const int n = all - p0 < held ? all - p0 : held, cols = chunk_read_cols((long long)n * heads, vdim, sms);
+            e = launch_dependent(retention_pack_rows_kernel<T>, dim3(2 * n, heads, 4), 256, 0, stream, qkvg, freq, chunks,
+                                 seq_first_row, seq_start, seq_count, packed, heads, dim, vdim, rot_dims, act, k_scale,
+                                 seq_first_chunk, n_seqs, p0);
+            if (e == cudaSuccess)
+                e = launch_dependent(retention_update_split_kernel, dim3(n, heads, (vdim + most - 1) / most), kCrThreads,
+                                     kCrSmem, stream, (const float*)packed, chunk_state, decay, seq_first_chunk, n_seqs, p0,
+                                     seq_first_row, seq_start, seq_count, heads, dim, vdim, status);
+            if (e == cudaSuccess)
+                e = launch_dependent(retention_carry_kernel, dim3(n_seqs, heads, (dim * (vdim / 4) + 127) / 128), 128, 0,
+                                     stream, chunk_state, state, decay, seq_slots, seq_start, seq_count, seq_first_chunk, p0,
+                                     n, heads, dim, vdim, vdim, 2);
+            if (e == cudaSuccess)
+                e = launch_dependent(retention_read_split_kernel, dim3(n, heads, (vdim + cols - 1) / cols), kCrThreads,
+                                     kCrSmem, stream, (const float*)packed, (const float*)chunk_state, decay, seq_first_chunk,
+                                     n_seqs, p0, seq_first_row, seq_start, seq_count, o_raw, heads, dim, vdim, cols, status);
+        }
+        return e == cudaSuccess ? NNIS_OK : (int)e;
+    }
     const int vp = (vdim + 3) & ~3, bv = vp > 64 ? 128 : 64;
     const int pack_smem = 2 * kChunkTokens * (dim + 1) * 4, update_smem = kChunkTokens * (64 + bv) * 4;
     const int read_smem = (bv == 128 ? chunk_read_floats<128>() : chunk_read_floats<64>()) * 4;
@@ -510,7 +698,7 @@ static int launch_chunks(const T* qkvg, const float* freq, const float* decay, f
         if (e == cudaSuccess)
             e = launch_dependent(retention_carry_kernel, dim3(n_seqs, heads, (dim * (vp / 4) + 127) / 128), 128, 0, stream,
                                  chunk_state, state, decay, seq_slots, seq_start, seq_count, seq_first_chunk, c0, n, heads,
-                                 dim, vdim, vp);
+                                 dim, vdim, vp, 1);
         if (e == cudaSuccess)
             e = launch_dependent(read, dim3(n, heads, v_tiles), 128, read_smem, stream, (const float*)packed,
                                  (const float*)chunk_state, decay, own, seq_first_row, seq_start, seq_count, o_raw, heads,
@@ -629,13 +817,13 @@ static int launch_retention(const void* qkvg, const float* freq, const float* de
                             const int* chunks, int n_chunks, const int* seq_first_chunk, int wave, float* packed,
                             float* chunk_state, float* o_raw, void* out, int n_tokens, int n_units, int heads, int dim,
                             int vdim, int rot_dims, float eps, int act, float k_scale, const float* norm_w,
-                            int gate_kind, cudaStream_t stream) {
+                            int gate_kind, int sms, int* status, cudaStream_t stream) {
     dim3 grid(n_units, heads, (vdim + 31) / 32);
     cudaError_t le = cudaSuccess;
     if (chunks) {  // a prompt step, chunks of tokens side by side
         int rc = launch_chunks<T>((const T*)qkvg, freq, decay, state, seq_slots, seq_first_row, seq_start, seq_count,
                                   chunks, n_chunks, seq_first_chunk, wave, packed, chunk_state, o_raw, n_units, heads, dim,
-                                  vdim, rot_dims, act, k_scale, stream);
+                                  vdim, rot_dims, act, k_scale, sms, status, stream);
         if (rc != NNIS_OK) return rc;
     } else if (seq_first_row && (dim == 32 || dim == 64 || dim == 128 || dim == 256)) {
         constexpr int C = kRetChunk;
@@ -694,8 +882,8 @@ NNIS_API int nnis_retention(const void* qkvg, const float* freq, const float* de
                             const int* chunks, int n_chunks, const int* seq_first_chunk, int wave, float* packed,
                             float* chunk_state, float* o_raw, void* out, int n_tokens, int n_units, int heads, int dim,
                             int vdim, int rot_dims, float eps, int act, float k_scale, const float* norm_w,
-                            int gate_kind, int dtype, cudaStream_t stream) {
-    if (n_tokens <= 0 || n_units <= 0 || heads <= 0 || dim <= 0 || vdim <= 0 || rot_dims < 0 ||
+                            int gate_kind, int dtype, int sms, int* status, cudaStream_t stream) {
+    if (n_tokens <= 0 || sms <= 0 || n_units <= 0 || heads <= 0 || dim <= 0 || vdim <= 0 || rot_dims < 0 ||
         (rot_dims & 1) || rot_dims > dim || !(eps > 0.f) || !qkvg || !freq || !decay || !state ||
         !token_pos || !token_seq || !seq_slots || !o_raw || !out)
         return NNIS_ERR_ARGUMENT;
@@ -708,10 +896,10 @@ NNIS_API int nnis_retention(const void* qkvg, const float* freq, const float* de
     if (dtype == NNIS_DTYPE_F32)
         return launch_retention<float>(qkvg, freq, decay, state, token_pos, token_seq, seq_slots,
                                        seq_first_row, seq_start, seq_count, chunks, n_chunks,
-                                       seq_first_chunk, wave, packed, chunk_state, o_raw, out, n_tokens, n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, stream);
+                                       seq_first_chunk, wave, packed, chunk_state, o_raw, out, n_tokens, n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, sms, status, stream);
     if (dtype == NNIS_DTYPE_BF16)
         return launch_retention<bf16>(qkvg, freq, decay, state, token_pos, token_seq, seq_slots,
                                       seq_first_row, seq_start, seq_count, chunks, n_chunks,
-                                      seq_first_chunk, wave, packed, chunk_state, o_raw, out, n_tokens, n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, stream);
+                                      seq_first_chunk, wave, packed, chunk_state, o_raw, out, n_tokens, n_units, heads, dim, vdim, rot_dims, eps, act, k_scale, norm_w, gate_kind, sms, status, stream);
     return NNIS_ERR_UNSUPPORTED;
 }

@@ -380,6 +380,42 @@ def test_retention_chunks_in_waves(wave, monkeypatch):
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
 
 
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (64, 200), (128, 264), (128, 384)])
+@pytest.mark.parametrize("dtype,act", [("float32", True), ("bfloat16", False)])
+def test_retention_of_prompts_in_pairs_of_chunks(dim, vdim, dtype, act):
+    """The sizes that go to the tensor cores: tiles of 128 columns half full, full, one CTA's two and more."""
+    test_retention_of_prompts_in_chunks(dim, vdim, dtype, act, False)
+
+
+@pytest.mark.parametrize("wave", [2, 3, 5])
+def test_retention_pairs_of_chunks_in_waves(wave, monkeypatch):
+    """The same bits however many pairs the scratch holds, with more sequences than a warp looks through at once."""
+    o = ops()
+    g = torch.Generator().manual_seed(wave)
+    H, dim, vdim, new = 2, 64, 72, [130, 64, 1, 300] + [3, 70, 129] * 12
+    starts = [0, 5, 0, 64] + [0, 9, 0] * 12
+    n, seqs = sum(new), len(new)
+    rows, decay = torch.randn(n, 2 * H * (dim + vdim), generator=g).to(DEV), torch.tensor([0.97, 0.5], device=DEV)
+    begin, freq = torch.randn(seqs, H, dim, vdim, generator=g), torch.ones(1, device=DEV)
+    for s, st in enumerate(starts):
+        begin[s] *= st > 0
+    chunks, first = (torch.from_numpy(t).to(DEV) for t in o.scan_segments(new, o.RETENTION_CHUNK))
+    tables = [i32(x) for x in ([st + t for st, c in zip(starts, new) for t in range(c)],
+                               [i for i, c in enumerate(new) for _ in range(c)], range(seqs),
+                               [sum(new[:i]) for i in range(seqs)], starts, new)]
+    got = []
+    for scratch in (o.RETENTION_SCRATCH, 4 * wave * H * (64 * (3 * dim + vdim) + dim * vdim)):
+        monkeypatch.setattr(o, "RETENTION_SCRATCH", scratch)
+        sizes = o.retention_scratch(len(chunks), H, dim, vdim)
+        state, o_raw = begin.to(DEV), torch.full((n, H * vdim), 5.0, device=DEV)
+        o.retention(rows, freq, decay, state, *tables, o_raw, torch.empty(n, H * vdim, device=DEV), H, dim, vdim, 0, 1e-5,
+                    chunks=chunks, seq_first_chunk=first, packed=torch.full((sizes[0],), math.nan, device=DEV),
+                    chunk_state=torch.full((sizes[1],), math.nan, device=DEV))
+        got.append((o_raw, state))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert got[0][0].isfinite().all() and got[0][1].isfinite().all()
+
+
 @pytest.mark.parametrize("dim,vdim,taps", [(64, 30, 4), (128, 128, 4), (64, 200, 1), (128, 64, 3)])
 @pytest.mark.parametrize("slow", [True, False])
 def test_delta_rule_of_prompts_in_chunks(dim, vdim, taps, slow):
