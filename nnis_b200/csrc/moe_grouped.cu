@@ -251,6 +251,53 @@ moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ place,
     }
 }
 
+// The same four columns at a time, the rows of up to four of the token's experts asked for at once; the same bits.  Bound by
+// memory: 2,048 tokens of 2,048 values and four experts each (67 MB of rows) 27 -> 16 us.
+__global__ void __launch_bounds__(256)
+moe_combine_quads_kernel(const float* __restrict__ y, const int* __restrict__ place, const float* __restrict__ weights,
+                         float* __restrict__ residual, int width, int top, const float* __restrict__ pass_weight,
+                         const bf16* __restrict__ x) {
+    const long long n = blockIdx.x;
+    for (int c = threadIdx.x * 4; c < width; c += 1024) {
+        float4 r = load4(residual + (size_t)n * width + c), sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (pass_weight) {
+            const float p = pass_weight[n];
+            const float4 v = load4(x + (size_t)n * width + c);
+            sum = make_float4(p * v.x, p * v.y, p * v.z, p * v.w);
+        }
+        for (int s0 = 0; s0 < top; s0 += 4) {
+            float4 v[4];
+            bool there[4];
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                const int at = s0 + s < top ? place[n * top + s0 + s] : -1;
+                there[s] = at >= 0;
+                v[s] = there[s] ? load4(y + (size_t)at * width + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                if (!there[s]) continue;
+                if (weights) {
+                    const float w = weights[n * top + s0 + s];
+                    sum = make_float4(fmaf(w, v[s].x, sum.x), fmaf(w, v[s].y, sum.y), fmaf(w, v[s].z, sum.z),
+                                      fmaf(w, v[s].w, sum.w));
+                } else {
+                    sum = make_float4(sum.x + v[s].x, sum.y + v[s].y, sum.z + v[s].z, sum.w + v[s].w);
+                }
+            }
+        }
+        r = make_float4(r.x + sum.x, r.y + sum.y, r.z + sum.z, r.w + sum.w);
+        store4(residual + (size_t)n * width + c, r);
+    }
+}
+
+static void launch_combine(const float* y, const int* place, const float* weights, float* residual, int n_tokens, int width,
+                           int top, const float* pass_weight, const bf16* x, cudaStream_t stream) {
+    const bool quads = width % 4 == 0 && ((uintptr_t)y | (uintptr_t)residual) % 16 == 0 && (!pass_weight || (uintptr_t)x % 8 == 0);
+    (quads ? moe_combine_quads_kernel : moe_combine_kernel)<<<n_tokens, 256, 0, stream>>>(y, place, weights, residual, width,
+                                                                                          top, pass_weight, x);
+}
+
 }  // namespace nnis
 
 using namespace nnis;
@@ -333,8 +380,7 @@ NNIS_API int nnis_moe_grouped(const void* x, const void* w_up, const void* w_dow
         (const float*)nullptr, act_kind);
     grouped_mma_kernel<1><<<dim3(tiles, (width + 63) / 64), 128, smem, stream>>>(
         (const bf16*)act, ff, perm, top, (const bf16*)w_down, tile_expert, y, width, ff, 0, 0, 0, 0);
-    moe_combine_kernel<<<n_tokens, 256, 0, stream>>>(y, place, weights, residual, width, top, pass_weight,
-                                                     (const bf16*)x);
+    launch_combine(y, place, weights, residual, n_tokens, width, top, pass_weight, (const bf16*)x, stream);
     NNIS_RETURN_LAUNCH();
 }
 
@@ -363,9 +409,8 @@ NNIS_API int nnis_moe_grouped_gated(const void* x, const void* w_gu, const void*
         weight_on_output ? (const float*)nullptr : weights);
     grouped_mma_kernel<1><<<dim3(tiles, (width + 63) / 64), 128, kGroupedSmem, stream>>>(
         (const bf16*)act, ff, perm, top, (const bf16*)w_down, tile_expert, y, width, ff, 0, 0, 0, 0);
-    moe_combine_kernel<<<n_tokens, 256, 0, stream>>>(y, place, weight_on_output ? weights : (const float*)nullptr,
-                                                     residual, width, top, weight_on_output ? pass_weight : nullptr,
-                                                     (const bf16*)x);
+    launch_combine(y, place, weight_on_output ? weights : (const float*)nullptr, residual, n_tokens, width, top,
+                   weight_on_output ? pass_weight : nullptr, (const bf16*)x, stream);
     NNIS_RETURN_LAUNCH();
 }
 
@@ -405,8 +450,7 @@ NNIS_API int nnis_moe_grouped_tc(const void* x, const void* w_up, const void* w_
     code = nnis_gemm_tc_grouped(act, w_down, y, rows, width, ff, experts, tile_expert, 0, sm_count, status, pdl,
                                 stream);
     if (code != NNIS_OK) return code;
-    moe_combine_kernel<<<n_tokens, 256, 0, stream>>>(y, place, weights, residual, width, top, pass_weight,
-                                                     (const bf16*)x);
+    launch_combine(y, place, weights, residual, n_tokens, width, top, pass_weight, (const bf16*)x, stream);
     NNIS_RETURN_LAUNCH();
 }
 
@@ -441,8 +485,7 @@ NNIS_API int nnis_moe_grouped_gated_tc(const void* x, const void* w_gu, const vo
     code = nnis_gemm_tc_grouped(act, w_down, y, rows, width, ff, experts, tile_expert, 0, sm_count, status, pdl,
                                 stream);
     if (code != NNIS_OK) return code;
-    moe_combine_kernel<<<n_tokens, 256, 0, stream>>>(y, place, weight_on_output ? weights : (const float*)nullptr,
-                                                     residual, width, top, weight_on_output ? pass_weight : nullptr,
-                                                     (const bf16*)x);
+    launch_combine(y, place, weight_on_output ? weights : (const float*)nullptr, residual, n_tokens, width, top,
+                   weight_on_output ? pass_weight : nullptr, (const bf16*)x, stream);
     NNIS_RETURN_LAUNCH();
 }
