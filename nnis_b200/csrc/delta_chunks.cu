@@ -19,7 +19,7 @@
 // keep): a token costs 2.2 dim vdim + 64 (dim + vdim) multiply-adds or so instead of 2.3 times three dim vdim, all but the chain side
 // by side, and a thread's 8 x 8 outputs share what is read.
 // Two prompts of 2,048 and 555 tokens, 32 heads over 16 key heads of 128 x 128, on a B200: prep 201, walk 707, prefix 270
-// and apply 235 us before; now pack 79, solve 148, chain 256 and read 132.
+// and apply 235 us before; now pack 60, solve 147, chain 255 and read 133.
 #include "async_copy.cuh"
 #include "common.cuh"
 #include "linear_chunks.cuh"
@@ -45,7 +45,8 @@ __device__ __forceinline__ DeltaChunk delta_chunk(const int* chunks, const int* 
 __host__ __device__ __forceinline__ size_t delta_qk_floats(int dim) { return (size_t)3 * kDC * dim; }
 
 // A CTA per (chunk, piece): q heads, k heads, value heads, and last the gates of all heads.  A thread walks 16 tokens of
-// a channel; with TAPS (the taps when there are 4, else 0) the inputs before a token stay in registers.
+// a channel; with TAPS (the taps when there are 4, else 0) the inputs before a token stay in registers.  Instructions bound it
+// (104 a value with a division for each place and a test for each input, 79 us on the prompts above; 60 us now).
 template <int TAPS>
 __global__ void __launch_bounds__(256)
 delta_pack_kernel(const float* __restrict__ a, const float* __restrict__ conv_w, const float* __restrict__ tail,
@@ -104,13 +105,32 @@ delta_pack_kernel(const float* __restrict__ a, const float* __restrict__ conv_w,
     auto input = [&](int t, int c) {
         return ch.start + t >= 0 ? a[(size_t)(ch.first + t) * row_len + c] : old[(size_t)(L + ch.start + t) * conv_cols + c];
     };
-    for (int it = tid; it < width * 4; it += 256) {
-        const int ci = it % width, t0 = it / width * 16, c = c0 + ci;
+    // (places of 64 x n values, 256 apart: no division in the loops)
+    struct Walk {
+        int t, j, dt, dj, n;
+        __device__ Walk(int at, int n) : t(at / n), j(at % n), dt(256 / n), dj(256 % n), n(n) {}
+        __device__ void step() {
+            t += dt;
+            j += dj;
+            if (j >= n) {
+                j -= n;
+                ++t;
+            }
+        }
+    };
+    for (Walk at(tid, width); at.t < 4; at.step()) {
+        const int ci = at.j, t0 = at.t * 16, c = c0 + ci;
         if (TAPS == 4) {
             const float4 w = *reinterpret_cast<const float4*>(conv_w + (size_t)c * 4);
             float x[19];
+            if (t0 + 16 <= ch.count && ch.start + t0 >= 3) {
+                const float* from = a + (size_t)(ch.first + t0 - 3) * row_len + c;
 #pragma unroll
-            for (int i = 0; i < 19; ++i) x[i] = t0 < ch.count && t0 + i - 3 < ch.count ? input(t0 + i - 3, c) : 0.f;
+                for (int i = 0; i < 19; ++i, from += row_len) x[i] = *from;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 19; ++i) x[i] = t0 < ch.count && t0 + i - 3 < ch.count ? input(t0 + i - 3, c) : 0.f;
+            }
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 float acc = fmaf(w.x, x[i], 0.f);
@@ -131,10 +151,8 @@ delta_pack_kernel(const float* __restrict__ a, const float* __restrict__ conv_w,
     __syncthreads();
     if (!head) {
         float* to = values + ((size_t)blockIdx.x * H + (piece - 2 * G)) * kDC * vp;
-        for (int it = tid; it < kDC * vp; it += 256) {
-            const int t = it / vp, j = it - t * vp;
-            to[it] = j < vdim ? pack_y[t * ld + j] : 0.f;
-        }
+        int it = tid;
+        for (Walk at(tid, vp); at.t < kDC; at.step(), it += 256) to[it] = at.j < vdim ? pack_y[at.t * ld + at.j] : 0.f;
         return;
     }
     for (int t = warp; t < kDC; t += 8) {
@@ -152,10 +170,8 @@ delta_pack_kernel(const float* __restrict__ a, const float* __restrict__ conv_w,
     }
     if (piece < G) return;
     to += (size_t)kDC * dim;
-    for (int it = tid; it < kDC * dim; it += 256) {
-        const int t = it / dim, d = it - t * dim;
-        to[it] = pack_y[t * ld + d] * scale[t];
-    }
+    int it = tid;
+    for (Walk at(tid, dim); at.t < kDC; at.step(), it += 256) to[it] = pack_y[at.t * ld + at.j] * scale[at.t];
 }
 
 // W [dim][64] (a row per value of the key) and U0 [64][vp].  128 threads, two columns each of the right sides
