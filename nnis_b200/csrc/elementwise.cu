@@ -339,20 +339,27 @@ __global__ void add_rows_kernel(float* __restrict__ a, const float* __restrict__
 // of a gate that scales the expert's whole output.  u float32 [n, inter + gated]
 // (`gated` columns beyond the activation's: the gate, then padding).
 // ---------------------------------------------------------------------------
+// Four values a thread, 256 apart, all asked for at once, the gate once a thread (a thread a value, its row by a division of 64
+// bits: 13 us for 2,048 rows of 1,408; now 5.5).
 template <typename T>
-__global__ void relu2_gate_kernel(const float* __restrict__ u, T* __restrict__ out, size_t n_rows,
-                                  int inter, int gated) {
+__global__ void __launch_bounds__(256)
+relu2_gate_kernel(const float* __restrict__ u, T* __restrict__ out, int inter, int gated) {
     pdl_wait();
     pdl_launch_dependents();
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n_rows * (size_t)inter) return;
-    size_t n = idx / inter;
-    int i = (int)(idx - n * inter);
+    const size_t n = blockIdx.x;
     const float* row = u + n * (size_t)(inter + gated);
-    float a = fmaxf(row[i], 0.f);
-    float v = a * a;
-    if (gated) v *= 1.0f / (1.0f + expf(-row[inter]));
-    out[idx] = from_float<T>(v);
+    const int i0 = blockIdx.y * 1024 + threadIdx.x;
+    float x[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) x[e] = i0 + e * 256 < inter ? row[i0 + e * 256] : 0.f;
+    const float scale = gated ? 1.0f / (1.0f + expf(-row[inter])) : 1.0f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float a = fmaxf(x[e], 0.f);
+        float v = a * a;
+        if (gated) v *= scale;
+        if (i0 + e * 256 < inter) out[n * inter + i0 + e * 256] = from_float<T>(v);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -536,15 +543,13 @@ NNIS_API int nnis_group_rmsnorm(const float* x, const int* rows, const float* w,
 NNIS_API int nnis_relu2_gate(const float* u, void* out, int out_dtype, long long n_rows, int inter,
                              int gated, cudaStream_t stream) {
     if (n_rows <= 0 || inter <= 0 || gated < 0) return NNIS_ERR_ARGUMENT;
-    size_t total = (size_t)n_rows * inter;
-    unsigned blocks = (unsigned)((total + 255) / 256);
+    const dim3 grid((unsigned)n_rows, (inter + 1023) / 1024);
+    if (n_rows > 0x7fffffffLL || grid.y > 65535) return NNIS_ERR_UNSUPPORTED;
     cudaError_t e;
     if (out_dtype == NNIS_DTYPE_F32)
-        e = launch_dependent(relu2_gate_kernel<float>, blocks, 256, 0, stream, u, (float*)out, (size_t)n_rows, inter,
-                             gated);
+        e = launch_dependent(relu2_gate_kernel<float>, grid, 256, 0, stream, u, (float*)out, inter, gated);
     else if (out_dtype == NNIS_DTYPE_BF16)
-        e = launch_dependent(relu2_gate_kernel<bf16>, blocks, 256, 0, stream, u, (bf16*)out, (size_t)n_rows, inter,
-                             gated);
+        e = launch_dependent(relu2_gate_kernel<bf16>, grid, 256, 0, stream, u, (bf16*)out, inter, gated);
     else
         return NNIS_ERR_UNSUPPORTED;
     return e == cudaSuccess ? NNIS_OK : (int)e;
