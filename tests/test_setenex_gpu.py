@@ -302,6 +302,30 @@ def test_prompt_attention_on_the_tensor_cores(H, G, dk, dv, window, keep, distan
         assert torch.allclose(out.float(), other.float(), atol=3e-2, rtol=3e-2), with_bias
 
 
+@pytest.mark.parametrize("size", [0.2, 1.0, 30.0])
+def test_the_cap_on_scores_in_both_forms(size):
+    """Scores far below half the cap (by multiply-adds), on both sides of it from page to page, and up to the cap."""
+    from nnis_b200.csrc import ops
+    g = torch.Generator().manual_seed(6)
+    n, H, d, cap = 150, 2, 64, 5.0
+    q, k, v = (torch.randn(n, H, d, generator=g).bfloat16() for _ in range(3))
+    q = q * size
+    k[64:128] *= 4.0
+    cache = [torch.zeros(3, H, 64, d, dtype=torch.bfloat16) for _ in (k, v)]
+    for c, x in zip(cache, (k, v)):
+        for t in range(n):
+            c[t // 64, :, t % 64] = x[t]
+    s = torch.einsum("ihd,jhd->hij", q.double(), k.double()) * d ** -0.5
+    s = cap * torch.tanh(s / cap)
+    p = torch.softmax(s.masked_fill(torch.ones(n, n).triu(1).bool(), -math.inf), -1)
+    want = torch.einsum("hij,jhd->ihd", p, v.double()).reshape(n, -1)
+    out = torch.full((n, H * d), 9.0, dtype=torch.bfloat16, device=DEV)
+    ops.attention_sink_mma(q.reshape(n, -1).to(DEV), cache[0].to(DEV), cache[1].to(DEV), i32([(0, q0) for q0 in range(0, n, 64)]),
+                           i32([0]), i32([0]), i32([n]), i32([[0, 1, 2]]), None, None, out, H, H, 0, 0, d ** -0.5, cap)
+    # weights and outputs are rounded to bfloat16: 2^-8 of the values' size each
+    assert (out.cpu().double() - want).abs().max() < 2 * 2.0 ** -8 * v.double().abs().max()
+
+
 def test_head_norms_with_weights_before_the_cache():
     """qkv_prep with a weight per value of a head: q and k heads normed by themselves, before a rotation if
     there is one, values as they are."""
