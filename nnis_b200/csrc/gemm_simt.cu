@@ -2,8 +2,9 @@
 // W is stored [out, in] row-major as the checkpoint has it, so both operands
 // run along K.  Operands are float32 or bfloat16; products are accumulated in
 // float32 with fmaf, never through a reduced-precision tensor-core mode.  These
-// are the whole float32 path, and the fallback of the bfloat16 path for shapes
-// that the tcgen05 kernel refuses.
+// are the float32 path of single tokens and of the shapes and addresses that
+// gemm_split_f32.cu does not take, and the fallback of the bfloat16 path for
+// shapes that the tcgen05 kernel refuses.
 //
 // Output modes: 0 store in the operand dtype, 1 store float32, 2 add to a
 // float32 destination (the residual stream).
