@@ -7,8 +7,11 @@
 //
 // A CTA of 17 warps: one issues the products; sixteen split operands, read sums, and hold a token and 32 keys or columns each
 // thread.  Shared memory: the queries' parts (128 x 64 twice), which the scores and the state meet and the weights replace,
-// and a ring of two blocks for what they meet (128 x 64 keys, or 64 x 128 of the state or the values).  Splitting bounds it:
-// a block of 128 x 64 takes the sixteen warps about 1,200 cycles, its products 770.
+// and a ring of two blocks for what they meet (128 x 64 keys, or 64 x 128 of the state or the values).
+// What bounds it: the way of a block through its loads, the splitting, the fence and the sixteen warps' arrivals, 3,300 cycles (the
+// products of a block take 1,536, issued in 2,400), and 8,000 cycles of start and 6,000 of end: one CTA has the SM's shared
+// memory, so nothing hides them.  Asking for the next block's values after the hand-over instead of before the fence was slower
+// (retention's read 30.2 -> 32.4 us).
 #pragma once
 
 #include "split_parts.cuh"
