@@ -118,6 +118,8 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map, const bf16* __rest
                 else if (page_end == hi && row == r1 - 1)  // this step's row: written by the kernels just before
                     *at = *reinterpret_cast<const uint4*>(cache + ((size_t)table[first_page + it] * kLdPage + row) * dk + chunk * 8);
             }
+            // (a window's first page is one that the ring asks for again: these stores come before the copies over them)
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncthreads();
         }
         // scores of keys 8 warp .. 8 warp + 7

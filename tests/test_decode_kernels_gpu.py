@@ -196,6 +196,43 @@ def test_latent_attention_of_single_tokens(heads, dk, dv, window):
     o.check_status(DEV)
 
 
+@pytest.mark.parametrize("heads,dk,dv", [(16, 576, 512), (8, 288, 256), (17, 72, 64)])
+@pytest.mark.parametrize("window", [130, 330, 450])
+def test_latent_attention_of_single_tokens_under_windows_of_more_pages_than_the_ring(heads, dk, dv, window):
+    """The first page of a window has hidden rows, is zeroed there, and its place is filled again: against 64 bits, and the same
+    bits whatever the hidden rows hold."""
+    o = ops()
+    g = torch.Generator().manual_seed(heads + window)
+    lengths, cols = [700, 461, 512, 640, 333], 11
+    n = len(lengths)
+    rows = torch.randn(n, cols * 64, dk, generator=g).bfloat16()
+    table = torch.randperm(n * cols, generator=g).to(torch.int32).view(n, cols)
+    q = torch.randn(n, heads * dk, generator=g).bfloat16()
+    scale = dk ** -0.5
+    d = lambda t: t.to(DEV)
+    for splits in (1, 2):
+        first = None
+        for hidden in (0.0, 1e4, math.nan):
+            cache = torch.full((n * cols, 1, 64, dk), hidden, dtype=torch.bfloat16)
+            for t, length in enumerate(lengths):
+                for i in range(length - window if length > window else 0, length):
+                    cache[int(table[t, i // 64]), 0, i % 64] = rows[t, i]
+            out = torch.full((n, heads * dv), 9.0, dtype=torch.bfloat16, device=DEV)
+            partial = torch.full((n * heads * splits * (dv + 2),), math.nan, device=DEV) if splits > 1 else None
+            o.attention_latent_decode(d(q), d(cache), d(torch.tensor(lengths, dtype=torch.int32) - 1),
+                                      torch.arange(n, dtype=torch.int32, device=DEV), d(table), out, heads, dv, scale, splits,
+                                      partial, window)
+            first = out.clone() if first is None else first
+            assert torch.equal(out, first), (splits, hidden)
+        for t, length in enumerate(lengths):
+            seen = rows[t, max(0, length - window):length].double()
+            p = torch.softmax(q[t].double().view(heads, dk) @ seen.T * scale, 1)
+            # (weights and outputs rounded to bfloat16, half a unit in eight bits each: 2^-7 of sums of |p v| together)
+            bound = 2.0 ** -7 * (p @ seen[:, :dv].abs()) + 1e-4
+            assert ((first[t].cpu().double().view(heads, dv) - p @ seen[:, :dv]).abs() <= bound).all(), (t, splits)
+    o.check_status(DEV)
+
+
 @pytest.mark.parametrize("m", [1, 7, 8, 9, 16])
 @pytest.mark.parametrize("heads,n,k", [(3, 8, 32), (2, 40, 96), (5, 24, 160), (16, 512, 128), (4, 128, 512), (2, 16, 544), (3, 12, 64)])
 @pytest.mark.parametrize("gate", [False, True])

@@ -333,3 +333,14 @@ def test_units_of_the_float32_prompt_attention_cover_every_tile_once():
         for parts in seen.values():
             assert sorted(z for z, _ in parts) == list(range(parts[0][1])) and len({k for _, k in parts}) == 1
         assert max(k for _, _, _, k in units.tolist()) == slices
+
+
+def test_stores_into_the_latent_ring_are_fenced_before_the_copies_over_them():
+    """Ordinary stores and bulk copies to the same shared memory are ordered by a proxy fence of the storing threads alone; no
+    result shows that it is missing, so the kernel's text is looked at: from the zeroed rows to the next barrier."""
+    import os
+    from nnis_b200 import csrc
+    with open(os.path.join(os.path.dirname(csrc.__file__), "attention_latent_decode.cu")) as f:
+        text = f.read()
+    stores = text[text.index("if (row < r0 || row >= r1) *at ="):]
+    assert "fence.proxy.async.shared::cta" in stores[:stores.index("__syncthreads()")]
