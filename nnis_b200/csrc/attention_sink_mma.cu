@@ -15,22 +15,9 @@
 // their (token, head).  The host lists the tiles (sequence, first query).
 #include <float.h>
 
-#include "fma_pairs.cuh"
 #include "mma_helpers.cuh"
 
 namespace nnis {
-
-// tanh(x) / x - 1 for |x| <= 1/2 as x^2 (a + b x^2 + c x^4 + d x^6): a least maximum fit of the odd series, error 1.7e-8; with
-// float32's roundings tanh is within 2.8e-8 (1 - 2 / (1 + e^2x) by the special function units: 1.7e-7)
-constexpr float kTanhA = -0.33333149552345276f, kTanhB = 0.1332598775625229f, kTanhC = -0.05305294319987297f,
-                kTanhD = 0.017256978899240494f;
-
-// 2^x; results below 2^-126 are zero
-__device__ __forceinline__ float sink_ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 constexpr int kSinkRows = 64;   // query rows per CTA
 constexpr int kSinkPage = 64;
@@ -149,7 +136,6 @@ attn_sink_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cach
     l_run[0] = l_run[1] = (sink && (lane & 3) == 0) ? 1.f : 0.f;
     const float cap_in = cap > 0.f ? 2.0f * kLog2e / cap : 0.f, cap_out = cap * kLog2e;
     const float sc = scale * kLog2e;
-    const float cap_2 = cap > 0.f ? scale / cap * (scale / cap) : 0.f, small_score = cap > 0.f ? 0.5f * cap / fabsf(scale) : 0.f;
 
     for (int it = 0; it < n_pages; ++it) {
         cp_async_wait<kSinkStages - 2>();
@@ -198,52 +184,23 @@ attn_sink_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cach
         }
         uint32_t pa[4][4];
         float mx[2] = {-INFINITY, -INFINITY};
-        // cap * tanh(x / cap): where no score of the warp's page passes half the cap, by multiply-adds, two scores an
-        // instruction (by the two special functions of the general form 3,001 queries of 16 heads over 1,024 keys took 59.5
-        // us; 54.3 so: the chain through a page, at three CTAs an SM, bounds what is left)
-        float most = 0.f;
-        if (cap > 0.f) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
+        for (int j = 0; j < 8; ++j)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) most = fmaxf(most, fabsf(s[j][e]));
-        }
-        if (cap > 0.f && !__any_sync(0xffffffffu, most > small_score)) {
-            const unsigned long long a = both(kTanhA * cap_2), b = both(kTanhB * cap_2 * cap_2),
-                                     c = both(kTanhC * cap_2 * cap_2 * cap_2), d = both(kTanhD * cap_2 * cap_2 * cap_2 * cap_2);
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; e += 2) {
-                    const unsigned long long x = pair_of(s[j][e], s[j][e + 1]);
-                    const unsigned long long z = mul2(x, x), w = mul2(x, both(sc));
-                    unsigned long long p = c, r = b, t = a, v = w;
-                    fma2(p, z, d);
-                    fma2(r, z, p);
-                    fma2(t, z, r);
-                    fma2(v, mul2(w, z), t);
-                    s[j][e] = halves(v).x;
-                    s[j][e + 1] = halves(v).y;
+            for (int e = 0; e < 4; ++e) {
+                float v;
+                // cap * tanh(x / cap) = cap * (1 - 2 / (exp(2 x / cap) + 1)).  One form for every score: a polynomial for those
+                // below half the cap, chosen by the score alone (chosen by the page it let slots that nobody may read decide),
+                // took 3,001 queries of 16 heads over 1,024 keys 68 -> 65 us, and 68 -> 80 with scores that pass it.
+                if (cap > 0.f) {
+                    float e2 = exp2f(s[j][e] * scale * cap_in);
+                    v = cap_out * (1.0f - __fdividef(2.0f, e2 + 1.0f));
+                } else {
+                    v = s[j][e] * sc;
                 }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    if (cap > 0.f) {  // cap * tanh(x / cap) = cap * (1 - 2 / (exp(2 x / cap) + 1))
-                        float e2 = exp2f(s[j][e] * scale * cap_in);
-                        s[j][e] = cap_out * (1.0f - __fdividef(2.0f, e2 + 1.0f));
-                    } else {
-                        s[j][e] *= sc;
-                    }
-                }
-        }
-        if (BIAS) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) s[j][e] += near[(e >> 1) - j + 7][e & 1];
-        }
+                if (BIAS) v += near[(e >> 1) - j + 7][e & 1];
+                s[j][e] = v;
+            }
         if (!full) {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
@@ -271,8 +228,8 @@ attn_sink_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cach
         float psum[2] = {0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            float p0v = sink_ex2(s[j][0] - base[0]), p1v = sink_ex2(s[j][1] - base[0]);
-            float p2v = sink_ex2(s[j][2] - base[1]), p3v = sink_ex2(s[j][3] - base[1]);
+            float p0v = exp2f(s[j][0] - base[0]), p1v = exp2f(s[j][1] - base[0]);
+            float p2v = exp2f(s[j][2] - base[1]), p3v = exp2f(s[j][3] - base[1]);
             psum[0] += p0v + p1v;
             psum[1] += p2v + p3v;
             pa[j >> 1][(j & 1) * 2] = pack_bf16(p0v, p1v);

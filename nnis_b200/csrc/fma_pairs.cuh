@@ -11,10 +11,6 @@ __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b));
-    return a;
-}
 __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
     asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a) : "l"(b));
     return a;

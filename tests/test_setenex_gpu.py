@@ -304,7 +304,7 @@ def test_prompt_attention_on_the_tensor_cores(H, G, dk, dv, window, keep, distan
 
 @pytest.mark.parametrize("size", [0.2, 1.0, 30.0])
 def test_the_cap_on_scores_in_both_forms(size):
-    """Scores far below half the cap (by multiply-adds), on both sides of it from page to page, and up to the cap."""
+    """Scores far below the cap, on both sides of half of it from page to page, and up to it."""
     from nnis_b200.csrc import ops
     g = torch.Generator().manual_seed(6)
     n, H, d, cap = 150, 2, 64, 5.0
@@ -324,6 +324,40 @@ def test_the_cap_on_scores_in_both_forms(size):
                            i32([0]), i32([0]), i32([n]), i32([[0, 1, 2]]), None, None, out, H, H, 0, 0, d ** -0.5, cap)
     # weights and outputs are rounded to bfloat16: 2^-8 of the values' size each
     assert (out.cpu().double() - want).abs().max() < 2 * 2.0 ** -8 * v.double().abs().max()
+
+
+@pytest.mark.parametrize("chunk", [0, 96])
+def test_a_capped_score_hangs_on_nothing_but_itself(chunk):
+    """The same bits whatever lies in slots that no token has filled, whatever the rows beside a row hold, and in whatever
+    portions a prompt comes."""
+    from nnis_b200.csrc import ops
+    g = torch.Generator().manual_seed(8)
+    n, H, d, cap = 150, 2, 64, 5.0
+    q, k, v = (torch.randn(n, H, d, generator=g).bfloat16() for _ in range(3))
+    q[20] *= 40.0  # scores on both sides of half the cap, for the rows that see them
+
+    def run(q, portions, left):
+        cache = [torch.full((3, H, 64, d), fill, dtype=torch.bfloat16) for fill in (left, 3.0)]
+        for c, x in zip(cache, (k, v)):
+            for t in range(n):
+                c[t // 64, :, t % 64] = x[t]
+        outs = []
+        for a, b in portions:
+            out = torch.full((b - a, H * d), 9.0, dtype=torch.bfloat16, device=DEV)
+            ops.attention_sink_mma(q[a:b].reshape(b - a, -1).to(DEV), cache[0].to(DEV), cache[1].to(DEV),
+                                   i32([(0, q0) for q0 in range(0, b - a, 64)]), i32([0]), i32([a]), i32([b - a]),
+                                   i32([[0, 1, 2]]), None, None, out, H, H, 0, chunk, d ** -0.5, cap)
+            outs.append(out.cpu())
+        return torch.cat(outs)
+
+    first = run(q, [(0, n)], 0.0)
+    for left in (1e4, -1e30, math.nan):
+        assert torch.equal(run(q, [(0, n)], left), first), left
+    assert torch.equal(run(q, [(0, 7), (7, 70), (70, n)], 0.0), first)
+    other = q.clone()
+    other[[3, 77, 149]] *= 50.0
+    kept = [t for t in range(n) if t not in (3, 77, 149)]
+    assert torch.equal(run(other, [(0, n)], 0.0)[kept], first[kept])
 
 
 def test_head_norms_with_weights_before_the_cache():
