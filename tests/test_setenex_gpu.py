@@ -332,9 +332,10 @@ def test_a_capped_score_hangs_on_nothing_but_itself(chunk):
     portions a prompt comes."""
     from nnis_b200.csrc import ops
     g = torch.Generator().manual_seed(8)
-    n, H, d, cap = 150, 2, 64, 5.0
+    n, H, d, cap = 150, 2, 64, 8192.0
     q, k, v = (torch.randn(n, H, d, generator=g).bfloat16() for _ in range(3))
-    q[20] *= 40.0  # scores on both sides of half the cap, for the rows that see them
+    q[..., 0], k[..., 0] = 4096.0, 4.0  # scores of 2,048 and a little: 2^-24 of the cap is 2^-11 of a weight, and shows
+    q[20] *= 3.0  # scores on both sides of half the cap, for the rows that see them
 
     def run(q, portions, left):
         cache = [torch.full((3, H, 64, d), fill, dtype=torch.bfloat16) for fill in (left, 3.0)]
@@ -355,7 +356,7 @@ def test_a_capped_score_hangs_on_nothing_but_itself(chunk):
         assert torch.equal(run(q, [(0, n)], left), first), left
     assert torch.equal(run(q, [(0, 7), (7, 70), (70, n)], 0.0), first)
     other = q.clone()
-    other[[3, 77, 149]] *= 50.0
+    other[[3, 77, 149]] *= 8.0
     kept = [t for t in range(n) if t not in (3, 77, 149)]
     assert torch.equal(run(other, [(0, n)], 0.0)[kept], first[kept])
 
