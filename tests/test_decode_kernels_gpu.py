@@ -253,3 +253,20 @@ def test_small_matrix_per_head_on_few_rows(m, heads, n, k, gate):
         got = out.cpu().double().view(m, heads, out_head)
         assert torch.allclose(got[..., :n], want, rtol=2.0 ** -8, atol=1e-5)  # (one rounding to bfloat16)
         assert (got[..., n:] == 7.0).all()
+
+
+@pytest.mark.parametrize("m,heads,n,k", [(8, 4, 512, 128), (16, 4, 128, 256), (8, 4, 128, 512)])
+def test_small_matrix_per_head_no_further_from_64_bits_than_chains_of_multiply_adds(m, heads, n, k):
+    """Sums whose second half takes the first away again: what is left is the error of the sums alone."""
+    import numpy as np
+    o = ops()
+    g = torch.Generator().manual_seed(k)
+    a, w = torch.randn(m, heads, k // 2, generator=g).bfloat16(), torch.randn(heads, n, k // 2, generator=g).bfloat16()
+    a, w = torch.cat([a, -a], 2), torch.cat([w, w], 2)
+    out = torch.empty(m, heads * n, dtype=torch.bfloat16, device=DEV)
+    o.batched_linear(a.reshape(m, -1).to(DEV), k, w.to(DEV), out, n)
+    x, y = a.float().numpy(), w.float().numpy()
+    chain = np.zeros((m, heads, n), dtype=np.float32)
+    for i in range(k):  # (a product of two bfloat16 values is exact in float32: a chain of multiply-adds)
+        chain += x[:, :, None, i] * y[None, :, :, i]
+    assert float(out.double().norm()) <= float(np.linalg.norm(chain.astype(np.float64)))
