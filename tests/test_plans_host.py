@@ -260,6 +260,17 @@ def test_which_kernel_takes_the_projections_of_a_decode_step():
     assert o.gemm_tc_splits(64, 2048, 8192)[0] == 4 and o.gemm_tc_splits(2048, 576, 1536)[0] == 1
 
 
+def test_adding_projections_share_k_in_one_launch_where_two_launches_are_not_faster():
+    """Two parts of more CTAs than two an SM leave the product to two launches; more parts never do."""
+    from nnis_b200.csrc import ops as o
+    for m, n, k, one_launch in ((8, 2048, 2048, True), (8, 4096, 3072, True), (8, 6144, 3072, False), (1, 6144, 2048, False),
+                                (17, 2048, 3072, True), (17, 3072, 1792, False), (64, 1024, 2560, True), (64, 1536, 2048, False),
+                                (64, 2048, 3072, False), (64, 2048, 8192, True), (32, 4096, 4096, True), (8, 6144, 4096, True)):
+        floats, tiles = o.gemv_split_scratch(m, n, k)
+        assert (floats > 0) == (tiles > 0) == one_launch, (m, n, k)
+        assert o.gemv_slices(m, n, k) >= 2
+
+
 def test_which_retention_prompts_work_their_chunks_side_by_side(monkeypatch):
     from nnis_b200.csrc import ops as o
     side = lambda counts, heads=8, dim=128, vdim=256: o.retention_side_by_side(counts, heads, dim, vdim, 148)
