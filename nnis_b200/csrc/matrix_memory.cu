@@ -25,7 +25,7 @@
 //                  O_t = exp(m_before - M_t) S_before^T q_t + sum_{s <= t} exp(u_s - M_t) (q_t . k_s) v_s,
 //                  the denominator the same with n and without v.
 //   memory_chunk_split, memory_out_split: the two contractions by pairs of chunks on the tensor cores (chunk_read_split.cuh),
-//                  for heads of 64 or 128 keys.
+//                  for heads of 64 or 128 keys where that pays (memory_by_pairs).
 //   memory_finish  every head's o divided by its root mean square, times a weight per value, times
 //                  sigmoid(g), rounded once to the operand dtype.
 //
@@ -718,6 +718,23 @@ memory_finish_kernel(const float* __restrict__ o_raw, const float* __restrict__ 
     for (int i = lane; i < vdim; i += 32) dst[i] = from_float<T>((o[i] * s) * wh[i] * (1.0f / (1.0f + expf(-g[i]))));
 }
 
+// Whether a step's chunks go to the kernels by pairs: heads of 64 or 128 keys, whole groups of eight columns, and where those
+// are not slower than the kernels of single chunks, in us of a whole memory_prompt (pairs, single chunks):
+//   * not for 64 x 64 and smaller, of which single chunks fill an SM's shared memory several times (8 heads: 100 tokens 43, 39;
+//     8 x 300 66, 57; 64 x 64 105, 73; 4,000 tokens 82, 94);
+//   * not for chunks of 32 tokens and fewer on average, where a CTA's start is most of its time (1 x 16 tokens of 4 heads of
+//     128 x 256 41, 37; 64 x 10 of 8 of 64 x 128 105, 74; 1 x 40 44, 43), but for many of large heads (16 x 24 of 8 of 128 x 256
+//     62, 73; 16 x 10 of 4 49, 50);
+//   * not for more sequences of a single chunk than SMs with heads of 128 x 64 and less, as half of a CTA's tokens are missing
+//     (64 x 40 of 8 heads of 64 x 128 114, 104, of 128 x 32 111, 86; 64 x 100 154, 212).
+// 2,000 tokens of 8 heads: 64 x 128 53, 70; 128 x 32 55, 72; 128 x 256 75, 187.
+static bool memory_by_pairs(long long n_tokens, long long n_chunks, long long n_seqs, int H, int dim, int vdim, int sms) {
+    const long long state = (long long)dim * vdim;
+    if ((dim != 64 && dim != 128) || vdim % 8 || (dim == 64 && vdim <= 64)) return false;
+    if (n_tokens <= 32 * n_chunks && (state < 128 * 256 || n_chunks * H <= 64)) return false;
+    return state > 128 * 64 || 2 * n_seqs <= n_chunks || n_chunks * H <= sms;
+}
+
 template <int BV>
 static cudaError_t launch_memory_prompt(const float* a, int a_cols, float* state, float* norm_state, float* max_state,
                                         const int* chunks, int n_chunks, const int* seq_first_chunk, int n_seqs,
@@ -728,8 +745,8 @@ static cudaError_t launch_memory_prompt(const float* a, int a_cols, float* state
     double *b = gates, *u = gates + (size_t)n_tokens * H, *top = gates + (size_t)2 * n_tokens * H;
     double *ends = chunk_gates, *before = chunk_gates + (size_t)2 * n_chunks * H;
     const int v_tiles = (vdim + BV - 1) / BV, d_tiles = (dim + 63) / 64;
-    // Pairs of chunks on the tensor cores: heads of 64 or 128, rows on 32-byte boundaries, whole groups of eight columns.
-    const bool split = (dim == 64 || dim == 128) && vdim % 8 == 0 && a_cols % 8 == 0 &&
+    // (rows on 32-byte boundaries)
+    const bool split = memory_by_pairs(n_tokens, n_chunks, n_seqs, H, dim, vdim, sms) && a_cols % 8 == 0 &&
                        ((uintptr_t)a | (uintptr_t)chunk_state | (uintptr_t)o_raw) % 32 == 0;
     const int by = split ? 2 : 1, most_pairs = (n_chunks + n_seqs) / 2;
     if (split) {
@@ -811,6 +828,11 @@ NNIS_API int nnis_memory_step(const float* a, int a_cols, const float* i_bias, c
                            norm_state, max_state, token_pos, token_seq, seq_slots, o_raw, H, dim, vdim, cap, q_scale,
                            floor_add);
     return e == cudaSuccess ? NNIS_OK : (int)e;
+}
+
+// Whether nnis_memory_prompt takes rows, scratch and outputs on 32-byte boundaries to the tensor cores.
+NNIS_API int nnis_memory_by_pairs(int n_tokens, int n_chunks, int n_seqs, int H, int dim, int vdim, int sms) {
+    return memory_by_pairs(n_tokens, n_chunks, n_seqs, H, dim, vdim, sms) ? 1 : 0;
 }
 
 // Prompt steps.  chunks: int32 [n_chunks, 2] = (sequence, first token of the chunk among the sequence's tokens of this

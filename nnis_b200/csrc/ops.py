@@ -2586,6 +2586,12 @@ def memory_step(a: torch.Tensor, i_bias: torch.Tensor, f_bias: torch.Tensor, sta
                                    ctypes.c_float(floor), _stream()), "memory_step")
 
 
+def memory_by_pairs(counts, heads: int, dim: int, vdim: int, sms: int) -> bool:
+    """Whether ``memory_prompt`` works a step of these token counts by pairs of chunks on the tensor cores."""
+    chunks = sum(-(-int(c) // memory_chunk_tokens()) for c in counts)
+    return bool(_lib().nnis_memory_by_pairs(int(sum(counts)), chunks, len(counts), heads, dim, vdim, sms))
+
+
 def memory_prompt(a: torch.Tensor, i_bias: torch.Tensor, f_bias: torch.Tensor, state: torch.Tensor,
                   norm_state: torch.Tensor, max_state: torch.Tensor, chunks: torch.Tensor,
                   seq_first_chunk: torch.Tensor, seq_slots: torch.Tensor, seq_first_row: torch.Tensor,

@@ -302,6 +302,19 @@ def test_chunks_of_the_delta_rule_keep_their_scratch_within_its_bound():
     assert o.delta_wave(9, 4096, 4096, 128, 512) >= 1
 
 
+def test_which_prompts_of_the_matrix_memory_go_by_pairs_of_chunks():
+    """Not short ones, not heads of 64 x 64, not many sequences of one chunk with small heads."""
+    from nnis_b200.csrc import ops as o
+    pairs = lambda counts, heads=8, dim=128, vdim=256: o.memory_by_pairs(counts, heads, dim, vdim, 148)
+    assert pairs([2000]) and pairs([40]) and pairs([33]) and pairs([1500, 1500, 701]) and pairs([300, 1, 17])
+    assert not pairs([1]) and not pairs([32]) and not pairs([16, 24, 30]) and pairs([64]) and pairs([66])
+    assert pairs([24] * 16) and not pairs([24] * 8) and not pairs([24] * 64, vdim=128)
+    assert not pairs([2000], dim=64, vdim=64) and pairs([2000], dim=64, vdim=72) and pairs([2000], vdim=8)
+    assert not pairs([2000], dim=96) and not pairs([2000], vdim=100)
+    assert not pairs([64] * 64, dim=64, vdim=128) and pairs([64] * 64, dim=64, vdim=136) and pairs([100] * 64, dim=64, vdim=128)
+    assert pairs([64] * 16, vdim=64) and not pairs([64] * 19, vdim=64)
+
+
 def test_float32_prompts_take_tiles_where_these_pay():
     """Enough queries to a tile, or a long chain of keys on an empty device; the counts behind the rule are those of the
     tiles and of the keys that the queries see."""

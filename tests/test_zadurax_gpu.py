@@ -218,6 +218,22 @@ def test_the_memory_in_every_cut_in_pairs_of_chunks(H, d, dv, cap):
     test_the_memory_in_every_cut(H, d, dv, cap)
 
 
+@pytest.mark.parametrize("H, d, dv", [(2, 64, 72), (1, 128, 8), (3, 128, 256)])
+def test_pairs_of_chunks_of_short_sequences_beside_a_long_one(H, d, dv):
+    """A step of enough tokens a chunk goes by pairs, whatever the sequences beside the long one bring; so does the next."""
+    g = torch.Generator().manual_seed(H * 100 + dv)
+    run = MemoryRun(H, d, dv, 12.0, pad=(-2 * H) % 8, seed=d)
+    lengths, cut = (420, 2, 70, 66, 130, 18), (64, 1, 66, 65, 129, 1)
+    rows = [memory_rows(n, H, d, dv, run.pad, g) for n in lengths]
+    first, rest = [n - c for n, c in zip(lengths, cut)], list(cut)
+    assert run.ops.memory_by_pairs(first, H, d, dv, 148) and run.ops.memory_by_pairs(rest, H, d, dv, 148)
+    a = run.step([(s, r[:n]) for s, (r, n) in enumerate(zip(rows, first))])
+    b = run.step([(s, r[n:]) for s, (r, n) in enumerate(zip(rows, first))])
+    for r, x, y in zip(rows, a, b):
+        want, bound = run.plain(r)
+        close(torch.cat([x, y]), want, bound)
+
+
 @pytest.mark.parametrize("bad", [math.inf, math.nan])
 def test_values_that_are_no_numbers_stay_in_their_column(bad):
     H, d, dv, T = 2, 128, 256, 150
