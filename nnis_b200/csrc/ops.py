@@ -1541,7 +1541,12 @@ def retention(qkvg: torch.Tensor, freq: torch.Tensor, decay: torch.Tensor, state
                                  ctypes.c_float(dim ** -0.5 if key_scale is None else key_scale),
                                  _ptr(norm_weight), 1 if gate == "sigmoid" else 0, code_of(out.dtype),
                                  sm_count(out.device), _ptr(status_word(out.device)), _stream()),
-           "retention", 4 * -(-n_chunks // wave) + 1 if chunks is not None else 2)
+           "retention", retention_launches(n_chunks, units, heads, dim, vdim, wave) if chunks is not None else 2)
+
+
+def retention_launches(n_chunks: int, n_seqs: int, heads: int, dim: int, vdim: int, wave: int) -> int:
+    """Kernels that ``retention`` launches for a prompt step whose chunks are worked side by side, ``wave`` at a time."""
+    return int(_lib().nnis_retention_launches(n_chunks, n_seqs, heads, dim, vdim, wave))
 
 
 RETENTION_CHUNK = 64  # tokens of a chunk

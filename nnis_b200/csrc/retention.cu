@@ -498,8 +498,8 @@ retention_read_kernel(const float* __restrict__ packed, const float* __restrict_
     }
 }
 
-// Keys of 64 and 128, 64 values and more in whole groups of eight: `update` and `read` by pairs of chunks on the tensor cores
-// (with fewer values most of a tile of 128 columns would be padding).  A wave holds whole pairs, so that results have the same
+// Keys of 64 and 128, values in whole groups of eight: `update` and `read` by pairs of chunks on the tensor cores, where
+// retention_by_pairs says so.  A wave holds whole pairs, so that results have the same
 // bits however many fit it; its first chunk is the one at which the scratch begins.  A packed
 // (chunk, head) is then queries [64][dim], keys [64][dim] and values [64][vdim], rows of tokens that are not there left alone;
 // four CTAs a (chunk, head), 16 tokens each: 2,048 tokens, eight heads of 128 x 256, 37 -> 16 us (three layouts and powers of the
@@ -644,6 +644,17 @@ retention_read_split_kernel(const float* __restrict__ packed, const float* __res
         });
 }
 
+// Whether chunks go by pairs (with fewer than 64 values most of a tile of 128 columns would be padding).
+static bool retention_by_pairs(long long n_chunks, long long n_seqs, int heads, int dim, int vdim, int wave) {
+    if (vdim % 8 || (wave < 2 && n_chunks > 1)) return false;
+    return (dim == 128 || dim == 64) && vdim >= 64;
+}
+// Pairs: at most as many, and as many as the scratch holds at a time.
+static int retention_pairs(int n_chunks, int n_seqs) { return (n_chunks + n_seqs) / 2; }
+static int retention_pairs_held(int n_chunks, int n_seqs, int wave) {
+    return n_chunks <= wave ? retention_pairs(n_chunks, n_seqs) : wave / 2;
+}
+
 template <typename T>
 static int launch_chunks(const T* qkvg, const float* freq, const float* decay, float* state, const int* seq_slots,
                          const int* seq_first_row, const int* seq_start, const int* seq_count, const int* chunks,
@@ -651,13 +662,13 @@ static int launch_chunks(const T* qkvg, const float* freq, const float* decay, f
                          int n_seqs, int heads, int dim, int vdim, int rot_dims, int act, float k_scale, int sms, int* status,
                          cudaStream_t stream) {
     // (rows of q, k and v in whole groups of eight on 16-byte borders, float32 rows on 32-byte borders)
-    if ((dim == 64 || dim == 128) && vdim >= 64 && vdim % 8 == 0 && (wave >= 2 || n_chunks == 1) && (uintptr_t)qkvg % 16 == 0 &&
+    if (retention_by_pairs(n_chunks, n_seqs, heads, dim, vdim, wave) && (uintptr_t)qkvg % 16 == 0 &&
         ((uintptr_t)packed | (uintptr_t)chunk_state | (uintptr_t)o_raw) % 32 == 0) {
         cudaError_t e = cudaFuncSetAttribute(retention_update_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCrSmem);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(retention_read_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCrSmem);
-        const int all = (n_chunks + n_seqs) / 2, most = kCrTiles * kCrCols;  // pairs: at most as many
-        const int held = n_chunks <= wave ? all : wave / 2;
+        const int all = retention_pairs(n_chunks, n_seqs), most = kCrTiles * kCrCols;
+        const int held = retention_pairs_held(n_chunks, n_seqs, wave);
         for (int p0 = 0; p0 < all && e == cudaSuccess; p0 += held) {
             const int n = all - p0 < held ? all - p0 : held, cols = chunk_read_cols((long long)n * heads, vdim, sms);
             e = launch_dependent(retention_pack_rows_kernel<T>, dim3(2 * n, heads, 4), 256, 0, stream, qkvg, freq, chunks,
@@ -865,6 +876,14 @@ static int launch_retention(const void* qkvg, const float* freq, const float* de
 }  // namespace nnis
 
 using namespace nnis;
+
+// Kernels that a prompt step of these sizes launches, chunks side by side (qkvg on 16-byte, the scratch and o_raw on 32-byte
+// boundaries).
+NNIS_API int nnis_retention_launches(int n_chunks, int n_seqs, int heads, int dim, int vdim, int wave) {
+    if (!retention_by_pairs(n_chunks, n_seqs, heads, dim, vdim, wave)) return 4 * ((n_chunks + wave - 1) / wave) + 1;
+    const int all = retention_pairs(n_chunks, n_seqs), held = retention_pairs_held(n_chunks, n_seqs, wave);
+    return 4 * ((all + held - 1) / held) + 1;
+}
 
 // `seq_first_row` null: every row is a sequence of its own bringing one token
 // (`n_units` = n_tokens); else `n_units` sequences with their first row, first
