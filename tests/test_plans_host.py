@@ -286,9 +286,11 @@ def test_launches_of_retention_side_by_side_are_those_of_its_waves():
     """Four kernels a wave and the gate: waves of whole pairs where chunks go by pairs, of chunks where not."""
     from nnis_b200.csrc import ops as o
     launches = lambda chunks, seqs, dim, vdim, wave, heads=8: o.retention_launches(chunks, seqs, heads, dim, vdim, wave)
-    assert launches(32, 1, 128, 256, 32) == 5 and launches(100, 1, 128, 256, 3) == 4 * 50 + 1 and launches(100, 1, 128, 64, 2) == 4 * 50 + 1
+    assert launches(32, 1, 128, 256, 32) == 5 and launches(100, 1, 128, 256, 3) == 4 * 50 + 1 and launches(100, 1, 128, 8, 2) == 4 * 50 + 1
     assert launches(100, 1, 128, 256, 1) == 401 and launches(100, 1, 128, 250, 3) == 4 * 34 + 1 and launches(100, 1, 32, 64, 3) == 4 * 34 + 1
     assert launches(48, 16, 64, 256, 10) == 4 * 7 + 1  # 32 pairs at most, five at a time
+    # small heads: by pairs where sequences are long and many CTAs come of them
+    assert launches(63, 1, 64, 64, 6) == 4 * 11 + 1 and launches(12, 1, 64, 64, 6) == 4 * 2 + 1 and launches(48, 16, 64, 64, 10) == 4 * 5 + 1
 
 
 def test_chunks_of_recurrent_layers_keep_their_scratch_within_its_bound():

@@ -387,6 +387,42 @@ def test_retention_of_prompts_in_pairs_of_chunks(dim, vdim, dtype, act):
     test_retention_of_prompts_in_chunks(dim, vdim, dtype, act, False)
 
 
+@pytest.mark.parametrize("dim,vdim", [(128, 8), (128, 40), (128, 56)])
+@pytest.mark.parametrize("dtype,act", [("float32", True), ("bfloat16", False)])
+def test_retention_of_prompts_in_pairs_of_chunks_with_few_values(dim, vdim, dtype, act):
+    """A tile of 128 columns of which most are not there."""
+    test_retention_of_prompts_in_chunks(dim, vdim, dtype, act, False)
+
+
+@pytest.mark.parametrize("vdim", [8, 40, 64])
+def test_retention_of_long_prompts_in_pairs_of_chunks_with_small_heads(vdim):
+    """Heads of 64 keys and few values go by pairs where sequences are long and many CTAs come of them: against the kernel
+    that works the tokens in order."""
+    o = ops()
+    g = torch.Generator().manual_seed(vdim)
+    H, dim, new, starts = 4, 64, [1500, 129], [0, 70]
+    n = sum(new)
+    chunks, first = (torch.from_numpy(t).to(DEV) for t in o.scan_segments(new, o.RETENTION_CHUNK))
+    by_pairs, one_by_one = (o.retention_launches(c, s, H, dim, vdim, 20) for c, s in ((len(chunks), 2), (len(chunks), 9)))
+    assert (by_pairs, one_by_one) == (4 * 2 + 1, 4 * 2 + 1) and o.retention_launches(len(chunks), 2, H, dim, vdim, 3) == 4 * 14 + 1
+    rows = torch.randn(n, 2 * H * (dim + vdim), generator=g).to(DEV)
+    decay, freq = torch.tensor([0.97, 0.5, 0.999, 0.9], device=DEV), torch.ones(1, device=DEV)
+    begin = torch.randn(2, H, dim, vdim, generator=g)
+    begin[0] = 0.0
+    tables = [i32(x) for x in ([st + t for st, c in zip(starts, new) for t in range(c)], [0] * new[0] + [1] * new[1], [0, 1],
+                               [0, new[0]], starts, new)]
+    sizes = o.retention_scratch(len(chunks), H, dim, vdim)
+    got = []
+    for side in (dict(chunks=chunks, seq_first_chunk=first, packed=torch.full((sizes[0],), math.nan, device=DEV),
+                      chunk_state=torch.full((sizes[1],), math.nan, device=DEV)), {}):
+        state, o_raw = begin.to(DEV), torch.full((n, H * vdim), 5.0, device=DEV)
+        o.retention(rows, freq, decay, state, *tables, o_raw, torch.empty(n, H * vdim, device=DEV), H, dim, vdim, 0, 1e-5, **side)
+        got.append((o_raw, state))
+    o.check_status(DEV)
+    for x, y in zip(*got):  # (each within 2e-6 of 64 bits, as above)
+        assert float((x - y).abs().max() / y.abs().max()) < 4e-6
+
+
 @pytest.mark.parametrize("wave", [2, 3, 5])
 def test_retention_pairs_of_chunks_in_waves(wave, monkeypatch):
     """The same bits however many pairs the scratch holds, with more sequences than a warp looks through at once."""
