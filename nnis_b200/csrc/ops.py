@@ -846,28 +846,44 @@ def _f32_warps_time(counts, starts, window: int, heads: int) -> float:
     return 3.0 + max(0.165 * longest, 9.2e-5 * keys * heads)
 
 
-def attention_split_f32_plan(counts, starts, window: int, heads: int, sms: int):
-    """Work list of ``attention_split_f32`` (int32 [n, 4] = (sequence, first query of 128, slice, slices of the tile), most pages
-    first) and the most slices of a tile; None where a warp for every query (attention_generic.cu) is thought to be faster.
+SPLIT_F32_SCRATCH = 1 << 27  # bytes of the slices' records; 9 heads of 64 fill it with two slices of 28,000 tokens
 
-    A unit takes as long as its pages and two more, 3.1 us each; with more units than SMs the last ones end half a unit late;
-    records of slices have to be put together.  9 heads of 64 on a B200, us by warps, by tiles of 64 queries on the CUDA cores
-    and here: prompts of 509, 131 and 384 tokens 221 / 55 / 23, 1,024 497 / 88 / 38, 3 x 1,024 1,307 / 227 / 79, 64 13.7 / 11.5 / 8.8,
-    17 after 500 90 / 46 / 11, 64 after 2,000 358 / 49 / 19, 10 x 100 60 / 25 / 13; 17 6.6 / 9.4 / 7.7, 64 x 8 7.9 / 24 / 35,
-    300 in a window of 30 12.5 / 20 / 14."""
-    import numpy as np
-    tiles = []  # (sequence, first query, pages)
+
+def _f32_tiles(counts, starts, window: int):
+    """(sequence, first query, pages of 64 keys) of a step's tiles of 128 queries."""
+    tiles = []
     for i, (c, st) in enumerate(zip(counts, starts)):
         for q0 in range(0, int(c), 128):
             first, last = int(st) + q0, int(st) + min(q0 + 128, int(c)) - 1
             lo = max(0, first - window + 1) if window > 0 else 0
             tiles.append((i, q0, last // 64 - lo // 64 + 1))
+    return tiles
+
+
+def attention_split_f32_plan(counts, starts, window: int, heads: int, sms: int):
+    """Work list of ``attention_split_f32`` (int32 [n, 4] = (sequence, first query of 128, slice, slices of the tile), most pages
+    first) and the most slices of a tile; None where a warp for every query (attention_generic.cu) is thought to be faster.
+
+    A unit takes as long as its pages and two more, 3.1 us each; with more units than SMs the last ones end half a unit late;
+    records of slices have to be put together, which costs a launch, and their bytes twice, and they never fill more than
+    SPLIT_F32_SCRATCH.  9 heads of 64 on a B200, us by warps, by tiles of 64 queries on the CUDA cores
+    and here: prompts of 509, 131 and 384 tokens 221 / 55 / 23, 1,024 497 / 88 / 38, 3 x 1,024 1,307 / 227 / 79, 64 13.7 / 11.5 / 8.8,
+    17 after 500 90 / 46 / 11, 64 after 2,000 358 / 49 / 19, 10 x 100 60 / 25 / 13; 17 6.6 / 9.4 / 7.7, 64 x 8 7.9 / 24 / 35,
+    300 in a window of 30 12.5 / 20 / 14.  With the price of their bytes 3 x 1,024 of 9 heads, 2,048 after 2,048 and 8,192 of 32 heads
+    are no longer cut: 82 -> 79, 209 -> 191, 2,975 -> 2,865."""
+    import numpy as np
+    tiles = _f32_tiles(counts, starts, window)
     pages, most = sum(t[2] for t in tiles), max(t[2] for t in tiles)
+    rows = [min(128, int(counts[i]) - q0) for i, q0, _ in tiles]
+    record = 4 * heads * (64 + 2)  # bytes of a row's
     best = None
     for per in sorted({-(-most // s) for s in range(1, min(16, most) + 1)}):
+        if per < most and sum(rows) * record * -(-most // per) > SPLIT_F32_SCRATCH:
+            continue
         units = sum(-(-t[2] // per) for t in tiles)
         time = per + 2.0 if units * heads <= sms else max(per + 2.0, (pages + 2.0 * units) * heads / sms + (per + 2.0) / 2)
-        time += 1.6 if per < most else 0.0
+        if per < most:  # (20 MB are a unit's time at 6.5 TB/s)
+            time += 1.6 + 2 * record * sum(r * -(-t[2] // per) for r, t in zip(rows, tiles)) / 20e6
         if best is None or time < best[0]:
             best = time, per
     if 3.1 * best[0] > _f32_warps_time(counts, starts, window, heads):

@@ -345,6 +345,19 @@ def test_float32_prompts_take_tiles_where_these_pay():
             assert pays([c], [st], window, 1000) == (pages * 1000 <= keys * 2)
 
 
+def test_slices_of_the_float32_prompt_attention_keep_their_scratch_within_its_bound():
+    """Records are as many as the most slices of any tile for every row of the step; long steps are cut less, or not."""
+    from nnis_b200.csrc import ops as o
+    for heads in (1, 9, 32, 128):
+        for counts, starts in (([65536], [0]), ([16384], [49152]), ([8192], [0]), ([8192], [8192]), ([1] * 3000 + [128], [0] * 3000 + [60000]),
+                               ([4096] * 8, [0] * 8), ([30000], [0]), ([1024], [0])):
+            for sms in (40, 148, 1000):
+                plan = o.attention_split_f32_plan(counts, starts, 0, heads, sms)
+                if plan is not None and plan[1] > 1:
+                    assert 4 * sum(counts) * heads * plan[1] * (64 + 2) <= o.SPLIT_F32_SCRATCH <= 1 << 28
+    assert o.attention_split_f32_plan([1024], [0], 0, 9, 148)[1] > 1 and o.attention_split_f32_plan([65536], [0], 0, 9, 148)[1] == 1
+
+
 def test_units_of_the_float32_prompt_attention_cover_every_tile_once():
     import random
     from nnis_b200.csrc import ops as o
