@@ -1,5 +1,5 @@
-// Prompt attention in true float32 over the paged cache, for head sizes (and steps) that attention_split_f32.cu does not
-// take: 64 consecutive queries of a sequence and one query head
+// Prompt attention in true float32 over the paged cache, for head sizes that attention_split_f32.cu does not take and, with
+// heads of 64, for steps of many prompts that see one page each: 64 consecutive queries of a sequence and one query head
 // per CTA, a page of 64 keys at a time.  Both products are tiled in registers (4 queries x 4 keys, then 4 queries
 // x 4 or 8 output values a thread), so a key or value fetched once serves 64 queries; the any-size kernel
 // (attention_generic.cu), which this one takes prompts from, reads every key again for every query.  Scores,

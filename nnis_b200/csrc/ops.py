@@ -860,9 +860,15 @@ def _f32_tiles(counts, starts, window: int):
     return tiles
 
 
+def attention_f32_single_pages(counts, starts, window: int) -> bool:
+    """Whether no tile of a step sees more than one page: prompts of at most 64 tokens with little before them."""
+    return all(int(c) <= 64 for c in counts) and all(t[2] == 1 for t in _f32_tiles(counts, starts, window))
+
+
 def attention_split_f32_plan(counts, starts, window: int, heads: int, sms: int):
     """Work list of ``attention_split_f32`` (int32 [n, 4] = (sequence, first query of 128, slice, slices of the tile), most pages
-    first) and the most slices of a tile; None where a warp for every query (attention_generic.cu) is thought to be faster.
+    first) and the most slices of a tile; None where another kernel is thought to be faster: a warp for every query
+    (attention_generic.cu), or tiles of 64 queries on the CUDA cores (attention_tile_f32.cu) where each sees one page.
 
     A unit takes as long as its pages and two more, 3.1 us each; with more units than SMs the last ones end half a unit late;
     records of slices have to be put together, which costs a launch, and their bytes twice, and they never fill more than
@@ -870,7 +876,8 @@ def attention_split_f32_plan(counts, starts, window: int, heads: int, sms: int):
     and here: prompts of 509, 131 and 384 tokens 221 / 55 / 23, 1,024 497 / 88 / 38, 3 x 1,024 1,307 / 227 / 79, 64 13.7 / 11.5 / 8.8,
     17 after 500 90 / 46 / 11, 64 after 2,000 358 / 49 / 19, 10 x 100 60 / 25 / 13; 17 6.6 / 9.4 / 7.7, 64 x 8 7.9 / 24 / 35,
     300 in a window of 30 12.5 / 20 / 14.  With the price of their bytes 3 x 1,024 of 9 heads, 2,048 after 2,048 and 8,192 of 32 heads
-    are no longer cut: 82 -> 79, 209 -> 191, 2,975 -> 2,865."""
+    are no longer cut: 82 -> 79, 209 -> 191, 2,975 -> 2,865.  Of a tile with 64 tokens half is not there: 40 x 64 with 4, 9, 16 and
+    32 heads takes tiles of 64 queries 16.8, 22.6, 36 and 60 us, this kernel 17.3, 28, 46 and 84; 8 x 64 with 32 heads 17.9 and 18.6."""
     import numpy as np
     tiles = _f32_tiles(counts, starts, window)
     pages, most = sum(t[2] for t in tiles), max(t[2] for t in tiles)
@@ -886,7 +893,10 @@ def attention_split_f32_plan(counts, starts, window: int, heads: int, sms: int):
             time += 1.6 + 2 * record * sum(r * -(-t[2] // per) for r, t in zip(rows, tiles)) / 20e6
         if best is None or time < best[0]:
             best = time, per
-    if 3.1 * best[0] > _f32_warps_time(counts, starts, window, heads):
+    others = _f32_warps_time(counts, starts, window, heads)
+    if attention_f32_single_pages(counts, starts, window):
+        others = min(others, max(11.5, 7.5 + 0.041 * len(tiles) * heads * 148 / sms))
+    if 3.1 * best[0] > others:
         return None
     units = []
     for i, q0, n in tiles:

@@ -115,22 +115,29 @@ class Attention(Part):
         tcgen05 kernels (head sizes 64 and 128), shared by all layers with this window
         and number of heads, where they pay; else the 64-query tiles of the
         mma.sync kernel (head sizes 64 and 128), the same for every layer.  In float32
-        the units of the tensor cores' kernel (head size 64), else 64-query tiles, the ones
-        with the most keys first, where they pay."""
+        the units of the tensor cores' kernel (head size 64) where it pays; 64-query tiles, the ones
+        with the most keys first, for other head sizes and for steps of single pages, where those pay."""
         if self.dtype != torch.bfloat16:
-            name = self._split_f32_name()
-            if self._split_f32(self.heads * self.head_dim):  # (or a warp for every query)
-                plan = None if name + "/units" in have else ops.attention_split_f32_plan(
-                    counts, starts, self.window, self.heads, ops.sm_count(self.device))
-                return {} if plan is None else {
-                    name + "/units": plan[0], name + "/slices": np.asarray([plan[1]], dtype=np.int32)}
-            name = self._tile_f32_name()
+            split, name = self._split_f32(self.heads * self.head_dim), self._tile_f32_name()
+            tables: Dict[str, object] = {}
+            if split:
+                plan_name = self._split_f32_name()
+                if plan_name + "/planned" in have:  # (a step is looked at once, whatever comes of it)
+                    return {}
+                plan = ops.attention_split_f32_plan(counts, starts, self.window, self.heads, ops.sm_count(self.device))
+                tables[plan_name + "/planned"] = np.asarray([plan is not None], dtype=np.int32)
+                if plan is not None:
+                    tables.update({plan_name + "/units": plan[0],
+                                   plan_name + "/slices": np.asarray([plan[1]], dtype=np.int32)})
+                if plan is not None or not ops.attention_f32_single_pages(counts, starts, self.window):
+                    return tables
             if name in have or not self._tile_f32(self.heads * self.head_dim) \
                     or not ops.attention_tile_f32_pays(counts, starts, self.window, self.heads):
-                return {}
+                return tables
             tiles = sorted(((i, q0) for i, c in enumerate(counts) for q0 in range(0, int(c), 64)),
                            key=lambda t: -(starts[t[0]] + t[1]))
-            return {name: np.asarray(tiles, dtype=np.int32).reshape(-1, 2)}
+            tables[name] = np.asarray(tiles, dtype=np.int32).reshape(-1, 2)
+            return tables
         name = self._tc_plan_name()
         if ops.attention_prefill_tc_takes(self.head_dim, PAGE_SIZE, self.heads * self.head_dim) \
                 and ops.prefill_tc_pays(counts, starts, self.window):

@@ -345,6 +345,32 @@ def test_float32_prompts_take_tiles_where_these_pay():
             assert pays([c], [st], window, 1000) == (pages * 1000 <= keys * 2)
 
 
+def test_which_kernel_takes_a_float32_prompt_step_of_heads_of_64(monkeypatch):
+    """Tiles of 128 queries on the tensor cores, tiles of 64 for many prompts of one page, a warp a query for few short ones;
+    a step is planned once for all layers with its window and heads."""
+    import torch
+    from nnis_b200.csrc import ops as o
+    from nnis_b200.parts.attention import Attention
+    monkeypatch.setattr(o, "sm_count", lambda device: 148)
+    monkeypatch.setattr(o, "TC_ATTENTION", 1)
+
+    def kinds(counts, starts=None, heads=9, window=0):
+        part = Attention.__new__(Attention)
+        part.dtype, part.heads, part.head_dim, part.window, part.device = torch.float32, heads, 64, window, "cpu"
+        starts = starts or [0] * len(counts)
+        tables = part.step_tables(counts, starts)
+        assert part.step_tables(counts, starts, tuple(tables)) == {}
+        tiles = [v for k, v in tables.items() if k == part._tile_f32_name()]
+        if tiles:
+            assert sorted(tiles[0].tolist()) == [[i, q0] for i, c in enumerate(counts) for q0 in range(0, c, 64)]
+        units = any(k.endswith("/units") for k in tables)
+        assert not (units and tiles)
+        return "tcgen05" if units else "tiles" if tiles else "warps"
+    assert kinds([1024]) == kinds([64]) == kinds([100] * 10) == kinds([64] * 8) == kinds([17], [500]) == kinds([65] * 40) == "tcgen05"
+    assert kinds([64] * 40) == kinds([50] * 40) == kinds([40] * 8, heads=32) == kinds([64] * 40, heads=4) == "tiles"
+    assert kinds([17]) == kinds([8] * 64) == kinds([300], window=30) == kinds([20] * 40, heads=32) == "warps"
+
+
 def test_slices_of_the_float32_prompt_attention_keep_their_scratch_within_its_bound():
     """Records are as many as the most slices of any tile for every row of the step; long steps are cut less, or not."""
     from nnis_b200.csrc import ops as o
