@@ -152,11 +152,11 @@ moe_route_kernel(const T* __restrict__ h, const float* __restrict__ wr, const fl
     // the `top` largest, one after another; the lanes of one warp share the search
     float first = 0.f, total = 0.f;
     for (int s = 0; s < top; ++s) {
-        float best = -FLT_MAX;
+        float best = -INFINITY;
         int arg = 0x7fffffff;
         for (int e = lane; e < experts; e += 32) {
             float v = z[e];
-            if (v > best) {  // (ascending e: the lower index wins a tie)
+            if (v > best || (v == best && arg == 0x7fffffff)) {  // (ascending e: the lower index wins a tie, of -inf too)
                 best = v;
                 arg = e;
             }
@@ -170,7 +170,7 @@ moe_route_kernel(const T* __restrict__ h, const float* __restrict__ wr, const fl
                 arg = oa;
             }
         }
-        if (arg >= experts) {  // (no logit left that is a number: nothing to choose by, and the token's output shows it)
+        if (arg >= experts) {  // (all logits left are NaN: nothing to choose by, and the token's output shows it)
             arg = s;
             best = NAN;
         }
@@ -180,7 +180,7 @@ moe_route_kernel(const T* __restrict__ h, const float* __restrict__ wr, const fl
         if (lane == 0) {
             id[s] = arg;
             wt[s] = p;
-            z[arg] = -FLT_MAX;
+            z[arg] = NAN;  // (chosen: no comparison holds)
         }
         __syncwarp();
     }

@@ -44,6 +44,32 @@ def test_router_of_few_and_of_many_tokens(n, width, experts, top, sigmoid):
             assert torch.allclose(weights[t], share, atol=1e-4)
 
 
+@pytest.mark.parametrize("n", [3, 520])
+@pytest.mark.parametrize("hidden", [-math.inf, torch.finfo(torch.float32).min])
+@pytest.mark.parametrize("sigmoid", [False, True])
+def test_router_with_experts_that_are_masked_out(n, hidden, sigmoid):
+    """A bias of minus infinity, or of the type's lowest value, is a logit like any other: chosen last, by index, with no
+    weight; a token with fewer other logits than choices still has numbers."""
+    o = ops()
+    g = torch.Generator().manual_seed(n)
+    width, experts, top = 36, 40, 6
+    h, wr, br = torch.randn(n, width, generator=g), torch.randn(experts, width, generator=g), torch.full((experts,), hidden)
+    seen = [3, 17, 33, 38]
+    br[seen] = torch.randn(4, generator=g)
+    ids = torch.full((n, top), 77, dtype=torch.int32, device=DEV)
+    weights = torch.full((n, top), 7.0, device=DEV)
+    o.moe_route(h.to(DEV), wr.to(DEV), br.to(DEV), torch.zeros(n, dtype=torch.int32, device=DEV), ids, weights, top,
+                sigmoid_scores=sigmoid)
+    z = h.double() @ wr.double().t() + br.double()
+    order = torch.sort(z[:, seen], descending=True).indices
+    want = torch.tensor(seen)[order]
+    assert torch.equal(ids[:, :4].cpu().long(), want) and (ids[:, 4:].cpu() == torch.tensor([0, 1])).all()
+    got = z.gather(1, want)
+    share = torch.sigmoid(got) if sigmoid else torch.softmax(got, 1)
+    # (float32 sums of `width` products: 1e-4 of logits of about sqrt(width))
+    assert torch.allclose(weights[:, :4].cpu().double(), share, atol=1e-4) and (weights[:, 4:] == 0.0).all()
+
+
 @pytest.mark.parametrize("dim,rot,heads", [(16, 4, 3), (48, 16, 2), (144, 8, 5), (504, 8, 2)])
 @pytest.mark.parametrize("splits", [2, 8, 9, 64])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
