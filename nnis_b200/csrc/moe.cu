@@ -71,10 +71,10 @@ __device__ __forceinline__ float warp_row_dot(const T* __restrict__ a, const T* 
 }
 
 // A CTA of `blockDim.x` / 32 warps takes TOK tokens.  With one token a warp takes an output at a time, and the launch brings
-// 32 warps, so that one SM asks L2 for a matrix of 32 rows at once (8 tokens, 32 experts, width 2,048: 9.9 -> 5.3 us).  With eight tokens a warp takes EXP rows of the matrix and all tokens, so a piece of a row is fetched once
-// for eight tokens and a piece of a token once for EXP rows (2,048 tokens of that layer: @R2@: every token's CTA
-// fetched the whole matrix, half a gigabyte from L2).  A logit is the same chain of multiply-adds either way.  Then warp k
-// chooses for token k.
+// 32 warps, so that one SM asks L2 for a matrix of 32 rows at once (8 tokens, 32 experts, width 2,048: 9.9 -> 5.3 us).  With
+// eight tokens a warp takes EXP rows of the matrix and all tokens, so a piece of a row is fetched once for eight tokens and a
+// piece of a token once for EXP rows (2,048 tokens of that layer: 40 -> 16 us, as every token's CTA fetched the whole matrix,
+// half a gigabyte from L2).  A logit is the same chain of multiply-adds either way.  Then warp k chooses for token k.
 template <typename T, int TOK, int EXP>
 __global__ void __launch_bounds__(TOK == 1 ? 1024 : 256)
 moe_route_kernel(const T* __restrict__ h, const float* __restrict__ wr, const float* __restrict__ br,
@@ -459,9 +459,9 @@ using namespace nnis;
 
 NNIS_API int nnis_moe_route(const void* h, const float* wr, const float* br, const int* token_pos,
                             int* ids, float* weights, int n_tokens, int width, int experts, int top,
-                            int sigmoid_scores, int dtype, cudaStream_t stream) {
+                            int sigmoid_scores, int dtype, int sm_count, cudaStream_t stream) {
     if (n_tokens <= 0 || width <= 0 || experts <= 0 || top <= 0 || top > experts || !h || !wr || !ids ||
-        !weights || !token_pos)
+        !weights || !token_pos || sm_count <= 0)
         return NNIS_ERR_ARGUMENT;
     const size_t per = (size_t)experts * sizeof(float);
     if (per > 48 * 1024) return NNIS_ERR_UNSUPPORTED;
@@ -469,11 +469,12 @@ NNIS_API int nnis_moe_route(const void* h, const float* wr, const float* br, con
     // 10 at 300 (32 experts, width 2,048; 64 experts, width 1,536: 17 against 22 and 16)
     const bool several = n_tokens >= 512 && 8 * per <= 48 * 1024;
     const unsigned blocks = several ? (unsigned)((n_tokens + 7) / 8) : (unsigned)n_tokens;
-    const unsigned threads = several || n_tokens > 2 * 148 ? 256 : 32 * (unsigned)(experts < 32 ? (experts < 8 ? 8 : experts) : 32);
+    // a warp an expert, up to 32, while CTAs of 1,024 threads have an SM each, or share it by twos
+    const unsigned warps = several || n_tokens > 2 * sm_count ? 8 : (unsigned)(experts < 8 ? 8 : experts < 32 ? experts : 32);
     const size_t smem = several ? 8 * per : per;
     cudaError_t e;
 #define NNIS_ROUTE(T, TOK, EXP) \
-    launch_dependent(moe_route_kernel<T, TOK, EXP>, blocks, threads, smem, stream, (const T*)h, wr, br, token_pos, \
+    launch_dependent(moe_route_kernel<T, TOK, EXP>, blocks, 32 * warps, smem, stream, (const T*)h, wr, br, token_pos, \
                      ids, weights, n_tokens, width, experts, top, sigmoid_scores)
     if (dtype == NNIS_DTYPE_F32)
         e = several ? NNIS_ROUTE(float, 8, 4) : NNIS_ROUTE(float, 1, 1);

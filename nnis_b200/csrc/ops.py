@@ -1631,7 +1631,7 @@ def moe_route(h: torch.Tensor, w_router: torch.Tensor, b_router: Optional[torch.
           and weights.numel() >= n * top and 0 < top <= experts, "moe_route: ids int32, weights float32 [n, top]")
     _check(_lib().nnis_moe_route(_ptr(h), _ptr(w_router), _ptr(b_router), _ptr(token_pos), _ptr(ids),
                                  _ptr(weights), n, width, experts, top, 1 if sigmoid_scores else 0,
-                                 code_of(h.dtype), _stream()),
+                                 code_of(h.dtype), sm_count(h.device), _stream()),
            "moe_route")
 
 
