@@ -5,14 +5,14 @@
 // them: a token of 16 heads leaves three warps of four without rows, and the fourth multiplies a page's scores and values
 // alone, one after another (8 tokens x 16 heads of 512 + 64 over 2,048 keys: 24.5 us).  Here the eight warps share a page:
 // each takes eight of its keys for the scores, two of the 16 rows for the softmax (which meets in shared memory) and every
-// eighth tile of 16 values for the output, whose sums it keeps in registers.  Pages come by bulk copies, a row a copy
-// (rows are 16 bytes further apart in shared memory than in the cache, so that eight of them meet no bank twice), all that
-// the ring holds before the wait for the kernel before: only the row of this step's token and the queries are fetched
-// after it.  Rows that the token does not see are zero, whatever the page holds there.
-// What bounds it: a chain of few products and three barriers a page, and the slices' way into the merge.  16 heads of 512 + 64, merge included, in us in a
-// graph, the kernel of prompts -> here: 8 tokens over 2,048 keys in 16 slices 28.8 -> 15.9, over 512 in 8 17.2 -> 10.8; one
-// token over 2,048 26.9 -> 14.2; 32 tokens over 512 in 4 27.3 -> 14.0; a page of a slice 8 -> 2.6.  8 heads of 256 + 32, 8 tokens
-// over 2,048 keys in 16: 18.4 -> 10.2.
+// eighth tile of 16 values for the output, whose sums it keeps in registers.  Pages come by TMA, a copy for 64 of a row's
+// values (boxes of 64 rows of 128 bytes in the 128-byte swizzle, so that eight rows meet no bank twice; the queries' rows are
+// padded by 16 bytes instead), all that the ring holds before the wait for the kernel before: only the row of this step's
+// token and the queries are fetched after it.  Rows that the token does not see are zero, whatever the page holds there.
+// What bounds it: a chain of few products and three barriers a page, and the slices' way into the merge.  16 heads of 512 +
+// 64, merge included, in us in a graph, the kernel of prompts -> here: 8 tokens over 2,048 keys in 16 slices 28.8 -> 15.9,
+// over 512 in 8 17.2 -> 10.8; one token over 2,048 26.9 -> 14.2; 32 tokens over 512 in 4 27.3 -> 14.0; a page of a slice
+// 8 -> 2.6.  8 heads of 256 + 32, 8 tokens over 2,048 keys in 16: 18.4 -> 10.2.
 #include "attention_merge.cuh"
 #include "mma_helpers.cuh"
 #include "tcgen05_helpers.cuh"
@@ -34,8 +34,8 @@ __device__ __forceinline__ unsigned char* page_chunk(unsigned char* page, int ro
 
 template <int STAGES>
 __global__ void __launch_bounds__(kLdWarps * 32)
-latent_decode_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restrict__ q, const bf16* __restrict__ cache, const int* __restrict__ token_pos,
-                     const int* __restrict__ token_seq, const int* __restrict__ page_table, int table_cols,
+latent_decode_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restrict__ q, const bf16* __restrict__ cache,
+                     const int* __restrict__ token_pos, const int* __restrict__ token_seq, const int* __restrict__ page_table, int table_cols,
                      bf16* __restrict__ out, float* __restrict__ partial, int heads, int dk, int dv, int head_tiles,
                      float scale, int n_splits, int window, const float* __restrict__ gate,
                      const float* __restrict__ sink, int* __restrict__ status) {
@@ -52,7 +52,10 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map, const bf16* __rest
     const int n = blockIdx.x / head_tiles, h0 = (blockIdx.x - n * head_tiles) * kLdRows;
     const int rows = min(kLdRows, heads - h0), split = blockIdx.y;
     const int pos = token_pos[n];
-    if (pos < 0) return;  // (a padding row: the merge and the projections after it read nothing of it)
+    if (pos < 0) {  // (a padding row: the merge and the projections after it read nothing of it)
+        pdl_wait();  // (a grid of such rows alone must not be over before the kernel ahead, which later ones count on)
+        return;
+    }
     const int lo = window > 0 ? max(0, pos - window + 1) : 0, hi = pos + 1;  // keys that the token sees
     const int seen_page = lo / kLdPage, end_page = (hi - 1) / kLdPage + 1;
     const int per = (end_page - seen_page + n_splits - 1) / n_splits;

@@ -409,12 +409,24 @@ def test_units_of_the_float32_prompt_attention_cover_every_tile_once():
         assert max(k for _, _, _, k in units.tolist()) == slices
 
 
-def test_stores_into_the_latent_ring_are_fenced_before_the_copies_over_them():
-    """Ordinary stores and bulk copies to the same shared memory are ordered by a proxy fence of the storing threads alone; no
-    result shows that it is missing, so the kernel's text is looked at: from the zeroed rows to the next barrier."""
+def _latent_decode_source():
     import os
     from nnis_b200 import csrc
     with open(os.path.join(os.path.dirname(csrc.__file__), "attention_latent_decode.cu")) as f:
-        text = f.read()
+        return f.read()
+
+
+def test_stores_into_the_latent_ring_are_fenced_before_the_copies_over_them():
+    """Ordinary stores and bulk copies to the same shared memory are ordered by a proxy fence of the storing threads alone; no
+    result shows that it is missing, so the kernel's text is looked at: from the zeroed rows to the next barrier."""
+    text = _latent_decode_source()
     stores = text[text.index("if (row < r0 || row >= r1) *at ="):]
     assert "fence.proxy.async.shared::cta" in stores[:stores.index("__syncthreads()")]
+
+
+def test_padding_rows_of_latent_decode_wait_for_the_kernel_ahead_too():
+    """What comes after a kernel counts on all before it being over; a grid of padding rows alone (the run before a capture)
+    that returns at once would break the chain, and no result shows it."""
+    text = _latent_decode_source()
+    padding = text[text.index("if (pos < 0)"):]
+    assert "pdl_wait();" in padding[:padding.index("return;")]
