@@ -2,10 +2,11 @@
 // value taken as the exact sum of three bfloat16 values.
 //
 // A float32 value x has 24 significant bits.  h = bfloat16(x), m = bfloat16(x - h) and l = bfloat16(x - h - m) hold them
-// all (both differences are exact), and bfloat16 has float32's range of exponents, so no scaling is needed.  Of the nine
-// products of two such sums the six largest are made (h h, h m, m h, m m, h l, l h); what is left out is 2^-27 of a
-// product and less, where float32 rounds every sum at 2^-24.  The tensor cores cut their running sum off instead of
-// rounding it, so no sum stays there for long: 64 columns of K at a time, the small products first, and then the 64
+// all (both differences are exact) from 2^-109 on; bfloat16 has float32's range of exponents, so no scaling is needed, but
+// below that the last part falls under its smallest number, and what is lost is at most 2^-134 a value.  Of the nine
+// products of two such sums the six largest are made (h h, h m, m h, m m, h l, l h); what is left out (m l, l m, l l) is
+// 2^-26 of a product and less, where float32 rounds every sum at 2^-24.  The tensor cores cut their running sum off instead
+// of rounding it, so no sum stays there for long: 64 columns of K at a time, the small products first, and then the 64
 // columns' sum is added in registers, by an ordinary float32 addition.  Against 64-bit sums this is closer than the
 // chains of float32 multiply-adds of gemm_simt.cu (figures at the bottom of this comment).
 //
@@ -14,8 +15,8 @@
 //
 // One CTA works a tile of 128 x BN (BN 64 or 128), KS CTAs of a cluster share the tile's K and add their sums through
 // distributed shared memory, in the order of their ranks (the same bits every time).  Roles:
-//   warp 0       (BN = 64: two warps) allocates tensor memory; one lane issues tcgen05.mma (kind::f16, 128 x BN x 16), 24 for 64 columns of K,
-//                into one of four accumulators;
+//   warp 0       (BN = 64: two warps) allocates tensor memory; one lane issues tcgen05.mma (kind::f16, 128 x BN x 16),
+//                24 for 64 columns of K, into one of four accumulators;
 //   16 others    bring A and W, 32 bytes a load, one block of K ahead in registers, write the three parts of each value
 //                into swizzled shared memory (two or three blocks of K), and read the accumulator of two blocks before with
 //                tcgen05.ld and add it to their registers (a row and a quarter of the columns a thread); at the end they
@@ -29,8 +30,9 @@
 // 2,048 x 2,048 x 2,048 416 -> 123 (140 TFLOP/s of float32), 17 x 576 x 576 35 -> 14.  Distance from 64-bit sums (2-norm, K =
 // 576 / 1,536 / 5,632): 2.2e-7 / 3.5e-7 / 6.7e-7 there, 0.98e-7 / 1.1e-7 / 1.5e-7 here.
 // The gated product also applies silu and multiplies: a pass of 7 us over 1,024 x 3,072 less.
-// Level: tiles of 256 x 128 worked by pairs of CTAs (cta_group::2, 192 instead of 256 rows split a block: 49 and 50 us at 1,024 x
-// 3,072 x 576, 160 and 162 at 1,024 x 2,048 x 5,632); eight warps that split and eight that add (158 us at 1,024 x 2,048 x 5,632 here, 180 there).
+// Level: tiles of 256 x 128 worked by pairs of CTAs (cta_group::2, 192 instead of 256 rows split a block: 49 and 50 us at
+// 1,024 x 3,072 x 576, 160 and 162 at 1,024 x 2,048 x 5,632).  Slower: eight warps that split and eight that add (158 us at
+// 1,024 x 2,048 x 5,632 here, 180 there).
 // Every wait is bounded, as in gemm_tcgen05.cu.
 // NNIS: crates/nnis-kernels/src/gemm.rs:16-64 (tiled float32 product on CUDA cores).
 #include "split_parts.cuh"
