@@ -339,26 +339,30 @@ __global__ void add_rows_kernel(float* __restrict__ a, const float* __restrict__
 // of a gate that scales the expert's whole output.  u float32 [n, inter + gated]
 // (`gated` columns beyond the activation's: the gate, then padding).
 // ---------------------------------------------------------------------------
-// Four values a thread, 256 apart, all asked for at once, the gate once a thread (a thread a value, its row by a division of 64
-// bits: 13 us for 2,048 rows of 1,408; now 5.5).
-template <typename T>
+// 2^log_lanes threads a row and four values a thread, as far apart, all asked for at once, the gate once a thread.  Rows of 1,024
+// values and more take a CTA of 256 threads each, shorter ones share it (a thread a value, its row by a division of 64 bits: 12.5
+// us for 2,048 rows of 1,408, 21 for 20,000 of 256, 17.7 for 65,536 of 64; now 5.0, 6.9 and 5.9; a CTA a row took 21 and 69 for
+// the last two).
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(256)
-relu2_gate_kernel(const float* __restrict__ u, T* __restrict__ out, int inter, int gated) {
+relu2_gate_kernel(const float* __restrict__ u, T* __restrict__ out, long long n_rows, int inter, int gated, int log_lanes) {
     pdl_wait();
     pdl_launch_dependents();
-    const size_t n = blockIdx.x;
+    const int lanes = WIDE ? 256 : 1 << log_lanes;
+    const size_t n = WIDE ? blockIdx.x : (size_t)blockIdx.x * (256 >> log_lanes) + (threadIdx.x >> log_lanes);
+    if (!WIDE && n >= (size_t)n_rows) return;
     const float* row = u + n * (size_t)(inter + gated);
-    const int i0 = blockIdx.y * 1024 + threadIdx.x;
+    const int i0 = blockIdx.y * lanes * 4 + (WIDE ? threadIdx.x : threadIdx.x & (lanes - 1));
     float x[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) x[e] = i0 + e * 256 < inter ? row[i0 + e * 256] : 0.f;
+    for (int e = 0; e < 4; ++e) x[e] = i0 + e * lanes < inter ? row[i0 + e * lanes] : 0.f;
     const float scale = gated ? 1.0f / (1.0f + expf(-row[inter])) : 1.0f;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float a = fmaxf(x[e], 0.f);
         float v = a * a;
         if (gated) v *= scale;
-        if (i0 + e * 256 < inter) out[n * inter + i0 + e * 256] = from_float<T>(v);
+        if (i0 + e * lanes < inter) out[n * inter + i0 + e * lanes] = from_float<T>(v);
     }
 }
 
@@ -543,13 +547,18 @@ NNIS_API int nnis_group_rmsnorm(const float* x, const int* rows, const float* w,
 NNIS_API int nnis_relu2_gate(const float* u, void* out, int out_dtype, long long n_rows, int inter,
                              int gated, cudaStream_t stream) {
     if (n_rows <= 0 || inter <= 0 || gated < 0) return NNIS_ERR_ARGUMENT;
-    const dim3 grid((unsigned)n_rows, (inter + 1023) / 1024);
-    if (n_rows > 0x7fffffffLL || grid.y > 65535) return NNIS_ERR_UNSUPPORTED;
+    int log_lanes = 3;
+    while (log_lanes < 8 && (4 << log_lanes) < inter) ++log_lanes;
+    const long long rows = 256 >> log_lanes, blocks = (n_rows + rows - 1) / rows;
+    const dim3 grid((unsigned)blocks, (unsigned)(((long long)inter + (4 << log_lanes) - 1) / (4 << log_lanes)));
+    if (blocks > 0x7fffffffLL || grid.y > 65535) return NNIS_ERR_UNSUPPORTED;
     cudaError_t e;
     if (out_dtype == NNIS_DTYPE_F32)
-        e = launch_dependent(relu2_gate_kernel<float>, grid, 256, 0, stream, u, (float*)out, inter, gated);
+        e = launch_dependent(log_lanes == 8 ? relu2_gate_kernel<float, true> : relu2_gate_kernel<float, false>, grid, 256, 0,
+                             stream, u, (float*)out, n_rows, inter, gated, log_lanes);
     else if (out_dtype == NNIS_DTYPE_BF16)
-        e = launch_dependent(relu2_gate_kernel<bf16>, grid, 256, 0, stream, u, (bf16*)out, inter, gated);
+        e = launch_dependent(log_lanes == 8 ? relu2_gate_kernel<bf16, true> : relu2_gate_kernel<bf16, false>, grid, 256, 0,
+                             stream, u, (bf16*)out, n_rows, inter, gated, log_lanes);
     else
         return NNIS_ERR_UNSUPPORTED;
     return e == cudaSuccess ? NNIS_OK : (int)e;

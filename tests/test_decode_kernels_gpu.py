@@ -296,3 +296,21 @@ def test_small_matrix_per_head_no_further_from_64_bits_than_chains_of_multiply_a
     for i in range(k):  # (a product of two bfloat16 values is exact in float32: a chain of multiply-adds)
         chain += x[:, :, None, i] * y[None, :, :, i]
     assert float(out.double().norm()) <= float(np.linalg.norm(chain.astype(np.float64)))
+
+
+@pytest.mark.parametrize("inter", [1, 8, 31, 33, 64, 127, 700, 1024, 1025, 4100])
+@pytest.mark.parametrize("gated", [0, 1, 8])
+@pytest.mark.parametrize("n", [1, 33, 67])
+def test_square_of_relu_with_a_gate_for_rows_of_any_length(inter, gated, n):
+    """Several short rows a CTA, one long row a CTA and more: every value of every row, none beside it."""
+    o = ops()
+    g = torch.Generator().manual_seed(inter + n)
+    u = torch.randn(n, inter + gated, generator=g)
+    u[0, 0] = math.nan  # (not above zero: nothing)
+    want = torch.relu(torch.nan_to_num(u[:, :inter].double(), nan=0.0)).square()
+    if gated:
+        want = want * torch.sigmoid(u[:, inter:inter + 1].double())
+    for dtype, tol in ((torch.float32, 1e-6), (torch.bfloat16, 2.0 ** -8)):
+        kept = torch.full((n + 2, inter), 7.0, dtype=dtype, device=DEV)
+        o.relu2_gate(u.to(DEV), kept[:n])
+        assert torch.allclose(kept[:n].cpu().double(), want, rtol=tol, atol=1e-7) and (kept[n:] == 7.0).all()
