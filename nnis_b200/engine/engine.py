@@ -165,28 +165,26 @@ class Engine:
         slots = [s.slot for s in batch]
         counts, starts, token_arrays, wants = [], [], [], []
         for s in batch:
-            # (lists, what most callers have, are read and checked by native code; whatever it does not take, and whatever
-            # is wrong, is looked at here)
+            # (lists, what most callers have, are read and checked by native code, wanted places where there are enough of
+            # them: a call takes as long as 20 numbers here; whatever it does not take, and whatever is wrong, is looked at here)
             tok = ops.list_to_ints(s.tokens, vocab) if type(s.tokens) is list and s.tokens else None
-            want = ops.list_to_ints(s.want, tok.size) if tok is not None and type(s.want) is list else None
-            if want is not None:
-                token_arrays.append(tok)
-                wants.append(want)
-                counts.append(tok.size)
-                starts.append(self.cache.length(s.slot))
-                continue
-            tok = np.asarray(s.tokens, dtype=np.int64).reshape(-1)
-            if tok.size == 0:
-                raise StepError(f"slot {s.slot}: a sequence in a step brings at least one token")
-            if int(tok.min()) < 0 or int(tok.max()) >= vocab:
-                bad = int(tok[(tok < 0) | (tok >= vocab)][0])
-                raise StepError(f"slot {s.slot}: token {bad} is outside the vocabulary of {vocab}")
-            for w in s.want:
-                if not 0 <= int(w) < tok.size:
-                    raise StepError(f"slot {s.slot}: wanted place {w} is outside its "
-                                    f"{tok.size} tokens")
-            token_arrays.append(tok.astype(np.int32))
-            wants.append(np.asarray([int(w) for w in s.want], dtype=np.int32))
+            if tok is None:
+                tok = np.asarray(s.tokens, dtype=np.int64).reshape(-1)
+                if tok.size == 0:
+                    raise StepError(f"slot {s.slot}: a sequence in a step brings at least one token")
+                if int(tok.min()) < 0 or int(tok.max()) >= vocab:
+                    bad = int(tok[(tok < 0) | (tok >= vocab)][0])
+                    raise StepError(f"slot {s.slot}: token {bad} is outside the vocabulary of {vocab}")
+                tok = tok.astype(np.int32)
+            want = ops.list_to_ints(s.want, tok.size) if type(s.want) is list and len(s.want) >= 24 else None
+            if want is None:
+                for w in s.want:
+                    if not 0 <= int(w) < tok.size:
+                        raise StepError(f"slot {s.slot}: wanted place {w} is outside its "
+                                        f"{tok.size} tokens")
+                want = np.asarray([int(w) for w in s.want], dtype=np.int32)
+            token_arrays.append(tok)
+            wants.append(want)
             counts.append(int(tok.size))
             starts.append(self.cache.length(s.slot))
         new_lengths = [a + b for a, b in zip(starts, counts)]
