@@ -210,6 +210,14 @@ def gemm_split_f32_takes(a: torch.Tensor, w: torch.Tensor) -> bool:
     return a.shape[0] > 16 and a.shape[1] % 8 == 0 and (a.data_ptr() | w.data_ptr()) % 32 == 0
 
 
+def gemm_split_f32_pays(a: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether it should: a K below two blocks of 64 is over on the CUDA cores before the tensor cores have begun, unless
+    the output is large (rows x N x K, CUDA cores and here, us: 64 x 3,072 x 64 4.8 and 5.5, 32 x 49,152 x 96 20 and 27, 512 x
+    576 x 96 5.8 and 6.7; 100 x 8,192 x 64 6.8 and 6.2, 512 x 3,072 x 64 9.6 and 7.8, 32 x 8,192 x 128 6.9 and 6.9)."""
+    (m, k), n = a.shape, w.shape[0]
+    return gemm_split_f32_takes(a, w) and (k >= 128 or (m >= 96 and m * n >= 600000))
+
+
 def gemm_split_f32(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, mode: int,
                    shape: int = 0) -> None:
     """out (op)= a . w^T + bias for float32 operands on the tensor cores, every value as the exact sum of

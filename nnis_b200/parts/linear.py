@@ -37,7 +37,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], 
                 scratch = workspace.get("gemm_split_sums", (floats,), torch.float32)
                 tickets = workspace.zeros("gemm_split_tickets", (tiles,), torch.int32)
         ops.gemm_tc(x, weight, bias, out, mode, split_scratch=scratch, split_tickets=tickets)
-    elif x.dtype == torch.float32 and ops.gemm_split_f32_takes(x, weight):
+    elif x.dtype == torch.float32 and ops.gemm_split_f32_pays(x, weight):
         ops.gemm_split_f32(x, weight, bias, out, mode)
     else:
         ops.gemm_simt(x, weight, bias, out, mode)

@@ -115,7 +115,7 @@ class GatedMLP(Part):
             # tensor-core product with the activation in its epilogue
             ops.gemm_tc(x, self.w_gu, self.b_gu, act, ops.GEMM_GATED)
         elif self.activation == "silu" and self.dtype == torch.float32 and x is not None \
-                and ops.gemm_split_f32_takes(x, self.w_gu):
+                and ops.gemm_split_f32_pays(x, self.w_gu):
             ops.gemm_split_f32(x, self.w_gu, self.b_gu, act, ops.GEMM_GATED)
         elif self.activation == "gelu_tanh" and self.dtype == torch.bfloat16 \
                 and ops.gemm_tc_takes(n, 2 * self.inter, self.hidden):

@@ -345,6 +345,22 @@ def test_float32_prompts_take_tiles_where_these_pay():
             assert pays([c], [st], window, 1000) == (pages * 1000 <= keys * 2)
 
 
+def test_which_float32_products_run_on_the_tensor_cores():
+    """More rows than a decode step's kernel takes, whole groups of eight columns, 32-byte boundaries; a K below 128 only with a
+    large output."""
+    import torch
+    from nnis_b200.csrc import ops as o
+
+    def pays(m, n, k, off=0):
+        at = lambda rows: torch.empty(rows * k + 8)[off:off + rows * k].view(rows, k)
+        a, w = at(m), at(n)
+        assert off or a.data_ptr() % 32 == 0 == w.data_ptr() % 32
+        return o.gemm_split_f32_pays(a, w)
+    assert pays(17, 576, 576) and pays(17, 8, 128) and pays(512, 3072, 64) and pays(100, 8192, 96)
+    assert not pays(16, 576, 576) and not pays(17, 576, 580) and not pays(17, 576, 576, 1)
+    assert not pays(64, 3072, 64) and not pays(512, 576, 96) and not pays(64, 12000, 120)
+
+
 def test_which_kernel_takes_a_float32_prompt_step_of_heads_of_64(monkeypatch):
     """Tiles of 128 queries on the tensor cores, tiles of 64 for many prompts of one page, a warp a query for few short ones;
     a step is planned once for all layers with its window and heads."""
