@@ -1,8 +1,8 @@
 """y (op)= x . W^T + b: picks the kernel for a dtype and a shape.
 
-float32 operands of more than a decode step's rows run on the tensor cores as exact
-sums of three bfloat16 values each, the others on the CUDA cores; both keep 32-bit
-products.  bfloat16 operands take the tcgen05 kernel where its
+float32 operands of more than a decode step's rows, with a K of 128 and more or a large
+output, run on the tensor cores as exact sums of three bfloat16 values each, the others on
+the CUDA cores; both keep 32-bit products.  bfloat16 operands take the tcgen05 kernel where its
 tile rules hold and the row count makes it worthwhile, else the CUDA-core
 kernel.  NNIS makes the same kind of choice per projection family with its
 projection plans (crates/nnis-model/src/projection_plan.rs:10-90).

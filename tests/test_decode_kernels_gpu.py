@@ -101,6 +101,26 @@ def test_merge_of_slices(dim, rot, heads, splits, dtype):
                 assert torch.allclose(cut[t, h * dim:(h + 1) * dim].double(), s @ rows[:, :dim], atol=1e-5)
 
 
+@pytest.mark.parametrize("dim", [66, 96, 128])
+@pytest.mark.parametrize("splits", [3, 16])
+def test_merge_of_many_rows_has_the_bits_of_few(dim, splits):
+    """Rows of 65 to 128 values take a CTA each, or a warp each where they are many."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim)
+    n, heads, row = 270, 8, dim + 8
+    cache = torch.randn(n, 1, 64, row, generator=g).to(DEV)
+    q = torch.randn(n, heads * row, generator=g).to(DEV)
+    pos = torch.randint(0, 64, (n,), generator=g).to(torch.int32).to(DEV)
+    seq, table = torch.arange(n, dtype=torch.int32, device=DEV), torch.randperm(n, generator=g).to(torch.int32).view(n, 1).to(DEV)
+
+    def run(a, b):
+        out = torch.full((b - a, heads * dim), 9.0, device=DEV)
+        partial = torch.full(((b - a) * heads * splits * (dim + 2),), math.nan, device=DEV)
+        o.attention_latent(q[a:b], cache, pos[a:b], seq[:b - a], table[a:b], out, heads, dim, 0.2, splits, partial)
+        return out
+    assert torch.equal(run(0, n), torch.cat([run(0, 100), run(100, 249), run(249, n)]))
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 2048, 5632), (16, 520, 12288), (8, 2048, 5632), (20, 960, 2560), (33, 1024, 3200),
                                    (64, 2048, 8192), (5, 40, 12288)])
 @pytest.mark.parametrize("emits", [False, True])
