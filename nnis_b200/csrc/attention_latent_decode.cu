@@ -1,18 +1,18 @@
-// Latent attention of single tokens (bfloat16): every row of the step is one token, and a CTA works 16 of its heads over a
-// slice of its keys.
+// Latent attention of single tokens (bfloat16): every row of the step is one token, and a CTA works 16 of its heads over
+// a slice of its keys.
 //
-// The kernel of prompts (attention_latent_mma.cu) stacks (token, head) pairs into 64 or 128 rows and gives each warp 16 of
-// them: a token of 16 heads leaves three warps of four without rows, and the fourth multiplies a page's scores and values
-// alone, one after another (8 tokens x 16 heads of 512 + 64 over 2,048 keys: 24.5 us).  Here the eight warps share a page:
-// each takes eight of its keys for the scores, two of the 16 rows for the softmax (which meets in shared memory) and every
-// eighth tile of 16 values for the output, whose sums it keeps in registers.  Pages come by TMA, a copy for 64 of a row's
-// values (boxes of 64 rows of 128 bytes in the 128-byte swizzle, so that eight rows meet no bank twice; the queries' rows are
-// padded by 16 bytes instead), all that the ring holds before the wait for the kernel before: only the row of this step's
-// token and the queries are fetched after it.  Rows that the token does not see are zero, whatever the page holds there.
-// What bounds it: a chain of few products and three barriers a page, and the slices' way into the merge.  16 heads of 512 +
-// 64, merge included, in us in a graph, the kernel of prompts -> here: 8 tokens over 2,048 keys in 16 slices 28.8 -> 15.9,
-// over 512 in 8 17.2 -> 10.8; one token over 2,048 26.9 -> 14.2; 32 tokens over 512 in 4 27.3 -> 14.0; a page of a slice
-// 8 -> 2.6.  8 heads of 256 + 32, 8 tokens over 2,048 keys in 16: 18.4 -> 10.2.
+// The kernel of prompts (attention_latent_mma.cu) stacks (token, head) pairs into 64 or 128 rows and gives each warp 16
+// of them: a token of 16 heads leaves three warps of four without rows, and the fourth multiplies a page's scores and
+// values alone, one after another (8 tokens x 16 heads of 512 + 64 over 2,048 keys: 24.5 us).  Here the eight warps share
+// a page: each takes eight of its keys for the scores, two of the 16 rows for the softmax (which meets in shared memory)
+// and every eighth tile of 16 values for the output, whose sums it keeps in registers.  Pages come by TMA, a copy for 64
+// of a row's values (boxes of 64 rows of 128 bytes in the 128-byte swizzle, so that eight rows meet no bank twice; the
+// queries' rows are padded by 16 bytes instead), all that the ring holds before the wait for the kernel before: only the
+// row of this step's token and the queries are fetched after it.  Rows that the token does not see are zero, whatever the
+// page holds there.  What bounds it: a chain of few products and three barriers a page, and the slices' way into the
+// merge.  16 heads of 512 + 64, merge included, in us in a graph, the kernel of prompts -> here: 8 tokens over 2,048 keys
+// in 16 slices 28.8 -> 15.9, over 512 in 8 17.2 -> 10.8; one token over 2,048 26.9 -> 14.2; 32 tokens over 512 in 4 27.3
+// -> 14.0; a page of a slice 8 -> 2.6.  8 heads of 256 + 32, 8 tokens over 2,048 keys in 16: 18.4 -> 10.2.
 #include "attention_merge.cuh"
 #include "mma_helpers.cuh"
 #include "tcgen05_helpers.cuh"
@@ -35,7 +35,8 @@ __device__ __forceinline__ unsigned char* page_chunk(unsigned char* page, int ro
 template <int STAGES>
 __global__ void __launch_bounds__(kLdWarps * 32)
 latent_decode_kernel(const __grid_constant__ CUtensorMap map, const bf16* __restrict__ q, const bf16* __restrict__ cache,
-                     const int* __restrict__ token_pos, const int* __restrict__ token_seq, const int* __restrict__ page_table, int table_cols,
+                     const int* __restrict__ token_pos, const int* __restrict__ token_seq,
+                     const int* __restrict__ page_table, int table_cols,
                      bf16* __restrict__ out, float* __restrict__ partial, int heads, int dk, int dv, int head_tiles,
                      float scale, int n_splits, int window, const float* __restrict__ gate,
                      const float* __restrict__ sink, int* __restrict__ status) {

@@ -12,11 +12,12 @@
 namespace nnis {
 
 // At most 64 slices.  A warp works out the slices' weights exp(m_s - m) / l once (lane s holds slices s and s + 32); then
-// every thread sums its output values over the slices, in ascending order of slice.  Rows of at most 64 values take a warp
-// each, four to a CTA of 128 threads, rows of up to 128 where they are many and their slices few; others a CTA each (32 slices
-// of 128 values, 16 rows: a warp a row 3 us longer; 16,384 rows of 4 slices: a CTA a row 7 us longer of 263 with the attention).
-// Eight slices' values of a thread's pair are asked for together: one after another they were a trip to L2 each (128 rows of
-// 512 values, 16 slices: 9.5 -> 5.8 us; 9,216 rows of 64 values in a float32 prompt: 11.0 -> 5.4).
+// every thread sums its output values over the slices, in ascending order of slice.  Rows of at most 64 values take a
+// warp each, four to a CTA of 128 threads, rows of up to 128 where they are many and their slices few; others a CTA each
+// (32 slices of 128 values, 16 rows: a warp a row 3 us longer; 16,384 rows of 4 slices: a CTA a row 7 us longer of 263
+// with the attention).  Eight slices' values of a thread's pair are asked for together: one after another they were a trip
+// to L2 each (128 rows of 512 values, 16 slices: 9.5 -> 5.8 us; 9,216 rows of 64 values in a float32 prompt: 11.0
+// -> 5.4).
 template <typename T, bool WARP_ROWS>
 __global__ void __launch_bounds__(128)
 attn_merge_kernel(const float* __restrict__ partial, T* __restrict__ out, size_t n_rows, int d,

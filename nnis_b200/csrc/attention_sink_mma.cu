@@ -189,9 +189,10 @@ attn_sink_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cach
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 float v;
-                // cap * tanh(x / cap) = cap * (1 - 2 / (exp(2 x / cap) + 1)).  One form for every score: a polynomial for those
-                // below half the cap, chosen by the score alone (chosen by the page it let slots that nobody may read decide),
-                // took 3,001 queries of 16 heads over 1,024 keys 68 -> 65 us, and 68 -> 80 with scores that pass it.
+                // cap * tanh(x / cap) = cap * (1 - 2 / (exp(2 x / cap) + 1)).  One form for every score: a polynomial for
+                // those below half the cap, chosen by the score alone (chosen by the page it let slots that nobody may
+                // read decide), took 3,001 queries of 16 heads over 1,024 keys 68 -> 65 us, and 68 -> 80 with scores that
+                // pass it.
                 if (cap > 0.f) {
                     float e2 = exp2f(s[j][e] * scale * cap_in);
                     v = cap_out * (1.0f - __fdividef(2.0f, e2 + 1.0f));

@@ -117,12 +117,13 @@ batched_rows_kernel(const T* __restrict__ A, long long lda, long long a_bs, cons
 }
 
 // The same for bfloat16 on mma.sync tiles, at most 16 rows: a warp takes eight output columns of a head and all of K (at
-// most 16 pieces of 32 columns).  A lane's 16 bytes of a weight row stand for the column pairs of two steps of 16, the same
-// bytes of the rows of A go with them; the weights are asked for before the wait, all at once, and the rows after it.  The
-// tensor cores cut a running sum off instead of rounding it, so each 16 products leave them and are added in registers, in two
-// chains: 76 of 983,040 sums of 512 products were not rounded to the nearest bfloat16, 73 with the kernel above, 155 with
-// running sums.  That one fetches every row of A again for every output column and, with K = 128, has half of its lanes idle (8
-// rows x 16 heads, one launch after another, 512 x 128: 8.2 -> 1.8 us; 128 x 512: 5.8 -> 2.8).
+// most 16 pieces of 32 columns).  A lane's 16 bytes of a weight row stand for the column pairs of two steps of 16, the
+// same bytes of the rows of A go with them; the weights are asked for before the wait, all at once, and the rows after
+// it.  The tensor cores cut a running sum off instead of rounding it, so each 16 products leave them and are added in
+// registers, in two chains: 76 of 983,040 sums of 512 products were not rounded to the nearest bfloat16, 73 with the
+// kernel above, 155 with running sums.  That one fetches every row of A again for every output column and, with K = 128,
+// has half of its lanes idle (8 rows x 16 heads, one launch after another, 512 x 128: 8.2 -> 1.8 us; 128 x 512: 5.8 ->
+// 2.8).
 template <int PIECES>
 __global__ void __launch_bounds__(128)
 batched_rows_mma_kernel(const bf16* __restrict__ A, long long lda, long long a_bs, const bf16* __restrict__ W,

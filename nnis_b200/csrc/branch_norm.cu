@@ -168,11 +168,11 @@ sandwich_close_kernel(float* __restrict__ branch, const float* __restrict__ w, f
     }
 }
 
-// The same for rows of whole quads, at most Q a thread: all that the row needs is asked for at once (the weights before the
-// wait for the kernel ahead) and stays in registers, where the loops above wait for memory after each reduction.  Sums and
-// results have the same bits.  Bound by memory and its latency: 3,701 rows of 1,024 28 -> 9.6 us, 2,603 rows of 2,048
-// 24 -> 18 us (rows of more than 4,096 values would leave too few warps in flight: the loops).  2,000 rows of 4,096, one launch
-// after another, loops and here: no history 22.7 and 21.0, two terms 45 and 47, three 54 and 50.
+// The same for rows of whole quads, at most Q a thread: all that the row needs is asked for at once (the weights before
+// the wait for the kernel ahead) and stays in registers, where the loops above wait for memory after each reduction.
+// Sums and results have the same bits.  Bound by memory and its latency: 3,701 rows of 1,024 28 -> 9.6 us, 2,603 rows of
+// 2,048 24 -> 18 us (rows of more than 4,096 values would leave too few warps in flight: the loops).  2,000 rows of
+// 4,096, one launch after another, loops and here: no history 22.7 and 21.0, two terms 45 and 47, three 54 and 50.
 template <typename T, int Q>
 __global__ void __launch_bounds__(256)
 sandwich_close_quads_kernel(float* __restrict__ branch, const float* __restrict__ w, float eps, float* __restrict__ hidden,

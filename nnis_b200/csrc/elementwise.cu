@@ -339,10 +339,10 @@ __global__ void add_rows_kernel(float* __restrict__ a, const float* __restrict__
 // of a gate that scales the expert's whole output.  u float32 [n, inter + gated]
 // (`gated` columns beyond the activation's: the gate, then padding).
 // ---------------------------------------------------------------------------
-// 2^log_lanes threads a row and four values a thread, as far apart, all asked for at once, the gate once a thread.  Rows of 1,024
-// values and more take a CTA of 256 threads each, shorter ones share it (a thread a value, its row by a division of 64 bits: 12.5
-// us for 2,048 rows of 1,408, 21 for 20,000 of 256, 17.7 for 65,536 of 64; now 5.0, 6.9 and 5.9; a CTA a row took 21 and 69 for
-// the last two).
+// 2^log_lanes threads a row and four values a thread, as far apart, all asked for at once, the gate once a thread.  Rows
+// of 1,024 values and more take a CTA of 256 threads each, shorter ones share it (a thread a value, its row by a division
+// of 64 bits: 12.5 us for 2,048 rows of 1,408, 21 for 20,000 of 256, 17.7 for 65,536 of 64; now 5.0, 6.9 and 5.9; a CTA a
+// row took 21 and 69 for the last two).
 template <typename T, bool WIDE>
 __global__ void __launch_bounds__(256)
 relu2_gate_kernel(const float* __restrict__ u, T* __restrict__ out, long long n_rows, int inter, int gated, int log_lanes) {

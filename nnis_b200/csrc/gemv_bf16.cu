@@ -123,10 +123,11 @@ static int rowtile_slices(int M, int N, int K, int epilogue, int pro, int sm_cou
 }
 
 // Parts of K of the adding product where they run as one launch whose CTAs share a tile's K (0: not so), for products
-// that would else take several launches; the columns of a part and the units of a CTA.  Two launches of the kernel over tiles
-// of rows, whose CTAs are resident together, are faster than two parts of more than two CTAs an SM (M x N x K, two launches and
-// two parts: 64 x 2,048 x 2,048 9.7 and 11.9 us, 32 x 4,096 x 2,560 11.0 and 13.5, 1 x 6,144 x 2,048 6.9 and 10.5, 17 x 3,072 x
-// 3,072 11.4 and 11.7; with fewer CTAs 32 x 2,048 x 2,048 0.71 of the time, 8 x 3,072 x 2,560 0.82, 64 x 1,024 x 2,048 1.03).
+// that would else take several launches; the columns of a part and the units of a CTA.  Two launches of the kernel over
+// tiles of rows, whose CTAs are resident together, are faster than two parts of more than two CTAs an SM (M x N x K, two
+// launches and two parts: 64 x 2,048 x 2,048 9.7 and 11.9 us, 32 x 4,096 x 2,560 11.0 and 13.5, 1 x 6,144 x 2,048 6.9 and
+// 10.5, 17 x 3,072 x 3,072 11.4 and 11.7; with fewer CTAs 32 x 2,048 x 2,048 0.71 of the time, 8 x 3,072 x 2,560 0.82, 64
+// x 1,024 x 2,048 1.03).
 static int shared_parts(int M, int N, int K, int sm_count, int* columns, int* units) {
     int unused;
     GemvPlan p;

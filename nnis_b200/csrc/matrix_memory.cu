@@ -718,15 +718,15 @@ memory_finish_kernel(const float* __restrict__ o_raw, const float* __restrict__ 
     for (int i = lane; i < vdim; i += 32) dst[i] = from_float<T>((o[i] * s) * wh[i] * (1.0f / (1.0f + expf(-g[i]))));
 }
 
-// Whether a step's chunks go to the kernels by pairs: heads of 64 or 128 keys, whole groups of eight columns, and where those
-// are not slower than the kernels of single chunks, in us of a whole memory_prompt (pairs, single chunks):
-//   * not for 64 x 64 and smaller, of which single chunks fill an SM's shared memory several times (8 heads: 100 tokens 43, 39;
-//     8 x 300 66, 57; 64 x 64 105, 73; 4,000 tokens 82, 94);
-//   * not for chunks of 32 tokens and fewer on average, where a CTA's start is most of its time (1 x 16 tokens of 4 heads of
-//     128 x 256 41, 37; 64 x 10 of 8 of 64 x 128 105, 74; 1 x 40 44, 43), but for many of large heads (16 x 24 of 8 of 128 x 256
-//     62, 73; 16 x 10 of 4 49, 50);
-//   * not for more sequences of a single chunk than SMs with heads of 128 x 64 and less, as half of a CTA's tokens are missing
-//     (64 x 40 of 8 heads of 64 x 128 114, 104, of 128 x 32 111, 86; 64 x 100 154, 212).
+// Whether a step's chunks go to the kernels by pairs: heads of 64 or 128 keys, whole groups of eight columns, and where
+// those are not slower than the kernels of single chunks, in us of a whole memory_prompt (pairs, single chunks):
+//   * not for 64 x 64 and smaller, of which single chunks fill an SM's shared memory several times (8 heads: 100 tokens
+//     43, 39; 8 x 300 66, 57; 64 x 64 105, 73; 4,000 tokens 82, 94);
+//   * not for chunks of 32 tokens and fewer on average, where a CTA's start is most of its time (1 x 16 tokens of 4 heads
+//     of 128 x 256 41, 37; 64 x 10 of 8 of 64 x 128 105, 74; 1 x 40 44, 43), but for many of large heads (16 x 24 of 8 of
+//     128 x 256 62, 73; 16 x 10 of 4 49, 50);
+//   * not for more sequences of a single chunk than SMs with heads of 128 x 64 and less, as half of a CTA's tokens are
+//     missing (64 x 40 of 8 heads of 64 x 128 114, 104, of 128 x 32 111, 86; 64 x 100 154, 212).
 // 2,000 tokens of 8 heads: 64 x 128 53, 70; 128 x 32 55, 72; 128 x 256 75, 187.
 static bool memory_by_pairs(long long n_tokens, long long n_chunks, long long n_seqs, int H, int dim, int vdim, int sms) {
     const long long state = (long long)dim * vdim;

@@ -70,11 +70,12 @@ __device__ __forceinline__ float warp_row_dot(const T* __restrict__ a, const T* 
     return warp_sum(acc);
 }
 
-// A CTA of `blockDim.x` / 32 warps takes TOK tokens.  With one token a warp takes an output at a time, and the launch brings
-// 32 warps, so that one SM asks L2 for a matrix of 32 rows at once (8 tokens, 32 experts, width 2,048: 9.9 -> 5.3 us).  With
-// eight tokens a warp takes EXP rows of the matrix and all tokens, so a piece of a row is fetched once for eight tokens and a
-// piece of a token once for EXP rows (2,048 tokens of that layer: 40 -> 16 us, as every token's CTA fetched the whole matrix,
-// half a gigabyte from L2).  A logit is the same chain of multiply-adds either way.  Then warp k chooses for token k.
+// A CTA of `blockDim.x` / 32 warps takes TOK tokens.  With one token a warp takes an output at a time, and the launch
+// brings 32 warps, so that one SM asks L2 for a matrix of 32 rows at once (8 tokens, 32 experts, width 2,048: 9.9 -> 5.3
+// us).  With eight tokens a warp takes EXP rows of the matrix and all tokens, so a piece of a row is fetched once for
+// eight tokens and a piece of a token once for EXP rows (2,048 tokens of that layer: 40 -> 16 us, as every token's CTA
+// fetched the whole matrix, half a gigabyte from L2).  A logit is the same chain of multiply-adds either way.  Then warp
+// k chooses for token k.
 template <typename T, int TOK, int EXP>
 __global__ void __launch_bounds__(TOK == 1 ? 1024 : 256)
 moe_route_kernel(const T* __restrict__ h, const float* __restrict__ wr, const float* __restrict__ br,

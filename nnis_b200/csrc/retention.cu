@@ -644,10 +644,11 @@ retention_read_split_kernel(const float* __restrict__ packed, const float* __res
         });
 }
 
-// Whether chunks go by pairs: not for heads of 64 x 64 and smaller unless there is a CTA for two SMs of three and sequences
-// are long, as most of a tile of 128 columns is padding (8 heads of 64 x 64, us by pairs and by single chunks: 512 tokens 37, 35,
-// 16 x 130 66, 58, 40 x 70 95, 81; 1,000 40, 50, 4 x 400 43, 53, 4,000 79, 86; of 64 x 32 512 36, 34, 1,000 39, 49).  With 128 keys they
-// win with few values too (8 heads of 128 x 8: 512 tokens 42, 54, 16 x 130 71, 79, 4,000 89, 124).
+// Whether chunks go by pairs: not for heads of 64 x 64 and smaller unless there is a CTA for two SMs of three and
+// sequences are long, as most of a tile of 128 columns is padding (8 heads of 64 x 64, us by pairs and by single chunks:
+// 512 tokens 37, 35, 16 x 130 66, 58, 40 x 70 95, 81; 1,000 40, 50, 4 x 400 43, 53, 4,000 79, 86; of 64 x 32 512 36, 34,
+// 1,000 39, 49).  With 128 keys they win with few values too (8 heads of 128 x 8: 512 tokens 42, 54, 16 x 130 71, 79,
+// 4,000 89, 124).
 static bool retention_by_pairs(long long n_chunks, long long n_seqs, int heads, int dim, int vdim, int wave) {
     if (vdim % 8 || (wave < 2 && n_chunks > 1)) return false;
     return dim == 128 || (dim == 64 && (vdim > 64 || (n_chunks * heads >= 100 && n_chunks >= 4 * n_seqs)));
