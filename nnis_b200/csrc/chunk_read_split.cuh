@@ -94,13 +94,6 @@ __device__ __forceinline__ uint64_t chunk_desc_mn(uint32_t smem_byte_addr) {
     return (desc & ~((uint64_t)0x3FFF << 16)) | (uint64_t)(8192 >> 4) << 16;
 }
 
-// Eight values in one store; the address is a multiple of 32 bytes.
-__device__ __forceinline__ void store8(float* p, const float* v) {
-    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(pair_of(v[0], v[1])), "l"(pair_of(v[2], v[3])),
-                 "l"(pair_of(v[4], v[5])), "l"(pair_of(v[6], v[7]))
-                 : "memory");
-}
-
 // Every thread of the CTA calls it.  `prepare()` runs on every thread before anything that reads what an earlier kernel
 // wrote, and ends in a barrier of the CTA; `weigh(i, j, x)` is asked for j <= i < count alone; `norm` (null: none) is a vector
 // whose product with every query is wanted; `finish(i, c, x, sum, dot)` takes eight outputs of a token from column c of the

@@ -11,6 +11,13 @@ __device__ __forceinline__ void load8(const float* p, unsigned long long (&v)[4]
     asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p));
 }
 
+// Eight values in one store; the address is a multiple of 32 bytes.
+__device__ __forceinline__ void store8(float* p, const float* v) {
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(pair_of(v[0], v[1])), "l"(pair_of(v[2], v[3])),
+                 "l"(pair_of(v[4], v[5])), "l"(pair_of(v[6], v[7]))
+                 : "memory");
+}
+
 // A pair of values' next bfloat16 parts, packed; what is left of the values stays in x.
 __device__ __forceinline__ uint32_t next_part(unsigned long long& x) {
     uint32_t p;

@@ -657,3 +657,53 @@ def test_qkv_products_on_pairs_of_ctas(nq, nkv, d, m, k):
     for whole, parts in zip(product(m), product(128)):
         assert torch.equal(whole, parts)
     o.check_status(DEV)
+
+
+@pytest.mark.parametrize("dim,vdim", [(64, 4), (64, 136), (128, 72), (128, 300)])
+def test_delta_rule_chunks_at_the_edges_of_their_tiles(dim, vdim):
+    """Columns that end inside an octet, a CTA's 64 and a tile of 128, chunks that end at their first and last token, a head
+    per key head: against the recurrence in 64 bits.  A value that is no number is felt by its own column from its token on."""
+    o = ops()
+    g = torch.Generator().manual_seed(dim + vdim)
+    H, G, taps, new, at = 2, 2, 1, [65, 1, 63, 128, 129], 100 + 129
+    n, channels = sum(new), 2 * G * dim + H * vdim
+    rows = torch.randn(n, channels + H * vdim + 2 * H, generator=g)
+    conv, a_log, bias = torch.ones(channels, taps, device=DEV), torch.tensor([-5.0, 0.5], device=DEV), torch.zeros(H, device=DEV)
+    begin, tails = torch.randn(len(new), H, dim, vdim, generator=g) * 0.3, torch.zeros(len(new), 1, channels, device=DEV)
+    first = [sum(new[:i]) for i in range(len(new))]
+    pos, seq = i32([t for c in new for t in range(c)]), i32([i for i, c in enumerate(new) for _ in range(c)])
+    chunks, first_chunk = (torch.from_numpy(t).to(DEV) for t in o.scan_segments(new, o.DELTA_CHUNK))
+
+    def run(x):
+        state, out = begin.to(DEV), torch.full((n, H * vdim), math.nan, device=DEV)
+        o.delta_prompt(x.to(DEV), conv, tails, a_log, bias, state, pos, seq, i32(range(len(new))), i32(first), i32(new), chunks,
+                       first_chunk, lambda name, shape, dtype: torch.full(shape, math.nan, dtype=dtype, device=DEV), out, H, G,
+                       dim, vdim, 1e-6, dim ** -0.5)
+        return out.view(n, H, vdim).cpu(), state.cpu()
+
+    out, state = run(rows)
+    x = torch.nn.functional.silu(rows[:, :channels].double())
+    q, k = (y / (y.pow(2).sum(-1, keepdim=True) + 1e-6).sqrt() for y in (x[:, :G * dim].view(n, G, dim), x[:, G * dim:2 * G * dim].view(n, G, dim)))
+    v, beta = x[:, 2 * G * dim:].view(n, H, vdim), torch.sigmoid(rows[:, -2 * H:-H].double())
+    decay = torch.exp(-torch.exp(a_log.cpu().double()) * torch.nn.functional.softplus(rows[:, -H:].double()))
+    want, finals = torch.empty(n, H, vdim, dtype=torch.float64), []
+    for i, c in enumerate(new):
+        S = begin[i].double()
+        for r in range(first[i], first[i] + c):
+            S = decay[r, :, None, None] * S
+            S = S + k[r][:, :, None] * (beta[r, :, None] * (v[r] - torch.einsum("hdv,hd->hv", S, k[r])))[:, None, :]
+            want[r] = torch.einsum("hdv,hd->hv", S, q[r]) * dim ** -0.5
+        finals.append(S)
+    finals = torch.stack(finals)
+    # (as test_delta_rule_of_prompts_in_chunks, and the float32 gates: a hundred roundings of logs of up to 5 a token, 1e-5 more)
+    assert (out.double() - want).abs().max() < 2e-5 * want.abs().max()
+    assert (state.double() - finals).abs().max() < 2e-5 * finals.abs().max()
+    rows[at, 2 * G * dim + vdim + 3] = math.nan  # the last prompt but one, its token 100; head 1, column 3
+    bad, bad_state = run(rows)
+    hit = torch.zeros(n, H, vdim, dtype=torch.bool)
+    hit[at:first[4], 1, 3] = True
+    # (the column's earlier tokens of that chunk are summed in another order)
+    assert torch.equal(torch.isnan(bad), hit) and (bad - out)[~hit].abs().max() < 1e-5 * out.abs().max()
+    hit = torch.zeros_like(state, dtype=torch.bool)
+    hit[3, 1, :, 3] = True
+    assert torch.equal(torch.isnan(bad_state), hit) and torch.equal(bad_state[~hit], state[~hit])
