@@ -8,7 +8,7 @@ from test_kernels_gpu import DEV, ops
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [0, 11, 12, 14, 21, 22, 24]
+SHAPES = [0, 11, 12, 14, 21, 22, 24, 31]
 # What is left out of a product is below 2^-26 of it; 64 columns' sum is cut off at most four times at 2^-23 of itself and
 # then added with a rounding of 2^-24 (K / 64 of them), one more for a bias or an addition into C.  The sums are random
 # walks, so 2-norms of errors add as squares: below 4e-7 of the result's for the K here.
