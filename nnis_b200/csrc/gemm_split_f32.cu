@@ -282,6 +282,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const SplitArgs g) 
                 const int row4 = (i * kSplitWorkers + worker) * 4;
                 store_parts(w_stages + (size_t)s * kStage + (row4 + r4) * 128 + ((unit ^ ((row4 & 4) + r4)) << 4), kPartW, v[i]);
                 load(i, kb + 1, wanted);
+                __syncwarp();  // (rows that do not exist load nothing; tensor memory is for whole warps)
             }
             fence_async_shared();
             tmem_store_wait();
