@@ -16,6 +16,10 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// The first 1,024-byte boundary at or after `smem` in shared memory, by an offset: a pointer that came out of an integer has no
+// space that the compiler knows, and is read and written by generic accesses with addresses of twice the registers.
+__device__ __forceinline__ unsigned char* shared_1024(unsigned char* smem) { return smem + (-smem_addr(smem) & 1023u); }
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t arrivals) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(arrivals));
 }

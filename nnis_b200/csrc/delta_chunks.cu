@@ -4,22 +4,23 @@
 //     u_i + sum_(j<i) beta_i e^(c_i - c_j) (k_i . k_j) u_j = beta_i (v_i - e^(c_i) S_0^T k_i)
 //     o_i = e^(c_i) S_0^T q_i + sum_(j<=i) e^(c_i - c_j) (q_i . k_j) u_j
 // so a chunk is a unit lower triangular system with two right sides, U = U0 - W S, and products:
-//   delta_pack    convolution, silu, unit vectors, beta and c of every chunk, in octets of eight neighbouring places;
+//   delta_pack    convolution, silu, unit vectors, beta and c of every chunk, in the tiles that the products' operands come from;
 //   delta_solve   a CTA per (chunk, head), all side by side: q_i . k_j and k_i . k_j, the triangle's inverse T, W and U0;
 //   delta_chain   a CTA per (sequence, head, 64 columns) walks the chunks: [q; W] S, U = U0 - W S, S <- e^c S + K^T (e^(c - c_j) U),
 //                 and the outputs.
 // More chunks than the scratch holds go through the kernels in waves, the slot's state from one to the next (the same
 // bits: the state is float32 there too).
 // Every product of matrices is six products of bfloat16 parts on the tensor cores, exact parts of float32 values, summed in
-// float32 64 places at a time (split_parts.cuh); the triangle is inverted in float32, c is double (differences of sums of up to
-// 64 logs keep float32's digits), a decay of zero counts as e^-200, which is zero in float32 and leaves the tokens after it
-// exact.  Distance from 64 bits 1.7e-7 to 4.9e-7 of the outputs' norm where float32 sums on the CUDA cores had 2.1e-7 to 1.1e-6.
+// float32 in tensor memory over the 64 or 128 places of a chunk or a head (split_parts.cuh); the triangle is inverted in float32, c is
+// double, then two floats (differences of sums of up to 64 logs keep float32's digits), a decay of zero counts as e^-200, which is
+// zero in float32 and leaves the tokens after it exact.  Distance from 64 bits 1.7e-7 to 5.2e-7 of the outputs' norm where float32
+// sums on the CUDA cores had 1.8e-7 to 1.1e-6.
 //
 // Against the walk in runs with a transition matrix per run (delta_rule.cu, which other key sizes and short prompts
 // keep): a token costs 2.2 dim vdim + 64 (dim + vdim) multiply-adds or so instead of 2.3 times three dim vdim, all but the chain side
 // by side.
 // Two prompts of 2,048 and 555 tokens, 32 heads over 16 key heads of 128 x 128, on a B200: with float32 multiply-adds, in four
-// kernels (substitution, states, reads), 61 + 148 + 255 + 133 us; now pack 56, solve 109, chain 178.
+// kernels (substitution, states, reads), 61 + 148 + 255 + 133 us; now pack 57, solve 91, chain 128.
 #include "async_copy.cuh"
 #include "common.cuh"
 #include "split_parts.cuh"
@@ -42,8 +43,12 @@ __device__ __forceinline__ DeltaChunk delta_chunk(const int* chunks, const int* 
     return m;
 }
 
-// A packed (chunk, key head), octets of eight neighbouring places of one token: queries [dim / 8][64][8], keys [dim / 8][64][8],
-// and of eight neighbouring tokens: keys [64 / 8][dim][8]; and (chunk, head): values [vp / 8][64][8].
+// Rows of a chunk in tiles of 32 columns, a row of 128 bytes a token with its 16-byte words swizzled: a warp that has a column a lane
+// and one that has a row a lane both meet every bank once.  A packed (chunk, key head): queries and keys [dim / 32][64][32], keys
+// with a row a place and a column a token [2][dim][32]; and (chunk, head): values, then U0 [vp / 32][64][32], W [dim / 32][64][32].
+__host__ __device__ __forceinline__ int delta_at(int c, int t, int rows) {
+    return ((c >> 5) * rows + t) * 32 + ((((c >> 2) & 7) ^ (t & 7)) << 2) + (c & 3);
+}
 __host__ __device__ __forceinline__ size_t delta_qk_floats(int dim) { return (size_t)3 * kDC * dim; }
 
 // A CTA per (chunk, piece): q heads, k heads, value heads, and last the gates of all heads.  A thread walks 16 tokens of
@@ -151,16 +156,20 @@ delta_pack_kernel(const float* __restrict__ a, const float* __restrict__ conv_w,
         }
     }
     __syncthreads();
-    if (!head) {
-        float* to = values + ((size_t)blockIdx.x * H + (piece - 2 * G)) * kDC * vp;
-        for (int it = tid; it < kDC * vp / 8; it += 256) {
-            const int t = it & (kDC - 1), j0 = (it >> 6) * 8;
-            const float* from = pack_y + t * ld + j0;
-            float x[8];
+    // (four columns an item, eight neighbours to a row of a tile)
+    auto put_rows = [&](float* to, int cols, int there, auto scale_of) {
+        for (int it = tid; it < kDC * cols / 4; it += 256) {
+            const int t = (it >> 3) & (kDC - 1), c = (it >> 9) * 32 + (((it ^ t) & 7) << 2);
+            const float* from = pack_y + t * ld + c;
+            const float f = scale_of(t);
+            float x[4];
 #pragma unroll
-            for (int e = 0; e < 8; ++e) x[e] = j0 + e < vdim ? from[e] : 0.f;
-            store8(to + it * 8, x);
+            for (int e = 0; e < 4; ++e) x[e] = c + e < there ? from[e] * f : 0.f;
+            store4(to + it * 4, make_float4(x[0], x[1], x[2], x[3]));
         }
+    };
+    if (!head) {
+        put_rows(values + ((size_t)blockIdx.x * H + (piece - 2 * G)) * kDC * vp, vp, vdim, [](int) { return 1.f; });
         return;
     }
     for (int t = warp; t < kDC; t += 8) {
@@ -172,24 +181,14 @@ delta_pack_kernel(const float* __restrict__ a, const float* __restrict__ conv_w,
     __syncthreads();
     const int g = piece < G ? piece : piece - G;
     float* to = qk + ((size_t)blockIdx.x * G + g) * delta_qk_floats(dim) + (piece < G ? 0 : (size_t)kDC * dim);
-    for (int it = tid; it < kDC * dim / 8; it += 256) {
-        const int t = it & (kDC - 1);
-        const float* from = pack_y + t * ld + (it >> 6) * 8;
-        float x[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = from[e] * scale[t];
-        store8(to + it * 8, x);
-    }
+    put_rows(to, dim, dim, [&](int t) { return scale[t]; });
     if (piece < G) return;
     to += (size_t)kDC * dim;
     const int shift = dim == 128 ? 7 : 6;  // (dim is 64 or 128)
-    for (int it = tid; it < kDC * dim / 8; it += 256) {
-        const int d = it & (dim - 1), t0 = (it >> shift) * 8;
-        const float* from = pack_y + t0 * ld + d;
-        float x[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = from[e * ld] * scale[t0 + e];
-        store8(to + it * 8, x);
+    for (int it = tid; it < kDC * dim / 4; it += 256) {
+        const int d = (it >> 3) & (dim - 1), t = (it >> (3 + shift)) * 32 + (((it ^ d) & 7) << 2);
+        const float* from = pack_y + t * ld + d;
+        store4(to + it * 4, make_float4(from[0] * scale[t], from[ld] * scale[t + 1], from[2 * ld] * scale[t + 2], from[3 * ld] * scale[t + 3]));
     }
 }
 
@@ -199,28 +198,27 @@ __host__ __device__ __forceinline__ int delta_score(int octet, int i) {
     return 8 * (64 * octet - 4 * octet * (octet - 1)) + (i - 8 * octet) * 8;
 }
 
-// Shared memory of the solve: two blocks of 64 places of dim, three parts each, a part [64 queries | 64 keys] of 128-byte rows.
-// Once the products q . k and k . k are made, the queries' tiles hold the rest: T beta's parts in the first block's, the
-// triangle itself (float32) in two of the second's and what its inversion multiplies in the third; the values' parts replace
-// the keys'.
-constexpr uint32_t kDsTile = 64 * 128, kDsPart = 2 * kDsTile, kDsBlock = 3 * kDsPart, kDsSmem = 2 * kDsBlock + 1024;
-constexpr int kDsThreads = 256;
+// Shared memory of the solve: for every 64 places of dim three parts, each a tile of queries and one of keys (64 rows of 128
+// bytes).  Once the products q . k and k . k are made, the queries' tiles hold the parts of T beta (first block), the triangle itself
+// in float32 (two of the second's) and what its inversion multiplies (the third); the keys' first ones the parts of T beta e^c,
+// the scores follow.
+constexpr uint32_t kDsTile = 64 * 128, kDsPart = 2 * kDsTile, kDsBlock = 3 * kDsPart, kDsSmem = 2 * kDsBlock + kDeltaScores * 4 + 1024;
+constexpr int kDsThreads = 512;
 
 struct DeltaSolveShared {
-    uint64_t done[4];
+    uint64_t done[2];  // in turn: a warp that still waits for one product is not overtaken by the next one's end
     uint32_t tmem;
     volatile int abort_flag;
-    double cs[kDC];
-    float bs[kDC], bg[kDC];
+    float ch[kDC], cl[kDC], bs[kDC], bg[kDC];  // the summed logs as two floats, beta, beta e^c
 };
 
 // (i, j) of the triangle, by words of 16 bytes that neighbouring rows keep in different banks
 __device__ __forceinline__ int delta_tri(int i, int j) { return (i >> 5) * (int)(kDsPart / 4) + (i & 31) * kDC + (j ^ ((i & 7) << 2)); }
 
-// T = (1 + L)^-1 in place of -L, a unit lower triangle of 64, by 256 threads: the four triangles of 16 on its diagonal a column
-// a thread, then twice the lower left square as T22 (-L21) T11.  Sums over m stop at the row's own place, so a row that
-// holds no numbers is felt by the rows after it alone.  The entries of T are bounded by one (unit keys, beta at most one), so the
-// inverse costs no digits against a substitution.
+// T = (1 + L)^-1 in place of -L, a unit lower triangle of 64, by 512 threads: the four triangles of 16 on its diagonal a column
+// a thread, then twice the lower left square as T22 (-L21) T11.  What a row gets comes from rows up to its own alone, also where
+// they hold no numbers.  The entries of T are bounded by one (unit keys, beta at most one), so the inverse costs no digits
+// against a substitution.
 __device__ __forceinline__ void delta_invert(float* tri, float* mid) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (warp < 4) {
@@ -237,8 +235,8 @@ __device__ __forceinline__ void delta_invert(float* tri, float* mid) {
                 for (int e = 0; e < 4; ++e) {
                     const int m = m4 * 4 + e;
                     if (m >= i) continue;
-                    if (e & 1) b = m >= c ? fmaf(lv[e], x[m], b) : b;
-                    else a = m >= c ? fmaf(lv[e], x[m], a) : a;
+                    if (e & 1) b = fmaf(lv[e], x[m], b);
+                    else a = fmaf(lv[e], x[m], a);
                 }
             }
             x[i] = a + b;
@@ -250,100 +248,125 @@ __device__ __forceinline__ void delta_invert(float* tri, float* mid) {
     }
     __syncthreads();
     {
-        const int pair = tid >> 7, i = (tid & 127) >> 3, j = (tid & 7) * 2, r0 = pair * 32 + 16, c0 = pair * 32;
+        const int pair = tid >> 8, i = (tid & 255) >> 4, j = tid & 15, r0 = pair * 32 + 16, c0 = pair * 32;
         float a = 0.f, b = 0.f;
 #pragma unroll
-        for (int m = 0; m < 16; ++m) {
-            const float l = tri[delta_tri(r0 + i, c0 + m)];
-            const float2 t = load2(tri + delta_tri(c0 + m, c0 + j));
-            a = m >= j ? fmaf(l, t.x, a) : a;
-            b = m >= j + 1 ? fmaf(l, t.y, b) : b;
+        for (int m = 0; m < 16; m += 4) {
+            const float4 l = load4(tri + delta_tri(r0 + i, c0 + m));
+            a = fmaf(l.x, tri[delta_tri(c0 + m, c0 + j)], a);
+            b = fmaf(l.y, tri[delta_tri(c0 + m + 1, c0 + j)], b);
+            a = fmaf(l.z, tri[delta_tri(c0 + m + 2, c0 + j)], a);
+            b = fmaf(l.w, tri[delta_tri(c0 + m + 3, c0 + j)], b);
         }
-        store2(mid + pair * 512 + i * 16 + j, a, b);
+        mid[pair * 256 + i * 16 + j] = a + b;
         __syncthreads();
-        a = b = 0.f;
+        a = 0.f;
 #pragma unroll
-        for (int m = 0; m < 16; ++m) {
-            const float t = tri[delta_tri(r0 + i, r0 + m)];
-            const float2 y = load2(mid + pair * 512 + m * 16 + j);
-            a = m <= i ? fmaf(t, y.x, a) : a;
-            b = m <= i ? fmaf(t, y.y, b) : b;
+        for (int m = 0; m < 16; m += 4) {
+            const float4 t = load4(tri + delta_tri(r0 + i, r0 + m));
+            const float tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float y = mid[pair * 256 + (m + e) * 16 + j];
+                a = m + e <= i ? fmaf(tv[e], y, a) : a;
+            }
         }
-        store2(tri + delta_tri(r0 + i, c0 + j), a, b);
+        tri[delta_tri(r0 + i, c0 + j)] = a;
         __syncthreads();
     }
-    const int i = tid >> 3, j = (tid & 7) * 4;
-    float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int m = 0; m < 32; ++m) {
-        const float l = tri[delta_tri(32 + i, m)];
-        const float4 t = load4(tri + delta_tri(m, j));
-        y.x = m >= j ? fmaf(l, t.x, y.x) : y.x;
-        y.y = m >= j + 1 ? fmaf(l, t.y, y.y) : y.y;
-        y.z = m >= j + 2 ? fmaf(l, t.z, y.z) : y.z;
-        y.w = m >= j + 3 ? fmaf(l, t.w, y.w) : y.w;
-    }
-    store4(mid + i * 32 + j, y);
-    __syncthreads();
-    y = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int m = 0; m < 32; ++m) {
-        const float t = tri[delta_tri(32 + i, 32 + m)];
-        const float4 z = load4(mid + m * 32 + j);
-        if (m <= i) {
-            y.x = fmaf(t, z.x, y.x);
-            y.y = fmaf(t, z.y, y.y);
-            y.z = fmaf(t, z.z, y.z);
-            y.w = fmaf(t, z.w, y.w);
+    // (32 x 32 outputs, 2 x 4 a thread: half the words of shared memory that 1 x 2 would read)
+    const int i = (tid >> 3) * 2, j = (tid & 7) * 4;
+    float y[2][4] = {};
+    if (tid < 128) {
+#pragma unroll
+        for (int m = 0; m < 32; m += 4) {
+            const float4 l0 = load4(tri + delta_tri(32 + i, m)), l1 = load4(tri + delta_tri(33 + i, m));
+            const float a[4] = {l0.x, l0.y, l0.z, l0.w}, b[4] = {l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float4 t = load4(tri + delta_tri(m + e, j));
+                y[0][0] = fmaf(a[e], t.x, y[0][0]), y[0][1] = fmaf(a[e], t.y, y[0][1]), y[0][2] = fmaf(a[e], t.z, y[0][2]), y[0][3] = fmaf(a[e], t.w, y[0][3]);
+                y[1][0] = fmaf(b[e], t.x, y[1][0]), y[1][1] = fmaf(b[e], t.y, y[1][1]), y[1][2] = fmaf(b[e], t.z, y[1][2]), y[1][3] = fmaf(b[e], t.w, y[1][3]);
+            }
         }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) store4(mid + (i + r) * 32 + j, make_float4(y[r][0], y[r][1], y[r][2], y[r][3]));
     }
-    store4(tri + delta_tri(32 + i, j), y);
+    __syncthreads();
+    if (tid < 128) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[r][e] = 0.f;
+#pragma unroll
+        for (int m = 0; m < 32; m += 4) {
+            const float4 t0 = load4(tri + delta_tri(32 + i, 32 + m)), t1 = load4(tri + delta_tri(33 + i, 32 + m));
+            const float a[4] = {t0.x, t0.y, t0.z, t0.w}, b[4] = {t1.x, t1.y, t1.z, t1.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float4 z = load4(mid + (m + e) * 32 + j);
+                if (m + e <= i) y[0][0] = fmaf(a[e], z.x, y[0][0]), y[0][1] = fmaf(a[e], z.y, y[0][1]), y[0][2] = fmaf(a[e], z.z, y[0][2]), y[0][3] = fmaf(a[e], z.w, y[0][3]);
+                if (m + e <= i + 1) y[1][0] = fmaf(b[e], z.x, y[1][0]), y[1][1] = fmaf(b[e], z.y, y[1][1]), y[1][2] = fmaf(b[e], z.z, y[1][2]), y[1][3] = fmaf(b[e], z.w, y[1][3]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) store4(tri + delta_tri(32 + i + r, j), make_float4(y[r][0], y[r][1], y[r][2], y[r][3]));
+    }
     __syncthreads();
 }
 
-// A CTA per (chunk, head), two to an SM: the scores P, W and U0, and for the chain e^(c - c_j) and e^(c_j) in the place of the
-// logs.  What is multiplied on the tensor cores: [q; k] k^T (128 x 64, a sum of 64 places at a time), k^T (T e^c beta)^T and
-// v^T (T beta)^T (128 x 64 each).  Rows that no number comes out of are made again by multiply-adds over their own tokens.
+// A CTA per (chunk, head), two to an SM: the scores, W and U0, and for the chain e^(c_last - c_j) and e^(c_j) in the place of the
+// logs.  On the tensor cores: [q; k] k^T (128 x 64, a sum of 64 places at a time), then columns of k and v (128, as the left side
+// in tensor memory) times the 64 rows of a triangle.  A column that no number comes out of is made again by multiply-adds over
+// each token's own past.
 template <int DIM>
 __global__ void __launch_bounds__(kDsThreads, 2)
 delta_solve_kernel(const float* __restrict__ qk, float* u, const float* __restrict__ beta, double* logs,
                    float* __restrict__ w_out, float* __restrict__ scores, int H, int G, int vp, int* __restrict__ status) {
     extern __shared__ unsigned char solve_smem[];
     __shared__ DeltaSolveShared sh;
-    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(solve_smem) + 1023) & ~(uintptr_t)1023);
+    unsigned char* base = shared_1024(solve_smem);
     constexpr int BLOCKS = DIM / 64;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), h = blockIdx.y, g = h / (H / G);
     const size_t unit = (size_t)blockIdx.x * H + h;
     float* tri = reinterpret_cast<float*>(base + kDsBlock);
     float* mid = reinterpret_cast<float*>(base + kDsBlock + 2 * kDsPart);
+    float* own_scores = reinterpret_cast<float*>(base + 2 * kDsBlock);
     pdl_wait();
     if (tid == 0) {
-        for (int i = 0; i < 4; ++i) mbar_init(&sh.done[i], 1);
+        mbar_init(&sh.done[0], 1);
+        mbar_init(&sh.done[1], 1);
         sh.abort_flag = 0;
         mbar_fence_init();
     }
     if (warp == 0) tmem_alloc(&sh.tmem, 256);
     const float* q = qk + ((size_t)blockIdx.x * G + g) * delta_qk_floats(DIM);
     const float* k = q + (size_t)kDC * DIM;
-    // rows of the queries and keys, eight values an item: token `it % 64`, places from 8 (it / 64 % (dim / 8))
+    // rows of the queries and keys, eight values an item, eight neighbours to 64 places of a token
+    {
+        unsigned long long v[2 * BLOCKS][4];
+        const int o = tid & 7, t = tid >> 3;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const float* from = half ? k : q;
-        constexpr int ITEMS = kDC * DIM / 8 / kDsThreads;
-        unsigned long long v[ITEMS][4];
+        for (int e = 0; e < 2 * BLOCKS; ++e) {
+            const int b = e >> 1;
+            load8((e & 1 ? k : q) + (size_t)((b * 2 + (o >> 2)) * kDC + t) * 32 + (((o & 3) * 2 ^ (t & 6)) << 2), v[e]);
+        }
 #pragma unroll
-        for (int e = 0; e < ITEMS; ++e) load8(from + (size_t)(e * kDsThreads + tid) * 8, v[e]);
-#pragma unroll
-        for (int e = 0; e < ITEMS; ++e) {
-            const int it = e * kDsThreads + tid, t = it & (kDC - 1), o = it >> 6;
-            store_parts(base + (o >> 3) * kDsBlock + half * kDsTile + t * 128 + (((o & 7) ^ (t & 7)) << 4), kDsPart, v[e]);
+        for (int e = 0; e < 2 * BLOCKS; ++e) {
+            if (t & 1) {  // (an octet's two words lie the other way round)
+                const unsigned long long a = v[e][0], c = v[e][1];
+                v[e][0] = v[e][2], v[e][1] = v[e][3], v[e][2] = a, v[e][3] = c;
+            }
+            store_parts(base + (e >> 1) * kDsBlock + (e & 1) * kDsTile + t * 128 + ((o ^ (t & 7)) << 4), kDsPart, v[e]);
         }
     }
     if (tid < kDC) {
         const double c = logs[unit * kDC + tid];
-        sh.cs[tid] = c;
-        sh.bs[tid] = beta[unit * kDC + tid];
-        sh.bg[tid] = sh.bs[tid] * expf((float)c);
+        const float b = beta[unit * kDC + tid];
+        sh.ch[tid] = (float)c;
+        sh.cl[tid] = (float)(c - (double)(float)c);
+        sh.bs[tid] = b;
+        sh.bg[tid] = b * expf((float)c);
     }
     fence_async_shared();
     tc_fence_before();
@@ -351,14 +374,82 @@ delta_solve_kernel(const float* __restrict__ qk, float* u, const float* __restri
     tc_fence_after();
     pdl_launch_dependents();  // (the next kernel's CTAs may start, and wait: every CTA of this one has its tensor memory)
     const uint32_t tmem = __shfl_sync(0xffffffffu, sh.tmem, 0);
-    const int row = (warp & 3) * 32 + lane, cg = warp >> 2;
+    // this thread's column of k or v (with 16 tokens), or row of the scores (with 16 keys)
+    const int row = (warp & 3) * 32 + lane, cg = warp >> 2, t0 = cg * 16;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     bool ok = true;
-    int waits = 0;
+    uint32_t made = 0, seen = 0;  // products
     auto wait_done = [&] {
-        ok = __all_sync(0xffffffffu, mbar_wait(&sh.done[waits & 3], (uint32_t)(waits >> 2) & 1u)) && ok;
-        ++waits;
+        ok = __all_sync(0xffffffffu, mbar_wait(&sh.done[seen & 1u], (seen >> 1) & 1u)) && ok;
+        ++seen;
         tc_fence_after();
+    };
+    auto hand_over = [&] {
+        __syncwarp();
+        fence_async_shared();
+        tmem_store_wait();
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+    };
+    auto decay = [&](int i, int j) { return expf((sh.ch[i] - sh.ch[j]) + (sh.cl[i] - sh.cl[j])); };
+    auto collect = [&](uint32_t place, float (&x)[16]) {
+        uint32_t y[16];
+        tmem_load16_issue(tmem + lanes + place + (uint32_t)t0, y);
+        tmem_load_wait();
+#pragma unroll
+        for (int e = 0; e < 16; ++e) x[e] = __uint_as_float(y[e]);
+    };
+    // parts of this thread's 16 tokens of a column, at three places of tensor memory
+    auto keep_left = [&](const float (&x)[16], uint32_t p0, uint32_t p1, uint32_t p2) {
+        unsigned long long v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = pair_of(x[2 * e], x[2 * e + 1]);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            uint32_t r[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) r[e] = p < 2 ? next_part(v[e]) : last_part(v[e]);
+            tmem_store_issue(tmem + lanes + (p == 0 ? p0 : p == 1 ? p1 : p2) + (uint32_t)cg * 8, r);
+        }
+    };
+    // 128 columns, parts of 64 tokens at three places, times the 64 rows of a triangle
+    auto multiply = [&](uint32_t to, uint32_t p0, uint32_t p1, uint32_t p2, const unsigned char* rows) {
+        if (warp == 0) {
+            constexpr uint32_t id = instr_desc(128, 64);
+            const uint64_t db = smem_desc_k128(smem_addr(rows));
+#pragma unroll
+            for (int p = 0; p < kSplitProducts; ++p)
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    const uint32_t a = split_part_a(p) == 0 ? p0 : split_part_a(p) == 1 ? p1 : p2;
+                    warp_mma_ts(tmem + to, tmem + a + s * 8, desc_advance(db, split_part_b(p) * kDsPart + s * 32), id, (p | s) != 0);
+                }
+            warp_commit(&sh.done[made & 1u]);
+        }
+        ++made;
+    };
+    // what sums over tokens gave no number is made again, a token's own past alone
+    auto mend = [&](float (&x)[16], bool there, const float* from, int c, const float* by) {
+        bool fine = true;
+#pragma unroll
+        for (int e = 0; e < 16; ++e) fine = fine && isfinite(x[e]);
+        tc_fence_before();
+        const bool any = __syncthreads_or(there && !fine);
+        tc_fence_after();
+        if (!any) return;
+        if (there && !fine) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) x[e] = 0.f;
+#pragma unroll 1
+            for (int j = 0; j < t0 + 16; ++j) {
+                const float y = from[delta_at(c, j, kDC)] * by[j];
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                    if (j <= t0 + e) x[e] = fmaf(tri[delta_tri(t0 + e, j)], y, x[e]);
+            }
+        }
+        __syncthreads();  // (four threads read a column that they may write in place)
     };
     if (warp == 0) {
         constexpr uint32_t id = instr_desc(128, 64);
@@ -370,164 +461,118 @@ delta_solve_kernel(const float* __restrict__ qk, float* u, const float* __restri
 #pragma unroll
                 for (int s = 0; s < 4; ++s)
                     warp_mma(tmem + b * 64, desc_advance(da, b * kDsBlock + split_part_a(p) * kDsPart + s * 32),
-                           desc_advance(db, b * kDsBlock + split_part_b(p) * kDsPart + s * 32), id, (p | s) != 0);
+                             desc_advance(db, b * kDsBlock + split_part_b(p) * kDsPart + s * 32), id, (p | s) != 0);
         warp_commit(&sh.done[0]);
     }
+    ++made;
+    float* values = u + unit * kDC * vp;
+    float v[16];
+    auto load_column = [&](const float* from, int c, bool there) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = there ? from[delta_at(c, t0 + e, kDC)] : 0.f;
+    };
+    // (columns of tensor memory: 0 to 127 q . k and k . k, then W and the values' first two parts; 128 to 223 the keys, then U0)
+    load_column(k, row, row < DIM);
+    keep_left(v, 128, 160, 192);
     if (tid < kDC) {  // (the logs are in shared memory)
         float* factors = reinterpret_cast<float*>(logs + unit * kDC);
-        factors[tid] = expf((float)(sh.cs[kDC - 1] - sh.cs[tid]));
-        factors[kDC + tid] = expf((float)sh.cs[tid]);
+        factors[tid] = decay(kDC - 1, tid);
+        factors[kDC + tid] = expf(sh.ch[tid]);
     }
+    load_column(values, row, row < vp);
     wait_done();
-    {   // scores of the queries (rows 0 to 63), and the system's triangle of the keys (rows 64 to 127)
-        float x[32];
+    __syncthreads();  // the queries' tiles are done with
+    {
+        float x[16];
+        collect(0, x);
+        if (BLOCKS > 1) {
+            float y[16];
+            collect(64, y);
 #pragma unroll
-        for (int b = 0; b < BLOCKS; ++b)
-#pragma unroll
-            for (int c = 0; c < 32; c += 16) {
-                uint32_t t[16];
-                tmem_load16_issue(tmem + lanes + (uint32_t)(b * 64 + cg * 32 + c), t);
-                tmem_load_wait();
-#pragma unroll
-                for (int e = 0; e < 16; ++e) x[c + e] = b ? x[c + e] + __uint_as_float(t[e]) : __uint_as_float(t[e]);
-            }
-        tc_fence_before();
+            for (int e = 0; e < 16; ++e) x[e] += y[e];
+        }
         const int i = row & 63;
-        const double ci = sh.cs[i];
+        const bool before = (i | 31) < t0;  // (of the whole warp: its rows come before its keys)
         if (row < 64) {
-            float* to = scores + unit * kDeltaScores;
 #pragma unroll
-            for (int o = 0; o < 4; ++o) {
-                const int j8 = cg * 4 + o;
-                if (i < j8 * 8) continue;
-                float y[8];
+            for (int o = 0; o < 2; ++o) {
+                if (i < t0 + o * 8) continue;
+                float* to = own_scores + delta_score(cg * 2 + o, i);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
-                    const int j = j8 * 8 + e;
-                    y[e] = j <= i ? x[o * 8 + e] * expf((float)(ci - sh.cs[j])) : 0.f;
+                    const int j = t0 + o * 8 + e;
+                    x[o * 8 + e] = j <= i ? x[o * 8 + e] * decay(i, j) : 0.f;
                 }
-                store8(to + delta_score(j8, i), y);
+                store4(to, make_float4(x[o * 8], x[o * 8 + 1], x[o * 8 + 2], x[o * 8 + 3]));
+                store4(to + 4, make_float4(x[o * 8 + 4], x[o * 8 + 5], x[o * 8 + 6], x[o * 8 + 7]));
             }
         } else {
             const float bi = sh.bs[i];
 #pragma unroll
-            for (int j4 = 0; j4 < 8; ++j4) {
-                float y[4];
+            for (int e = 0; e < 16; e += 4) {
+                float y[4] = {0.f, 0.f, 0.f, 0.f};
+                if (!before)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int j = cg * 32 + j4 * 4 + e;
-                    y[e] = j < i ? -x[j4 * 4 + e] * (bi * expf((float)(ci - sh.cs[j]))) : 0.f;
-                }
-                store4(tri + delta_tri(i, cg * 32 + j4 * 4), make_float4(y[0], y[1], y[2], y[3]));
+                    for (int f = 0; f < 4; ++f) {
+                        const int j = t0 + e + f;
+                        y[f] = j < i ? -x[e + f] * (bi * decay(i, j)) : 0.f;
+                    }
+                store4(tri + delta_tri(i, t0 + e), make_float4(y[0], y[1], y[2], y[3]));
             }
         }
     }
-    __syncthreads();
-    delta_invert(tri, mid);
-    // parts of T with its columns weighed
-    auto keep_triangle = [&](const float* by) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int it = e * kDsThreads + tid, i = it & (kDC - 1), o = it >> 6;
-            const float4 a = load4(tri + delta_tri(i, o * 8)), b = load4(tri + delta_tri(i, o * 8 + 4));
-            float y[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-            unsigned long long v[4];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) y[j] = o * 8 + j <= i ? y[j] * by[o * 8 + j] : 0.f;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = pair_of(y[2 * j], y[2 * j + 1]);
-            store_parts(base + i * 128 + ((o ^ (i & 7)) << 4), kDsPart, v);
-        }
-    };
-    auto hand_over = [&] {
-        fence_async_shared();
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-    };
-    // 128 columns of k or v (rows of the result) times the triangle's 64 rows (its columns)
-    auto multiply = [&](uint32_t to, int bar) {
-        if (warp == 0) {
-            constexpr uint32_t id = instr_desc(128, 64) | (1u << 15);
-            const uint64_t mn = smem_desc_mn128(smem_addr(base) + kDsTile);
-            const uint64_t da = (mn & ~((uint64_t)0x3FFF << 16)) | (uint64_t)(kDsBlock >> 4) << 16;
-            const uint64_t db = smem_desc_k128(smem_addr(base));
-#pragma unroll
-            for (int p = 0; p < kSplitProducts; ++p)
-#pragma unroll
-                for (int s = 0; s < 4; ++s)
-                    warp_mma(tmem + to, desc_advance(da, split_part_a(p) * kDsPart + s * 2048),
-                           desc_advance(db, split_part_b(p) * kDsPart + s * 32), id, (p | s) != 0);
-            warp_commit(&sh.done[bar & 3]);
-        }
-    };
-    // what this thread's column `c` of `rows` (octets, [64][8] each) gives tokens cg 32 .. of the result
-    auto collect = [&](uint32_t place, const float* rows, int c, bool there, const float* by, float* to) {
-        float x[32];
-#pragma unroll
-        for (int e0 = 0; e0 < 32; e0 += 16) {
-            uint32_t t[16];
-            tmem_load16_issue(tmem + lanes + place + (uint32_t)(cg * 32 + e0), t);
-            tmem_load_wait();
-#pragma unroll
-            for (int e = 0; e < 16; ++e) x[e0 + e] = __uint_as_float(t[e]);
-        }
-        tc_fence_before();
-        bool fine = true;
-#pragma unroll
-        for (int e = 0; e < 32; ++e) fine = fine && isfinite(x[e]);
-        if (__syncthreads_or(there && !fine)) {
-            const float* from = rows + (size_t)(c >> 3) * kDC * 8 + (c & 7);
-            if (there && !fine) {
-#pragma unroll
-                for (int e = 0; e < 32; ++e) x[e] = 0.f;
-#pragma unroll 1
-                for (int j = 0; j < kDC; ++j) {
-                    const float y = from[j * 8] * by[j];
-#pragma unroll
-                    for (int e = 0; e < 32; ++e)
-                        if (j <= cg * 32 + e) x[e] = fmaf(tri[delta_tri(cg * 32 + e, j)], y, x[e]);
-                }
-            }
-            __syncthreads();  // (two threads read a column that they may write in place)
-        }
-        if (!there) return;
-        float* out = to + (size_t)(c >> 3) * kDC * 8 + (c & 7);
-#pragma unroll
-        for (int e = 0; e < 32; ++e) out[(cg * 32 + e) * 8] = x[e];
-    };
-    keep_triangle(sh.bg);
     hand_over();
-    multiply(128, 1);
-    float* values = u + unit * kDC * vp;
-    const int tiles = (vp + 127) / 128;
-    unsigned long long v[4][4];
-    auto load_values = [&](int tile) {
+    if (tid == 0) {  // (the scores leave as they lie)
+        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(scores + unit * kDeltaScores),
+                     "r"(smem_addr(own_scores)), "r"((uint32_t)(kDeltaScores * 4))
+                     : "memory");
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+    __syncwarp();  // (tensor memory is for whole warps)
+    keep_left(v, 64, 96, 224);
+    delta_invert(tri, mid);
+    const int ti = tid & (kDC - 1), to8 = tid >> 6;  // an octet of the triangle's row
+    auto keep_triangle = [&](unsigned char* to, const float* by) {
+        const float4 a = load4(tri + delta_tri(ti, to8 * 8)), b = load4(tri + delta_tri(ti, to8 * 8 + 4));
+        float y[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        unsigned long long p[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int o = tile * 16 + ((e * kDsThreads + tid) >> 6);
-            if (o * 8 < vp) load8(values + ((size_t)o * kDC + (tid & (kDC - 1))) * 8, v[e]);
-            else v[e][0] = v[e][1] = v[e][2] = v[e][3] = 0ull;
-        }
+        for (int j = 0; j < 8; ++j) y[j] = to8 * 8 + j <= ti ? y[j] * by[to8 * 8 + j] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) p[j] = pair_of(y[2 * j], y[2 * j + 1]);
+        store_parts(to + ti * 128 + ((to8 ^ (ti & 7)) << 4), kDsPart, p);
     };
-    load_values(0);
-    wait_done();  // (the keys and the triangle's parts are done with)
-    keep_triangle(sh.bs);
+    keep_triangle(base + kDsTile, sh.bg);
+    keep_triangle(base, sh.bs);
+    hand_over();
+    multiply(0, 128, 160, 192, base + kDsTile);
+    wait_done();
+    multiply(128, 64, 96, 224, base);
+    float x[16];
+    collect(0, x);
+    mend(x, row < DIM, k, row, sh.bg);
+    if (row < DIM)
+#pragma unroll
+        for (int e = 0; e < 16; ++e) w_out[unit * kDC * DIM + delta_at(row, t0 + e, kDC)] = x[e];
+    const int tiles = (vp + 127) / 128;
 #pragma unroll 1
     for (int tile = 0; tile < tiles; ++tile) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int it = e * kDsThreads + tid, t = it & (kDC - 1), o = it >> 6;
-            store_parts(base + kDsTile + (o >> 3) * kDsBlock + t * 128 + (((o & 7) ^ (t & 7)) << 4), kDsPart, v[e]);
+        const int c = tile * 128 + row;
+        if (tile > 0) {
+            keep_left(v, 64, 96, 224);
+            hand_over();
+            multiply(128, 64, 96, 224, base);
         }
-        hand_over();
-        multiply(192, 2 + tile);
-        if (tile == 0) collect(128, k, row, row < DIM, sh.bg, w_out + unit * kDC * DIM);
-        if (tile + 1 < tiles) load_values(tile + 1);
+        if (tile + 1 < tiles) load_column(values, c + 128, c + 128 < vp);
         wait_done();
-        collect(192, values, tile * 128 + row, tile * 128 + row < vp, sh.bs, values);
+        collect(128, x);
+        mend(x, c < vp, values, c, sh.bs);
+        if (c < vp)
+#pragma unroll
+            for (int e = 0; e < 16; ++e) values[delta_at(c, t0 + e, kDC)] = x[e];
     }
     if (!ok) sh.abort_flag = 1;
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -537,24 +582,24 @@ delta_solve_kernel(const float* __restrict__ qk, float* u, const float* __restri
     if (tid == 0 && sh.abort_flag && status) atomicExch(status, 3);
 }
 
-// Tensor memory of the chain, in columns: the parts of [q; W] and of the weighed keys (both the products' left sides), the sums
-// of 64 places of [q; W] S each, and those of the scores times U.  What the keys add to the state takes the first sums' place.
+// Tensor memory of the chain, in columns: the parts of [q; W], of the weighed keys and of the scores (the products' left sides),
+// [q; W] S, whose place then takes what the keys add to the state, and the scores times U.
 template <int DIM>
 struct DeltaChainPlaces {
-    static constexpr uint32_t rows_part = DIM / 2, keys = 3 * rows_part, keys_part = kDC / 2, sums = keys + 3 * keys_part,
-                              outs = sums + DIM, all = outs + 64;
+    static constexpr uint32_t rows_part = DIM / 2, keys = 3 * rows_part, keys_part = kDC / 2, scores = keys + 3 * keys_part,
+                              sums = scores + 3 * keys_part, outs = sums + 64, all = outs + 64;
     static_assert(all <= 512);
 };
 constexpr int kDtCols = 64, kDtWorkers = 16, kDtThreads = 32 * (1 + kDtWorkers);
-constexpr uint32_t kDtPart = 64 * 128, kDtFactors = 2 * kDC * 4;  // bytes of a part of U or the scores; of a chunk's decays
+constexpr uint32_t kDtPart = 64 * 128, kDtFactors = 2 * kDC * 4;  // bytes of a part of U; of a chunk's decays
 
-// Shared memory of the chain: parts of S (64-column rows), of U and of the scores, then what the next step splits, as it lies
-// in memory: a row of q and W, the keys, the scores, U0.
+// Shared memory of the chain: parts of S (64-column rows) and of U, then what the next step splits, as it lies in memory: rows of q
+// and W, the keys, U0, the scores, the decays of two steps; and a step's outputs on their way.
 template <int DIM>
 struct DeltaChainSmem {
-    static constexpr uint32_t s_part = DIM * 128, u = 3 * s_part, p = u + 3 * kDtPart, rows = p + 3 * kDtPart,
-                              keys = rows + 2 * kDC * DIM * 4, scores = keys + kDC * DIM * 4, u0 = scores + kDeltaScores * 4,
-                              factors = u0 + kDC * kDtCols * 4, all = factors + 2 * kDtFactors + 1024;
+    static constexpr uint32_t s_part = DIM * 128, u = 3 * s_part, rows = u + 3 * kDtPart, keys = rows + 2 * kDC * DIM * 4,
+                              u0 = keys + kDC * DIM * 4, out = u0 + kDC * kDtCols * 4, scores = out + kDC * kDtCols * 4,
+                              factors = scores + kDeltaScores * 4, all = factors + 2 * kDtFactors + 1024;
 };
 
 struct DeltaChainShared {
@@ -567,11 +612,15 @@ struct DeltaChainShared {
 // A CTA per (sequence, head, 64 columns) walks the chunks: one warp brings the operands and issues the products, sixteen hold the
 // state, 16 values a thread (place `row` of the key, columns 16 cg ..), and split what is multiplied.  A step: [q; W] S; U = U0 - W S,
 // split; K^T (e^(c - c_j) U) into the state, which is split for the next step, and P U beside it for the outputs.
-// What bounds it: the two products that wait for each other, 1,445 + 722 cycles of the tensor cores at 64 columns, and the way of
-// their sums through the threads to the next one's operand, twice a step.
+// What bounds it: the two products that wait for each other, 1,445 + 722 cycles of the tensor cores at 64 columns (1,700 and 1,100 to
+// 1,500 beside the copies and splits that share shared memory with them), and the way of their sums through the threads to the
+// next one's operand, 1,100 cycles each: 6,800 cycles a step.  Against a first form, 10,000 cycles a step: left sides in tensor memory
+// instead of the scores in shared memory, rows of 128 swizzled bytes instead of octets, and outputs stored by TMA (row by row from
+// the threads they held up the loads of shared memory of the other warps: 152 us of the kernel, 128 so).  Also tried: P W and P U0
+// made by the solve so that the outputs are P U0 + (e^c q - P W) S: solve 161, chain 157.
 template <int DIM>
 __global__ void __launch_bounds__(kDtThreads, 1)
-delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, const float* __restrict__ u0,
+delta_chain_kernel(const __grid_constant__ CUtensorMap map_o, const float* __restrict__ qk, const float* __restrict__ w, const float* __restrict__ u0,
                    const float* __restrict__ scores, const double* __restrict__ logs, float* __restrict__ state,
                    const int* __restrict__ seq_slots, const int* __restrict__ seq_first_row, const int* __restrict__ seq_count,
                    const int* __restrict__ seq_first_chunk, float* __restrict__ o_raw, int wave0, int wave_n, int H, int G,
@@ -580,7 +629,7 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, co
     using Smem = DeltaChainSmem<DIM>;
     extern __shared__ unsigned char chain_smem[];
     __shared__ DeltaChainShared sh;
-    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(chain_smem) + 1023) & ~(uintptr_t)1023);
+    unsigned char* base = shared_1024(chain_smem);
     pdl_wait();
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -623,7 +672,6 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, co
     if (warp == 0) {
         constexpr uint32_t id = instr_desc(128, 64) | (1u << 16);
         const uint64_t ds = smem_desc_mn128(smem_addr(base)), du = smem_desc_mn128(smem_addr(base + Smem::u));
-        const uint64_t dp = smem_desc_k128(smem_addr(base + Smem::p));
         const uint32_t u0_bytes = (uint32_t)min(kDtCols, vp - col0) * kDC * 4;
         auto bring_rows = [&](int c) {
             if (lane || c >= c1) return;
@@ -652,14 +700,12 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, co
             const uint32_t parity = (uint32_t)(c - c0) & 1u;
             if (!wait(&sh.state_in, parity)) break;
             bring_rows(c + 1);  // (this step's are in tensor memory)
-#pragma unroll 1
-            for (int b = 0; b < DIM / 64; ++b)
 #pragma unroll
-                for (int p = 0; p < kSplitProducts; ++p)
+            for (int p = 0; p < kSplitProducts; ++p)
 #pragma unroll
-                    for (int s = 0; s < 4; ++s)
-                        warp_mma_ts(tmem + At::sums + b * 64, tmem + split_part_a(p) * At::rows_part + b * 32 + s * 8,
-                                    desc_advance(ds, b * 8192 + split_part_b(p) * Smem::s_part + s * 2048), id, (p | s) != 0);
+                for (int s = 0; s < DIM / 16; ++s)
+                    warp_mma_ts(tmem + At::sums, tmem + split_part_a(p) * At::rows_part + s * 8,
+                                desc_advance(ds, split_part_b(p) * Smem::s_part + s * 2048), id, (p | s) != 0);
             warp_commit(&sh.sums_done);
             if (!wait(&sh.u_in, parity)) break;
             bring_keys(c + 1);
@@ -674,8 +720,8 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, co
             for (int p = 0; p < kSplitProducts; ++p)
 #pragma unroll
                 for (int s = 0; s < 4; ++s)
-                    warp_mma(tmem + At::outs, desc_advance(dp, split_part_a(p) * kDtPart + s * 32),
-                             desc_advance(du, split_part_b(p) * kDtPart + s * 2048), id, (p | s) != 0);
+                    warp_mma_ts(tmem + At::outs, tmem + At::scores + split_part_a(p) * At::keys_part + s * 8,
+                                desc_advance(du, split_part_b(p) * kDtPart + s * 2048), id, (p | s) != 0);
             warp_commit(&sh.outs_done);
         }
         if (!ok) sh.abort_flag = 1;
@@ -683,7 +729,7 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, co
     } else {
         const int worker = warp - 1, cg = worker >> 2, row = (warp & 3) * 32 + lane, t = row & 63;
         const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-        const bool writes = row >= 64;  // a token's row of W S; else of its query
+        const bool writes = (warp & 2) != 0;  // a token's row of W S; else of its query
         const int n_cols = vdim - col0 - cg * 16;
         bool ok = true;
         auto wait = [&](uint64_t* bar, int step) {
@@ -704,55 +750,61 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, co
                 store_parts(to + r * 128 + (((cg * 2 + o) ^ (r & 7)) << 4), part, v);
             }
         };
-        auto shared_octet = [&](uint32_t at, unsigned long long (&v)[4]) {
-            const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(base + at), b = *reinterpret_cast<const ulonglong2*>(base + at + 16);
-            v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+        // four neighbouring places of a row of a tile (`word` of its eight)
+        auto shared_word = [&](uint32_t tile, int r, int word) {
+            return *reinterpret_cast<const ulonglong2*>(base + tile + (uint32_t)r * 128 + (uint32_t)((word ^ (r & 7)) << 4));
         };
-        constexpr int RO = DIM / 32;  // octets of its row of q or W that a thread splits
-        auto keep_rows = [&] {
-            unsigned long long v[RO][4];
-#pragma unroll
-            for (int o = 0; o < RO; ++o)
-                shared_octet(Smem::rows + (writes ? kDC * DIM * 4 : 0) + (uint32_t)((cg * RO + o) * kDC + t) * 32, v[o]);
-            uint32_t r[4 * RO];
-#pragma unroll
-            for (int p = 0; p < 3; ++p) {
-#pragma unroll
-                for (int e = 0; e < 4 * RO; ++e) r[e] = p < 2 ? next_part(v[e >> 2][e & 3]) : last_part(v[e >> 2][e & 3]);
-                tmem_store_issue(tmem + lanes + p * At::rows_part + cg * 4 * RO, r);
-            }
-        };
-        const int pj = (worker * 32 + lane) >> 6, pi = (worker * 32 + lane) & 63;
-        auto keep_keys = [&](int step) {  // weighed, and the scores
-            const uint32_t factors = Smem::factors + (uint32_t)(step & 1) * kDtFactors;
-            unsigned long long v[2][4];
-#pragma unroll
-            for (int o = 0; o < 2; ++o) {
-                if (row < DIM) {
-                    unsigned long long f[4];
-                    shared_octet(Smem::keys + (uint32_t)((cg * 2 + o) * DIM + row) * 32, v[o]);
-                    shared_octet(factors + (uint32_t)(cg * 2 + o) * 32, f);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float2 y = halves(v[o][e]), z = halves(f[e]);
-                        v[o][e] = pair_of(y.x * z.x, y.y * z.y);
-                    }
-                } else {
-                    v[o][0] = v[o][1] = v[o][2] = v[o][3] = 0ull;
-                }
-            }
+        auto keep_left = [&](uint32_t at, uint32_t part, unsigned long long (&v)[8]) {
             uint32_t r[8];
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
 #pragma unroll
-                for (int e = 0; e < 8; ++e) r[e] = p < 2 ? next_part(v[e >> 2][e & 3]) : last_part(v[e >> 2][e & 3]);
-                tmem_store_issue(tmem + lanes + At::keys + p * At::keys_part + cg * 8, r);
+                for (int e = 0; e < 8; ++e) r[e] = p < 2 ? next_part(v[e]) : last_part(v[e]);
+                tmem_store_issue(tmem + lanes + at + p * part, r);
             }
-            if (pi >= pj * 8) shared_octet(Smem::scores + (uint32_t)delta_score(pj, pi) * 4, v[0]);
-            else v[0][0] = v[0][1] = v[0][2] = v[0][3] = 0ull;
-            store_parts(base + Smem::p + pi * 128 + ((pj ^ (pi & 7)) << 4), kDtPart, v[0]);
+        };
+        auto keep_rows = [&] {  // DIM / 4 places of its row of q or W
+            const uint32_t from = Smem::rows + (writes ? kDC * DIM * 4 : 0);
+#pragma unroll
+            for (int i = 0; i < DIM / 64; ++i) {
+                const int w0 = cg * (DIM / 16) + i * 4;
+                unsigned long long v[8];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const ulonglong2 a = shared_word(from + (uint32_t)((w0 + e) >> 3) * 8192, t, (w0 + e) & 7);
+                    v[2 * e] = a.x, v[2 * e + 1] = a.y;
+                }
+                keep_left(cg * (DIM / 8) + i * 8, At::rows_part, v);
+            }
+        };
+        auto keep_keys = [&](int step) {  // weighed, and the scores
+            const float* left = reinterpret_cast<const float*>(base + Smem::factors + (uint32_t)(step & 1) * kDtFactors) + cg * 16;
+            unsigned long long v[8];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (row < DIM) {
+                    const ulonglong2 a = shared_word(Smem::keys + (uint32_t)((cg >> 1) * DIM) * 128, row, (cg & 1) * 4 + e);
+                    const float2 x = halves(a.x), y = halves(a.y);
+                    const float4 f = load4(left + e * 4);
+                    v[2 * e] = pair_of(x.x * f.x, x.y * f.y), v[2 * e + 1] = pair_of(y.x * f.z, y.y * f.w);
+                } else {
+                    v[2 * e] = v[2 * e + 1] = 0ull;
+                }
+            }
+            keep_left(At::keys + cg * 8, At::keys_part, v);
+            if (writes) return;
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const ulonglong2* from = reinterpret_cast<const ulonglong2*>(base + Smem::scores + (uint32_t)delta_score(cg * 2 + o, max(t, (cg * 2 + o) * 8)) * 4);
+                const bool there = t >= (cg * 2 + o) * 8;
+                const ulonglong2 a = from[0], b = from[1];
+                v[o * 4] = there ? a.x : 0ull, v[o * 4 + 1] = there ? a.y : 0ull;
+                v[o * 4 + 2] = there ? b.x : 0ull, v[o * 4 + 3] = there ? b.y : 0ull;
+            }
+            keep_left(At::scores + cg * 8, At::keys_part, v);
         };
         const bool wide = (vdim & 3) == 0;
+        const int worker_of_out = cg * 2 + (warp & 1);
         const int first_row = seq_first_row[seq], count = seq_count[seq];
         auto put_outs = [&](int c) {
             const int at = (c - first_chunk) * kDC + t;
@@ -760,26 +812,42 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, co
             uint32_t y[16];
             tmem_load16_issue(tmem + lanes + At::outs + (uint32_t)(cg * 16), y);
             tmem_load_wait();
-            if (at >= count) return;
 #pragma unroll
             for (int e = 0; e < 16; ++e) x[e] = fmaf(x[e], carry, __uint_as_float(y[e]));
             if (sh.any_bad)
 #pragma unroll
                 for (int e = 0; e < 16; ++e)
                     if (at >= sh.bad[cg * 16 + e]) x[e] = __int_as_float(0x7fc00000);
-            float* to = o_raw + ((size_t)(first_row + at) * H + h) * vdim + col0 + cg * 16;
+            if (wide && n_cols >= 16 && (c - first_chunk) * kDC + (t | 31) < count) {  // the warp's 32 rows of 64 bytes, as one store
+                unsigned char* mine = base + Smem::out + (uint32_t)(worker_of_out * 2048);
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                __syncwarp();
 #pragma unroll
-            for (int e = 0; e < 16; e += 4) {
-                if (wide) {
-                    if (e < n_cols) store4(to + e, make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]));
-                } else {
+                for (int e = 0; e < 4; ++e)
+                    store4(reinterpret_cast<float*>(mine + lane * 64 + ((e ^ ((lane >> 1) & 3)) << 4)),
+                           make_float4(x[e * 4], x[e * 4 + 1], x[e * 4 + 2], x[e * 4 + 3]));
+                fence_async_shared();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_2d(&map_o, h * vdim + col0 + cg * 16, first_row + (c - first_chunk) * kDC + (t & 32), mine);
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+            } else if (at < count) {
+                float* to = o_raw + ((size_t)(first_row + at) * H + h) * vdim + col0 + cg * 16;
 #pragma unroll
-                    for (int i = e; i < e + 4; ++i)
-                        if (i < n_cols) to[i] = x[i];
+                for (int e = 0; e < 16; e += 4) {
+                    if (wide) {
+                        if (e < n_cols) store4(to + e, make_float4(x[e], x[e + 1], x[e + 2], x[e + 3]));
+                    } else {
+#pragma unroll
+                        for (int i = e; i < e + 4; ++i)
+                            if (i < n_cols) to[i] = x[i];
+                    }
                 }
             }
         };
         auto hand_over = [&](uint64_t* bar) {
+            __syncwarp();
             fence_async_shared();
             tmem_store_wait();
             tc_fence_before();
@@ -804,26 +872,21 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, co
             const float keep = *reinterpret_cast<const float*>(base + Smem::factors + (uint32_t)(step & 1) * kDtFactors + (2 * kDC - 1) * 4);
             if (writes) {
 #pragma unroll
-                for (int o = 0; o < 2; ++o) {
-                    unsigned long long v[4] = {0ull, 0ull, 0ull, 0ull};
-                    if (col0 + (cg * 2 + o) * 8 < vp) shared_octet(Smem::u0 + (uint32_t)((cg * 2 + o) * kDC + t) * 32, v);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float2 y = halves(v[e]);
-                        x[o * 8 + 2 * e] = y.x, x[o * 8 + 2 * e + 1] = y.y;
-                    }
+                for (int e = 0; e < 4; ++e) {
+                    ulonglong2 a = make_ulonglong2(0ull, 0ull);
+                    if (col0 + cg * 16 < vp) a = shared_word(Smem::u0 + (uint32_t)(cg >> 1) * 8192, t, (cg & 1) * 4 + e);
+                    const float2 y = halves(a.x), z = halves(a.y);
+                    x[e * 4] = y.x, x[e * 4 + 1] = y.y, x[e * 4 + 2] = z.x, x[e * 4 + 3] = z.y;
                 }
             }
             if (!wait(&sh.sums_done, step)) break;
             {
-                uint32_t y[16], z[16];
+                uint32_t y[16];
                 tmem_load16_issue(tmem + lanes + At::sums + (uint32_t)(cg * 16), y);
-                if (DIM > 64) tmem_load16_issue(tmem + lanes + At::sums + 64 + (uint32_t)(cg * 16), z);
                 tmem_load_wait();
                 float sum[16];
 #pragma unroll
-                for (int e = 0; e < 16; ++e)
-                    sum[e] = DIM > 64 ? __uint_as_float(y[e]) + __uint_as_float(z[e]) : __uint_as_float(y[e]);
+                for (int e = 0; e < 16; ++e) sum[e] = __uint_as_float(y[e]);
                 if (writes) {
                     bool fine = true;
 #pragma unroll
@@ -870,6 +933,7 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, co
         }
         if (ok && wait(&sh.outs_done, c1 - 1 - c0) && !writes) put_outs(c1 - 1);
         if (!ok) sh.abort_flag = 1;
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         if (row < DIM)
 #pragma unroll
             for (int e = 0; e < 16; ++e)
@@ -884,6 +948,16 @@ delta_chain_kernel(const float* __restrict__ qk, const float* __restrict__ w, co
     if (tid == 0 && sh.abort_flag && status) atomicExch(status, 3);
 }
 
+// Rows of the outputs for stores of 32 rows x 16 columns, 64 bytes a row, swizzled by fours of words.
+static bool delta_out_map(CUtensorMap* map, float* o_raw, int rows, int cols) {
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * 4};
+    const cuuint32_t box[2] = {16, 32}, elem[2] = {1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, o_raw, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <typename K>
 static cudaError_t most_shared(K kernel, int bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -893,7 +967,7 @@ static cudaError_t most_shared(K kernel, int bytes) {
 
 // a, conv_w, tail, a_log, dt_bias as for nnis_delta_prep (the tail is read; nnis_delta_conv_tail moves it on); dim 64 or
 // 128; chunks int32 [n_chunks, 2] = (sequence, first token of the chunk among the step's), 64 tokens each, with
-// seq_first_chunk [n_seqs + 1].  Float32 scratch on 32-byte boundaries, vp = vdim rounded up to a multiple of eight: qk [wave, G,
+// seq_first_chunk [n_seqs + 1].  Float32 scratch on 32-byte boundaries, vp = vdim rounded up to a multiple of 32: qk [wave, G,
 // 192 dim], u [wave, H, 64 vp], w [wave, H, 64 dim], scores [wave, H, 2304], beta [wave, H, 64]; double logs [wave, H, 64]
 // (of n_chunks, if these are fewer): `wave` chunks are worked at a time.  o_raw float32 [n, H vdim].
 NNIS_API int nnis_delta_prompt(const float* a, const float* conv_w, const float* tail, const float* a_log,
@@ -901,9 +975,9 @@ NNIS_API int nnis_delta_prompt(const float* a, const float* conv_w, const float*
                                const int* seq_count, const int* chunks, int n_chunks, const int* seq_first_chunk, int wave,
                                float* qk, float* u, float* w, float* scores, float* beta, double* logs, float* o_raw,
                                int n_seqs, int H, int G, int dim, int vdim, int taps, float unit_eps, float q_scale,
-                               int* status, cudaStream_t stream) {
+                               int n, int* status, cudaStream_t stream) {
     using namespace nnis;
-    if (n_seqs <= 0 || n_chunks <= 0 || wave <= 0 || H <= 0 || G <= 0 || H % G || vdim <= 0 || taps < 1 || !(unit_eps > 0.f) || !a ||
+    if (n <= 0 || n_seqs <= 0 || n_chunks <= 0 || wave <= 0 || H <= 0 || G <= 0 || H % G || vdim <= 0 || taps < 1 || !(unit_eps > 0.f) || !a ||
         !conv_w || !tail || !a_log || !dt_bias || !state || !seq_slots || !seq_first_row || !seq_count || !chunks ||
         !seq_first_chunk || !qk || !u || !w || !scores || !beta || !logs || !o_raw)
         return NNIS_ERR_ARGUMENT;
@@ -911,7 +985,7 @@ NNIS_API int nnis_delta_prompt(const float* a, const float* conv_w, const float*
     if (((uintptr_t)conv_w | (uintptr_t)o_raw) % 16 ||
         ((uintptr_t)qk | (uintptr_t)u | (uintptr_t)w | (uintptr_t)scores | (uintptr_t)logs) % 32)
         return NNIS_ERR_ALIGNMENT;
-    const int vp = (vdim + 7) & ~7, width = dim > vdim ? dim : vdim;
+    const int vp = (vdim + 31) & ~31, width = dim > vdim ? dim : vdim;
     const int pack_smem = kDC * (width + 1) * 4;
     const int chain_smem = (int)(dim == 128 ? DeltaChainSmem<128>::all : DeltaChainSmem<64>::all);
     auto pack = taps == 4 ? delta_pack_kernel<4> : delta_pack_kernel<0>;
@@ -920,24 +994,26 @@ NNIS_API int nnis_delta_prompt(const float* a, const float* conv_w, const float*
     cudaError_t e = most_shared(pack, pack_smem);
     if (e == cudaSuccess) e = most_shared(solve, (int)kDsSmem);
     if (e == cudaSuccess) e = most_shared(chain, chain_smem);
+    CUtensorMap map_o = {};
+    if (vdim % 4 == 0 && !delta_out_map(&map_o, o_raw, n, H * vdim)) return NNIS_ERR_UNSUPPORTED;
     for (int c0 = 0; c0 < n_chunks && e == cudaSuccess; c0 += wave) {
-        const int n = n_chunks - c0 < wave ? n_chunks - c0 : wave;
+        const int n_own = n_chunks - c0 < wave ? n_chunks - c0 : wave;
         const int* own = chunks + 2 * c0;
-        e = launch_dependent(pack, dim3(n, 2 * G + H + 1), 256, pack_smem, stream, a, conv_w, tail, a_log, dt_bias, own,
+        e = launch_dependent(pack, dim3(n_own, 2 * G + H + 1), 256, pack_smem, stream, a, conv_w, tail, a_log, dt_bias, own,
                              seq_slots, seq_first_row, seq_count, qk, u, beta, logs, H, G, dim, vdim, vp, taps, unit_eps,
                              q_scale);
         // (values become U0 in place, logs the decays that the chain takes: a CTA of the solve reads its own before it writes them)
         if (e == cudaSuccess)
-            e = launch_dependent(solve, dim3(n, H), kDsThreads, kDsSmem, stream, (const float*)qk, u, (const float*)beta, logs,
+            e = launch_dependent(solve, dim3(n_own, H), kDsThreads, kDsSmem, stream, (const float*)qk, u, (const float*)beta, logs,
                                  w, scores, H, G, vp, status);
         // (the chain numbers the chunks of all waves, so its scratch begins where the first wave's would)
         const size_t gone = (size_t)c0 * H;
         if (e == cudaSuccess)
-            e = launch_dependent(chain, dim3((vdim + kDtCols - 1) / kDtCols, H, n_seqs), kDtThreads, chain_smem, stream,
+            e = launch_dependent(chain, dim3((vdim + kDtCols - 1) / kDtCols, H, n_seqs), kDtThreads, chain_smem, stream, map_o,
                                  (const float*)(qk - (size_t)c0 * G * delta_qk_floats(dim)),
                                  (const float*)(w - gone * dim * kDC), (const float*)(u - gone * kDC * vp),
                                  (const float*)(scores - gone * kDeltaScores), (const double*)(logs - gone * kDC), state,
-                                 seq_slots, seq_first_row, seq_count, seq_first_chunk, o_raw, c0, n, H, G, vdim, vp, status);
+                                 seq_slots, seq_first_row, seq_count, seq_first_chunk, o_raw, c0, n_own, H, G, vdim, vp, status);
     }
     return e == cudaSuccess ? NNIS_OK : (int)e;
 }

@@ -2359,7 +2359,7 @@ DELTA_SCRATCH = 1 << 29  # bytes; 32 heads over 16 of 128 x 128 fill it with 5,8
 def delta_wave(n_chunks: int, heads: int, kv_heads: int, dim: int, vdim: int) -> int:
     """How many of a prompt step's chunks are worked at a time: all of them as long as the scratch holds them."""
     vp = -(-vdim // 8) * 8
-    floats = 3 * kv_heads * DELTA_CHUNK * dim + heads * (DELTA_CHUNK * (vp + dim + 3) + max(dim * vp, DELTA_SCORES))
+    floats = 3 * kv_heads * DELTA_CHUNK * dim + heads * (DELTA_CHUNK * (vp + dim + 3) + dim * vp)
     return max(1, min(n_chunks, DELTA_SCRATCH // (4 * floats)))
 
 
@@ -2391,8 +2391,8 @@ def delta_prompt(a: torch.Tensor, conv_w: torch.Tensor, tail: torch.Tensor, a_lo
     seqs, c = seq_first_row.numel(), chunks.shape[0]
     _need(chunks.dtype == seq_first_chunk.dtype == torch.int32 and chunks.dim() == 2 and chunks.shape[1] == 2
           and seq_first_chunk.numel() == seqs + 1, "delta_prompt: chunks int32 [n, 2], seq_first_chunk [sequences + 1]")
-    vp, f = -(-vdim // 8) * 8, torch.float32
-    wave = delta_wave(c, heads, kv_heads, dim, vdim)
+    vp, f = -(-vdim // 32) * 32, torch.float32
+    wave = delta_wave(c, heads, kv_heads, dim, max(vp, DELTA_CHUNK))  # (the scores where a state of 64 columns was counted)
     scratch = [buffer("delta_chunk_qk", (wave, kv_heads, 3 * DELTA_CHUNK * dim), f),
                buffer("delta_chunk_u", (wave, heads, DELTA_CHUNK, vp), f), buffer("delta_chunk_w", (wave, heads, dim, DELTA_CHUNK), f),
                buffer("delta_chunk_scores", (wave, heads, DELTA_SCORES), f), buffer("delta_chunk_beta", (wave, heads, DELTA_CHUNK), f),
@@ -2400,7 +2400,7 @@ def delta_prompt(a: torch.Tensor, conv_w: torch.Tensor, tail: torch.Tensor, a_lo
     _check(_lib().nnis_delta_prompt(_ptr(a), _ptr(conv_w), _ptr(tail), _ptr(a_log), _ptr(dt_bias), _ptr(state),
                                     _ptr(seq_slots), _ptr(seq_first_row), _ptr(seq_count), _ptr(chunks), c,
                                     _ptr(seq_first_chunk), wave, *(_ptr(t) for t in scratch), _ptr(o_raw), seqs, heads, kv_heads,
-                                    dim, vdim, taps, ctypes.c_float(unit_eps), ctypes.c_float(q_scale), _ptr(status_word(a.device)), _stream()),
+                                    dim, vdim, taps, ctypes.c_float(unit_eps), ctypes.c_float(q_scale), n, _ptr(status_word(a.device)), _stream()),
            "delta_prompt", 3 * -(-c // wave))
     _check(_lib().nnis_delta_conv_tail(_ptr(a), _ptr(tail), _ptr(token_pos), _ptr(token_seq), _ptr(seq_slots),
                                        _ptr(seq_first_row), _ptr(seq_count), seqs, heads, kv_heads, dim, vdim, taps,
