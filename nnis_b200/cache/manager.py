@@ -33,6 +33,7 @@ from typing import Dict, List, Optional, Sequence, Tuple, Union
 
 import torch
 
+from ..csrc import ops
 from .slots import CacheFull, FreeList, SlotError
 
 PAGE_SIZE = 64
@@ -150,6 +151,7 @@ class CacheManager:
             self.groups.append(g)
         self._states: List[torch.Tensor] = []
         self._slot_states: Dict[int, List[torch.Tensor]] = {}
+        self._slot_pieces: Dict[int, ops.Pieces] = {}
         for i, r in enumerate(requests):
             if isinstance(r, KVRequest):
                 gi, j = group_of[i]
@@ -189,7 +191,8 @@ class CacheManager:
         for g in self.groups:
             g.tables[slot] = []
         if self._states:
-            torch._foreach_zero_(self._states_of(slot))
+            pieces = self._pieces_of(slot)
+            pieces.clear() if pieces else torch._foreach_zero_(self._states_of(slot))
         return slot
 
     def _states_of(self, slot: int) -> List[torch.Tensor]:
@@ -198,6 +201,15 @@ class CacheManager:
         if views is None:
             views = self._slot_states[slot] = [t[slot] for t in self._states]
         return views
+
+    def _pieces_of(self, slot: int):
+        """The same for one launch over all of them; None without a device (host tests)."""
+        if self.device.type != "cuda":
+            return None
+        pieces = self._slot_pieces.get(slot)
+        if pieces is None:
+            pieces = self._slot_pieces[slot] = ops.Pieces(self._states_of(slot))
+        return pieces
 
     def release(self, slot: int) -> None:
         if not self.slots.is_held(slot):
@@ -301,8 +313,9 @@ class CacheManager:
         model (with keys and values alone it is a truncation)."""
         if not self.slots.is_held(slot):
             raise SlotError(f"slot {slot} is not held")
+        pieces = self._pieces_of(slot) if self._states else None
         return CacheSnapshot(slot, self.owners[slot], self.lengths[slot],
-                             [t.clone() for t in self._states_of(slot)])
+                             pieces.copies() if pieces else [t.clone() for t in self._states_of(slot)])
 
     def restore(self, snapshot: CacheSnapshot) -> None:
         """Back to the snapshot: later positions are forgotten, the state is what it
@@ -316,8 +329,13 @@ class CacheManager:
                             f"sequence only {self.lengths[slot]}")
         if snapshot.length < self.lengths[slot]:
             self._forget_from(slot, snapshot.length)
-        for t, kept in zip(self._states_of(slot), snapshot.states):
-            t.copy_(kept)
+        pieces = self._pieces_of(slot) if snapshot.states else None
+        if pieces and all(k.device == t.device and k.dtype == t.dtype and k.shape == t.shape and k.is_contiguous()
+                          for k, t in zip(snapshot.states, pieces.tensors)):
+            pieces.take_back(snapshot.states)
+        else:
+            for t, kept in zip(self._states_of(slot), snapshot.states):
+                t.copy_(kept)
 
     def page_table(self, group: int, slot: int) -> List[int]:
         return self.groups[group].tables[slot]

@@ -105,6 +105,34 @@ def copy_async(dst: torch.Tensor, src: torch.Tensor) -> None:
         raise KernelError(f"copy_async: CUDA error {code}")
 
 
+class Pieces:
+    """Contiguous tensors of one device that are copied or cleared together, one launch for up to 32 of them."""
+
+    def __init__(self, tensors):
+        self.tensors, n = list(tensors), len(tensors)
+        _need(all(t.is_contiguous() and t.is_cuda for t in self.tensors), "pieces: contiguous CUDA tensors")
+        self.ptrs = (ctypes.c_void_p * max(n, 1))(*(t.data_ptr() for t in self.tensors))
+        self.bytes = (ctypes.c_longlong * max(n, 1))(*(t.numel() * t.element_size() for t in self.tensors))
+
+    def _run(self, src, dst) -> None:
+        if self.tensors:
+            _check(_lib().nnis_copy_pieces(src, dst, self.bytes, len(self.tensors), sm_count(self.tensors[0].device), _stream()),
+                   "copy_pieces", -(-len(self.tensors) // 32))
+
+    def clear(self) -> None:
+        self._run(None, self.ptrs)
+
+    def copies(self) -> list:
+        """New tensors that hold what these hold."""
+        out = [torch.empty_like(t) for t in self.tensors]
+        self._run(self.ptrs, (ctypes.c_void_p * max(len(out), 1))(*(t.data_ptr() for t in out)))
+        return out
+
+    def take_back(self, kept) -> None:
+        """What ``copies`` returned, into these again."""
+        self._run((ctypes.c_void_p * max(len(kept), 1))(*(t.data_ptr() for t in kept)), self.ptrs)
+
+
 def list_to_ints(values: list, limit: int):
     """A list of whole numbers from 0 to below ``limit`` as an int32 array; None where it holds anything else (the
     caller then looks at it number by number)."""
