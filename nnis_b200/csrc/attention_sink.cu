@@ -118,6 +118,92 @@ qkv_prep_kernel(const float* __restrict__ a, const float* __restrict__ wq, const
             gate_out[(size_t)n * H + i] = 1.0f / (1.0f + expf(-row[nq + nk + nv + i]));
 }
 
+// The same where everything lies by fours: two tokens a CTA, 128 threads each, four neighbouring values a thread and load, a
+// token's cosines and sines made once for all its heads.  3,001 tokens of 16 + 4 + 4 heads of 64 on a B200: 23 us with a thread a
+// pair, two stores of two bytes and a cosine and a sine for every pair of every head; 13.6 here, of which 3 are the hand-over from
+// the product before.  Level or slower: the first values asked for before the cosines (15.2 us), 64 threads a token (14.4).
+constexpr int kPrepTurns = 128;  // pairs of a head that turn
+template <typename T>
+__global__ void __launch_bounds__(256)
+qkv_prep_quads_kernel(const float* __restrict__ a, const float* __restrict__ wq, const float* __restrict__ wk,
+                      const float* __restrict__ freq, const int* __restrict__ token_pos,
+                      const int* __restrict__ token_seq, const int* __restrict__ page_table, int table_cols,
+                      T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache,
+                      float* __restrict__ gate_out, int n_tokens, int H, int G, int dk, int dv, int rot, int gated, int page_size,
+                      float eps) {
+    __shared__ float red[2][8];
+    __shared__ float2 turns[2][kPrepTurns];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int half = threadIdx.x >> 7, t = threadIdx.x & 127, n = blockIdx.x * 2 + half;
+    const int pos = n < n_tokens ? token_pos[n] : -1;
+    const int nq = H * dk, nk = G * dk, nv = G * dv;
+    const float* row = a + (size_t)(pos < 0 ? 0 : n) * (nq + nk + nv + (gated ? H : 0));
+    const int quads = (nq + nk + nv) >> 2;
+    size_t cache_row = 0;
+    if (nk && pos >= 0) {
+        const int page = page_table[(size_t)token_seq[n] * table_cols + pos / page_size];
+        cache_row = (size_t)page * G * page_size + (pos % page_size);
+    }
+    for (int i = t; i < rot >> 1; i += 128) {
+        const float ang = (float)pos * freq[i];
+        turns[half][i] = make_float2(cosf(ang), sinf(ang));
+    }
+    if (wq || wk) {
+        float sq = 0.f, sk = 0.f;
+        if (wq) for (int i = t; i < nq; i += 128) sq = fmaf(row[i], row[i], sq);
+        if (wk) for (int i = t; i < nk; i += 128) sk = fmaf(row[nq + i], row[nq + i], sk);
+        sq = warp_sum(sq);
+        sk = warp_sum(sk);
+        if ((threadIdx.x & 31) == 0) {
+            red[0][threadIdx.x >> 5] = sq;
+            red[1][threadIdx.x >> 5] = sk;
+        }
+    }
+    __syncthreads();
+    if (pos < 0) return;
+    float inv_q = 1.0f, inv_k = 1.0f;
+    if (wq || wk) {
+        float sq = 0.f, sk = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            sq += red[0][half * 4 + w];
+            sk += red[1][half * 4 + w];
+        }
+        if (wq) inv_q = 1.0f / sqrtf(sq / (float)nq + eps);
+        if (wk && nk) inv_k = 1.0f / sqrtf(sk / (float)nk + eps);
+    }
+    auto put = [&](int i, const float4& v) {
+        if (4 * i >= nq + nk) {
+            const int e = 4 * i - nq - nk, head = e / dv, within = e - head * dv;
+            store4(v_cache + (cache_row + (size_t)head * page_size) * dv + within, v);
+            return;
+        }
+        const bool is_q = 4 * i < nq;
+        const int e = is_q ? 4 * i : 4 * i - nq;  // element index within q or k
+        const float* wn = is_q ? wq : wk;
+        const float inv = is_q ? inv_q : inv_k;
+        float x[4] = {v.x * inv, v.y * inv, v.z * inv, v.w * inv};
+        if (wn)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) x[k] *= wn[e + k];
+        const int head = e / dk, within = e - head * dk;
+#pragma unroll
+        for (int k = 0; k < 4; k += 2)
+            if (within + k < rot) {
+                const float2 cs = turns[half][(within + k) >> 1];
+                const float y0 = x[k] * cs.x - x[k + 1] * cs.y, y1 = x[k + 1] * cs.x + x[k] * cs.y;
+                x[k] = y0;
+                x[k + 1] = y1;
+            }
+        T* dst = is_q ? q_out + (size_t)n * nq + e : k_cache + (cache_row + (size_t)head * page_size) * dk + within;
+        store4(dst, make_float4(x[0], x[1], x[2], x[3]));
+    };
+    for (int i = t; i < quads; i += 128) put(i, load4(row + 4 * i));
+    if (gated)
+        for (int i = t; i < H; i += 128) gate_out[(size_t)n * H + i] = 1.0f / (1.0f + expf(-row[nq + nk + nv + i]));
+}
+
 // A warp per head of q and of k.  pairing 0: values (2i, 2i + 1) turn together; 1: values (i, i + rot / 2).
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -608,6 +694,24 @@ NNIS_API int nnis_qkv_prep(const float* a, const float* wq, const float* wk, con
     if (G > 0 && (!k_cache || !v_cache || !page_table || !token_seq || page_size <= 0)) return NNIS_ERR_ARGUMENT;
     if (gated && !gate_out) return NNIS_ERR_ARGUMENT;
     cudaError_t e;
+    // (a row of the input, of q and of both caches starts by fours of values, and so does every head)
+    const int row_len = H * dk + G * (dk + dv) + (gated ? H : 0);
+    const uintptr_t out = (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache;
+    if (dk % 4 == 0 && dv % 4 == 0 && row_len % 4 == 0 && rot / 2 <= kPrepTurns && (uintptr_t)a % 16 == 0 &&
+        out % (dtype == NNIS_DTYPE_F32 ? 16 : 8) == 0) {
+        const unsigned blocks = (unsigned)((n_tokens + 1) / 2);
+        if (dtype == NNIS_DTYPE_F32)
+            e = launch_dependent(qkv_prep_quads_kernel<float>, blocks, 256, 0, stream, a, wq, wk, freq, token_pos, token_seq, page_table,
+                                 table_cols, (float*)q_out, (float*)k_cache, (float*)v_cache, gate_out, n_tokens, H, G, dk, dv, rot,
+                                 gated, page_size, eps);
+        else if (dtype == NNIS_DTYPE_BF16)
+            e = launch_dependent(qkv_prep_quads_kernel<bf16>, blocks, 256, 0, stream, a, wq, wk, freq, token_pos, token_seq, page_table,
+                                 table_cols, (bf16*)q_out, (bf16*)k_cache, (bf16*)v_cache, gate_out, n_tokens, H, G, dk, dv, rot,
+                                 gated, page_size, eps);
+        else
+            return NNIS_ERR_UNSUPPORTED;
+        return e == cudaSuccess ? NNIS_OK : (int)e;
+    }
     if (dtype == NNIS_DTYPE_F32)
         e = launch_dependent(qkv_prep_kernel<float>, (unsigned)n_tokens, 256, 0, stream, a, wq, wk, freq, token_pos,
                              token_seq, page_table, table_cols, (float*)q_out, (float*)k_cache, (float*)v_cache,

@@ -402,6 +402,48 @@ __global__ void rope_part_kernel(const T* src, long long src_row, int src_head, 
     }
 }
 
+// The same where everything lies by fours: two tokens a CTA, 128 threads each, four pairs (two with `neighbours`) or four passing
+// values a thread, a token's cosines and sines made once for all its heads.  3,359 tokens of 16 heads of 64 on a B200: 10.0 us a
+// pair a thread, 4.4 here.
+constexpr int kRopeTurns = 128;
+template <typename T>
+__global__ void __launch_bounds__(256)
+rope_part_quads_kernel(const T* src, long long src_row, int src_head, int src_off, T* dst, long long dst_row, int dst_head,
+                       int dst_off, const int* __restrict__ token_pos, const float* __restrict__ freq, int n_tokens, int heads,
+                       int len, int dims, int neighbours) {
+    __shared__ float2 turns[2][kRopeTurns];
+    pdl_wait();
+    pdl_launch_dependents();
+    const int side = threadIdx.x >> 7, t = threadIdx.x & 127, n = blockIdx.x * 2 + side, half = dims >> 1;
+    const int pos = n < n_tokens ? max(token_pos[n], 0) : 0;
+    for (int i = t; i < half; i += 128) {
+        const float ang = (float)pos * freq[i];
+        turns[side][i] = make_float2(cosf(ang), sinf(ang));
+    }
+    __syncthreads();
+    if (n >= n_tokens) return;
+    // items of a head: turned quads (of both halves, or of neighbours), then passing ones
+    const int turned = neighbours ? dims >> 2 : half >> 2, items = turned + ((len - dims) >> 2);
+    for (int it = t; it < heads * items; it += 128) {
+        const int h = it / items, j = it - h * items;
+        const T* s = src + (size_t)n * src_row + (size_t)h * src_head + src_off;
+        T* d = dst + (size_t)n * dst_row + (size_t)h * dst_head + dst_off;
+        if (j >= turned) {
+            const int at = dims + 4 * (j - turned);
+            store4(d + at, load4(s + at));
+        } else if (neighbours) {
+            const float4 x = load4(s + 4 * j);
+            const float2 f = turns[side][2 * j], g = turns[side][2 * j + 1];
+            store4(d + 4 * j, make_float4(x.x * f.x - x.y * f.y, x.y * f.x + x.x * f.y, x.z * g.x - x.w * g.y, x.w * g.x + x.z * g.y));
+        } else {
+            const float4 a = load4(s + 4 * j), b = load4(s + half + 4 * j);
+            const float2 f0 = turns[side][4 * j], f1 = turns[side][4 * j + 1], f2 = turns[side][4 * j + 2], f3 = turns[side][4 * j + 3];
+            store4(d + 4 * j, make_float4(a.x * f0.x - b.x * f0.y, a.y * f1.x - b.y * f1.y, a.z * f2.x - b.z * f2.y, a.w * f3.x - b.w * f3.y));
+            store4(d + half + 4 * j, make_float4(b.x * f0.x + a.x * f0.y, b.y * f1.x + a.y * f1.y, b.z * f2.x + a.z * f2.y, b.w * f3.x + a.w * f3.y));
+        }
+    }
+}
+
 }  // namespace nnis
 
 using namespace nnis;
@@ -570,6 +612,19 @@ NNIS_API int nnis_rope_part(const void* src, long long src_row, int src_head, in
                             int dtype, cudaStream_t stream) {
     if (n_tokens <= 0 || heads <= 0 || len <= 0 || dims < 0 || (dims & 1) || dims > len || !freq)
         return NNIS_ERR_ARGUMENT;
+    // (every head's part starts by fours, and so do its halves and what passes)
+    const bool quads = n_tokens > 2 && len % 4 == 0 && dims % (neighbours ? 4 : 8) == 0 && dims / 2 <= kRopeTurns &&
+                       !((src_row | dst_row | src_head | dst_head | src_off | dst_off) & 3) &&
+                       ((uintptr_t)src | (uintptr_t)dst) % (dtype == NNIS_DTYPE_F32 ? 16 : 8) == 0;
+    if (quads && (dtype == NNIS_DTYPE_F32 || dtype == NNIS_DTYPE_BF16)) {
+        const unsigned blocks = (unsigned)((n_tokens + 1) / 2);
+        const cudaError_t q = dtype == NNIS_DTYPE_F32
+            ? launch_dependent(rope_part_quads_kernel<float>, blocks, 256, 0, stream, (const float*)src, src_row, src_head, src_off,
+                               (float*)dst, dst_row, dst_head, dst_off, token_pos, freq, n_tokens, heads, len, dims, neighbours)
+            : launch_dependent(rope_part_quads_kernel<bf16>, blocks, 256, 0, stream, (const bf16*)src, src_row, src_head, src_off,
+                               (bf16*)dst, dst_row, dst_head, dst_off, token_pos, freq, n_tokens, heads, len, dims, neighbours);
+        return q == cudaSuccess ? NNIS_OK : (int)q;
+    }
     int work = heads * (len - dims / 2);
     int threads = work >= 256 ? 256 : (work >= 128 ? 128 : 64);
     cudaError_t e;
