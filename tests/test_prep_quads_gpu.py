@@ -63,3 +63,27 @@ def test_heads_prepared_by_fours(dtype, H, G, dk, dv, rot, gated, normed, n):
     for got, want in zip(*out):
         assert (got.float() - want.float()).abs().max() <= BOUND[dtype] * max(1.0, float(want.float().abs().max()))
         assert torch.equal(got == 9.0, want == 9.0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq,nkv,d,rotate", [(9, 3, 64, 1), (2, 0, 8, 1), (1, 1, 136, 1), (0, 2, 16, 0), (4, 4, 128, 0)])
+@pytest.mark.parametrize("n", [1, 71])
+def test_heads_rotated_and_stored_by_fours(dtype, nq, nkv, d, rotate, n):
+    from nnis_b200.csrc import ops
+    g = torch.Generator().manual_seed(nq + d + n)
+    qkv = torch.randn(n, (nq + 2 * nkv) * d, generator=g).to(dtype).to(DEV)
+    pos = torch.arange(50, 50 + n, dtype=torch.int32)
+    pos[n // 2] = -1 if n > 1 else 50
+    pos, seq = pos.to(DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+    table = torch.tensor([[2, 0, 1]], dtype=torch.int32, device=DEV)
+    angle = torch.rand(128, d // 2, generator=g) * 6
+    cos, sin, P, out = angle.cos().to(DEV), angle.sin().to(DEV), ops._ptr, []
+    for x in (qkv.clone(), off(qkv)):
+        kc, vc = (torch.full((3, max(nkv, 1), 64, d), 9.0, dtype=dtype, device=DEV) for _ in range(2))
+        code = ops._lib().nnis_rope_store(P(x), 0 if dtype == torch.float32 else 1, P(pos), P(seq), P(table), 3, P(cos), P(sin), P(kc), P(vc),
+                                          n, nq, nkv, d, 64, rotate, ops._stream())
+        assert code == 0
+        out.append((x, kc, vc))
+    for got, want in zip(*out):
+        assert (got.float() - want.float()).abs().max() <= BOUND[dtype] * max(1.0, float(want.float().abs().max()))
+        assert torch.equal(got == 9.0, want == 9.0)
