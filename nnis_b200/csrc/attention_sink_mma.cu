@@ -33,6 +33,8 @@ attn_sink_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cach
                      const float* __restrict__ sink, const float* __restrict__ gate, bf16* __restrict__ out,
                      int nq, int nkv, int window, int chunk, float scale, float cap, int gate_elems, int dk_real,
                      int dv_real, int keep, const float* __restrict__ bias, int bias_len) {
+    pdl_wait();
+    pdl_launch_dependents();
     constexpr int NT = DV / 8, KS = DK / 16;
     const int dk = PAD ? dk_real : DK, dv = PAD ? dv_real : DV;
     const int KCH = dk >> 3, VCH = dv >> 3;  // 16-byte chunks of a row
@@ -298,9 +300,9 @@ static int launch_sink_mma(dim3 grid, cudaStream_t stream, const bf16* q, const 
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    kernel<<<grid, 128, smem, stream>>>(q, k, v, tiles, first_row, start, count, table, cols, sink, gate, out, nq,
-                                        nkv, window, chunk, scale, cap, gate_elems, dk, dv, keep, bias, bias_len);
-    NNIS_RETURN_LAUNCH();
+    const cudaError_t e = launch_dependent(kernel, grid, 128, smem, stream, q, k, v, tiles, first_row, start, count, table, cols, sink, gate,
+                                           out, nq, nkv, window, chunk, scale, cap, gate_elems, dk, dv, keep, bias, bias_len);
+    return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 
 }  // namespace nnis

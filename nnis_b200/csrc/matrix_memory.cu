@@ -175,6 +175,8 @@ memory_gates_kernel(const float* __restrict__ a, int a_cols, const float* __rest
                     const int* __restrict__ seq_count, double* __restrict__ b, double* __restrict__ u,
                     double* __restrict__ top, double* __restrict__ ends, double* __restrict__ before, int H,
                     int gate_off, float cap) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const MemChunk ch = mem_chunk(chunks, seq_first_row, seq_count, blockIdx.x);
     for (int h = blockIdx.y * 8 + warp; h < H; h += gridDim.y * 8) {
@@ -237,6 +239,8 @@ memory_chunk_kernel(const float* __restrict__ a, int a_cols, const double* __res
                     const double* __restrict__ ends, const int* __restrict__ chunks,
                     const int* __restrict__ seq_first_row, const int* __restrict__ seq_count,
                     float* __restrict__ chunk_state, float* __restrict__ chunk_norm, int H, int dim, int vdim) {
+    pdl_wait();
+    pdl_launch_dependents();
     constexpr int TX = BV / 4, RM = BV / 16, STEP = 32;
     __shared__ __align__(16) float Ks[STEP][64];
     __shared__ __align__(16) float Vs[STEP][BV];
@@ -331,6 +335,8 @@ memory_chunk_split_kernel(const float* __restrict__ a, int a_cols, const double*
                           const int* __restrict__ seq_first_row, const int* __restrict__ seq_count,
                           float* __restrict__ chunk_state, float* __restrict__ chunk_norm, int H, int dim, int vdim,
                           int* __restrict__ status) {
+    pdl_wait();
+    pdl_launch_dependents();
     constexpr int C = kMemChunk;
     extern __shared__ __align__(1024) unsigned char sum_smem[];
     __shared__ ChunkReadShared sh;
@@ -373,6 +379,8 @@ __global__ void __launch_bounds__(32)
 memory_chain_kernel(const double* __restrict__ ends, double* before, float* __restrict__ factors,
                     float* __restrict__ max_state, const int* __restrict__ seq_slots, const int* __restrict__ seq_start,
                     const int* __restrict__ seq_count, const int* __restrict__ seq_first_chunk, int H, int by) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int seq = blockIdx.x, h = blockIdx.y, lane = threadIdx.x;
     const int c0 = seq_first_chunk[seq], c1 = seq_first_chunk[seq + 1];
     if (c1 <= c0) return;
@@ -404,6 +412,8 @@ memory_carry_kernel(float* chunk_state, float* chunk_norm, float* state, float* 
                     const float* __restrict__ factors, const int* __restrict__ seq_slots,
                     const int* __restrict__ seq_start, const int* __restrict__ seq_count,
                     const int* __restrict__ seq_first_chunk, int H, int dim, int vdim, int by) {
+    pdl_wait();
+    pdl_launch_dependents();
     constexpr int AHEAD = 8;
     struct alignas(4 * V) Pack { float x[V]; };
     const int seq = blockIdx.x, h = blockIdx.y, per = dim * vdim;
@@ -446,6 +456,8 @@ memory_out_kernel(const float* __restrict__ a, int a_cols, const double* __restr
                   const int* __restrict__ chunks, const int* __restrict__ seq_first_row,
                   const int* __restrict__ seq_start, const int* __restrict__ seq_count, float* __restrict__ o_raw,
                   int H, int dim, int vdim, float q_scale, float floor_add) {
+    pdl_wait();
+    pdl_launch_dependents();
     constexpr int C = kMemChunk, STEP = 32, LD = C + 4, TX = BV / 4, RM = BV / 16;
     extern __shared__ __align__(16) float smem[];
     float* Qs = smem;               // [STEP][LD], by place in dim
@@ -607,6 +619,8 @@ memory_out_split_kernel(const float* __restrict__ a, int a_cols, const double* _
                         const int* __restrict__ seq_first_chunk, int n_seqs, const int* __restrict__ seq_first_row,
                         const int* __restrict__ seq_start, const int* __restrict__ seq_count, float* __restrict__ o_raw,
                         int H, int dim, int vdim, int cols, float q_scale, float floor_add, int* __restrict__ status) {
+    pdl_wait();
+    pdl_launch_dependents();
     constexpr int C = kMemChunk;
     extern __shared__ __align__(1024) unsigned char out_smem[];
     __shared__ ChunkReadShared sh;
@@ -748,51 +762,50 @@ static cudaError_t launch_memory_prompt(const float* a, int a_cols, float* state
     // (rows on 32-byte boundaries)
     const bool split = memory_by_pairs(n_tokens, n_chunks, n_seqs, H, dim, vdim, sms) && a_cols % 8 == 0 &&
                        ((uintptr_t)a | (uintptr_t)chunk_state | (uintptr_t)o_raw) % 32 == 0;
+    // (the prompt's five kernels take 3 to 25 us each: every one is launched beside the end of the
+    // one before and waits for it first thing; prompts of 1500, 1500 and 701 tokens, 16 heads of 64, by
+    // graph take 203 us so, 207 with plain launches)
     const int by = split ? 2 : 1, most_pairs = (n_chunks + n_seqs) / 2;
+    cudaError_t e = cudaSuccess;
     if (split) {
-        cudaError_t e = cudaFuncSetAttribute(memory_chunk_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCrSmem);
+        e = cudaFuncSetAttribute(memory_chunk_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCrSmem);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(memory_out_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCrSmem);
         if (e != cudaSuccess) return e;
-        memory_chunk_split_kernel<<<dim3(most_pairs, H, (vdim + kCrTiles * kCrCols - 1) / (kCrTiles * kCrCols)), kCrThreads,
-                                    kCrSmem, stream>>>(a, a_cols, u, ends, seq_first_chunk, n_seqs, seq_first_row,
-                                                       seq_count, chunk_state, chunk_norm, H, dim, vdim, status);
+        e = launch_dependent(memory_chunk_split_kernel, dim3(most_pairs, H, (vdim + kCrTiles * kCrCols - 1) / (kCrTiles * kCrCols)),
+                             kCrThreads, kCrSmem, stream, a, a_cols, u, ends, seq_first_chunk, n_seqs, seq_first_row, seq_count,
+                             chunk_state, chunk_norm, H, dim, vdim, status);
     } else {
-        memory_chunk_kernel<BV><<<dim3(n_chunks, H, v_tiles * d_tiles), 256, 0, stream>>>(
-            a, a_cols, u, ends, chunks, seq_first_row, seq_count, chunk_state, chunk_norm, H, dim, vdim);
+        e = launch_dependent(memory_chunk_kernel<BV>, dim3(n_chunks, H, v_tiles * d_tiles), 256, 0, stream, a, a_cols, u, ends, chunks,
+                             seq_first_row, seq_count, chunk_state, chunk_norm, H, dim, vdim);
     }
+    if (e != cudaSuccess) return e;
     float* factors = reinterpret_cast<float*>(chunk_gates + (size_t)3 * n_chunks * H);
-    memory_chain_kernel<<<dim3(n_seqs, H), 32, 0, stream>>>(ends, before, factors, max_state, seq_slots, seq_start,
-                                                            seq_count, seq_first_chunk, H, by);
-    const int elems = dim * vdim + dim;
-    if (dim % 4 == 0)
-        memory_carry_kernel<4><<<dim3(n_seqs, H, (elems / 4 + 255) / 256), 256, 0, stream>>>(
-            chunk_state, chunk_norm, state, norm_state, factors, seq_slots, seq_start, seq_count, seq_first_chunk, H, dim,
-            vdim, by);
-    else
-        memory_carry_kernel<1><<<dim3(n_seqs, H, (elems + 255) / 256), 256, 0, stream>>>(
-            chunk_state, chunk_norm, state, norm_state, factors, seq_slots, seq_start, seq_count, seq_first_chunk, H, dim,
-            vdim, by);
+    e = launch_dependent(memory_chain_kernel, dim3(n_seqs, H), 32, 0, stream, ends, before, factors, max_state, seq_slots, seq_start,
+                         seq_count, seq_first_chunk, H, by);
+    if (e != cudaSuccess) return e;
+    const int elems = dim * vdim + dim, each = dim % 4 == 0 ? 4 : 1;
+    e = launch_dependent(each == 4 ? memory_carry_kernel<4> : memory_carry_kernel<1>, dim3(n_seqs, H, (elems / each + 255) / 256), 256, 0,
+                         stream, chunk_state, chunk_norm, state, norm_state, factors, seq_slots, seq_start, seq_count,
+                         seq_first_chunk, H, dim, vdim, by);
+    if (e != cudaSuccess) return e;
     if (split) {
         const int cols = chunk_read_cols((long long)most_pairs * H, vdim, sms);
-        memory_out_split_kernel<<<dim3(most_pairs, H, (vdim + cols - 1) / cols), kCrThreads, kCrSmem, stream>>>(
-            a, a_cols, b, u, top, ends, before, chunk_state, chunk_norm, seq_first_chunk, n_seqs, seq_first_row, seq_start,
-            seq_count, o_raw, H, dim, vdim, cols, q_scale, floor_add, status);
-        return cudaGetLastError();
+        return launch_dependent(memory_out_split_kernel, dim3(most_pairs, H, (vdim + cols - 1) / cols), kCrThreads, kCrSmem, stream, a,
+                                a_cols, b, u, top, ends, before, chunk_state, chunk_norm, seq_first_chunk, n_seqs, seq_first_row,
+                                seq_start, seq_count, o_raw, H, dim, vdim, cols, q_scale, floor_add, status);
     }
     const size_t smem = (size_t)(2 * 32 * (kMemChunk + 4) + kMemChunk * (kMemChunk + 4) + 32 * BV) * sizeof(float);
     auto kernel = memory_out_kernel<BV>;
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
     cudaError_t carve = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                              cudaSharedmemCarveoutMaxShared);  // three CTAs an SM
     if (carve != cudaSuccess) return carve;
-    kernel<<<dim3(n_chunks, H, v_tiles), 256, smem, stream>>>(a, a_cols, b, u, top, before, chunk_state, chunk_norm,
-                                                              chunks, seq_first_row, seq_start, seq_count, o_raw, H,
-                                                              dim, vdim, q_scale, floor_add);
-    return cudaGetLastError();
+    return launch_dependent(kernel, dim3(n_chunks, H, v_tiles), 256, smem, stream, a, a_cols, b, u, top, before, chunk_state, chunk_norm,
+                            chunks, seq_first_row, seq_start, seq_count, o_raw, H, dim, vdim, q_scale, floor_add);
 }
 
 template <typename T>
@@ -856,10 +869,11 @@ NNIS_API int nnis_memory_prompt(const float* a, int a_cols, const float* i_bias,
     if (sms <= 0) return NNIS_ERR_ARGUMENT;
     double *b = gates, *u = gates + (size_t)n_tokens * H, *top = gates + (size_t)2 * n_tokens * H;
     double *ends = chunk_gates, *before = chunk_gates + (size_t)2 * n_chunks * H;
-    memory_gates_kernel<<<dim3(n_chunks, (H + 7) / 8), 256, 0, stream>>>(
-        a, a_cols, i_bias, f_bias, max_state, chunks, seq_slots, seq_first_row, seq_start, seq_count, b, u, top, ends,
-        before, H, 2 * H * (dim + vdim), cap);
-    cudaError_t e = vdim > 64
+    cudaError_t e = launch_dependent(memory_gates_kernel, dim3(n_chunks, (H + 7) / 8), 256, 0, stream, a, a_cols, i_bias, f_bias, max_state,
+                                     chunks, seq_slots, seq_first_row, seq_start, seq_count, b, u, top, ends, before, H,
+                                     2 * H * (dim + vdim), cap);
+    if (e != cudaSuccess) return (int)e;
+    e = vdim > 64
         ? launch_memory_prompt<128>(a, a_cols, state, norm_state, max_state, chunks, n_chunks, seq_first_chunk, n_seqs,
                                     seq_slots, seq_first_row, seq_start, seq_count, gates, chunk_gates, n_tokens,
                                     chunk_state, chunk_norm, o_raw, H, dim, vdim, q_scale, floor_add, sms, status, stream)

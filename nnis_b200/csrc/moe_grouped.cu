@@ -34,6 +34,8 @@ constexpr int kGroupRows = 64;
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int* __restrict__ ids, int n_pairs, int experts, int max_tiles, int tile_rows,
                 int* __restrict__ perm, int* __restrict__ place, int* __restrict__ tile_expert) {
+    pdl_wait();
+    pdl_launch_dependents();
     extern __shared__ int sort_smem[];
     int* count = sort_smem;             // [experts]
     int* first = count + experts;       // [experts + 1]: first row of each padded run
@@ -238,6 +240,8 @@ __global__ void __launch_bounds__(256)
 moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ place,
                    const float* __restrict__ weights, float* __restrict__ residual, int width, int top,
                    const float* __restrict__ pass_weight, const bf16* __restrict__ x) {
+    pdl_wait();
+    pdl_launch_dependents();
     const long long n = blockIdx.x;
     for (int c = threadIdx.x; c < width; c += 256) {
         // (pairs without an expert hand the token's input on: their weights' sum times the input)
@@ -257,6 +261,8 @@ __global__ void __launch_bounds__(256)
 moe_combine_quads_kernel(const float* __restrict__ y, const int* __restrict__ place, const float* __restrict__ weights,
                          float* __restrict__ residual, int width, int top, const float* __restrict__ pass_weight,
                          const bf16* __restrict__ x) {
+    pdl_wait();
+    pdl_launch_dependents();
     const long long n = blockIdx.x;
     for (int c = threadIdx.x * 4; c < width; c += 1024) {
         float4 r = load4(residual + (size_t)n * width + c), sum = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -291,11 +297,11 @@ moe_combine_quads_kernel(const float* __restrict__ y, const int* __restrict__ pl
     }
 }
 
-static void launch_combine(const float* y, const int* place, const float* weights, float* residual, int n_tokens, int width,
-                           int top, const float* pass_weight, const bf16* x, cudaStream_t stream) {
+static cudaError_t launch_combine(const float* y, const int* place, const float* weights, float* residual, int n_tokens, int width,
+                                  int top, const float* pass_weight, const bf16* x, cudaStream_t stream) {
     const bool quads = width % 4 == 0 && ((uintptr_t)y | (uintptr_t)residual) % 16 == 0 && (!pass_weight || (uintptr_t)x % 8 == 0);
-    (quads ? moe_combine_quads_kernel : moe_combine_kernel)<<<n_tokens, 256, 0, stream>>>(y, place, weights, residual, width,
-                                                                                          top, pass_weight, x);
+    return launch_dependent(quads ? moe_combine_quads_kernel : moe_combine_kernel, n_tokens, 256, 0, stream, y, place, weights, residual,
+                            width, top, pass_weight, x);
 }
 
 }  // namespace nnis
@@ -370,8 +376,9 @@ NNIS_API int nnis_moe_grouped(const void* x, const void* w_up, const void* w_dow
     if (((uintptr_t)x | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)act) % 16) return NNIS_ERR_ALIGNMENT;
     const long long pairs = (long long)n_tokens * top;
     const int tiles = nnis_moe_grouped_tiles(pairs, experts);
-    moe_sort_kernel<<<1, 1024, (3 * experts + 1) * sizeof(int), stream>>>(ids, (int)pairs, experts, tiles,
-                                                                         kGroupRows, perm, place, tile_expert);
+    const cudaError_t sorted = launch_dependent(moe_sort_kernel, 1, 1024, (3 * experts + 1) * sizeof(int), stream, ids, (int)pairs,
+                                                experts, tiles, kGroupRows, perm, place, tile_expert);
+    if (sorted != cudaSuccess) return (int)sorted;
     const size_t smem = kGroupedSmem;
     int code = configure_grouped();
     if (code != NNIS_OK) return code;
@@ -380,8 +387,8 @@ NNIS_API int nnis_moe_grouped(const void* x, const void* w_up, const void* w_dow
         (const float*)nullptr, act_kind);
     grouped_mma_kernel<1><<<dim3(tiles, (width + 63) / 64), 128, smem, stream>>>(
         (const bf16*)act, ff, perm, top, (const bf16*)w_down, tile_expert, y, width, ff, 0, 0, 0, 0);
-    launch_combine(y, place, weights, residual, n_tokens, width, top, pass_weight, (const bf16*)x, stream);
-    NNIS_RETURN_LAUNCH();
+    const cudaError_t last = launch_combine(y, place, weights, residual, n_tokens, width, top, pass_weight, (const bf16*)x, stream);
+    return last == cudaSuccess ? NNIS_OK : (int)last;
 }
 
 // Gated experts with the scores on their inputs: w_gu [experts, 2 ff, width] with the gate's and
@@ -400,8 +407,9 @@ NNIS_API int nnis_moe_grouped_gated(const void* x, const void* w_gu, const void*
     if (((uintptr_t)x | (uintptr_t)w_gu | (uintptr_t)w_down | (uintptr_t)act) % 16) return NNIS_ERR_ALIGNMENT;
     const long long pairs = (long long)n_tokens * top;
     const int tiles = nnis_moe_grouped_tiles(pairs, experts);
-    moe_sort_kernel<<<1, 1024, (3 * experts + 1) * sizeof(int), stream>>>(ids, (int)pairs, experts, tiles,
-                                                                         kGroupRows, perm, place, tile_expert);
+    const cudaError_t sorted = launch_dependent(moe_sort_kernel, 1, 1024, (3 * experts + 1) * sizeof(int), stream, ids, (int)pairs,
+                                                experts, tiles, kGroupRows, perm, place, tile_expert);
+    if (sorted != cudaSuccess) return (int)sorted;
     int code = configure_grouped();
     if (code != NNIS_OK) return code;
     grouped_mma_kernel<3><<<dim3(tiles, (2 * ff + 63) / 64), 128, kGroupedSmem, stream>>>(
@@ -409,9 +417,9 @@ NNIS_API int nnis_moe_grouped_gated(const void* x, const void* w_gu, const void*
         weight_on_output ? (const float*)nullptr : weights);
     grouped_mma_kernel<1><<<dim3(tiles, (width + 63) / 64), 128, kGroupedSmem, stream>>>(
         (const bf16*)act, ff, perm, top, (const bf16*)w_down, tile_expert, y, width, ff, 0, 0, 0, 0);
-    launch_combine(y, place, weight_on_output ? weights : (const float*)nullptr, residual, n_tokens, width, top,
+    const cudaError_t last = launch_combine(y, place, weight_on_output ? weights : (const float*)nullptr, residual, n_tokens, width, top,
                    weight_on_output ? pass_weight : nullptr, (const bf16*)x, stream);
-    NNIS_RETURN_LAUNCH();
+    return last == cudaSuccess ? NNIS_OK : (int)last;
 }
 
 // The same with both products on the tcgen05 kernel (nnis_gemm_tc_grouped): runs padded to
@@ -439,9 +447,10 @@ NNIS_API int nnis_moe_grouped_tc(const void* x, const void* w_up, const void* w_
     const long long pairs = (long long)n_tokens * top;
     const int tiles = nnis_moe_grouped_tiles_tc(pairs, experts);
     const int rows = tiles * 128;
-    moe_sort_kernel<<<1, 1024, (3 * experts + 1) * sizeof(int), stream>>>(ids, (int)pairs, experts, tiles, 128, perm,
-                                                                         place, tile_expert);
-    cudaError_t e = launch_dependent(moe_gather_kernel, (unsigned)rows, 256, 0, stream, (const bf16*)x,
+    cudaError_t e = launch_dependent(moe_sort_kernel, 1, 1024, (3 * experts + 1) * sizeof(int), stream, ids, (int)pairs, experts, tiles,
+                                     128, perm, place, tile_expert);
+    if (e != cudaSuccess) return (int)e;
+    e = launch_dependent(moe_gather_kernel, (unsigned)rows, 256, 0, stream, (const bf16*)x,
                                      (const int*)perm, top, (bf16*)x_sorted, width);
     if (e != cudaSuccess) return (int)e;
     int code = nnis_gemm_tc_grouped(x_sorted, w_up, act, rows, ff, width, experts, tile_expert, act_kind, sm_count, status,
@@ -450,8 +459,8 @@ NNIS_API int nnis_moe_grouped_tc(const void* x, const void* w_up, const void* w_
     code = nnis_gemm_tc_grouped(act, w_down, y, rows, width, ff, experts, tile_expert, 0, sm_count, status, pdl,
                                 stream);
     if (code != NNIS_OK) return code;
-    launch_combine(y, place, weights, residual, n_tokens, width, top, pass_weight, (const bf16*)x, stream);
-    NNIS_RETURN_LAUNCH();
+    const cudaError_t last = launch_combine(y, place, weights, residual, n_tokens, width, top, pass_weight, (const bf16*)x, stream);
+    return last == cudaSuccess ? NNIS_OK : (int)last;
 }
 
 // Gated experts with the scores on their inputs, both products on the tcgen05 kernel: the first
@@ -471,9 +480,10 @@ NNIS_API int nnis_moe_grouped_gated_tc(const void* x, const void* w_gu, const vo
     const long long pairs = (long long)n_tokens * top;
     const int tiles = nnis_moe_grouped_tiles_tc(pairs, experts);
     const int rows = tiles * 128;
-    moe_sort_kernel<<<1, 1024, (3 * experts + 1) * sizeof(int), stream>>>(ids, (int)pairs, experts, tiles, 128, perm,
-                                                                         place, tile_expert);
-    cudaError_t e = launch_dependent(moe_gather_kernel, (unsigned)rows, 256, 0, stream, (const bf16*)x,
+    cudaError_t e = launch_dependent(moe_sort_kernel, 1, 1024, (3 * experts + 1) * sizeof(int), stream, ids, (int)pairs, experts, tiles,
+                                     128, perm, place, tile_expert);
+    if (e != cudaSuccess) return (int)e;
+    e = launch_dependent(moe_gather_kernel, (unsigned)rows, 256, 0, stream, (const bf16*)x,
                                      (const int*)perm, top, (bf16*)x_sorted, width);
     if (e != cudaSuccess) return (int)e;
     int code = nnis_gemm_tc_grouped(x_sorted, w_gu, up, rows, 2 * ff, width, experts, tile_expert, 0, sm_count, status,
@@ -485,7 +495,7 @@ NNIS_API int nnis_moe_grouped_gated_tc(const void* x, const void* w_gu, const vo
     code = nnis_gemm_tc_grouped(act, w_down, y, rows, width, ff, experts, tile_expert, 0, sm_count, status, pdl,
                                 stream);
     if (code != NNIS_OK) return code;
-    launch_combine(y, place, weight_on_output ? weights : (const float*)nullptr, residual, n_tokens, width, top,
+    const cudaError_t last = launch_combine(y, place, weight_on_output ? weights : (const float*)nullptr, residual, n_tokens, width, top,
                    weight_on_output ? pass_weight : nullptr, (const bf16*)x, stream);
-    NNIS_RETURN_LAUNCH();
+    return last == cudaSuccess ? NNIS_OK : (int)last;
 }
