@@ -17,9 +17,11 @@ namespace nnis {
 // (32 slices of 128 values, 16 rows: a warp a row 3 us longer; 16,384 rows of 4 slices: a CTA a row 7 us longer of 263
 // with the attention).  Eight slices' values of a thread's pair are asked for together: one after another they were a trip
 // to L2 each (128 rows of 512 values, 16 slices: 9.5 -> 5.8 us; 9,216 rows of 64 values in a float32 prompt: 11.0
-// -> 5.4).
-template <typename T, bool WARP_ROWS>
-__global__ void __launch_bounds__(128)
+// -> 5.4).  EARLY: rows that the device takes all at once, where these trips are the whole time: sixteen slices' values are asked
+// for beside the maxima and sums, needed or not, and rows beyond 256 values take 256 threads, a pair each (128 rows of 512 values,
+// 16 slices, one launch after another: 3.7 -> 2.4 us; behind latent attention 6.1 -> 2.9).
+template <typename T, bool WARP_ROWS, int THREADS, bool EARLY>
+__global__ void __launch_bounds__(THREADS)
 attn_merge_kernel(const float* __restrict__ partial, T* __restrict__ out, size_t n_rows, int d,
                   int n_splits, const float* __restrict__ row_gate, int pairs) {
     __shared__ float shares[WARP_ROWS ? 4 : 1][64];
@@ -30,6 +32,15 @@ attn_merge_kernel(const float* __restrict__ partial, T* __restrict__ out, size_t
     if (row >= n_rows) return;  // (whole warps)
     float* share = shares[WARP_ROWS ? warp : 0];
     const float* rec = partial + row * n_splits * (size_t)(d + 2);
+    const int first = WARP_ROWS ? lane : (int)threadIdx.x;
+    constexpr int kThreads = WARP_ROWS ? 32 : THREADS, kMost = EARLY ? 16 : 8;
+    float2 v[kMost];
+    if (EARLY && pairs) {
+#pragma unroll
+        for (int k = 0; k < kMost; ++k)
+            v[k] = k < n_splits && first * 2 < d ? *reinterpret_cast<const float2*>(rec + (size_t)k * (d + 2) + 2 + first * 2)
+                                                 : make_float2(0.f, 0.f);
+    }
     if (WARP_ROWS || warp == 0) {
         float ms[2], ls[2];
         float m = -FLT_MAX;
@@ -55,23 +66,21 @@ attn_merge_kernel(const float* __restrict__ partial, T* __restrict__ out, size_t
     }
     if (WARP_ROWS) __syncwarp();
     else __syncthreads();
-    const int first = WARP_ROWS ? lane : (int)threadIdx.x;
-    constexpr int kThreads = WARP_ROWS ? 32 : 128;
     if (pairs) {
         for (int i = first * 2; i < d; i += kThreads * 2) {
             float2 o = make_float2(0.f, 0.f);
-            for (int s0 = 0; s0 < n_splits; s0 += 8) {
-                // (slices that hold nothing for the row have weight zero and are never read)
-                float2 v[8];
-                float w[8];
+            for (int s0 = 0; s0 < n_splits; s0 += kMost) {
+                // (slices that hold nothing for the row have weight zero and are never added)
+                float w[kMost];
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
+                for (int k = 0; k < kMost; ++k) {
                     w[k] = s0 + k < n_splits ? share[s0 + k] : 0.f;
-                    v[k] = w[k] != 0.f ? *reinterpret_cast<const float2*>(rec + (size_t)(s0 + k) * (d + 2) + 2 + i)
-                                       : make_float2(0.f, 0.f);
+                    if (!EARLY || s0 || i != first * 2)
+                        v[k] = w[k] != 0.f ? *reinterpret_cast<const float2*>(rec + (size_t)(s0 + k) * (d + 2) + 2 + i)
+                                           : make_float2(0.f, 0.f);
                 }
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
+                for (int k = 0; k < kMost; ++k) {
                     if (w[k] != 0.f) {
                         o.x = fmaf(w[k], v[k].x, o.x);
                         o.y = fmaf(w[k], v[k].y, o.y);
@@ -98,10 +107,18 @@ static cudaError_t launch_merge(const float* partial, T* out, size_t rows, int d
     // (records of an even number of floats start on 8-byte boundaries if the first does)
     const int pairs = d % 2 == 0 && (uintptr_t)partial % 8 == 0 && (uintptr_t)out % (2 * sizeof(T)) == 0;
     const bool warp_rows = d <= 64 || (d <= 128 && rows >= 2000 && n_splits <= 16);
-    return warp_rows ? launch_dependent(attn_merge_kernel<T, true>, (unsigned)((rows + 3) / 4), 128, 0, stream, partial, out,
+    // Early, us, late -> early, 16 slices: 592 rows of 96 / 256 / 512 values 2.8 -> 2.6, 3.2 -> 2.8, 4.5 -> 3.7; 1,776 rows 3.6 -> 4.6,
+    // 4.9 -> 5.2 (a second wave, whose CTAs are fewer an SM).  Up to eight slices are one trip late too: level or slower up to 256 values (592
+    // rows 2.2 -> 2.5), of 512 values 128 rows 2.6 -> 2.3 and 592 rows 3.0 -> 3.3.  More than sixteen are slower (32: 3.6 -> 5.1).
+    const bool wide = d > 256;
+    if (!warp_rows && pairs && n_splits <= 16 && (n_splits > 8 ? rows <= 1184 : wide && rows <= 296)) {
+        return launch_dependent(wide ? attn_merge_kernel<T, false, 256, true> : attn_merge_kernel<T, false, 128, true>, (unsigned)rows,
+                                wide ? 256 : 128, 0, stream, partial, out, rows, d, n_splits, row_gate, pairs);
+    }
+    return warp_rows ? launch_dependent(attn_merge_kernel<T, true, 128, false>, (unsigned)((rows + 3) / 4), 128, 0, stream, partial, out,
                                         rows, d, n_splits, row_gate, pairs)
-                     : launch_dependent(attn_merge_kernel<T, false>, (unsigned)rows, 128, 0, stream, partial, out, rows, d,
-                                       n_splits, row_gate, pairs);
+                     : launch_dependent(attn_merge_kernel<T, false, 128, false>, (unsigned)rows, 128, 0, stream, partial, out, rows,
+                                        d, n_splits, row_gate, pairs);
 }
 
 }  // namespace nnis

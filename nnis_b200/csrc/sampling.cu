@@ -11,12 +11,15 @@
 // on the host sampler.
 #include <float.h>
 
+#include "async_copy.cuh"
 #include "common.cuh"
 
 namespace nnis {
 
 __global__ void __launch_bounds__(256)
 argmax_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float best_v[256];
     __shared__ int best_i[256];
     const float* row = logits + (size_t)blockIdx.x * vocab;
@@ -56,6 +59,8 @@ __global__ void __launch_bounds__(256)
 sample_temperature_kernel(const float* __restrict__ logits, const float* __restrict__ temperature,
                           unsigned long long* __restrict__ rng_state, int* __restrict__ out,
                           int vocab) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ double sums[256];
     __shared__ float red[256];
     __shared__ double target_s;
@@ -110,6 +115,8 @@ sample_temperature_kernel(const float* __restrict__ logits, const float* __restr
 // and live rows (position >= 0) move on by one.
 __global__ void advance_kernel(int* __restrict__ tokens, int* __restrict__ pos,
                                const int* __restrict__ picked, int n) {
+    pdl_wait();
+    pdl_launch_dependents();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || pos[i] < 0) return;
     tokens[i] = picked[i];
@@ -120,21 +127,21 @@ __global__ void advance_kernel(int* __restrict__ tokens, int* __restrict__ pos,
 
 NNIS_API int nnis_advance(int* tokens, int* pos, const int* picked, int n, cudaStream_t stream) {
     if (n <= 0) return NNIS_ERR_ARGUMENT;
-    nnis::advance_kernel<<<(n + 127) / 128, 128, 0, stream>>>(tokens, pos, picked, n);
-    NNIS_RETURN_LAUNCH();
+    const cudaError_t e = nnis::launch_dependent(nnis::advance_kernel, (n + 127) / 128, 128, 0, stream, tokens, pos, picked, n);
+    return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 
 NNIS_API int nnis_argmax(const float* logits, int* out, int n_rows, int vocab, cudaStream_t stream) {
     if (n_rows <= 0 || vocab <= 0) return NNIS_ERR_ARGUMENT;
-    nnis::argmax_kernel<<<n_rows, 256, 0, stream>>>(logits, out, vocab);
-    NNIS_RETURN_LAUNCH();
+    const cudaError_t e = nnis::launch_dependent(nnis::argmax_kernel, n_rows, 256, 0, stream, logits, out, vocab);
+    return e == cudaSuccess ? NNIS_OK : (int)e;
 }
 
 NNIS_API int nnis_sample_temperature(const float* logits, const float* temperature,
                                      unsigned long long* rng_state, int* out, int n_rows, int vocab,
                                      cudaStream_t stream) {
     if (n_rows <= 0 || vocab <= 0 || !temperature || !rng_state) return NNIS_ERR_ARGUMENT;
-    nnis::sample_temperature_kernel<<<n_rows, 256, 0, stream>>>(logits, temperature, rng_state, out,
-                                                               vocab);
-    NNIS_RETURN_LAUNCH();
+    const cudaError_t e = nnis::launch_dependent(nnis::sample_temperature_kernel, n_rows, 256, 0, stream, logits, temperature,
+                                                 rng_state, out, vocab);
+    return e == cudaSuccess ? NNIS_OK : (int)e;
 }
