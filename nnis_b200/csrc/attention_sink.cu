@@ -131,7 +131,7 @@ qkv_prep_quads_kernel(const float* __restrict__ a, const float* __restrict__ wq,
                       T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache,
                       float* __restrict__ gate_out, int n_tokens, int H, int G, int dk, int dv, int rot, int gated, int page_size,
                       float eps) {
-    __shared__ float red[2][8];
+    __shared__ float red[2][2][8];
     __shared__ float2 turns[2][kPrepTurns];
     pdl_wait();
     pdl_launch_dependents();
@@ -150,14 +150,26 @@ qkv_prep_quads_kernel(const float* __restrict__ a, const float* __restrict__ wq,
         turns[half][i] = make_float2(cosf(ang), sinf(ang));
     }
     if (wq || wk) {
-        float sq = 0.f, sk = 0.f;
-        if (wq) for (int i = t; i < nq; i += 128) sq = fmaf(row[i], row[i], sq);
-        if (wk) for (int i = t; i < nk; i += 128) sk = fmaf(row[nq + i], row[nq + i], sk);
-        sq = warp_sum(sq);
-        sk = warp_sum(sk);
-        if ((threadIdx.x & 31) == 0) {
-            red[0][threadIdx.x >> 5] = sq;
-            red[1][threadIdx.x >> 5] = sk;
+        // (the same partial sums as the general kernel's 256 threads, two a thread, met in the same order: the same bits)
+        auto add_squares = [&](const float* x, int n, float (&s)[2]) {
+#pragma unroll 4
+            for (int i = t; i < n; i += 256) {
+                const float u = x[i], v = i + 128 < n ? x[i + 128] : 0.f;
+                s[0] = fmaf(u, u, s[0]);
+                s[1] = fmaf(v, v, s[1]);
+            }
+        };
+        float sq[2] = {0.f, 0.f}, sk[2] = {0.f, 0.f};
+        if (wq) add_squares(row, nq, sq);
+        if (wk) add_squares(row + nq, nk, sk);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            sq[e] = warp_sum(sq[e]);
+            sk[e] = warp_sum(sk[e]);
+            if ((t & 31) == 0) {
+                red[half][0][e * 4 + (t >> 5)] = sq[e];
+                red[half][1][e * 4 + (t >> 5)] = sk[e];
+            }
         }
     }
     __syncthreads();
@@ -166,9 +178,9 @@ qkv_prep_quads_kernel(const float* __restrict__ a, const float* __restrict__ wq,
     if (wq || wk) {
         float sq = 0.f, sk = 0.f;
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {
-            sq += red[0][half * 4 + w];
-            sk += red[1][half * 4 + w];
+        for (int w = 0; w < 8; ++w) {
+            sq += red[half][0][w];
+            sk += red[half][1][w];
         }
         if (wq) inv_q = 1.0f / sqrtf(sq / (float)nq + eps);
         if (wk && nk) inv_k = 1.0f / sqrtf(sk / (float)nk + eps);

@@ -87,3 +87,28 @@ def test_heads_rotated_and_stored_by_fours(dtype, nq, nkv, d, rotate, n):
     for got, want in zip(*out):
         assert (got.float() - want.float()).abs().max() <= BOUND[dtype] * max(1.0, float(want.float().abs().max()))
         assert torch.equal(got == 9.0, want == 9.0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,dk,dv,rot,gated,normed", [(16, 4, 64, 64, 64, True, True), (4, 1, 128, 64, 32, False, True),
+                                                        (3, 3, 20, 8, 16, False, True), (8, 8, 128, 128, 128, False, False)])
+def test_heads_prepared_by_fours_have_the_general_kernels_bits(dtype, H, G, dk, dv, rot, gated, normed):
+    """A prompt's layer gives the same whether its rows lie by fours or not: norms sum in one order."""
+    import ctypes
+    from nnis_b200.csrc import ops
+    n = 601
+    g = torch.Generator().manual_seed(H + dk)
+    a = (torch.randn(n, H * dk + G * (dk + dv) + (H if gated else 0), generator=g) * 3).to(DEV)
+    pos, seq = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+    table = torch.randperm(10, generator=g).to(torch.int32)[None].to(DEV)
+    freq, wq, wk = torch.rand(rot // 2, generator=g).to(DEV), torch.rand(H * dk, generator=g).to(DEV), torch.rand(G * dk, generator=g).to(DEV)
+    out, P = [], ops._ptr
+    for x in (a, off(a)):
+        q, gate = torch.full((n, H * dk), 9.0, dtype=dtype, device=DEV), torch.full((n, H), 9.0, device=DEV)
+        kc, vc = (torch.full((10, G, 64, d), 9.0, dtype=dtype, device=DEV) for d in (dk, dv))
+        assert ops._lib().nnis_qkv_prep(P(x), P(wq) if normed else None, P(wk) if normed else None, P(freq), P(pos), P(seq), P(table), 10,
+                                        P(q), P(kc), P(vc), P(gate), n, H, G, dk, dv, rot, int(gated), 64, ctypes.c_float(1e-5),
+                                        0 if dtype == torch.float32 else 1, ops._stream()) == 0
+        out.append((q, kc, vc, gate))
+    for got, want in zip(*out):
+        assert torch.equal(got, want)
