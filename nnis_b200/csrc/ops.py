@@ -110,14 +110,20 @@ class Pieces:
 
     def __init__(self, tensors):
         self.tensors, n = list(tensors), len(tensors)
-        _need(all(t.is_contiguous() and t.is_cuda for t in self.tensors), "pieces: contiguous CUDA tensors")
+        _need(all(t.is_contiguous() and t.is_cuda and t.device == self.tensors[0].device for t in self.tensors),
+              "pieces: contiguous CUDA tensors of one device")
         self.ptrs = (ctypes.c_void_p * max(n, 1))(*(t.data_ptr() for t in self.tensors))
         self.bytes = (ctypes.c_longlong * max(n, 1))(*(t.numel() * t.element_size() for t in self.tensors))
 
     def _run(self, src, dst) -> None:
-        if self.tensors:
-            _check(_lib().nnis_copy_pieces(src, dst, self.bytes, len(self.tensors), sm_count(self.tensors[0].device), _stream()),
-                   "copy_pieces", -(-len(self.tensors) // 32))
+        if not self.tensors:
+            return
+        device = self.tensors[0].device
+        if torch.cuda.current_device() != device.index:  # (a program of several engines: launched where the tensors are)
+            with torch.cuda.device(device):
+                return self._run(src, dst)
+        _check(_lib().nnis_copy_pieces(src, dst, self.bytes, len(self.tensors), sm_count(device), _stream()),
+               "copy_pieces", -(-len(self.tensors) // 32))
 
     def clear(self) -> None:
         self._run(None, self.ptrs)

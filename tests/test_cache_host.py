@@ -254,3 +254,37 @@ def test_a_slots_version_tells_copies_of_its_page_table_when_they_are_stale():
     assert c.versions[a] == v0 + 2
     c.release(b)
     c.check()
+
+
+def test_states_are_cleared_and_copied_on_their_own_device(monkeypatch):
+    """A program of two engines: whichever device is current, the launch is on the device and stream of the states."""
+    import contextlib
+    import types
+
+    from nnis_b200.csrc import ops
+    current, launched = [1], []
+
+    @contextlib.contextmanager
+    def on(device):
+        before, current[0] = current[0], torch.device(device).index
+        yield
+        current[0] = before
+
+    class Fake:
+        is_cuda, device = True, torch.device("cuda", 0)
+        is_contiguous = lambda self: True
+        data_ptr = lambda self: 4096
+        numel = lambda self: 8
+        element_size = lambda self: 4
+
+    lib = types.SimpleNamespace(nnis_copy_pieces=lambda *args: launched.append((current[0], args[-1].value)) or 0)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
+    monkeypatch.setattr(torch.cuda, "device", on)
+    monkeypatch.setattr(torch, "empty_like", lambda t: Fake())
+    monkeypatch.setattr(ops, "_raw_stream", lambda device: 100 + device)
+    monkeypatch.setattr(ops, "_lib", lambda: lib)
+    monkeypatch.setattr(ops, "sm_count", lambda device: 148)
+    pieces = ops.Pieces([Fake(), Fake()])
+    pieces.clear()
+    pieces.take_back(pieces.copies())
+    assert launched == [(0, 100)] * 3 and current == [1]
