@@ -330,8 +330,9 @@ class CacheManager:
         if snapshot.length < self.lengths[slot]:
             self._forget_from(slot, snapshot.length)
         pieces = self._pieces_of(slot) if snapshot.states else None
-        if pieces and all(k.device == t.device and k.dtype == t.dtype and k.shape == t.shape and k.is_contiguous()
-                          for k, t in zip(snapshot.states, pieces.tensors)):
+        if pieces and len(snapshot.states) == len(pieces.tensors) and \
+                all(k.device == t.device and k.dtype == t.dtype and k.shape == t.shape and k.is_contiguous()
+                    for k, t in zip(snapshot.states, pieces.tensors)):
             pieces.take_back(snapshot.states)
         else:
             for t, kept in zip(self._states_of(slot), snapshot.states):

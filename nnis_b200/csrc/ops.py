@@ -136,6 +136,7 @@ class Pieces:
 
     def take_back(self, kept) -> None:
         """What ``copies`` returned, into these again."""
+        _need(len(kept) == len(self.tensors), "pieces: as many tensors as there are pieces")
         self._run((ctypes.c_void_p * max(len(kept), 1))(*(t.data_ptr() for t in kept)), self.ptrs)
 
 

@@ -288,3 +288,23 @@ def test_states_are_cleared_and_copied_on_their_own_device(monkeypatch):
     pieces.clear()
     pieces.take_back(pieces.copies())
     assert launched == [(0, 100)] * 3 and current == [1]
+
+
+def test_a_snapshot_with_fewer_states_is_copied_as_far_as_it_goes(monkeypatch):
+    """A launch over all pieces would read beyond the list of what is kept."""
+    import types
+    c = make(requests=[StateRequest((3,)), StateRequest((2,))], max_slots=2)
+    s = c.acquire()
+    for i in (0, 1):
+        c.view(i).state[s] = 1.0 + i
+    snap = c.snapshot(s)
+    taken = []
+    pieces = types.SimpleNamespace(tensors=c._states_of(s), take_back=taken.append)
+    monkeypatch.setattr(c, "_pieces_of", lambda slot: pieces)
+    c.restore(snap)
+    assert taken == [snap.states]
+    snap.states = snap.states[:1]
+    for i in (0, 1):
+        c.view(i).state[s] = 9.0
+    c.restore(snap)
+    assert len(taken) == 1 and c.view(0).state[s].tolist() == [1.0] * 3 and c.view(1).state[s].tolist() == [9.0] * 2
