@@ -186,33 +186,41 @@ class Engine:
             starts.append(self.cache.length(s.slot))
         return token_arrays, wants, counts, starts
 
+    def _write(self, head: np.ndarray, tail: np.ndarray, token_arrays, wants, counts, slots, widths) -> None:
+        """Of a step's tables what its shape does not name: the tokens into ``head``, and into ``tail``, as they lie behind
+        positions and sequences, the slots, the wanted rows and every group's page table, ``widths`` columns each."""
+        o = 0
+        for tok in token_arrays:
+            head[o:o + tok.size] = tok
+            o += tok.size
+        o = len(slots)
+        tail[:o] = slots
+        row = 0
+        for want, count in zip(wants, counts):
+            np.add(want, row, out=tail[o:o + want.size])
+            o += want.size
+            row += count
+        for g, width in enumerate(widths):
+            for slot in slots:
+                table = self.cache.page_table(g, slot)[:width]
+                tail[o:o + len(table)] = table
+                tail[o + len(table):o + width] = -1
+                o += width
+
     def _refill(self, batch: Sequence[SequenceStep], entry: dict):
         """``prepare`` for a captured step: what its key names (positions, counts, plans) stands in a pinned buffer of the
         step's own, so tokens, slots, wanted rows and pages are written over it and the whole is copied; a prompt of 3,700
-        tokens in three sequences: 150 us less of the host than tables made anew and views of them that nobody asks for."""
+        tokens in three sequences: 150 us less of the host than tables made anew and views of them that nobody asks for.
+        None where the batch brings another number of tokens than was captured (a key counts what ``len`` says)."""
         token_arrays, wants, counts, starts = self._read(batch)
+        if counts != entry["counts"]:
+            return None
         slots = [s.slot for s in batch]
         new_lengths = [a + b for a, b in zip(starts, counts)]
         self.cache.reserve(slots, new_lengths)
         entry["free"].synchronize()  # (the copy out of the buffer of its last replay)
-        ints, o = entry["ints_np"], 0
-        for tok in token_arrays:
-            ints[o:o + tok.size] = tok
-            o += tok.size
-        o *= 3  # (positions and sequences)
-        ints[o:o + len(slots)] = slots
-        o += len(slots)
-        row = 0
-        for want, count in zip(wants, counts):
-            np.add(want, row, out=ints[o:o + want.size])
-            o += want.size
-            row += count
-        for g, width in enumerate(entry["widths"]):
-            for slot in slots:
-                table = self.cache.page_table(g, slot)[:width]
-                ints[o:o + len(table)] = table
-                ints[o + len(table):o + width] = -1
-                o += width
+        ints, n = entry["ints_np"], sum(counts)
+        self._write(ints[:n], ints[3 * n:], token_arrays, wants, counts, slots, entry["widths"])
         entry["dev"].copy_(entry["ints"], non_blocking=True)
         self.h2d_bytes += 4 * ints.size
         entry["free"].record()
@@ -233,17 +241,11 @@ class Engine:
         pos = np.concatenate([np.arange(a, e, dtype=np.int32) for a, e in zip(starts, new_lengths)])
         seq = np.repeat(np.arange(b, dtype=np.int32), counts)
         first_rows = np.concatenate([[0], np.cumsum(counts)[:-1]]).astype(np.int32)
-        want_rows = np.concatenate([first_rows[i] + w for i, w in enumerate(wants)]).astype(np.int32, copy=False)
-        parts = [np.concatenate(token_arrays), pos, seq, i32(slots), want_rows]
-        cols = []
-        for g in range(len(self.cache.groups)):
-            width = max(1, max(-(-L // PAGE_SIZE) for L in new_lengths))
-            table = np.full((b, width), -1, dtype=np.int32)
-            for r, slot in enumerate(slots):
-                t = self.cache.page_table(g, slot)[:width]
-                table[r, :len(t)] = t
-            parts.append(table.reshape(-1))
-            cols.append(width)
+        n_want = sum(w.size for w in wants)
+        cols = [max(1, max(-(-L // PAGE_SIZE) for L in new_lengths))] * len(self.cache.groups)
+        changing = np.empty(n + b + n_want + b * sum(cols), dtype=np.int32)
+        self._write(changing[:n], changing[n:], token_arrays, wants, counts, slots, cols)
+        parts = [changing[:n], pos, seq, changing[n:]]
         decode = all(c == 1 for c in counts)
         if not decode:
             parts += [first_rows, i32(starts), i32(counts)]
@@ -263,7 +265,7 @@ class Engine:
             return out
 
         d_tokens, d_pos, d_seq, d_slots = take(n), take(n), take(n), take(b)
-        d_want = take(want_rows.size)
+        d_want = take(n_want)
         d_tables = [take(b * c).view(b, c) for c in cols]
         ctx = StepContext(
             n_tokens=n, n_seqs=b, tokens=d_tokens, token_pos=d_pos, token_seq=d_seq,
@@ -298,10 +300,11 @@ class Engine:
         entry = self._step_graphs.get(key) if key is not None else None
         if entry is not None:
             self._step_graphs[key] = self._step_graphs.pop(key)  # most recently used last
-            slots, new_lengths = self._refill(batch, entry)
-            entry["graph"].replay()
-            self.cache.commit(slots, new_lengths)
-            return entry["logits"].clone()
+            refilled = self._refill(batch, entry)
+            if refilled is not None:
+                entry["graph"].replay()
+                self.cache.commit(*refilled)
+                return entry["logits"].clone()
         if key is not None and key in self._seen_shapes:
             return self._capture_step(batch, key)
         if key is not None:
@@ -343,7 +346,7 @@ class Engine:
         free.record()
         self._step_graphs[key] = {"graph": graph, "workspace": workspace, "logits": logits, "dev": dev, "ints": ints,
                                   "ints_np": ints.numpy(), "free": free,
-                                  "widths": [t.shape[1] for t in ctx.page_tables]}
+                                  "counts": list(ctx.host_counts), "widths": [t.shape[1] for t in ctx.page_tables]}
         return result
 
     def step_in_portions(self, batch: Sequence[SequenceStep], max_step_tokens: int) -> torch.Tensor:

@@ -219,6 +219,44 @@ def test_recurring_prompt_shapes_are_replayed_from_a_graph(models, dtype, tmp_pa
     assert any(e["graph"] is not None for e in engine._step_graphs.values())
 
 
+def test_a_replayed_step_takes_its_own_places_slots_and_tokens(models, monkeypatch):
+    """What a captured shape does not name comes from the step at hand: other wanted places of the same number, slots in
+    another order with other pages, and tokens whose ``len`` is not their number, which no replay may take."""
+    from nnis_b200.engine import SequenceStep
+    from nnis_b200.engine import engine as module
+    rng, vocab = random.Random(21), CONFIGS["A"]["vocab_size"]
+    engine = engine_for(models, "A", "bfloat16")
+    wants = [([0, 150, 255], [39]), ([0, 150, 255], [39]), ([7, 8, 201], [0]), ([254, 1, 64], [17]), ([0, 63, 128], [39])]
+    prompts = [(random_tokens(rng, 256, vocab), random_tokens(rng, 40, vocab)) for _ in wants]
+
+    def run():
+        out, held = [], []
+        for i, ((a, b), (wa, wb)) in enumerate(zip(prompts, wants)):
+            slots = [engine.acquire_slot(), engine.acquire_slot()]
+            if i % 2:
+                slots.reverse()
+            out.append(engine.step([SequenceStep(slots[0], a, wa), SequenceStep(slots[1], b, wb)]))
+            held.append(slots.pop(i % 2))  # the other stays, so that slots and pages differ from round to round
+            engine.release_slot(slots[0])
+        for slot in held:
+            engine.release_slot(slot)
+        # an array of rows: 256 by ``len``, 512 tokens
+        slots = [engine.acquire_slot(), engine.acquire_slot()]
+        rows = np.asarray(prompts[0][0] + prompts[1][0]).reshape(256, 2)
+        out.append(engine.step([SequenceStep(slots[0], rows, [0, 300, 511]), SequenceStep(slots[1], prompts[0][1], [39])]))
+        assert engine.cache.length(slots[0]) == 512
+        for slot in slots:
+            engine.release_slot(slot)
+        return out
+
+    before = len(engine._step_graphs)
+    got = run()
+    assert len(engine._step_graphs) == min(before + 1, module.MAX_STEP_GRAPHS)
+    monkeypatch.setattr(module, "GRAPH_MIN_TOKENS", 1 << 30)
+    for x, y in zip(got, run()):
+        assert torch.equal(x, y)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_prompts_in_portions_give_the_logits_of_one_step(models, dtype):
     """Long batches of prompts are run as several steps of a bounded number of tokens;
