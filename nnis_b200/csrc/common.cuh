@@ -94,6 +94,14 @@ __device__ __forceinline__ float warp_max(float v) {
 // (NNIS_PDL=0 turns it off everywhere); defined in elementwise.cu.
 bool dependent_launches();
 
+// The current device's SMs (a B200's where it cannot be asked).
+inline int device_sms() {
+    int device = 0, sms = 0;
+    const bool known = cudaGetDevice(&device) == cudaSuccess &&
+                       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && sms > 0;
+    return known ? sms : 148;
+}
+
 // Launch `kernel` as a programmatic dependent of the kernel before it on the stream: it may
 // be scheduled while that kernel still runs and waits for it with griddepcontrol.wait (the
 // kernel must call pdl_wait() before it touches anything a kernel of the step writes).
