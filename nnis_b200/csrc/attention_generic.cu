@@ -149,6 +149,12 @@ static int launch_attention(const void* q, int q_stride, const void* k_cache, co
 }  // namespace nnis
 
 // The merge alone, for kernels that write the same partial records.
+NNIS_API int nnis_attention_merge_f32(const float* partial, void* out, long long n_rows, int d,
+                                      int n_splits, cudaStream_t stream) {
+    if (n_splits > 64) return NNIS_ERR_UNSUPPORTED;
+    const cudaError_t e = nnis::launch_merge<float>(partial, (float*)out, (size_t)n_rows, d, n_splits, nullptr, stream);
+    return e == cudaSuccess ? NNIS_OK : (int)e;
+}
 NNIS_API int nnis_attention_merge_bf16(const float* partial, void* out, long long n_rows, int d,
                                        int n_splits, cudaStream_t stream) {
     if (n_splits > 64) return NNIS_ERR_UNSUPPORTED;

@@ -17,7 +17,7 @@ namespace nnis {
 // (32 slices of 128 values, 16 rows: a warp a row 3 us longer; 16,384 rows of 4 slices: a CTA a row 7 us longer of 263
 // with the attention).  Eight slices' values of a thread's pair are asked for together: one after another they were a trip
 // to L2 each (128 rows of 512 values, 16 slices: 9.5 -> 5.8 us; 9,216 rows of 64 values in a float32 prompt: 11.0
-// -> 5.4).  EARLY: rows that the device takes all at once, where these trips are the whole time: sixteen slices' values are asked
+// -> 5.4).  EARLY: few rows, where these trips are the whole time: sixteen slices' values are asked
 // for beside the maxima and sums, needed or not, and rows beyond 256 values take 256 threads, a pair each (128 rows of 512 values,
 // 16 slices, one launch after another: 3.7 -> 2.4 us; behind latent attention 6.1 -> 2.9).
 template <typename T, bool WARP_ROWS, int THREADS, bool EARLY>
@@ -107,11 +107,25 @@ static cudaError_t launch_merge(const float* partial, T* out, size_t rows, int d
     // (records of an even number of floats start on 8-byte boundaries if the first does)
     const int pairs = d % 2 == 0 && (uintptr_t)partial % 8 == 0 && (uintptr_t)out % (2 * sizeof(T)) == 0;
     const bool warp_rows = d <= 64 || (d <= 128 && rows >= 2000 && n_splits <= 16);
-    // Early, us, late -> early, 16 slices: 592 rows of 96 / 256 / 512 values 2.8 -> 2.6, 3.2 -> 2.8, 4.5 -> 3.7; 1,776 rows 3.6 -> 4.6,
-    // 4.9 -> 5.2 (a second wave, whose CTAs are fewer an SM).  Up to eight slices are one trip late too: level or slower up to 256 values (592
-    // rows 2.2 -> 2.5), of 512 values 128 rows 2.6 -> 2.3 and 592 rows 3.0 -> 3.3.  More than sixteen are slower (32: 3.6 -> 5.1).
-    const bool wide = d > 256;
-    if (!warp_rows && pairs && n_splits <= 16 && (n_splits > 8 ? rows <= 1184 : wide && rows <= 296)) {
+    // Early as long as the device holds all rows beside the next kernel's CTAs (float32 outputs take more registers: three instead of four CTAs an
+    // SM).  us late -> early, bfloat16 / float32: 16 slices of 128 values, 444 rows 2.66 -> 2.32 / 2.66 -> 2.31, 592 rows 2.75 -> 2.45 / 2.72 -> 2.85, 740 rows
+    // 2.85 -> 3.01; of 512 values 444 rows 4.19 -> 3.38 / 4.19 -> 3.12, 592 rows 4.41 -> 3.53 / 4.49 -> 4.50, 740 rows 4.66 -> 4.85; of 1,024 values 296 rows
+    // 6.28 -> 5.85, 370 rows 6.66 -> 6.83.  From 6 rows an SM on the late form is in its second wave, the early one up to 8 (7) not in its third: 1,036 rows of
+    // 256 values 4.67 -> 3.43 / 4.69 -> 3.27, of 512 7.72 -> 5.57 / 7.72 -> 6.45 (level at 128 values; 320 values of float32, 9 slices, 5.58 -> 5.84).  Up to eight
+    // slices are one trip late too: level or slower up to 256 values (592 rows 2.14 -> 2.40), of 512 values 296 rows 2.76 -> 2.55 / 2.76 -> 2.86, 128 rows
+    // 2.56 -> 2.20 / 2.56 -> 2.20, of 1,024 slower (3.58 -> 4.04).  More than sixteen are slower (32: 3.6 -> 5.1).
+    const bool wide = d > 256, f32 = sizeof(T) == 4;
+    bool early = !warp_rows && pairs && n_splits <= 16;
+    if (early) {
+        const size_t sms = (size_t)device_sms(), held = f32 ? 3 : 4;
+        if (n_splits > 8) {
+            const bool second = d > 128 && d <= 512 && (d <= 256 || d >= 384) && rows > 6 * sms && rows <= (f32 ? 7 : 8) * sms;
+            early = rows <= (d > 512 ? 2 : held) * sms || second;
+        } else {
+            early = wide && d <= 512 && rows <= held / 2 * sms;
+        }
+    }
+    if (early) {
         return launch_dependent(wide ? attn_merge_kernel<T, false, 256, true> : attn_merge_kernel<T, false, 128, true>, (unsigned)rows,
                                 wide ? 256 : 128, 0, stream, partial, out, rows, d, n_splits, row_gate, pairs);
     }
