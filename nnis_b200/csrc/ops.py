@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import math
 import os
 from typing import Optional
 
@@ -2388,14 +2389,21 @@ DELTA_CHUNK_MIN, DELTA_STEP_MIN = 192, 256
 
 
 DELTA_SCORES = 2304      # floats that the scores of a chunk and head take
-DELTA_SCRATCH = 1 << 29  # bytes; 32 heads over 16 of 128 x 128 fill it with 5,800 tokens
+DELTA_SCRATCH = 1 << 29  # bytes; 32 heads over 16 of 128 x 128 fill it with 8,500 tokens
+
+
+def delta_scratch(wave: int, heads: int, kv_heads: int, dim: int, vdim: int) -> list:
+    """(name, shape, dtype) of the scratch of ``wave`` chunks that are worked at a time."""
+    vp, f = -(-vdim // 32) * 32, torch.float32
+    return [("delta_chunk_qk", (wave, kv_heads, 3 * DELTA_CHUNK * dim), f), ("delta_chunk_u", (wave, heads, DELTA_CHUNK, vp), f),
+            ("delta_chunk_w", (wave, heads, dim, DELTA_CHUNK), f), ("delta_chunk_scores", (wave, heads, DELTA_SCORES), f),
+            ("delta_chunk_beta", (wave, heads, DELTA_CHUNK), f), ("delta_chunk_logs", (wave, heads, DELTA_CHUNK), torch.float64)]
 
 
 def delta_wave(n_chunks: int, heads: int, kv_heads: int, dim: int, vdim: int) -> int:
     """How many of a prompt step's chunks are worked at a time: all of them as long as the scratch holds them."""
-    vp = -(-vdim // 8) * 8
-    floats = 3 * kv_heads * DELTA_CHUNK * dim + heads * (DELTA_CHUNK * (vp + dim + 3) + dim * vp)
-    return max(1, min(n_chunks, DELTA_SCRATCH // (4 * floats)))
+    one = sum(math.prod(shape) * dtype.itemsize for _, shape, dtype in delta_scratch(1, heads, kv_heads, dim, vdim))
+    return max(1, min(n_chunks, DELTA_SCRATCH // one))
 
 
 def delta_takes_chunks(dim: int, vdim: int) -> bool:
@@ -2426,12 +2434,8 @@ def delta_prompt(a: torch.Tensor, conv_w: torch.Tensor, tail: torch.Tensor, a_lo
     seqs, c = seq_first_row.numel(), chunks.shape[0]
     _need(chunks.dtype == seq_first_chunk.dtype == torch.int32 and chunks.dim() == 2 and chunks.shape[1] == 2
           and seq_first_chunk.numel() == seqs + 1, "delta_prompt: chunks int32 [n, 2], seq_first_chunk [sequences + 1]")
-    vp, f = -(-vdim // 32) * 32, torch.float32
-    wave = delta_wave(c, heads, kv_heads, dim, max(vp, DELTA_CHUNK))  # (the scores where a state of 64 columns was counted)
-    scratch = [buffer("delta_chunk_qk", (wave, kv_heads, 3 * DELTA_CHUNK * dim), f),
-               buffer("delta_chunk_u", (wave, heads, DELTA_CHUNK, vp), f), buffer("delta_chunk_w", (wave, heads, dim, DELTA_CHUNK), f),
-               buffer("delta_chunk_scores", (wave, heads, DELTA_SCORES), f), buffer("delta_chunk_beta", (wave, heads, DELTA_CHUNK), f),
-               buffer("delta_chunk_logs", (wave, heads, DELTA_CHUNK), torch.float64)]
+    wave = delta_wave(c, heads, kv_heads, dim, vdim)
+    scratch = [buffer(*asked) for asked in delta_scratch(wave, heads, kv_heads, dim, vdim)]
     _check(_lib().nnis_delta_prompt(_ptr(a), _ptr(conv_w), _ptr(tail), _ptr(a_log), _ptr(dt_bias), _ptr(state),
                                     _ptr(seq_slots), _ptr(seq_first_row), _ptr(seq_count), _ptr(chunks), c,
                                     _ptr(seq_first_chunk), wave, *(_ptr(t) for t in scratch), _ptr(o_raw), seqs, heads, kv_heads,

@@ -1,4 +1,5 @@
 """Work lists that the host makes for kernels: checked without a GPU."""
+import math
 
 
 def test_prompt_attention_plan_cuts_tiles_without_empty_chunks():
@@ -309,7 +310,8 @@ def test_chunks_of_the_delta_rule_keep_their_scratch_within_its_bound():
     from nnis_b200.csrc import ops as o
     assert o.delta_wave(52, 32, 16, 128, 128) == 52   # 3,300 tokens
     wave = o.delta_wave(4096, 32, 16, 128, 128)
-    assert 4 * wave * (3 * 16 * 64 * 128 + 32 * (64 * (128 + 128 + 3) + 128 * 128)) <= o.DELTA_SCRATCH < 1 << 30 and wave > 52
+    asked = lambda n: sum(math.prod(shape) * dtype.itemsize for _, shape, dtype in o.delta_scratch(n, 32, 16, 128, 128))
+    assert asked(wave) <= o.DELTA_SCRATCH < 1 << 30 and asked(wave + 1) > o.DELTA_SCRATCH and 64 * wave > 8500
     assert o.delta_wave(9, 4096, 4096, 128, 512) >= 1
 
 

@@ -516,13 +516,18 @@ def test_delta_rule_chunks_in_waves(wave, monkeypatch):
     tables = [i32(x) for x in ([t + 9 for c in new for t in range(c)], [i for i, c in enumerate(new) for _ in range(c)],
                                [0, 1, 2, 3], [sum(new[:i]) for i in range(len(new))], new)]
     got = []
-    for scratch in (o.DELTA_SCRATCH, 4 * wave * (3 * G * 64 * dim + H * (64 * (vdim + dim + 3) + dim * vdim))):
+    held = sum(math.prod(shape) * dtype.itemsize for _, shape, dtype in o.delta_scratch(wave, H, G, dim, vdim))
+    for scratch in (o.DELTA_SCRATCH, held):
         monkeypatch.setattr(o, "DELTA_SCRATCH", scratch)
-        assert o.delta_wave(len(chunks), H, G, dim, vdim) == (len(chunks) if not got else wave)
+        asked = []
+
+        def buffer(name, shape, dtype):
+            asked.append(shape[0])
+            return torch.full(shape, math.nan, dtype=dtype, device=DEV)
+
         state, tail, o_raw = begin.to(DEV), tails.to(DEV), torch.full((n, H * vdim), 5.0, device=DEV)
-        o.delta_prompt(rows, conv, tail, a_log, bias, state, *tables, chunks, first,
-                       lambda name, shape, dtype: torch.full(shape, math.nan, dtype=dtype, device=DEV), o_raw, H, G, dim,
-                       vdim, 1e-6, 1.0)
+        o.delta_prompt(rows, conv, tail, a_log, bias, state, *tables, chunks, first, buffer, o_raw, H, G, dim, vdim, 1e-6, 1.0)
+        assert asked == [wave if got else len(chunks)] * 6
         got.append((o_raw, state, tail))
     for one, other in zip(*got):
         assert torch.equal(one, other)
