@@ -712,3 +712,32 @@ def test_delta_rule_chunks_at_the_edges_of_their_tiles(dim, vdim):
     hit = torch.zeros_like(state, dtype=torch.bool)
     hit[3, 1, :, 3] = True
     assert torch.equal(torch.isnan(bad_state), hit) and torch.equal(bad_state[~hit], state[~hit])
+
+
+def test_a_chunks_decays_are_rounded_once():
+    """e^(c_last - c_j) of every chunk, as the solve leaves it for the walk, against 64-bit sums of the same logs: the difference is rounded
+    to float32 once (half a unit in its last place) and the exponential is two units off at most."""
+    o = ops()
+    g = torch.Generator().manual_seed(3)
+    H, G, dim, vdim, taps, n = 16, 1, 64, 32, 1, 512
+    channels = 2 * G * dim + H * vdim
+    rows = torch.randn(n, channels + H * vdim + 2 * H, generator=g).to(DEV)
+    conv, tails = torch.ones(channels, taps, device=DEV), torch.zeros(1, 1, channels, device=DEV)
+    a_log, bias = torch.linspace(-4.0, 0.5, H).to(DEV), torch.zeros(H, device=DEV)
+    tables = [i32(x) for x in (range(n), [0] * n, [0], [0], [n])]
+    qkv, beta_g = torch.empty(n, channels, device=DEV), torch.empty(n, 2 * H, device=DEV)
+    o.delta_prep(rows, conv, tails.clone(), a_log, bias, *tables, qkv, beta_g, H, G, dim, vdim, 1e-6, 1.0)
+    chunks, first = (torch.from_numpy(t).to(DEV) for t in o.scan_segments([n], o.DELTA_CHUNK))
+    held = {}
+
+    def buffer(name, shape, dtype):
+        held[name] = torch.full(shape, math.nan, dtype=dtype, device=DEV)
+        return held[name]
+
+    o.delta_prompt(rows, conv, tails, a_log, bias, torch.zeros(1, H, dim, vdim, device=DEV), *tables, chunks, first, buffer,
+                   torch.empty(n, H * vdim, device=DEV), H, G, dim, vdim, 1e-6, 1.0)
+    got = held["delta_chunk_logs"].cpu().view(torch.float32).view(n // 64, H, 128)[..., :64].double()
+    c = torch.log(beta_g[:, H:].cpu().double()).view(n // 64, 64, H).cumsum(1).transpose(1, 2)
+    d = c[..., -1:] - c
+    half_unit = torch.exp2(torch.floor(torch.log2(d.abs().clamp(min=2.0**-126))) - 24)
+    assert (d < -32).sum() > 500 and ((got / d.exp() - 1).abs() <= 1.01 * half_unit + 2.0**-22)[d > -80].all()
