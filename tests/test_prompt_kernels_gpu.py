@@ -453,10 +453,11 @@ def test_retention_pairs_of_chunks_in_waves(wave, monkeypatch):
 
 
 @pytest.mark.parametrize("dim,vdim,taps", [(64, 30, 4), (128, 128, 4), (64, 200, 1), (128, 64, 3)])
-@pytest.mark.parametrize("slow", [True, False])
-def test_delta_rule_of_prompts_in_chunks(dim, vdim, taps, slow):
+@pytest.mark.parametrize("slow,alike", [(True, False), (False, False), (True, True)])
+def test_delta_rule_of_prompts_in_chunks(dim, vdim, taps, slow, alike):
     """Against the walk token by token and the recurrence in 64 bits: sequences of one token, a chunk, a chunk and one,
-    several, that go on from states and convolution inputs; decays near one, and fast ones among which some are zero."""
+    several, that go on from states and convolution inputs; decays near one, and fast ones among which some are zero; keys nearly
+    alike with strong writes, which the triangle's inverse has to stand."""
     o = ops()
     g = torch.Generator().manual_seed(dim + vdim + taps)
     H, G, new = 4, 2, [1, 64, 65, 200, 130]
@@ -464,6 +465,9 @@ def test_delta_rule_of_prompts_in_chunks(dim, vdim, taps, slow):
     rows = torch.randn(n, channels + H * vdim + 2 * H, generator=g)
     if not slow:
         rows[70:90, -1] = 1e4  # the last head's decay is zero there
+    if alike:
+        rows[:, G * dim:2 * G * dim] += 3.0 * torch.randn(1, G * dim, generator=g)
+        rows[:, -2 * H:-H] += 4.0
     conv = torch.randn(channels, taps, generator=g).to(DEV)
     a_log = (torch.empty(H).uniform_(-7.0, -4.0, generator=g) if slow else torch.empty(H).uniform_(-1.0, 1.0, generator=g)).to(DEV)
     bias = torch.empty(H).uniform_(-1.0, 1.0, generator=g).to(DEV)
@@ -496,6 +500,8 @@ def test_delta_rule_of_prompts_in_chunks(dim, vdim, taps, slow):
             want[row] = torch.einsum("hdv,hd->hv", S, q[row])
             row += 1
         finals[int(slots[i])] = S
+    if alike:
+        assert (k[70:100, None] * k[None, 70:100]).sum(-1).mean() > 0.5
     # (a few hundred float32 roundings of values of order one, on either way: 1e-5 of the largest is some 80 ulps)
     for y, s in ((walked, state), (got, state2)):
         assert (y.cpu().double() - want.reshape(n, -1)).abs().max() < 1e-5 * want.abs().max()
