@@ -2380,11 +2380,14 @@ def delta_scan(qkv: torch.Tensor, beta_g: torch.Tensor, state: torch.Tensor, tok
 
 
 DELTA_CHUNK = 64       # tokens of a chunk of delta_prompt
-# Steps whose longest sequence has more tokens run in chunks, if they have DELTA_STEP_MIN tokens together: shorter steps are
-# launched one by one, where the three launches and two tables more cost 40 us.  Whole prompts of one layer, 16 heads
-# with keys of 64 / 32 with keys of 128, values of 128, us walked (beyond 256 tokens in runs) and in chunks: 200 tokens 351 / 354 and
-# 391 / 394, 255 tokens 355 / 371 and 387 / 396, replayed 256 tokens 276 / 364 and 175 / 254, 2 x 200 tokens 274 / 418 and
-# 225 / 346, 3 x 300 tokens 370 / 775 and 286 / 485; 4 x 128 tokens 278 / 382 and 301 / 402.
+# Steps whose longest sequence has more tokens run in chunks, if they have DELTA_STEP_MIN tokens together: shorter
+# steps are launched one by one, where the two launches and two tables more cost 45 us.  Whole prompts of one layer,
+# 16 heads over 8 with keys of 64 / 32 over 16 with keys of 128, values of 128, us walked (beyond 256 tokens in
+# runs) -> in chunks: 65 tokens 335 -> 385 / 340 -> 388, 255 tokens 348 -> 397 / 358 -> 398; replayed from 256
+# tokens on: 256 tokens 263 -> 111 / 332 -> 160, 2 x 200 248 -> 129 / 347 -> 211, 3 x 300 327 -> 168 / 705 -> 302.
+# Replayed steps of shorter sequences would gain as well since the chunks run on the tensor cores (2 x 128 tokens
+# 182 -> 115 / 250 -> 165, 4 x 64 157 -> 153 / 217 -> 198): their line is that of the kernels before, where they
+# were slower.
 DELTA_CHUNK_MIN, DELTA_STEP_MIN = 192, 256
 
 
