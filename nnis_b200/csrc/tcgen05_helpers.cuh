@@ -79,8 +79,8 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_
 }
 // The same from a whole warp, one lane of which issues, A in shared or in tensor memory (a row a lane, two neighbouring places of K
 // a column): descriptors that the compiler knows to be the warp's stay in uniform
-// registers.  A product of 128 x 64 x 16 with A in tensor memory is issued every 30 cycles so, every 49 by one lane that runs
-// alone; with A in shared memory it takes 47 either way (what its operands' 6 KB are read in), one of 128 columns 61.
+// registers.  A product of 128 x N x 16 takes N / 2 cycles with A in tensor memory and 32 + N / 4 with A in shared memory (its 4 KB are
+// read again by every product) up to N = 128; one lane that runs alone issues one every 44 cycles at best.
 __device__ __forceinline__ void warp_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
@@ -117,14 +117,6 @@ __device__ __forceinline__ void tmem_store_issue(uint32_t taddr, const uint32_t 
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]),
                  "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
-}
-__device__ __forceinline__ void tmem_store_issue(uint32_t taddr, const uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-          "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-        : "memory");
 }
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Makes this thread's writes to shared memory visible to tcgen05.mma and TMA.
