@@ -13,14 +13,14 @@
 // Every product of matrices is six products of bfloat16 parts on the tensor cores, exact parts of float32 values, summed in
 // float32 in tensor memory over the 64 or 128 places of a chunk or a head (split_parts.cuh); the triangle is inverted in float32, c is
 // double, then two floats (differences of sums of up to 64 logs keep float32's digits), a decay of zero counts as e^-200, which is
-// zero in float32 and leaves the tokens after it exact.  Distance from 64 bits 1.7e-7 to 5.2e-7 of the outputs' norm where float32
-// sums on the CUDA cores had 1.8e-7 to 1.1e-6.
+// zero in float32 and leaves the tokens after it exact.  Distance from 64 bits, independent keys to nearly parallel ones, of the outputs'
+// norm 1.6e-7 to 5.2e-7 where float32 sums on the CUDA cores had 1.8e-7 to 1.1e-6, of the states' 0.9e-7 to 4.9e-7 (1.2e-7 to 1.0e-6).
 //
 // Against the walk in runs with a transition matrix per run (delta_rule.cu, which other key sizes and short prompts
 // keep): a token costs 2.2 dim vdim + 64 (dim + vdim) multiply-adds or so instead of 2.3 times three dim vdim, all but the chain side
 // by side.
 // Two prompts of 2,048 and 555 tokens, 32 heads over 16 key heads of 128 x 128, on a B200: with float32 multiply-adds, in four
-// kernels (substitution, states, reads), 61 + 148 + 255 + 133 us; now pack 57, solve 91, chain 128.
+// kernels (substitution, states, reads), 61 + 148 + 255 + 133 us; now pack 57, solve 92, chain 128.
 #include "async_copy.cuh"
 #include "common.cuh"
 #include "split_parts.cuh"
@@ -53,7 +53,7 @@ __host__ __device__ __forceinline__ size_t delta_qk_floats(int dim) { return (si
 
 // A CTA per (chunk, piece): q heads, k heads, value heads, and last the gates of all heads.  A thread walks 16 tokens of
 // a channel; with TAPS (the taps when there are 4, else 0) the inputs before a token stay in registers.  Instructions bound it
-// (104 a value with a division for each place and a test for each input, 79 us on the prompts above; 60 us now).
+// (104 a value with a division for each place and a test for each input, 79 us on the prompts above; 57 us now).
 template <int TAPS>
 __global__ void __launch_bounds__(256)
 delta_pack_kernel(const float* __restrict__ a, const float* __restrict__ conv_w, const float* __restrict__ tail,
@@ -617,7 +617,7 @@ struct DeltaChainShared {
 // A CTA per (sequence, head, 64 columns) walks the chunks: one warp brings the operands and issues the products, sixteen hold the
 // state, 16 values a thread (place `row` of the key, columns 16 cg ..), and split what is multiplied.  A step: [q; W] S; U = U0 - W S,
 // split; K^T (e^(c - c_j) U) into the state, which is split for the next step, and P U beside it for the outputs.
-// What bounds it: the two products that wait for each other, 1,445 + 722 cycles of the tensor cores at 64 columns (1,700 and 1,100 to
+// What bounds it: the two products that wait for each other, 1,536 + 768 cycles of the tensor cores at 64 columns (1,700 and 1,100 to
 // 1,500 beside the copies and splits that share shared memory with them), and the way of their sums through the threads to the
 // next one's operand, 1,100 cycles each: 6,800 cycles a step.  Against a first form, 10,000 cycles a step: left sides in tensor memory
 // instead of the scores in shared memory, rows of 128 swizzled bytes instead of octets, and outputs stored by TMA (row by row from

@@ -25,7 +25,7 @@
 //
 // What bounds it: shared memory and L1, 128 bytes a cycle.  With A's parts in shared memory too the products read 8 KB every 64 cycles
 // (BN = 128) beside 96 KB of parts written and 64 KB loaded for 64 columns of K, 2,750 cycles a block; in tensor memory A is written
-// (TMA) and read once as float32, and a block moves 250 KB instead of 350: 2,400 cycles, the products alone 1,405.  Adding
+// (TMA) and read once as float32, and a block moves 250 KB instead of 350: 2,400 cycles, the products alone 1,536.  Adding
 // under the splitting is 3 % faster than before or after it, and costs a tile of 192 columns registers that it has not: that one
 // adds after it.  Rows x N x K on a B200, cold L2, A's parts in shared memory -> here: 1,024 x 3,072 x 576 51 -> 35 us (128 tiles of 192
 // columns in one wave where 192 of 128 are two), 1,024 x 576 x 1,536 30 -> 25, 1,024 x 576 x 576 19.5 -> 17.4,

@@ -762,9 +762,9 @@ static cudaError_t launch_memory_prompt(const float* a, int a_cols, float* state
     // (rows on 32-byte boundaries)
     const bool split = memory_by_pairs(n_tokens, n_chunks, n_seqs, H, dim, vdim, sms) && a_cols % 8 == 0 &&
                        ((uintptr_t)a | (uintptr_t)chunk_state | (uintptr_t)o_raw) % 32 == 0;
-    // (the prompt's five kernels take 3 to 25 us each: every one is launched beside the end of the
-    // one before and waits for it first thing; prompts of 1500, 1500 and 701 tokens, 16 heads of 64, by
-    // graph take 203 us so, 207 with plain launches)
+    // (the prompt's five kernels take 2 to 35 us each: every one is launched beside the end of the
+    // one before and waits for it first thing; a layer of width 1,024, 4 heads of 128 x 256, prompts of
+    // 1,500, 1,500 and 701 tokens, by graph: 203 us so, 207 with plain launches)
     const int by = split ? 2 : 1, most_pairs = (n_chunks + n_seqs) / 2;
     cudaError_t e = cudaSuccess;
     if (split) {
