@@ -107,13 +107,15 @@ static cudaError_t launch_merge(const float* partial, T* out, size_t rows, int d
     // (records of an even number of floats start on 8-byte boundaries if the first does)
     const int pairs = d % 2 == 0 && (uintptr_t)partial % 8 == 0 && (uintptr_t)out % (2 * sizeof(T)) == 0;
     const bool warp_rows = d <= 64 || (d <= 128 && rows >= 2000 && n_splits <= 16);
-    // Early as long as the device holds all rows beside the next kernel's CTAs (float32 outputs take more registers: three instead of four CTAs an
-    // SM).  us late -> early, bfloat16 / float32: 16 slices of 128 values, 444 rows 2.66 -> 2.32 / 2.66 -> 2.31, 592 rows 2.75 -> 2.45 / 2.72 -> 2.85, 740 rows
-    // 2.85 -> 3.01; of 512 values 444 rows 4.19 -> 3.38 / 4.19 -> 3.12, 592 rows 4.41 -> 3.53 / 4.49 -> 4.50, 740 rows 4.66 -> 4.85; of 1,024 values 296 rows
-    // 6.28 -> 5.85, 370 rows 6.66 -> 6.83.  From 6 rows an SM on the late form is in its second wave, the early one up to 8 (7) not in its third: 1,036 rows of
-    // 256 values 4.67 -> 3.43 / 4.69 -> 3.27, of 512 7.72 -> 5.57 / 7.72 -> 6.45 (level at 128 values; 320 values of float32, 9 slices, 5.58 -> 5.84).  Up to eight
-    // slices are one trip late too: level or slower up to 256 values (592 rows 2.14 -> 2.40), of 512 values 296 rows 2.76 -> 2.55 / 2.76 -> 2.86, 128 rows
-    // 2.56 -> 2.20 / 2.56 -> 2.20, of 1,024 slower (3.58 -> 4.04).  More than sixteen are slower (32: 3.6 -> 5.1).
+    // Early as long as the device holds all rows beside the next kernel's CTAs (float32 outputs take more registers: three
+    // instead of four CTAs an SM).  us late -> early, bfloat16 / float32: 16 slices of 128 values, 444 rows 2.66 -> 2.32 /
+    // 2.66 -> 2.31, 592 rows 2.75 -> 2.45 / 2.72 -> 2.85, 740 rows 2.85 -> 3.01; of 512 values 444 rows 4.19 -> 3.38 / 4.19
+    // -> 3.12, 592 rows 4.41 -> 3.53 / 4.49 -> 4.50, 740 rows 4.66 -> 4.85; of 1,024 values 296 rows 6.28 -> 5.85, 370 rows
+    // 6.66 -> 6.83.  From 6 rows an SM on the late form is in its second wave, the early one up to 8 (7) not in its third:
+    // 1,036 rows of 256 values 4.67 -> 3.43 / 4.69 -> 3.27, of 512 7.72 -> 5.57 / 7.72 -> 6.45 (level at 128 values; 320
+    // values of float32, 9 slices, 5.58 -> 5.84).  Up to eight slices are one trip late too: level or slower up to 256
+    // values (592 rows 2.14 -> 2.40), of 512 values 296 rows 2.76 -> 2.55 / 2.76 -> 2.86, 128 rows 2.56 -> 2.20 / 2.56 ->
+    // 2.20, of 1,024 slower (3.58 -> 4.04).  More than sixteen are slower (32: 3.6 -> 5.1).
     const bool wide = d > 256, f32 = sizeof(T) == 4;
     bool early = !warp_rows && pairs && n_splits <= 16;
     if (early) {

@@ -709,11 +709,11 @@ NNIS_API int nnis_qkv_prep(const float* a, const float* wq, const float* wk, con
     // (a row of the input, of q and of both caches starts by fours of values, and so does every head)
     const int row_len = H * dk + G * (dk + dv) + (gated ? H : 0);
     const uintptr_t out = (uintptr_t)q_out | (uintptr_t)k_cache | (uintptr_t)v_cache;
-    // Few tokens leave a token's 128 threads more turns than 256 would have, behind a barrier for the angles: by fours from 1.5 tokens an SM on,
-    // with norms of wide rows from 3; rows of up to 512 quads without norms always.  us in general / by fours, bfloat16, one launch after another:
-    // 384 quads 8 tokens 3.07 / 2.93; 768 quads 8 tokens 3.60 / 3.99, 256 4.30 / 4.25, 512 7.98 / 4.66; 1,280 quads 128 tokens 5.92 / 6.07,
-    // 256 6.50 / 6.09; with norms 384 quads 128 tokens 4.36 / 4.47, 370 5.02 / 4.76, 768 quads 8 tokens 5.04 / 5.64, 444 6.22 / 6.36, 512
-    // 9.16 / 6.36.
+    // Few tokens leave a token's 128 threads more turns than 256 would have, behind a barrier for the angles: by fours from
+    // 1.5 tokens an SM on, with norms of wide rows from 3; rows of up to 512 quads without norms always.  us in general /
+    // by fours, bfloat16, one launch after another: 384 quads 8 tokens 3.07 / 2.93; 768 quads 8 tokens 3.60 / 3.99, 256
+    // 4.30 / 4.25, 512 7.98 / 4.66; 1,280 quads 128 tokens 5.92 / 6.07, 256 6.50 / 6.09; with norms 384 quads 128 tokens
+    // 4.36 / 4.47, 370 5.02 / 4.76, 768 quads 8 tokens 5.04 / 5.64, 444 6.22 / 6.36, 512 9.16 / 6.36.
     const bool normed = wq || wk, narrow = (H * dk + G * (dk + dv)) / 4 <= 512;
     const bool pays = (narrow && !normed) || 2LL * n_tokens > (normed && !narrow ? 6LL : 3LL) * device_sms();
     if (pays && dk % 4 == 0 && dv % 4 == 0 && row_len % 4 == 0 && rot / 2 <= kPrepTurns && (uintptr_t)a % 16 == 0 &&

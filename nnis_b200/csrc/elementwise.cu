@@ -603,8 +603,9 @@ NNIS_API int nnis_rope_store(void* qkv, int dtype, const int* token_pos, const i
     if (rotate && (!cos_t || !sin_t)) return NNIS_ERR_ARGUMENT;
     const uintptr_t rows = (uintptr_t)qkv | (uintptr_t)k_cache | (uintptr_t)v_cache;
     const uintptr_t turns = rotate ? (uintptr_t)cos_t | (uintptr_t)sin_t : 0;
-    // A token of fewer than 64 items leaves most of its 128 threads idle, which many tokens feel: us in general / by fours, 2 + 1 + 1 heads
-    // of 64 (40 items), bfloat16, 740 tokens 2.71 / 2.50, 1,024 2.84 / 3.01, 3,001 3.95 / 4.56; 2 + 2 + 2 heads (64 items) 3,001 5.12 / 4.06.
+    // A token of fewer than 64 items leaves most of its 128 threads idle, which many tokens feel: us in general / by fours,
+    // 2 + 1 + 1 heads of 64 (40 items), bfloat16, 740 tokens 2.71 / 2.50, 1,024 2.84 / 3.01, 3,001 3.95 / 4.56; 2 + 2 + 2
+    // heads (64 items) 3,001 5.12 / 4.06.
     const bool pays = (nq + nkv) * (d / 8) + nkv * (d / 4) >= 64 || n_tokens <= 5LL * device_sms();
     if (pays && d % 8 == 0 && turns % 16 == 0 && rows % (dtype == NNIS_DTYPE_F32 ? 16 : 8) == 0 &&
         (dtype == NNIS_DTYPE_F32 || dtype == NNIS_DTYPE_BF16)) {
@@ -674,10 +675,10 @@ NNIS_API int nnis_rope_part(const void* src, long long src_row, int src_head, in
     if (n_tokens <= 0 || heads <= 0 || len <= 0 || dims < 0 || (dims & 1) || dims > len || !freq)
         return NNIS_ERR_ARGUMENT;
     // (every head's part starts by fours, and so do its halves and what passes)
-    // (short steps are over before the barrier behind the angles pays.  us in general / by fours, bfloat16, halves: 16 heads of 64, 8 tokens 1.75 / 1.67
-    // (float32 1.69 / 1.69), 256 2.10 / 1.85; 8 heads 128 tokens 1.54 / 1.79, 512 1.89 / 1.93, 740 2.55 / 1.96; neighbours: 16 heads 8 tokens 1.74 /
-    // 1.99, 296 2.10 / 2.16, 512 2.66 / 2.30; 12 heads 444 tokens 2.14 / 2.29, 512 2.39 / 2.26; a head of 64, halves: 1,536 tokens 1.91 / 1.93, 2,560
-    // 2.98 / 2.92)
+    // (short steps are over before the barrier behind the angles pays.  us in general / by fours, bfloat16, halves: 16
+    // heads of 64, 8 tokens 1.75 / 1.67 (float32 1.69 / 1.69), 256 2.10 / 1.85; 8 heads 128 tokens 1.54 / 1.79, 512 1.89 /
+    // 1.93, 740 2.55 / 1.96; neighbours: 16 heads 8 tokens 1.74 / 1.99, 296 2.10 / 2.16, 512 2.66 / 2.30; 12 heads 444
+    // tokens 2.14 / 2.29, 512 2.39 / 2.26; a head of 64, halves: 1,536 tokens 1.91 / 1.93, 2,560 2.98 / 2.92)
     const bool pays = (long long)n_tokens * heads * len >= (neighbours ? 3LL << 17 : 1LL << 18) || n_tokens > 16LL * device_sms();
     const bool quads = pays && len % 4 == 0 && dims % (neighbours ? 4 : 8) == 0 && dims / 2 <= kRopeTurns &&
                        !((src_row | dst_row | src_head | dst_head | src_off | dst_off) & 3) &&
